@@ -299,10 +299,12 @@ int pbf_kernel_launches(pbf_handle* h, uint64_t* out);
 int pbf_set_use_graph(pbf_handle* h, int on);
 /* Execution options (results do not depend on them; no reference counterpart):
  *   PBF_OPT_SPATIAL_ORDER  the neighbour passes' walk.
- *                          4: particles taken in the Morton order of their
- *                          cells, one thread each, each of the 27 hashed
- *                          buckets tested in chunks of 8 before the pair body
- *                          runs on the hits.
+ *                          4: the 27 hashed buckets.  Up to 2^18 particles a
+ *                          group of 8 to 32 lanes walks them per particle;
+ *                          above, particles are taken in the Morton order of
+ *                          their cells, one thread each, each bucket tested
+ *                          in chunks of 8 before the pair body runs on the
+ *                          hits.
  *                          8: data relabelled by the slot of each particle's
  *                          cell in a dense window of the box (z, y, x), so
  *                          the three x-adjacent cells of a row are one label
@@ -311,10 +313,11 @@ int pbf_set_use_graph(pbf_handle* h, int on);
  *                          particle within reach has moved 0.9 h since the
  *                          predict near a colliding cell; the hashed buckets
  *                          elsewhere.  Same pairs, same order as the buckets.
- *                          -1 (default): mode 8 from 2^19 particles, mode 4
- *                          below (where mode 8's relabelling launches cost
- *                          more than its walk saves); APBF and windows over
- *                          2^26 cells run mode 4.  Modes 4 and 8 give
+ *                          -1 (default): mode 8 from 2^19 particles, or from
+ *                          3 * 2^16 when the window has at most 8 cells per
+ *                          particle, mode 4 below (where mode 8's relabelling
+ *                          launches cost more than its walk saves); APBF and
+ *                          windows over 2^26 cells run mode 4.  Modes 4 and 8 give
  *                          bit-identical results (same pairs, order and pair
  *                          arithmetic).  Other values: PBF_ERR_INVALID. */
 #define PBF_OPT_SPATIAL_ORDER 1
@@ -383,6 +386,9 @@ int pbf_batch_device_ptrs(pbf_batch* b, void** pos4, void** vel4);
 int pbf_batch_kernel_launches(const pbf_batch* b, uint64_t* count);
 
 /* Options.  None changes results, only speed.
+ *                           (block, order and persistence shape the neighbour passes of
+ *                           mode 4 above 2^18 particles in all; up to there a group of
+ *                           lanes walks the buckets per particle, in sorted order)
  *   PBF_BOPT_BLOCK          threads per block of the neighbour passes: 64, 128 (default), 256
  *   PBF_BOPT_ORDER          1 (default): threads take particles in the scene-prefixed
  *                           Morton order of their cells; 0: sorted (hash) order
@@ -390,7 +396,8 @@ int pbf_batch_kernel_launches(const pbf_batch* b, uint64_t* count);
  *                           particles; 0 (default): one thread per particle
  *   PBF_BOPT_USE_GRAPH      1 (default): replay the step from a CUDA graph
  *   PBF_BOPT_NEIGHBOUR_MODE -1 (default): automatic (the autotuner's pick once it has run,
- *                           before that 8 from 2^19 particles when the windows fit, else 4);
+ *                           before that 8 above 2^18 particles when the windows fit and,
+ *                           below 2^19, have at most 8 cells per particle, else 4);
  *                           4: every scene walks its 27 hashed buckets (block, order and
  *                           persistence apply); 8: a dense cell window per scene (the walls'
  *                           box plus 6 cells each side, at most 2^26 cells in all, APBF off),

@@ -102,6 +102,30 @@ struct HashWalk {
     }
 };
 
+// What the lambda pass makes of a particle's sums: rho, sg = sum |gradW|^2,
+// g = sum gradW and, with s_corr on, sc = sum (W / W(dq))^n gradW.  Outputs
+// as lambda_core's.
+__device__ __forceinline__ float4 lambda_finish(const DevParams& P, float4 xi, float rho, float sg, float3 g, float3 sc,
+                                                bool scorr, float& rho_out, float3& g_out, float& den_out,
+                                                float3& b_out)
+{
+    const float lam_gx = g.x, lam_gy = g.y, lam_gz = g.z;  // sum_j gradW_ij, unscaled
+    float gx = g.x, gy = g.y, gz = g.z;
+    gx *= P.inv_rho0;
+    gy *= P.inv_rho0;
+    gz *= P.inv_rho0;
+    const float C = fmaxf(rho / P.rho0 - 1.0f, -P.cohesion);
+    sg = sg * P.inv_rho0_sq + (gx * gx + gy * gy + gz * gz);
+    rho_out = rho;
+    g_out = make_float3(gx, gy, gz);
+    den_out = sg + P.eps;
+    const float lam = -C / den_out;
+    const float kc = scorr ? -P.k_corr : 0.f;
+    b_out = make_float3(__fmaf_rn(lam, lam_gx, kc * sc.x), __fmaf_rn(lam, lam_gy, kc * sc.y),
+                        __fmaf_rn(lam, lam_gz, kc * sc.z));
+    return make_float4(xi.x, xi.y, xi.z, lam);
+}
+
 // ---- CS_ComputeLambdas.glsl:108-162 -----------------------------------------------------------
 // Returns (x*, lambda); also rho, grad C_i (the scaled sum of spiky
 // gradients), the denominator sum |grad C|^2 + eps that lambda divides by
@@ -149,21 +173,8 @@ __device__ __forceinline__ float4 lambda_core(const DevParams& P, XS X, float4 x
                  }
              }
          });
-    const float lam_gx = gxy.x, lam_gy = gxy.y, lam_gz = gz;  // sum_j gradW_ij, unscaled
-    float gx = gxy.x, gy = gxy.y;
-    gx *= P.inv_rho0;
-    gy *= P.inv_rho0;
-    gz *= P.inv_rho0;
-    const float C = fmaxf(rho / P.rho0 - 1.0f, -P.cohesion);
-    sg = sg * P.inv_rho0_sq + (gx * gx + gy * gy + gz * gz);
-    rho_out = rho;
-    g_out = make_float3(gx, gy, gz);
-    den_out = sg + P.eps;
-    const float lam = -C / den_out;
-    const float kc = scorr ? -P.k_corr : 0.f;
-    b_out = make_float3(__fmaf_rn(lam, lam_gx, kc * sxy.x), __fmaf_rn(lam, lam_gy, kc * sxy.y),
-                        __fmaf_rn(lam, lam_gz, kc * sz));
-    return make_float4(xi.x, xi.y, xi.z, lam);
+    return lambda_finish(P, xi, rho, sg, make_float3(gxy.x, gxy.y, gz), make_float3(sxy.x, sxy.y, sz), scorr, rho_out,
+                         g_out, den_out, b_out);
 }
 
 __device__ __forceinline__ float4 lambda_particle_x(const DevParams& P, const int2* __restrict__ table,
@@ -206,30 +217,13 @@ __device__ __forceinline__ float scorr_term(const DevParams& P, float r2)
     return 0.0f;
 }
 
-// ---- CS_ComputeDeltaP.glsl:120-166 + CS_ApplyDeltaP.glsl:80-124 --------------------------------
-// Returns (x* + dp, lambda); dp_raw = dp before the 0.5 h clamp.  b is the
-// lambda pass's b_out for this particle: the shader's per-pair factor
-// (lambda_i + lambda_j + s_corr) * gradW_ij is summed as b + sum_j lambda_j *
-// gradW_ij, so the pair body here loads and scales only lambda_j.
-template <class XS, class Walk>
-__device__ __forceinline__ float4 deltap_core(const DevParams& P, const SdfDev& sdf, XS X, float4 xi, Walk&& walk,
-                                              float3& dp_raw, float3 b)
+// The corrected position from a particle's delta-p sum d (before the 1/rho0
+// scale): clamp, obstacle projection.
+__device__ __forceinline__ float4 deltap_finish(const DevParams& P, const SdfDev& sdf, float4 xi, float3 d,
+                                                float3& dp_raw)
 {
     const float li = xi.w;
-    float dz = b.z;
-    float2 dxy = make_float2(b.x, b.y);
-    const float2 xyi = make_float2(xi.x, xi.y);
-    walk([&](float r2) { return r2 <= P.h2 && r2 >= 1e-10f; },
-         [&](int k) {
-             const float4 xj = X[k];
-             const float2 rxy = sub_f32x2(xyi, make_float2(xj.x, xj.y));
-             const float rx = rxy.x, ry = rxy.y, rz = xi.z - xj.z;
-             const float r2 = rx * rx + ry * ry + rz * rz;
-             const float g = spiky_scale(P, r2) * xj.w;
-             dxy = fma_f32x2(rxy, g, dxy);
-             dz = __fmaf_rn(rz, g, dz);
-         });
-    float dx = dxy.x, dy = dxy.y;
+    float dx = d.x, dy = d.y, dz = d.z;
     // rounded products (not fused into the x + dp below)
     dx = __fmul_rn(dx, P.inv_rho0);
     dy = __fmul_rn(dy, P.inv_rho0);
@@ -250,6 +244,31 @@ __device__ __forceinline__ float4 deltap_core(const DevParams& P, const SdfDev& 
     return make_float4(p.x, p.y, p.z, li);
 }
 
+// ---- CS_ComputeDeltaP.glsl:120-166 + CS_ApplyDeltaP.glsl:80-124 --------------------------------
+// Returns (x* + dp, lambda); dp_raw = dp before the 0.5 h clamp.  b is the
+// lambda pass's b_out for this particle: the shader's per-pair factor
+// (lambda_i + lambda_j + s_corr) * gradW_ij is summed as b + sum_j lambda_j *
+// gradW_ij, so the pair body here loads and scales only lambda_j.
+template <class XS, class Walk>
+__device__ __forceinline__ float4 deltap_core(const DevParams& P, const SdfDev& sdf, XS X, float4 xi, Walk&& walk,
+                                              float3& dp_raw, float3 b)
+{
+    float dz = b.z;
+    float2 dxy = make_float2(b.x, b.y);
+    const float2 xyi = make_float2(xi.x, xi.y);
+    walk([&](float r2) { return r2 <= P.h2 && r2 >= 1e-10f; },
+         [&](int k) {
+             const float4 xj = X[k];
+             const float2 rxy = sub_f32x2(xyi, make_float2(xj.x, xj.y));
+             const float rx = rxy.x, ry = rxy.y, rz = xi.z - xj.z;
+             const float r2 = rx * rx + ry * ry + rz * rz;
+             const float g = spiky_scale(P, r2) * xj.w;
+             dxy = fma_f32x2(rxy, g, dxy);
+             dz = __fmaf_rn(rz, g, dz);
+         });
+    return deltap_finish(P, sdf, xi, make_float3(dxy.x, dxy.y, dz), dp_raw);
+}
+
 __device__ __forceinline__ float4 deltap_particle_x(const DevParams& P, const int2* __restrict__ table,
                                                     uint32_t mask, const SdfDev& sdf,
                                                     const float4* __restrict__ xin, int s, float3& dp_raw)
@@ -267,49 +286,12 @@ __device__ __forceinline__ float4 deltap_particle(const DevParams& P, const int2
     return deltap_particle_x(P, table, mask, sdf, xin, s, dp);
 }
 
-// ---- CS_Integrate.glsl:135-280 (pre-dispatch neighbour velocities) ---------------------------
-// From x* (x4), the predicted velocity v0, the substep start p0 and the
-// neighbours' (X, V): the committed position xo (w = p0.w), velocity vo
-// (w = v0.w) and, when vorticity is on, omega4 = (omega, |omega|).
-template <class XS, class VS, class P0, class Walk>
-__device__ __forceinline__ void integrate_core(const DevParams& P, const float* bmin, const float* bmax,
-                                               const SdfDev& sdf, XS X, VS V, float4 x4, float4 v0, P0&& p0_load,
-                                               Walk&& walk, float4& xo, float4& vo, float4& omega4)
+// The committed state from a particle's XSPH sum f and curl sum c.
+__device__ __forceinline__ void integrate_finish(const DevParams& P, const float* bmin, const float* bmax,
+                                                 const SdfDev& sdf, float4 x4, float4 v0, float4 p0, float3 f,
+                                                 float3 c, float4& xo, float4& vo, float4& omega4)
 {
-    float fz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
-    float2 fxy = make_float2(0.f, 0.f);
-    const float2 xyi = make_float2(x4.x, x4.y), vxy0 = make_float2(v0.x, v0.y);
-    if (P.visc_on || P.vort_on) {
-        walk([&](float r2) { return r2 <= P.h2; },
-             [&](int k) {
-                 const float4 xj = X[k];
-                 const float2 rxy = sub_f32x2(xyi, make_float2(xj.x, xj.y));
-                 const float rx = rxy.x, ry = rxy.y, rz = x4.z - xj.z;
-                 const float r2 = rx * rx + ry * ry + rz * rz;
-                 const float4 vj = V[k];
-                 const float2 uxy = sub_f32x2(make_float2(vj.x, vj.y), vxy0);
-                 const float ux = uxy.x, uy = uxy.y, uz = vj.z - v0.z;
-                 if (P.visc_on) {
-                     const float w = poly6_in(P, r2) * P.inv_rho0;
-                     fxy = fma_f32x2(uxy, w, fxy);
-                     fz = __fmaf_rn(uz, w, fz);
-                 }
-                 if (P.vort_on && r2 >= 1e-10f) {
-                     const float sc = spiky_scale(P, r2);
-                     const float2 axy = mul_f32x2(rxy, sc);
-                     const float ax = axy.x, ay = axy.y, az = rz * sc;
-                     // a*b - c*d with the rounding fixed (one product rounded,
-                     // one fused), so every instantiation gives the same bits
-                     cx += __fmaf_rn(uy, az, -__fmul_rn(uz, ay));
-                     cy += __fmaf_rn(uz, ax, -__fmul_rn(ux, az));
-                     cz += __fmaf_rn(ux, ay, -__fmul_rn(uy, ax));
-                 }
-             });
-    }
-    // the substep-start position is needed only now: loaded after the walk,
-    // it holds no registers across it
-    const float4 p0 = p0_load();
-    const float fx = fxy.x, fy = fxy.y;
+    const float fx = f.x, fy = f.y, fz = f.z, cx = c.x, cy = c.y, cz = c.z;
     float3 x = make_float3(x4.x, x4.y, x4.z);
     float vdx = 0.f, vdy = 0.f, vdz = 0.f;
     if (P.visc_on) {
@@ -354,6 +336,51 @@ __device__ __forceinline__ void integrate_core(const DevParams& P, const float* 
     vo = make_float4(vx, vy, vz, v0.w);
 }
 
+// ---- CS_Integrate.glsl:135-280 (pre-dispatch neighbour velocities) ---------------------------
+// From x* (x4), the predicted velocity v0, the substep start p0 and the
+// neighbours' (X, V): the committed position xo (w = p0.w), velocity vo
+// (w = v0.w) and, when vorticity is on, omega4 = (omega, |omega|).
+template <class XS, class VS, class P0, class Walk>
+__device__ __forceinline__ void integrate_core(const DevParams& P, const float* bmin, const float* bmax,
+                                               const SdfDev& sdf, XS X, VS V, float4 x4, float4 v0, P0&& p0_load,
+                                               Walk&& walk, float4& xo, float4& vo, float4& omega4)
+{
+    float fz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
+    float2 fxy = make_float2(0.f, 0.f);
+    const float2 xyi = make_float2(x4.x, x4.y), vxy0 = make_float2(v0.x, v0.y);
+    if (P.visc_on || P.vort_on) {
+        walk([&](float r2) { return r2 <= P.h2; },
+             [&](int k) {
+                 const float4 xj = X[k];
+                 const float2 rxy = sub_f32x2(xyi, make_float2(xj.x, xj.y));
+                 const float rx = rxy.x, ry = rxy.y, rz = x4.z - xj.z;
+                 const float r2 = rx * rx + ry * ry + rz * rz;
+                 const float4 vj = V[k];
+                 const float2 uxy = sub_f32x2(make_float2(vj.x, vj.y), vxy0);
+                 const float ux = uxy.x, uy = uxy.y, uz = vj.z - v0.z;
+                 if (P.visc_on) {
+                     const float w = poly6_in(P, r2) * P.inv_rho0;
+                     fxy = fma_f32x2(uxy, w, fxy);
+                     fz = __fmaf_rn(uz, w, fz);
+                 }
+                 if (P.vort_on && r2 >= 1e-10f) {
+                     const float sc = spiky_scale(P, r2);
+                     const float2 axy = mul_f32x2(rxy, sc);
+                     const float ax = axy.x, ay = axy.y, az = rz * sc;
+                     // a*b - c*d with the rounding fixed (one product rounded,
+                     // one fused), so every instantiation gives the same bits
+                     cx += __fmaf_rn(uy, az, -__fmul_rn(uz, ay));
+                     cy += __fmaf_rn(uz, ax, -__fmul_rn(ux, az));
+                     cz += __fmaf_rn(ux, ay, -__fmul_rn(uy, ax));
+                 }
+             });
+    }
+    // the substep-start position is needed only now: loaded after the walk,
+    // it holds no registers across it
+    integrate_finish(P, bmin, bmax, sdf, x4, v0, p0_load(), make_float3(fxy.x, fxy.y, fz), make_float3(cx, cy, cz), xo,
+                     vo, omega4);
+}
+
 // Commits x and v of slot s: writes pos/vel at the particle id, sx0[s] = x
 // and somega[s] = (omega, |omega|).
 __device__ __forceinline__ void integrate_particle(const DevParams& P, const int2* __restrict__ table, uint32_t mask,
@@ -373,6 +400,28 @@ __device__ __forceinline__ void integrate_particle(const DevParams& P, const int
     pos[id] = xo;
     vel[id] = vo;
     sx0[s] = xo;
+}
+
+// The confinement increment from a particle's sum e of |omega_j| gradW; false
+// when it is too short for a direction.
+template <class WL>
+__device__ __forceinline__ bool vorticity_finish(const DevParams& P, float3 e, WL&& w_load, float3& dv)
+{
+    float ex = e.x, ey = e.y, ez = e.z;
+    ex *= P.inv_rho0;
+    ey *= P.inv_rho0;
+    ez *= P.inv_rho0;
+    const float el = sqrtf(ex * ex + ey * ey + ez * ez);
+    if (el < 1e-6f) return false;
+    const float4 w = w_load();  // the particle's own omega, loaded after the walk
+    const float nx = ex / el, ny = ey / el, nz = ez / el;
+    const float crx = __fmaf_rn(ny, w.z, -__fmul_rn(nz, w.y)), cry = __fmaf_rn(nz, w.x, -__fmul_rn(nx, w.z)),
+                crz = __fmaf_rn(nx, w.y, -__fmul_rn(ny, w.x));
+    // rounded products: the caller adds dv to v, and a fused multiply-add
+    // there would round differently from one kernel to another
+    dv = make_float3(__fmul_rn(P.vort_eps * crx, P.dt), __fmul_rn(P.vort_eps * cry, P.dt),
+                     __fmul_rn(P.vort_eps * crz, P.dt));
+    return true;
 }
 
 // ---- CS_VorticityConfinement.glsl:133-167 (pass 1) ----------------------------------------------
@@ -396,21 +445,7 @@ __device__ __forceinline__ bool vorticity_core(const DevParams& P, XS X, MS OMAG
              exy = fma_f32x2(rxy, sc, exy);
              ez = __fmaf_rn(rz, sc, ez);
          });
-    float ex = exy.x, ey = exy.y;
-    ex *= P.inv_rho0;
-    ey *= P.inv_rho0;
-    ez *= P.inv_rho0;
-    const float el = sqrtf(ex * ex + ey * ey + ez * ez);
-    if (el < 1e-6f) return false;
-    const float4 w = w_load();  // the particle's own omega, loaded after the walk
-    const float nx = ex / el, ny = ey / el, nz = ez / el;
-    const float crx = __fmaf_rn(ny, w.z, -__fmul_rn(nz, w.y)), cry = __fmaf_rn(nz, w.x, -__fmul_rn(nx, w.z)),
-                crz = __fmaf_rn(nx, w.y, -__fmul_rn(ny, w.x));
-    // rounded products: the caller adds dv to v, and a fused multiply-add
-    // there would round differently from one kernel to another
-    dv = make_float3(__fmul_rn(P.vort_eps * crx, P.dt), __fmul_rn(P.vort_eps * cry, P.dt),
-                     __fmul_rn(P.vort_eps * crz, P.dt));
-    return true;
+    return vorticity_finish(P, make_float3(exy.x, exy.y, ez), w_load, dv);
 }
 
 __device__ __forceinline__ void vorticity_particle(const DevParams& P, const int2* __restrict__ table, uint32_t mask,

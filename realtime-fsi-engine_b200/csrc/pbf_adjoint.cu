@@ -82,19 +82,13 @@ int pbf_batch::ad_alloc()
 
 int pbf_batch::record_body()
 {
-    const DevParams P = dev_params();
-    BatchLaunch L = launch;
-    L.sms = num_sms;
     for (uint32_t sub = 0; sub < cfg.substep_iterations; ++sub) {
         ACK(cudaMemcpyAsync(cp_pos + (size_t)sub * n, pos, sizeof(float4) * n, cudaMemcpyDeviceToDevice, stream));
         ACK(cudaMemcpyAsync(cp_vel + (size_t)sub * n, vel, sizeof(float4) * n, cudaMemcpyDeviceToDevice, stream));
         const int rc = substep_body(pos, vel, pos, vel);
         if (rc) return rc;
     }
-    if (cfg.enable_vorticity) {
-        launch_b_vorticity(P, L, scenes_dev, scene_of, sx0, somega, ids, vel, table, order, stream);
-        ++launches;
-    }
+    if (cfg.enable_vorticity) vorticity_pass();
     return PBF_OK;
 }
 
@@ -140,8 +134,12 @@ int pbf_batch::backward_body()
         const bool last = (sub == (int)S - 1) && vort;
         if (last) {
             // committed state and omega of the last substep, for the vorticity reverse
-            launch_b_integrate(P, L, scenes_dev, scene_of, sx[0], sv, sx0, somega, ids, tpos, tvel, table, order,
-                               stream);
+            if (const int G = coop_lanes(n))
+                launch_c_integrate(G, P, scenes_dev, scene_of, sx[0], sv, sx0, somega, ids, tpos, tvel, table, order,
+                                   stream);
+            else
+                launch_b_integrate(P, L, scenes_dev, scene_of, sx[0], sv, sx0, somega, ids, tpos, tvel, table, order,
+                                   stream);
             launch_ad_vorticity(P, scenes_dev, scene_of, order, table, sx0, somega, ids, vb, pbs, omb, stream);
             launches += 2;
         }

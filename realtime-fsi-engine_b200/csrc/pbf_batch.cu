@@ -76,7 +76,7 @@ pbf_batch::~pbf_batch()
     bfree(pos); bfree(vel); bfree(pred); bfree(aos); bfree(scene_of); bfree(scenes_dev);
     bfree(keys); bfree(ka); bfree(ia); bfree(kb); bfree(ib); bfree(hist); bfree(totals); bfree(table);
     bfree(mcode); bfree(mka); bfree(mia); bfree(mkb); bfree(mib);
-    bfree(sx[0]); bfree(sx[1]); bfree(sv); bfree(sx0); bfree(somega); bfree(dpb); bfree(rho); bfree(lod);
+    bfree(sx[0]); bfree(sx[1]); bfree(sv); bfree(sx0); bfree(somega); bfree(dpb); bfree(rho); bfree(lod); bfree(chits); bfree(chit_len);
     bfree(save_pos); bfree(save_vel);
     dense_free();
     ad_free();
@@ -232,36 +232,64 @@ int pbf_batch::substep_body(const float4* src_pos, const float4* src_vel, float4
     const int sms = num_sms;
     BatchLaunch L = launch;
     L.sms = sms;
+    const int G = coop_lanes(n);
     const uint32_t max_iter = derived.enable_apbf ? derived.max_lod : cfg.solver_iterations;
     launch_b_predict(P, scenes_dev, scene_of, src_pos, src_vel, keys, sms, stream);
     launch_radix_sort(n, key_bits, keys, ka, ia, kb, ib, hist, totals, &skeys, &ids, stream, &launches);
     BCK(cudaMemsetAsync(table, 0xFF, sizeof(int2) * (size_t)table_size, stream));
     launch_build_table(n, skeys, table, sms, stream);
-    launch_b_reorder(P, scenes_dev, scene_of, ids, src_pos, src_vel, sx[0], sv, sx0, lod, morton ? mcode : nullptr,
+    const bool sorted = morton && !G;  // a group of lanes per particle needs no processing order
+    launch_b_reorder(P, scenes_dev, scene_of, ids, src_pos, src_vel, sx[0], sv, sx0, lod, sorted ? mcode : nullptr,
                      mbits, sms, stream);
     launches += 3;
     order = nullptr;
-    if (morton) {
+    if (sorted) {
         uint32_t* msorted = nullptr;
         launch_radix_sort(n, order_bits, mcode, mka, mia, mkb, mib, hist, totals, &msorted, &order, stream,
                           &launches);
     }
     for (uint32_t it = 1; it <= max_iter; ++it) {
-        launch_b_lambda(P, L, scenes_dev, scene_of, sx[0], sx[1], rho, table, lod, it, order, stream);
-        launch_b_deltap(P, L, scenes_dev, scene_of, sx[1], sx[0], table, lod, it, order, stream);
+        if (G) {
+            launch_c_lambda(G, P, scenes_dev, scene_of, sx[0], sx[1], rho, table, lod, it, order, chits, chit_len,
+                            stream);
+            launch_c_deltap(G, P, scenes_dev, scene_of, sx[1], sx[0], table, lod, it, order, chits, chit_len, stream);
+        } else {
+            launch_b_lambda(P, L, scenes_dev, scene_of, sx[0], sx[1], rho, table, lod, it, order, stream);
+            launch_b_deltap(P, L, scenes_dev, scene_of, sx[1], sx[0], table, lod, it, order, stream);
+        }
         launches += 2;
     }
-    launch_b_integrate(P, L, scenes_dev, scene_of, sx[0], sv, sx0, somega, ids, dst_pos, dst_vel, table, order,
-                       stream);
+    if (G)
+        launch_c_integrate(G, P, scenes_dev, scene_of, sx[0], sv, sx0, somega, ids, dst_pos, dst_vel, table, order,
+                           stream);
+    else
+        launch_b_integrate(P, L, scenes_dev, scene_of, sx[0], sv, sx0, somega, ids, dst_pos, dst_vel, table, order,
+                           stream);
     ++launches;
     return PBF_OK;
+}
+
+// The vorticity pass over the hashed buckets of the last substep.
+void pbf_batch::vorticity_pass()
+{
+    const DevParams P = dev_params();
+    BatchLaunch L = launch;
+    L.sms = num_sms;
+    if (const int G = coop_lanes(n))
+        launch_c_vorticity(G, P, scenes_dev, scene_of, sx0, somega, ids, vel, table, order, stream);
+    else
+        launch_b_vorticity(P, L, scenes_dev, scene_of, sx0, somega, ids, vel, table, order, stream);
+    ++launches;
 }
 
 int pbf_batch::effective_mode() const
 {
     if (neighbour_mode == 4 || neighbour_mode == 8) return neighbour_mode;
     if (tuned_mode) return tuned_mode;
-    return dense_fits() && n >= (1u << 19) ? 8 : 4;
+    // mode 8 where mode 4 leaves its groups of lanes (k_coop.cu: 146,319
+    // particles in 40 scenes 1219 us a step against 2069 in mode 8, 162,133 in 14
+    // scenes 1396 against 1954) and the windows have at most 8 cells per particle
+    return dense_fits() && n > (1u << 18) && (n >= (1u << 19) || dense_total <= 8ull * n) ? 8 : 4;
 }
 
 void pbf_batch::dense_free()
@@ -424,17 +452,11 @@ int pbf_batch::dense_step_body()
 int pbf_batch::step_body()
 {
     if (effective_mode() == 8) return dense_step_body();
-    const DevParams P = dev_params();
-    BatchLaunch L = launch;
-    L.sms = num_sms;
     for (uint32_t sub = 0; sub < cfg.substep_iterations; ++sub) {
         const int rc = substep_body(pos, vel, pos, vel);
         if (rc) return rc;
     }
-    if (cfg.enable_vorticity) {
-        launch_b_vorticity(P, L, scenes_dev, scene_of, sx0, somega, ids, vel, table, order, stream);
-        ++launches;
-    }
+    if (cfg.enable_vorticity) vorticity_pass();
     return PBF_OK;
 }
 
@@ -539,9 +561,10 @@ extern "C" int pbf_batch_create(const pbf_fluid_config* cfg, const pbf_scene_des
         (rc = balloc(b->ib, c)) || (rc = balloc(b->hist, (size_t)256 * sort_num_tiles((uint32_t)c))) ||
         (rc = balloc(b->totals, 256)) || (rc = balloc(b->table, std::max<uint32_t>(b->table_size, 1u))) ||
         (rc = balloc(b->mcode, c)) || (rc = balloc(b->mka, c)) || (rc = balloc(b->mia, c)) ||
-        (rc = balloc(b->mkb, c)) || (rc = balloc(b->mib, c)) || (rc = balloc(b->sx[0], c)) ||
-        (rc = balloc(b->sx[1], c)) || (rc = balloc(b->sv, c)) || (rc = balloc(b->sx0, c)) ||
-        (rc = balloc(b->somega, c)) || (rc = balloc(b->dpb, c)) || (rc = balloc(b->rho, c)) || (rc = balloc(b->lod, c))) {
+        (rc = balloc(b->mkb, c)) || (rc = balloc(b->mib, c)) || (rc = balloc(b->sx[0], c + kCoopPad)) ||
+        (rc = balloc(b->sx[1], c + kCoopPad)) || (rc = balloc(b->sv, c)) || (rc = balloc(b->sx0, c + kCoopPad)) ||
+        (rc = balloc(b->somega, c)) || (rc = balloc(b->dpb, c)) || (rc = balloc(b->rho, c)) || (rc = balloc(b->lod, c)) ||
+        (coop_lanes((uint32_t)c) && ((rc = balloc(b->chits, c * kCoopList)) || (rc = balloc(b->chit_len, c))))) {
         delete b;
         return rc;
     }

@@ -142,6 +142,7 @@ struct pbf_batch {
     float4* dpb = nullptr;  // lambda-independent part of each delta-p sum (DevParams::dpb)
     float* rho = nullptr;
     uint32_t* lod = nullptr;
+    uint32_t *chits = nullptr, *chit_len = nullptr;  // small batches: hits of a lambda pass (k_coop.cu)
     // autotuner state snapshot
     float4 *save_pos = nullptr, *save_vel = nullptr;
 
@@ -203,6 +204,7 @@ struct pbf_batch {
     void invalidate_graph();
     int step_body();
     int step();
+    void vorticity_pass();
     int substep_body(const float4* src_pos, const float4* src_vel, float4* dst_pos, float4* dst_vel);
     int ad_alloc();
     void ad_free();

@@ -275,13 +275,18 @@ int pbf_handle::ensure_capacity(uint32_t need_n)
         const size_t c = need_n;
         if ((rc = dalloc(pos, c)) || (rc = dalloc(vel, c)) || (rc = dalloc(pred, c)) || (rc = dalloc(aos, 3 * c)) ||
             (rc = dalloc(keys, c)) || (rc = dalloc(ka, c)) || (rc = dalloc(mcode, c)) || (rc = dalloc(mka, c)) ||
-            (rc = dalloc(mia, c)) || (rc = dalloc(mkb, c)) || (rc = dalloc(mib, c)) || (rc = dalloc(ia, c)) || (rc = dalloc(kb, c)) || (rc = dalloc(ib, c)) || (rc = dalloc(sx[0], c)) ||
-            (rc = dalloc(sx[1], c)) || (rc = dalloc(sv, c)) || (rc = dalloc(sx0, c)) || (rc = dalloc(somega, c)) || (rc = dalloc(dpb, c)) ||
+            (rc = dalloc(mia, c)) || (rc = dalloc(mkb, c)) || (rc = dalloc(mib, c)) || (rc = dalloc(ia, c)) || (rc = dalloc(kb, c)) || (rc = dalloc(ib, c)) || (rc = dalloc(sx[0], c + kCoopPad)) ||
+            (rc = dalloc(sx[1], c + kCoopPad)) || (rc = dalloc(sv, c)) || (rc = dalloc(sx0, c + kCoopPad)) || (rc = dalloc(somega, c)) || (rc = dalloc(dpb, c)) ||
             (rc = dalloc(rho, c)) || (rc = dalloc(lod, c)) || (rc = dalloc(cand, 2 * c)) ||
             (rc = dalloc(ct_counts, (size_t)contact_num_blocks(need_n) + 1)))
             return rc;
         if ((rc = dalloc(hist, (size_t)256 * sort_num_tiles(need_n)))) return rc;
         cap_n = need_n;
+    }
+    if (coop_lanes(need_n) && need_n > cap_chits) {
+        cap_chits = 0;
+        if ((rc = dalloc(chits, (size_t)need_n * kCoopList)) || (rc = dalloc(chit_len, need_n))) return rc;
+        cap_chits = need_n;
     }
     if (!totals && (rc = dalloc(totals, 256))) return rc;
     if (!scalars && (rc = dalloc(scalars, 8))) return rc;
@@ -312,7 +317,7 @@ pbf_handle::~pbf_handle()
     for (cudaEvent_t e : event_pool) cudaEventDestroy(e);
     dfree(pos); dfree(vel); dfree(pred); dfree(aos); dfree(keys);
     dfree(mcode); dfree(mka); dfree(mia); dfree(mkb); dfree(mib); dfree(ka); dfree(ia); dfree(kb); dfree(ib);
-    dfree(sx[0]); dfree(sx[1]); dfree(sv); dfree(sx0); dfree(somega); dfree(dpb); dfree(rho); dfree(lod);
+    dfree(sx[0]); dfree(sx[1]); dfree(sv); dfree(sx0); dfree(somega); dfree(dpb); dfree(rho); dfree(lod); dfree(chits); dfree(chit_len);
     dfree(hist); dfree(totals); dfree(table); dfree(cand); dfree(ct_counts); dfree(scalars);
     dfree(lx[0]); dfree(lx[1]); dfree(lxb); dfree(lv); dfree(lx0); dfree(lom); dfree(lrho);
     dfree(lid); dfree(lkey); dfree(inv); dfree(dkey_id);
@@ -379,19 +384,22 @@ int pbf_handle::prof_collect()
 // Mode 8 (dense-window runs) needs label arrays without APBF's per-particle
 // skips and a dense window of the box within 2^26 cells; otherwise the
 // handle runs mode 4 (hashed buckets).  Automatic choice (the default,
-// pass_mode < 0): mode 8 from 2^19 particles, below which its extra
-// relabelling launches cost more than its walk saves (measured crossover
-// between 2.6e5 and 8.8e5 particles), mode 4 below.
+// pass_mode < 0): mode 8 from 2^19 particles, and from 3 * 2^16 where the
+// window has at most 8 cells per particle (its per-substep tables are cleared
+// and scanned whole).  Below, its relabelling launches cost more than its walk
+// saves over mode 4's groups of lanes (k_coop.cu): one step of 151,250
+// particles 1401 us in mode 4 and 1710 in mode 8, 180,000 1653 and 1802,
+// 262,144 2335 and 2202.
 int pbf_handle::effective_mode() const
 {
-    const int mode = pass_mode >= 0 ? pass_mode : (n >= (1u << 19) ? 8 : 4);
-    if (mode == 8 && (derived.enable_apbf || n >= (1u << 27))) return 4;
-    if (mode == 8) {
-        int g0[3];
-        uint32_t nd[3];
-        if (!dense_window(g0, nd)) return 4;
-    }
-    return mode;
+    if (pass_mode >= 0 && pass_mode != 8) return pass_mode;
+    const bool automatic = pass_mode < 0;
+    if ((automatic && n < 3u * (1u << 16)) || derived.enable_apbf || n >= (1u << 27)) return 4;
+    int g0[3];
+    uint32_t nd[3];
+    if (!dense_window(g0, nd)) return 4;
+    const bool roomy = (uint64_t)nd[0] * nd[1] * nd[2] > 8ull * n;
+    return automatic && n < (1u << 19) && roomy ? 4 : 8;
 }
 
 int pbf_handle::ensure_label_capacity()
@@ -701,39 +709,57 @@ int pbf_handle::stage(int st, uint32_t iter)
             prof_end(PBF_STAGE_REORDER);
             break;
         }
-        launch_reorder(P, ids, pos, vel, sx[0], sv, sx0, lod, mcode, sms, stream);
+        // (a group of lanes per particle reads a bucket as one line whatever
+        // the order of the groups: no processing order to sort for)
+        launch_reorder(P, ids, pos, vel, sx[0], sv, sx0, lod, coop_lanes(n) ? nullptr : mcode, sms, stream);
         ++launches;
-        {
+        if (!coop_lanes(n)) {
             uint32_t* msorted = nullptr;
             launch_radix_sort(n, 24, mcode, mka, mia, mkb, mib, hist, totals, &msorted, &order, stream, &launches);
         }
         label_space = false;
+        chit_iter = 0;
         last_x = 0;
         prof_end(PBF_STAGE_REORDER);
         break;
     case PBF_STAGE_LAMBDA:
         prof_begin(PBF_STAGE_LAMBDA);
-        launch_lambda_m(P, sx[0], sx[1], rho, table, lod, iter, order, stream);
+        if (const int G = coop_lanes(n))
+            launch_c_lambda(G, P, nullptr, nullptr, sx[0], sx[1], rho, table, lod, iter, order, chits, chit_len, stream);
+        else
+            launch_lambda_m(P, sx[0], sx[1], rho, table, lod, iter, order, stream);
         ++launches;
+        chit_iter = (int)iter;
         last_x = 1;
         prof_end(PBF_STAGE_LAMBDA);
         break;
     case PBF_STAGE_DELTAP:
         prof_begin(PBF_STAGE_DELTAP);
-        launch_deltap_m(P, sx[1], sx[0], table, lod, iter, order, stream);
+        if (const int G = coop_lanes(n))
+            launch_c_deltap(G, P, nullptr, nullptr, sx[1], sx[0], table, lod, iter, order,
+                            chit_iter == (int)iter ? chits : nullptr, chit_len, stream);
+        else
+            launch_deltap_m(P, sx[1], sx[0], table, lod, iter, order, stream);
         ++launches;
+        chit_iter = 0;
         last_x = 0;
         prof_end(PBF_STAGE_DELTAP);
         break;
     case PBF_STAGE_INTEGRATE:
         prof_begin(PBF_STAGE_INTEGRATE);
-        launch_integrate_m(P, sx[0], sv, sx0, somega, ids, pos, vel, table, order, stream);
+        if (const int G = coop_lanes(n))
+            launch_c_integrate(G, P, nullptr, nullptr, sx[0], sv, sx0, somega, ids, pos, vel, table, order, stream);
+        else
+            launch_integrate_m(P, sx[0], sv, sx0, somega, ids, pos, vel, table, order, stream);
         ++launches;
         prof_end(PBF_STAGE_INTEGRATE);
         break;
     case PBF_STAGE_VORTICITY:
         prof_begin(PBF_STAGE_VORTICITY);
-        launch_vorticity_m(P, sx0, somega, ids, vel, table, order, stream);
+        if (const int G = coop_lanes(n))
+            launch_c_vorticity(G, P, nullptr, nullptr, sx0, somega, ids, vel, table, order, stream);
+        else
+            launch_vorticity_m(P, sx0, somega, ids, vel, table, order, stream);
         ++launches;
         prof_end(PBF_STAGE_VORTICITY);
         break;

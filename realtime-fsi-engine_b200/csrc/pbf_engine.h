@@ -101,6 +101,10 @@ struct pbf_handle {
     float4* dpb = nullptr;     // lambda-independent part of each delta-p sum (DevParams::dpb)
     float* rho = nullptr;
     uint32_t* lod = nullptr;
+    // small scenes: the hits of the latest lambda pass (k_coop.cu)
+    uint32_t *chits = nullptr, *chit_len = nullptr;
+    uint32_t cap_chits = 0;
+    int chit_iter = 0;  // solver iteration that recorded them (0: none)
     // contacts
     float4* cand = nullptr;
     uint32_t* ct_counts = nullptr;

@@ -32,6 +32,31 @@ void launch_integrate_m(const DevParams& P, const float4* xs, const float4* sv, 
 void launch_vorticity_m(const DevParams& P, const float4* spos, const float4* somega, const uint32_t* ids,
                         float4* vel, const int2* table, const uint32_t* order, cudaStream_t st);
 
+// ---- k_coop.cu: the hashed buckets with a group of G lanes per particle ----
+// Lanes per particle for a scene (or batch) of n particles; 0: one thread per
+// particle (k_masked.cu, k_batch.cu).
+int coop_lanes(uint32_t n);
+// The hits of a lambda pass, kept for the delta-p pass of the same iteration:
+// kCoopList slots per sorted slot and their number (list, list_len; null: not kept).
+constexpr int kCoopList = 64;
+// Position arrays hold this many entries past the last sorted slot: a run of
+// up to 8 candidates is loaded whole.
+constexpr int kCoopPad = 8;
+struct SceneDev;  // pbf_batch.h
+// scenes/scene_of: the scenes of a batch (null: one scene, constants in P)
+void launch_c_lambda(int G, const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const float4* xin,
+                     float4* xout, float* rho, const int2* table, const uint32_t* lod, uint32_t iter,
+                     const uint32_t* order, uint32_t* list, uint32_t* list_len, cudaStream_t st);
+void launch_c_deltap(int G, const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const float4* xin,
+                     float4* xout, const int2* table, const uint32_t* lod, uint32_t iter, const uint32_t* order,
+                     const uint32_t* list, const uint32_t* list_len, cudaStream_t st);
+void launch_c_integrate(int G, const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const float4* xs,
+                        const float4* sv, float4* sx0, float4* somega, const uint32_t* ids, float4* pos, float4* vel,
+                        const int2* table, const uint32_t* order, cudaStream_t st);
+void launch_c_vorticity(int G, const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of,
+                        const float4* spos, const float4* somega, const uint32_t* ids, float4* vel, const int2* table,
+                        const uint32_t* order, cudaStream_t st);
+
 // ---- k_dense.cu: x-runs of a dense cell window over relabelled data ----------
 constexpr int kDenseListWords = 16;
 // Label-space position/velocity arrays hold this many entries past the last
@@ -41,7 +66,6 @@ constexpr int kLabelPad = 32;
 // predict-time cells of particles that move towards a wall (x* = x + v dt lies
 // beyond it until the walls clamp it).
 constexpr int kDenseMargin = 6;
-struct SceneDev;  // pbf_batch.h
 // A dense window per scene: one scene (scenes == null), or the scenes of a
 // batch, scene k's window occupying global slots [slot0_k, slot0_k + its
 // cells).  The window fields below describe one window; the passes of a batch

@@ -1,0 +1,82 @@
+"""Neighbour passes with a group of lanes per particle (k_coop.cu) against the
+dense-window passes (k_dense.cu), which walk the same pairs in another way:
+bit-identical.  Sizes at the edges of the group widths (32, 16 and 8 lanes,
+then one thread), buckets of more candidates than a group lists at a time and
+more hits than it keeps, and every s_corr branch."""
+import numpy as np
+import pytest
+
+import pbf_b200 as P
+from pbf_b200 import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def moving_block(n, d, h, seed, hash_size=None):
+    side = int(np.ceil(n ** (1.0 / 3.0)))
+    rng = np.random.default_rng(seed)
+    pos = scenes.lattice(side, side, side, d, (0.0, 0.0, 0.0), 0.0, 0)[:n]
+    pos = np.clip(pos + rng.uniform(-0.2 * d, 0.2 * d, pos.shape), 1e-4, None).astype(np.float32)
+    vel = (rng.normal(size=pos.shape) * 0.1 * d * 120.0).astype(np.float32)
+    box = 1.5 * side * d
+    cfg = scenes.base_config(h, d, (box, box, box), 2, 3, 1.0 / 60.0, n, hash_size)
+    return cfg, pos, vel
+
+
+def stepped(cfg, pos, vel, mode, steps=2):
+    fl = P.PBFluids(cfg)
+    fl.set_option(1, mode)
+    fl.setParticles(P.make_particles(pos, vel))
+    for _ in range(steps):
+        fl.step()
+    return fl.readbackParticles()
+
+
+def same(a, b):
+    return np.array_equal(a["pos"], b["pos"]) and np.array_equal(a["vel"], b["vel"])
+
+
+@pytest.mark.parametrize("n", [1, 2, 33, 1000, 4096, 4097, 8192, 8193, 1 << 18, (1 << 18) + 1])
+def test_group_widths_are_bit_identical_to_dense_windows(have_gpu, n):
+    cfg, pos, vel = moving_block(n, 0.02, 0.04, n)
+    assert same(stepped(cfg, pos, vel, 4), stepped(cfg, pos, vel, 8))
+
+
+@pytest.mark.parametrize("n", [3000, 6000, 9000])
+@pytest.mark.parametrize("d,hash_size", [(0.02, 64), (0.011, 1 << 15), (0.011, 16)])
+def test_long_buckets_and_many_hits(have_gpu, n, d, hash_size):
+    """64 buckets of a hundred particles and more, 200 hits a particle."""
+    cfg, pos, vel = moving_block(n, d, 0.04, 7, hash_size)
+    assert same(stepped(cfg, pos, vel, 4, 1), stepped(cfg, pos, vel, 8, 1))
+
+
+@pytest.mark.parametrize("n", [2000, 6000, 12000])
+@pytest.mark.parametrize("change", [dict(enable_scorr=0), dict(n_corr=3.0), dict(enable_viscosity=0),
+                                    dict(enable_vorticity=0), dict(enable_viscosity=0, enable_vorticity=0)])
+def test_options(have_gpu, n, change):
+    cfg, pos, vel = moving_block(n, 0.02, 0.04, 11)
+    for k, v in change.items():
+        setattr(cfg, k, v)
+    assert same(stepped(cfg, pos, vel, 4), stepped(cfg, pos, vel, 8))
+
+
+@pytest.mark.parametrize("sizes", [[1], [700, 1, 1500], [3000, 5200, 4100], [70000, 1, 131000]])
+def test_batches(have_gpu, sizes):
+    from pbf_b200 import batch as PB
+    cfg, sc = scenes.c3(5, len(sizes), sizes)
+    out = []
+    for mode in (4, 8):
+        b = PB.make_batch(cfg, sc)
+        b.set_option(P.BOPT_NEIGHBOUR_MODE, mode)
+        for _ in range(2):
+            b.step()
+        out.append(b.read_particles())
+    assert same(*out)
+
+
+def test_coincident_particles(have_gpu):
+    """r = 0 pairs: density without a gradient."""
+    cfg, pos, vel = moving_block(3000, 0.02, 0.04, 13)
+    pos[1::2] = pos[::2]
+    vel[1::2] = vel[::2]
+    assert same(stepped(cfg, pos, vel, 4), stepped(cfg, pos, vel, 8))
