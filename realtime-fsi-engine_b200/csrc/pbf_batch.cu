@@ -211,16 +211,32 @@ int pbf_batch::upload_scenes()
         w[7 * k + 6] = (int)d.slot0;
     }
     if (!fits) total = 1ull << 40;  // no dense windows (dense_fits() is false)
-    if (w != win || total != dense_total) dense_ready = false;
+    // Kernels read the scenes' constants from scenes_dev, so the captured graphs
+    // stay valid when only those change (a new graph costs 5 ms for a recorded
+    // step of 16 substeps); the windows and the Morton code widths are kernel
+    // arguments.
+    bool recapture = false;
+    if (w != win || total != dense_total) {
+        dense_ready = false;
+        recapture = true;
+    }
     win = w;
     dense_total = total;
     const uint32_t sbits = ceil_log2(scenes.size());
+    const uint32_t mbits_was = mbits, order_bits_was = order_bits;
     mbits = std::min<uint32_t>(std::max<uint32_t>(ceil_log2(max_span), 1u), 10u);
     while (sbits + 3 * mbits > 32) --mbits;
     order_bits = sbits + 3 * mbits;
+    if (mbits != mbits_was || order_bits != order_bits_was) recapture = true;
+    if (recapture) invalidate_graph();
+    if (hs.size() == scenes_host.size() &&
+        std::memcmp(hs.data(), scenes_host.data(), sizeof(SceneDev) * hs.size()) == 0)
+        return PBF_OK;
+    scenes_host.clear();
     BCK(cudaMemcpyAsync(scenes_dev, hs.data(), sizeof(SceneDev) * hs.size(), cudaMemcpyHostToDevice, stream));
     BCK(cudaStreamSynchronize(stream));
-    invalidate_graph();
+    scenes_host.swap(hs);
+    ++scenes_gen;
     return PBF_OK;
 }
 
@@ -689,6 +705,8 @@ extern "C" int pbf_batch_set_sdf_grid(pbf_batch* b, uint32_t scene, const float*
     launch_sdf_slab_min(s.grid, dims[0], dims[1], dims[2], s.slab_min, b->stream);
     ++b->launches;
     s.sdf_on = true;
+    ++b->scenes_gen;  // the grid's contents
+    BCK(cudaStreamSynchronize(b->stream));
     return b->upload_scenes();
 }
 

@@ -130,6 +130,8 @@ struct pbf_batch {
     float4 *pos = nullptr, *vel = nullptr, *pred = nullptr, *aos = nullptr;
     uint16_t* scene_of = nullptr;
     pbf::SceneDev* scenes_dev = nullptr;
+    std::vector<pbf::SceneDev> scenes_host;  // what scenes_dev holds
+    uint64_t scenes_gen = 0;                 // changes of the scenes' constants or SDF grids
     uint32_t* keys = nullptr;
     uint32_t *ka = nullptr, *ia = nullptr, *kb = nullptr, *ib = nullptr;
     uint32_t *skeys = nullptr, *ids = nullptr;
