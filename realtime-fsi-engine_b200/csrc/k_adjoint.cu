@@ -14,7 +14,7 @@
 //   dW/d(r^2)  = -3 K6 (h^2 - r^2)^2
 //   ds/d(r^2)  = Ks (h - q)(h + q) / (2 q^3)          (s = -Ks (h - q)^2 / q)
 //   adjoint of a = r s given a_bar: r_bar = s a_bar + 2 ds (r . a_bar) r
-#include "masked_body.cuh"
+#include "coop_walk.cuh"
 #include "pbf_batch.h"
 
 namespace pbf {
@@ -249,35 +249,19 @@ __global__ void __launch_bounds__(kAThreads) k_ad_vorticity(DevParams P, const S
 }
 
 // ---- CS_Integrate.glsl:135-280 reversed -------------------------------------------------------
-// (posb, velb) particle order (+ posb_s sorted, omb sorted when the vorticity
-// pass was reversed) -> gx (adjoint of x*), gv (of v'), x0b, tgrad.
-__global__ void __launch_bounds__(kAThreads, kAdjBlocks) k_ad_integrate(
-    DevParams P, const SceneDev* __restrict__ scenes, const uint16_t* __restrict__ scene_of,
-    const uint32_t* __restrict__ order, const int2* __restrict__ table, const float4* __restrict__ xs,
-    const float4* __restrict__ sv, const float4* __restrict__ cp_pos, const uint32_t* __restrict__ ids,
-    const float4* __restrict__ posb, const float4* __restrict__ velb, const float4* __restrict__ posb_s,
-    const float4* __restrict__ omb, const float4* __restrict__ somega, float4* __restrict__ gx,
-    float4* __restrict__ gv, float4* __restrict__ x0b, float* __restrict__ tgrad)
+// The per-particle part: from the adjoints of the committed state (pb, vb;
+// posb_s, omb of the vorticity reverse, or null) and the XSPH sum f, the own
+// adjoints of x* before the pair terms, x0 (written), the sums' adjoints vfb
+// (XSPH) and cb (curl), and the SDF translation's (tb).
+struct IntegrateAdjoint {
+    float3 own, vfb, cb, tb;
+};
+__device__ __forceinline__ IntegrateAdjoint integrate_adjoint(const DevParams& P, const SceneDev* SC, int s, uint32_t id,
+                                                              float4 x4, float4 p0, float3 f, float4 pb4, float4 vb4,
+                                                              const float4* posb_s, const float4* omb,
+                                                              const float4* __restrict__ somega, float4& x0b)
 {
-    AD_PROLOGUE
     const SdfDev sdf = load_sdf(SC);
-    const float4 x4 = __ldg(xs + s);
-    const float4 v0 = __ldg(sv + s);
-    const uint32_t id = __ldg(ids + s);
-    const float4 p0 = __ldg(cp_pos + id);
-    float fx = 0.f, fy = 0.f, fz = 0.f;
-    if (P.visc_on) {
-        masked_walk(P, tab, mask, xs, x4.x, x4.y, x4.z, s, [&](float r2) { return r2 <= P.h2; }, [&](int k) {
-            const float4 xj = __ldg(xs + k);
-            const float rx = x4.x - xj.x, ry = x4.y - xj.y, rz = x4.z - xj.z;
-            const float r2 = rx * rx + ry * ry + rz * rz;
-            const float4 vj = __ldg(sv + k);
-            const float w = poly6_in(P, r2) * P.inv_rho0;
-            fx += (vj.x - v0.x) * w;
-            fy += (vj.y - v0.y) * w;
-            fz += (vj.z - v0.z) * w;
-        });
-    }
     float bmin[3], bmax[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -298,9 +282,9 @@ __global__ void __launch_bounds__(kAThreads, kAdjBlocks) k_ad_integrate(
     if (sdf.enabled) col_sdf = sdf_project(sdf, x, nrm);
     float vdx = 0.f, vdy = 0.f, vdz = 0.f;
     if (P.visc_on) {
-        vdx = fx * P.viscosity;
-        vdy = fy * P.viscosity;
-        vdz = fz * P.viscosity;
+        vdx = f.x * P.viscosity;
+        vdy = f.y * P.viscosity;
+        vdz = f.z * P.viscosity;
     }
     const float v1x = (x.x - p0.x) * P.inv_dt + vdx, v1y = (x.y - p0.y) * P.inv_dt + vdy,
                 v1z = (x.z - p0.z) * P.inv_dt + vdz;
@@ -315,7 +299,6 @@ __global__ void __launch_bounds__(kAThreads, kAdjBlocks) k_ad_integrate(
     const float v3x = colx ? v2x * -P.damping : v2x, v3y = coly ? v2y * -P.damping : v2y,
                 v3z = colz ? v2z * -P.damping : v2z;
     // reverse
-    const float4 vb4 = __ldg(velb + id);
     float3 vb = make_float3(vb4.x, vb4.y, vb4.z);
     float3 nb = make_float3(0.f, 0.f, 0.f);
     if (col_sdf) {
@@ -334,7 +317,6 @@ __global__ void __launch_bounds__(kAThreads, kAdjBlocks) k_ad_integrate(
         const float k = 50.0f / len;
         vb = make_float3(k * (vb.x - ux * ub), k * (vb.y - uy * ub), k * (vb.z - uz * ub));
     }
-    const float4 pb4 = __ldg(posb + id);
     float3 xb = make_float3(pb4.x + vb.x * P.inv_dt, pb4.y + vb.y * P.inv_dt, pb4.z + vb.z * P.inv_dt);
     if (posb_s) {
         const float4 q = posb_s[s];
@@ -342,54 +324,94 @@ __global__ void __launch_bounds__(kAThreads, kAdjBlocks) k_ad_integrate(
         xb.y += q.y;
         xb.z += q.z;
     }
-    x0b[s] = make_float4(-vb.x * P.inv_dt, -vb.y * P.inv_dt, -vb.z * P.inv_dt, 0.0f);
-    float3 tb = make_float3(0.f, 0.f, 0.f);
-    if (col_sdf) project_vjp(sdf, xw, xb, nb, tb);
-    add_t(tgrad, sid, tb);
-    float3 own = make_float3(colx ? 0.f : xb.x, coly ? 0.f : xb.y, colz ? 0.f : xb.z);
-    float3 vfb = make_float3(0.f, 0.f, 0.f), cb = make_float3(0.f, 0.f, 0.f);
-    if (P.visc_on) vfb = make_float3(vb.x * P.viscosity, vb.y * P.viscosity, vb.z * P.viscosity);
+    x0b = make_float4(-vb.x * P.inv_dt, -vb.y * P.inv_dt, -vb.z * P.inv_dt, 0.0f);
+    IntegrateAdjoint r;
+    r.tb = make_float3(0.f, 0.f, 0.f);
+    if (col_sdf) project_vjp(sdf, xw, xb, nb, r.tb);
+    r.own = make_float3(colx ? 0.f : xb.x, coly ? 0.f : xb.y, colz ? 0.f : xb.z);
+    r.vfb = make_float3(0.f, 0.f, 0.f);
+    r.cb = make_float3(0.f, 0.f, 0.f);
+    if (P.visc_on) r.vfb = make_float3(vb.x * P.viscosity, vb.y * P.viscosity, vb.z * P.viscosity);
     if (P.vort_on && omb) {
         const float4 o = omb[s];
         const float4 w = __ldg(somega + s);
         float kx = 0.f;
         if (w.w > 0.0f) kx = o.w / w.w;
-        cb = make_float3((o.x + kx * w.x) * P.inv_rho0, (o.y + kx * w.y) * P.inv_rho0, (o.z + kx * w.z) * P.inv_rho0);
+        r.cb = make_float3((o.x + kx * w.x) * P.inv_rho0, (o.y + kx * w.y) * P.inv_rho0, (o.z + kx * w.z) * P.inv_rho0);
     }
-    float3 vown = make_float3(0.f, 0.f, 0.f);
-    const bool need_walk = P.visc_on || (P.vort_on && omb);
-    if (need_walk) {
+    return r;
+}
+
+// A pair's share: ub, rb of the own velocity difference and r = x_i - x_j.
+__device__ __forceinline__ void integrate_pair_adjoint(const DevParams& P, float4 x4, float4 v0, float4 xj, float4 vj,
+                                                       float3 vfb, float3 cb, bool curl, float3& ub, float3& rb)
+{
+    const float rx = x4.x - xj.x, ry = x4.y - xj.y, rz = x4.z - xj.z;
+    const float r2 = rx * rx + ry * ry + rz * rz;
+    const float ux = vj.x - v0.x, uy = vj.y - v0.y, uz = vj.z - v0.z;
+    ub = make_float3(0.f, 0.f, 0.f);
+    rb = make_float3(0.f, 0.f, 0.f);
+    if (P.visc_on) {
+        const float w = poly6_in(P, r2) * P.inv_rho0;
+        ub = make_float3(vfb.x * w, vfb.y * w, vfb.z * w);
+        const float kk = (vfb.x * ux + vfb.y * uy + vfb.z * uz) * P.inv_rho0 * poly6_d(P, r2) * 2.0f;
+        rb = make_float3(kk * rx, kk * ry, kk * rz);
+    }
+    if (curl && r2 >= 1e-10f) {
+        const float sg = spiky_scale(P, r2);
+        const float gx_ = rx * sg, gy_ = ry * sg, gz_ = rz * sg;
+        ub.x += gy_ * cb.z - gz_ * cb.y;
+        ub.y += gz_ * cb.x - gx_ * cb.z;
+        ub.z += gx_ * cb.y - gy_ * cb.x;
+        const float3 gb = make_float3(cb.y * uz - cb.z * uy, cb.z * ux - cb.x * uz, cb.x * uy - cb.y * ux);
+        const float3 r2b = grad_vjp(P, rx, ry, rz, r2, gb);
+        rb.x += r2b.x;
+        rb.y += r2b.y;
+        rb.z += r2b.z;
+    }
+}
+
+// (posb, velb) particle order (+ posb_s sorted, omb sorted when the vorticity
+// pass was reversed) -> gx (adjoint of x*), gv (of v'), x0b, tgrad.
+__global__ void __launch_bounds__(kAThreads, kAdjBlocks) k_ad_integrate(
+    DevParams P, const SceneDev* __restrict__ scenes, const uint16_t* __restrict__ scene_of,
+    const uint32_t* __restrict__ order, const int2* __restrict__ table, const float4* __restrict__ xs,
+    const float4* __restrict__ sv, const float4* __restrict__ cp_pos, const uint32_t* __restrict__ ids,
+    const float4* __restrict__ posb, const float4* __restrict__ velb, const float4* __restrict__ posb_s,
+    const float4* __restrict__ omb, const float4* __restrict__ somega, float4* __restrict__ gx,
+    float4* __restrict__ gv, float4* __restrict__ x0b, float* __restrict__ tgrad)
+{
+    AD_PROLOGUE
+    const float4 x4 = __ldg(xs + s);
+    const float4 v0 = __ldg(sv + s);
+    const uint32_t id = __ldg(ids + s);
+    const float4 p0 = __ldg(cp_pos + id);
+    float fx = 0.f, fy = 0.f, fz = 0.f;
+    if (P.visc_on) {
         masked_walk(P, tab, mask, xs, x4.x, x4.y, x4.z, s, [&](float r2) { return r2 <= P.h2; }, [&](int k) {
             const float4 xj = __ldg(xs + k);
             const float rx = x4.x - xj.x, ry = x4.y - xj.y, rz = x4.z - xj.z;
             const float r2 = rx * rx + ry * ry + rz * rz;
             const float4 vj = __ldg(sv + k);
-            const float ux = vj.x - v0.x, uy = vj.y - v0.y, uz = vj.z - v0.z;
-            float3 ub = make_float3(0.f, 0.f, 0.f), rb = make_float3(0.f, 0.f, 0.f);
-            if (P.visc_on) {
-                const float w = poly6_in(P, r2) * P.inv_rho0;
-                ub = make_float3(vfb.x * w, vfb.y * w, vfb.z * w);
-                const float kk = (vfb.x * ux + vfb.y * uy + vfb.z * uz) * P.inv_rho0 * poly6_d(P, r2) * 2.0f;
-                rb = make_float3(kk * rx, kk * ry, kk * rz);
-            }
-            if (P.vort_on && omb && r2 >= 1e-10f) {
-                const float sg = spiky_scale(P, r2);
-                const float gx_ = rx * sg, gy_ = ry * sg, gz_ = rz * sg;
-                ub.x += gy_ * cb.z - gz_ * cb.y;
-                ub.y += gz_ * cb.x - gx_ * cb.z;
-                ub.z += gx_ * cb.y - gy_ * cb.x;
-                const float3 gb = make_float3(cb.y * uz - cb.z * uy, cb.z * ux - cb.x * uz, cb.x * uy - cb.y * ux);
-                const float3 r2b = grad_vjp(P, rx, ry, rz, r2, gb);
-                rb.x += r2b.x;
-                rb.y += r2b.y;
-                rb.z += r2b.z;
-            }
-            own.x += rb.x;
-            own.y += rb.y;
-            own.z += rb.z;
-            vown.x -= ub.x;
-            vown.y -= ub.y;
-            vown.z -= ub.z;
+            const float w = poly6_in(P, r2) * P.inv_rho0;
+            fx += (vj.x - v0.x) * w;
+            fy += (vj.y - v0.y) * w;
+            fz += (vj.z - v0.z) * w;
+        });
+    }
+    float4 x0a;
+    const IntegrateAdjoint A = integrate_adjoint(P, SC, s, id, x4, p0, make_float3(fx, fy, fz), __ldg(posb + id),
+                                                 __ldg(velb + id), posb_s, omb, somega, x0a);
+    x0b[s] = x0a;
+    add_t(tgrad, sid, A.tb);
+    float3 own = A.own, vown = make_float3(0.f, 0.f, 0.f);
+    const bool curl = P.vort_on && omb;
+    if (P.visc_on || curl) {
+        masked_walk(P, tab, mask, xs, x4.x, x4.y, x4.z, s, [&](float r2) { return r2 <= P.h2; }, [&](int k) {
+            float3 ub, rb;
+            integrate_pair_adjoint(P, x4, v0, __ldg(xs + k), __ldg(sv + k), A.vfb, A.cb, curl, ub, rb);
+            own = make_float3(own.x + rb.x, own.y + rb.y, own.z + rb.z);
+            vown = make_float3(vown.x - ub.x, vown.y - ub.y, vown.z - ub.z);
             atomicAdd(gx + k, make_float4(-rb.x, -rb.y, -rb.z, 0.0f));
             atomicAdd(gv + k, make_float4(ub.x, ub.y, ub.z, 0.0f));
         });
@@ -399,6 +421,55 @@ __global__ void __launch_bounds__(kAThreads, kAdjBlocks) k_ad_integrate(
 }
 
 // ---- CS_ComputeDeltaP.glsl:120-166 + CS_ApplyDeltaP.glsl:80-124 reversed --------------------
+// The per-particle part: from the adjoint xb of this iteration's output x*
+// (in) the adjoint of x* + dp (out), of the scaled sum (returned), and the SDF
+// translation's (tb).
+__device__ __forceinline__ float3 deltap_adjoint(const DevParams& P, const SceneDev* SC, float4 xi, float4 dp,
+                                                 float3& xb, float3& tb)
+{
+    float dx = dp.x, dy = dp.y, dz = dp.z;
+    const float l2 = dx * dx + dy * dy + dz * dz;
+    const bool clamped = l2 > P.max_dp * P.max_dp;
+    if (clamped) {
+        const float sc = P.max_dp * rsqrtf(l2);
+        dx *= sc;
+        dy *= sc;
+        dz *= sc;
+    }
+    const float3 x = make_float3(xi.x + dx, xi.y + dy, xi.z + dz);
+    tb = make_float3(0.f, 0.f, 0.f);
+    const SdfDev sdf = load_sdf(SC);
+    if (sdf.enabled) project_vjp(sdf, x, xb, make_float3(0.f, 0.f, 0.f), tb);
+    float3 dpb = xb;
+    if (clamped) {
+        const float len = sqrtf(l2);
+        const float ux = dp.x / len, uy = dp.y / len, uz = dp.z / len;
+        const float ub = ux * xb.x + uy * xb.y + uz * xb.z;
+        const float k = P.max_dp / len;
+        dpb = make_float3(k * (xb.x - ux * ub), k * (xb.y - uy * ub), k * (xb.z - uz * ub));
+    }
+    return make_float3(dpb.x * P.inv_rho0, dpb.y * P.inv_rho0, dpb.z * P.inv_rho0);
+}
+
+// A pair's share: rb of r = x_i - x_j, ga of lambda_i and of lambda_j.
+__device__ __forceinline__ void deltap_pair_adjoint(const DevParams& P, float4 xi, float4 xj, float3 accb, float3& rb,
+                                                    float& ga)
+{
+    const float rx = xi.x - xj.x, ry = xi.y - xj.y, rz = xi.z - xj.z;
+    const float r2 = rx * rx + ry * ry + rz * rz;
+    const float sg = spiky_scale(P, r2);
+    float f = xi.w + xj.w;
+    if (P.scorr) f += scorr_term(P, r2);
+    ga = sg * (rx * accb.x + ry * accb.y + rz * accb.z);
+    rb = grad_vjp(P, rx, ry, rz, r2, make_float3(f * accb.x, f * accb.y, f * accb.z));
+    if (P.scorr) {
+        const float kk = ga * scorr_d(P, r2) * 2.0f;
+        rb.x += kk * rx;
+        rb.y += kk * ry;
+        rb.z += kk * rz;
+    }
+}
+
 // gin (adjoint of this iteration's output x*) -> gout.xyz (adjoint of the
 // input x*) and gout.w (adjoint of lambda), tgrad.
 __global__ void __launch_bounds__(kAThreads, kAdjBlocks) k_ad_deltap(DevParams P, const SceneDev* __restrict__ scenes,
@@ -413,62 +484,63 @@ __global__ void __launch_bounds__(kAThreads, kAdjBlocks) k_ad_deltap(DevParams P
     AD_PROLOGUE
     const float4 xi = __ldg(xl + s);
     const float4 g4 = gin[s];
-    const float4 dp = __ldg(auxd + s);
-    float dx = dp.x, dy = dp.y, dz = dp.z;
-    const float l2 = dx * dx + dy * dy + dz * dz;
-    const bool clamped = l2 > P.max_dp * P.max_dp;
-    if (clamped) {
-        const float sc = P.max_dp * rsqrtf(l2);
-        dx *= sc;
-        dy *= sc;
-        dz *= sc;
-    }
-    const float3 x = make_float3(xi.x + dx, xi.y + dy, xi.z + dz);
-    float3 xb = make_float3(g4.x, g4.y, g4.z);
-    const SdfDev sdf = load_sdf(SC);
-    if (sdf.enabled) {
-        float3 tb = make_float3(0.f, 0.f, 0.f);
-        project_vjp(sdf, x, xb, make_float3(0.f, 0.f, 0.f), tb);
-        add_t(tgrad, sid, tb);
-    }
-    float3 dpb = xb;
-    if (clamped) {
-        const float len = sqrtf(l2);
-        const float ux = dp.x / len, uy = dp.y / len, uz = dp.z / len;
-        const float ub = ux * xb.x + uy * xb.y + uz * xb.z;
-        const float k = P.max_dp / len;
-        dpb = make_float3(k * (xb.x - ux * ub), k * (xb.y - uy * ub), k * (xb.z - uz * ub));
-    }
-    const float3 accb = make_float3(dpb.x * P.inv_rho0, dpb.y * P.inv_rho0, dpb.z * P.inv_rho0);
-    float3 own = xb;
+    float3 own = make_float3(g4.x, g4.y, g4.z), tb;
+    const float3 accb = deltap_adjoint(P, SC, xi, __ldg(auxd + s), own, tb);
+    add_t(tgrad, sid, tb);
     float lown = 0.0f;
-    const float li = xi.w;
     masked_walk(P, tab, mask, xl, xi.x, xi.y, xi.z, s, [&](float r2) { return r2 <= P.h2 && r2 >= 1e-10f; },
                 [&](int k) {
-                    const float4 xj = __ldg(xl + k);
-                    const float rx = xi.x - xj.x, ry = xi.y - xj.y, rz = xi.z - xj.z;
-                    const float r2 = rx * rx + ry * ry + rz * rz;
-                    const float sg = spiky_scale(P, r2);
-                    float f = li + xj.w;
-                    if (P.scorr) f += scorr_term(P, r2);
-                    const float ga = sg * (rx * accb.x + ry * accb.y + rz * accb.z);
+                    float3 rb;
+                    float ga;
+                    deltap_pair_adjoint(P, xi, __ldg(xl + k), accb, rb, ga);
                     lown += ga;
-                    float3 rb = grad_vjp(P, rx, ry, rz, r2, make_float3(f * accb.x, f * accb.y, f * accb.z));
-                    if (P.scorr) {
-                        const float kk = ga * scorr_d(P, r2) * 2.0f;
-                        rb.x += kk * rx;
-                        rb.y += kk * ry;
-                        rb.z += kk * rz;
-                    }
-                    own.x += rb.x;
-                    own.y += rb.y;
-                    own.z += rb.z;
+                    own = make_float3(own.x + rb.x, own.y + rb.y, own.z + rb.z);
                     atomicAdd(gout + k, make_float4(-rb.x, -rb.y, -rb.z, ga));
                 });
     add_own(gout + s, own, lown);
 }
 
-// ---- CS_ComputeLambdas.glsl:108-162 reversed: gout.w (lambda adjoint) -> gout.xyz ---------------
+// ---- CS_ComputeLambdas.glsl:108-162 reversed ----------------------------------------------------
+// The adjoints of a particle's sums from lambda's (lb): rhob of rho, gsb of
+// sum gradW, k2 of sum |gradW|^2.
+struct LambdaAdjoint {
+    float rhob, k2;
+    float3 gsb;
+};
+__device__ __forceinline__ LambdaAdjoint lambda_adjoint(const DevParams& P, float lb, float4 aux, float rho)
+{
+    const float craw = rho / P.rho0 - 1.0f;
+    const float C = fmaxf(craw, -P.cohesion);
+    const float den = aux.w;
+    const float Cb = -lb / den;
+    const float Db = lb * C / (den * den);
+    LambdaAdjoint r;
+    r.rhob = (craw < -P.cohesion) ? 0.0f : Cb / P.rho0;
+    r.gsb = make_float3(Db * 2.0f * aux.x * P.inv_rho0, Db * 2.0f * aux.y * P.inv_rho0,
+                        Db * 2.0f * aux.z * P.inv_rho0);
+    r.k2 = Db * 2.0f * P.inv_rho0_sq;
+    return r;
+}
+
+// A pair's share of r = x_i - x_j.
+__device__ __forceinline__ float3 lambda_pair_adjoint(const DevParams& P, float4 xi, float4 xj, const LambdaAdjoint& A)
+{
+    const float rx = xi.x - xj.x, ry = xi.y - xj.y, rz = xi.z - xj.z;
+    const float r2 = rx * rx + ry * ry + rz * rz;
+    const float kp = A.rhob * poly6_d(P, r2) * 2.0f;
+    float3 rb = make_float3(kp * rx, kp * ry, kp * rz);
+    if (r2 >= 1e-10f) {
+        const float sg = spiky_scale(P, r2);
+        const float3 ab = make_float3(A.k2 * rx * sg + A.gsb.x, A.k2 * ry * sg + A.gsb.y, A.k2 * rz * sg + A.gsb.z);
+        const float3 r2b = grad_vjp(P, rx, ry, rz, r2, ab);
+        rb.x += r2b.x;
+        rb.y += r2b.y;
+        rb.z += r2b.z;
+    }
+    return rb;
+}
+
+// gout.w (adjoint of lambda) -> gout.xyz
 __global__ void __launch_bounds__(kAThreads, kAdjBlocks) k_ad_lambda(DevParams P, const SceneDev* __restrict__ scenes,
                                                          const uint16_t* __restrict__ scene_of,
                                                          const uint32_t* __restrict__ order,
@@ -481,38 +553,167 @@ __global__ void __launch_bounds__(kAThreads, kAdjBlocks) k_ad_lambda(DevParams P
     const float lb = gout[s].w;
     if (lb == 0.0f) return;
     const float4 xi = __ldg(xl + s);
-    const float4 aux = __ldg(auxl + s);
-    const float rho = __ldg(rhol + s);
-    const float craw = rho / P.rho0 - 1.0f;
-    const float C = fmaxf(craw, -P.cohesion);
-    const float den = aux.w;
-    const float Cb = -lb / den;
-    const float Db = lb * C / (den * den);
-    const float rhob = (craw < -P.cohesion) ? 0.0f : Cb / P.rho0;
-    const float3 gsb = make_float3(Db * 2.0f * aux.x * P.inv_rho0, Db * 2.0f * aux.y * P.inv_rho0,
-                                   Db * 2.0f * aux.z * P.inv_rho0);
-    const float k2 = Db * 2.0f * P.inv_rho0_sq;
+    const LambdaAdjoint A = lambda_adjoint(P, lb, __ldg(auxl + s), __ldg(rhol + s));
     float3 own = make_float3(0.f, 0.f, 0.f);
     masked_walk(P, tab, mask, xl, xi.x, xi.y, xi.z, s, [&](float r2) { return r2 <= P.h2; }, [&](int k) {
-        const float4 xj = __ldg(xl + k);
-        const float rx = xi.x - xj.x, ry = xi.y - xj.y, rz = xi.z - xj.z;
-        const float r2 = rx * rx + ry * ry + rz * rz;
-        const float kp = rhob * poly6_d(P, r2) * 2.0f;
-        float3 rb = make_float3(kp * rx, kp * ry, kp * rz);
-        if (r2 >= 1e-10f) {
-            const float sg = spiky_scale(P, r2);
-            const float3 ab = make_float3(k2 * rx * sg + gsb.x, k2 * ry * sg + gsb.y, k2 * rz * sg + gsb.z);
-            const float3 r2b = grad_vjp(P, rx, ry, rz, r2, ab);
-            rb.x += r2b.x;
-            rb.y += r2b.y;
-            rb.z += r2b.z;
-        }
-        own.x += rb.x;
-        own.y += rb.y;
-        own.z += rb.z;
+        const float3 rb = lambda_pair_adjoint(P, xi, __ldg(xl + k), A);
+        own = make_float3(own.x + rb.x, own.y + rb.y, own.z + rb.z);
         atomicAdd(gout + k, make_float4(-rb.x, -rb.y, -rb.z, 0.0f));
     });
     add_own(gout + s, own, 0.0f);
+}
+
+// ---- the same with a group of G lanes per particle (small batches) --------------------------------
+// The pairs come from the hits the recording passes kept, one per lane; where
+// a particle had more than fit, its buckets are walked.  One thread walking
+// the buckets took 36 us a pass at 32,768 particles whatever the pass does.
+struct CoopHits {
+    const uint32_t* list;      // kCoopList slots per sorted slot
+    const uint32_t* list_len;  // their number, kNoHits: walk
+};
+
+template <class F>
+struct CoopEach {  // coop_walk's hits one per lane, in no order
+    int gl, G;
+    F f;
+    template <class HitAt>
+    __device__ __forceinline__ void add(int cnt, HitAt&& hit)
+    {
+        for (int h = gl; h < cnt; h += G) f(hit(h));
+        __syncwarp();
+    }
+};
+
+// f(k) for every hit of particle s (itself left out), over the group's lanes
+template <int G, class F>
+__device__ __forceinline__ void coop_each(const DevParams& P, const int2* __restrict__ tab, uint32_t mask,
+                                          const float4* __restrict__ X, float4 xi, int s, bool on, CoopHits H,
+                                          CoopMem<G, 1>& M, F&& f)
+{
+    const int gl = threadIdx.x & (G - 1);
+    auto other = [&](int k) {
+        if (k != s) f(k);
+    };
+    const uint32_t len = on ? __ldg(H.list_len + s) : 0u;
+    if (__any_sync(0xffffffffu, len == kNoHits)) {
+        CoopEach<decltype(other)> each{gl, G, other};
+        coop_walk<G, 1>(P, tab, mask, X, xi, len == kNoHits, M, each, [&](float r2) { return r2 <= P.h2; }, nullptr,
+                        nullptr);
+    }
+    if (len != kNoHits) {
+        const uint32_t* mine = H.list + (size_t)s * kCoopList;
+        for (uint32_t h = gl; h < len; h += G) other((int)__ldg(mine + h));
+    }
+    __syncwarp();
+}
+
+template <int G>
+__device__ __forceinline__ float group_sum(float v)
+{
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o, G);
+    return v;
+}
+template <int G>
+__device__ __forceinline__ float3 group_sum(float3 v)
+{
+    return make_float3(group_sum<G>(v.x), group_sum<G>(v.y), group_sum<G>(v.z));
+}
+
+#define AD_COOP_PROLOGUE                                                                            \
+    __shared__ __align__(16) CoopMem<G, 1> mem[kCThreads / G];                                      \
+    const CoopParticle cp = coop_particle<G>(P.n, nullptr);                                         \
+    const int s = cp.s, gl = threadIdx.x & (G - 1);                                                 \
+    const int sid = (int)__ldg(scene_of + s);                                                       \
+    const SceneDev* SC = scenes + sid;                                                              \
+    const int2* tab = table + __ldg(&SC->table_off);                                                \
+    const uint32_t mask = __ldg(&SC->mask);
+
+template <int G>
+__global__ void __launch_bounds__(kCThreads, kCBlocks) k_ac_integrate(
+    DevParams P, const SceneDev* __restrict__ scenes, const uint16_t* __restrict__ scene_of,
+    const int2* __restrict__ table, CoopHits H, const float4* __restrict__ fsum, const float4* __restrict__ xs,
+    const float4* __restrict__ sv, const float4* __restrict__ cp_pos, const uint32_t* __restrict__ ids,
+    const float4* __restrict__ posb, const float4* __restrict__ velb, const float4* __restrict__ posb_s,
+    const float4* __restrict__ omb, const float4* __restrict__ somega, float4* __restrict__ gx,
+    float4* __restrict__ gv, float4* __restrict__ x0b, float* __restrict__ tgrad)
+{
+    AD_COOP_PROLOGUE
+    const float4 x4 = __ldg(xs + s), v0 = __ldg(sv + s), f4 = __ldg(fsum + s);
+    const uint32_t id = __ldg(ids + s);
+    float4 x0a;
+    const IntegrateAdjoint A = integrate_adjoint(P, SC, s, id, x4, __ldg(cp_pos + id), make_float3(f4.x, f4.y, f4.z),
+                                                 __ldg(posb + id), __ldg(velb + id), posb_s, omb, somega, x0a);
+    const bool curl = P.vort_on && omb;
+    float3 own = make_float3(0.f, 0.f, 0.f), vown = make_float3(0.f, 0.f, 0.f);
+    coop_each<G>(P, tab, mask, xs, x4, s, cp.live && (P.visc_on || curl), H, mem[threadIdx.x / G], [&](int k) {
+        float3 ub, rb;
+        integrate_pair_adjoint(P, x4, v0, __ldg(xs + k), __ldg(sv + k), A.vfb, A.cb, curl, ub, rb);
+        own = make_float3(own.x + rb.x, own.y + rb.y, own.z + rb.z);
+        vown = make_float3(vown.x - ub.x, vown.y - ub.y, vown.z - ub.z);
+        atomicAdd(gx + k, make_float4(-rb.x, -rb.y, -rb.z, 0.0f));
+        atomicAdd(gv + k, make_float4(ub.x, ub.y, ub.z, 0.0f));
+    });
+    own = group_sum<G>(own);
+    vown = group_sum<G>(vown);
+    if (!cp.live || gl != 0) return;
+    x0b[s] = x0a;
+    add_t(tgrad, sid, A.tb);
+    add_own(gx + s, make_float3(own.x + A.own.x, own.y + A.own.y, own.z + A.own.z), 0.0f);
+    add_own(gv + s, vown, 0.0f);
+}
+
+template <int G>
+__global__ void __launch_bounds__(kCThreads, kCBlocks) k_ac_deltap(
+    DevParams P, const SceneDev* __restrict__ scenes, const uint16_t* __restrict__ scene_of,
+    const int2* __restrict__ table, CoopHits H, const float4* __restrict__ xl, const float4* __restrict__ auxd,
+    const float4* __restrict__ gin, float4* __restrict__ gout, float* __restrict__ tgrad)
+{
+    AD_COOP_PROLOGUE
+    const float4 xi = __ldg(xl + s);
+    const float4 g4 = __ldg(gin + s);
+    float3 xb = make_float3(g4.x, g4.y, g4.z), tb;
+    const float3 accb = deltap_adjoint(P, SC, xi, __ldg(auxd + s), xb, tb);
+    float3 own = make_float3(0.f, 0.f, 0.f);
+    float lown = 0.0f;
+    coop_each<G>(P, tab, mask, xl, xi, s, cp.live, H, mem[threadIdx.x / G], [&](int k) {
+        const float4 xj = __ldg(xl + k);
+        const float rx = xi.x - xj.x, ry = xi.y - xj.y, rz = xi.z - xj.z;
+        if (!(rx * rx + ry * ry + rz * rz >= 1e-10f)) return;
+        float3 rb;
+        float ga;
+        deltap_pair_adjoint(P, xi, xj, accb, rb, ga);
+        lown += ga;
+        own = make_float3(own.x + rb.x, own.y + rb.y, own.z + rb.z);
+        atomicAdd(gout + k, make_float4(-rb.x, -rb.y, -rb.z, ga));
+    });
+    own = group_sum<G>(own);
+    lown = group_sum<G>(lown);
+    if (!cp.live || gl != 0) return;
+    add_t(tgrad, sid, tb);
+    add_own(gout + s, make_float3(own.x + xb.x, own.y + xb.y, own.z + xb.z), lown);
+}
+
+template <int G>
+__global__ void __launch_bounds__(kCThreads, kCBlocks) k_ac_lambda(
+    DevParams P, const SceneDev* __restrict__ scenes, const uint16_t* __restrict__ scene_of,
+    const int2* __restrict__ table, CoopHits H, const float4* __restrict__ xl, const float4* __restrict__ auxl,
+    const float* __restrict__ rhol, float4* __restrict__ gout)
+{
+    AD_COOP_PROLOGUE
+    (void)sid;
+    const float lb = gout[s].w;
+    const bool on = cp.live && lb != 0.0f;
+    const float4 xi = __ldg(xl + s);
+    const LambdaAdjoint A = lambda_adjoint(P, lb, __ldg(auxl + s), __ldg(rhol + s));
+    float3 own = make_float3(0.f, 0.f, 0.f);
+    coop_each<G>(P, tab, mask, xl, xi, s, on, H, mem[threadIdx.x / G], [&](int k) {
+        const float3 rb = lambda_pair_adjoint(P, xi, __ldg(xl + k), A);
+        own = make_float3(own.x + rb.x, own.y + rb.y, own.z + rb.z);
+        atomicAdd(gout + k, make_float4(-rb.x, -rb.y, -rb.z, 0.0f));
+    });
+    own = group_sum<G>(own);
+    if (on && gl == 0) add_own(gout + s, own, 0.0f);
 }
 
 // ---- CS_PredictAndHash.glsl:102,114 reversed (slot -> particle order) ----------------------------
@@ -575,6 +776,40 @@ void launch_ad_lambda(const DevParams& P, const SceneDev* scenes, const uint16_t
 {
     k_ad_lambda<<<agrid(P.n), kAThreads, 0, st>>>(P, scenes, scene_of, order, table, xl, auxl, rhol, gout);
 }
+
+#define PBF_AC_LAUNCH(KERNEL, ...)                                                                 \
+    do {                                                                                          \
+        const unsigned grid_ = (unsigned)(((uint64_t)P.n * (uint64_t)G + kCThreads - 1) / kCThreads); \
+        if (G == 32) KERNEL<32><<<grid_, kCThreads, 0, st>>>(__VA_ARGS__);                        \
+        else if (G == 16) KERNEL<16><<<grid_, kCThreads, 0, st>>>(__VA_ARGS__);                   \
+        else KERNEL<8><<<grid_, kCThreads, 0, st>>>(__VA_ARGS__);                                 \
+    } while (0)
+
+void launch_ac_integrate(int G, const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const int2* table,
+                         const uint32_t* list, const uint32_t* list_len, const float4* fsum, const float4* xs,
+                         const float4* sv, const float4* cp_pos, const uint32_t* ids, const float4* posb,
+                         const float4* velb, const float4* posb_s, const float4* omb, const float4* somega, float4* gx,
+                         float4* gv, float4* x0b, float* tgrad, cudaStream_t st)
+{
+    PBF_AC_LAUNCH(k_ac_integrate, P, scenes, scene_of, table, CoopHits{list, list_len}, fsum, xs, sv, cp_pos, ids, posb,
+                  velb, posb_s, omb, somega, gx, gv, x0b, tgrad);
+}
+
+void launch_ac_deltap(int G, const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const int2* table,
+                      const uint32_t* list, const uint32_t* list_len, const float4* xl, const float4* auxd,
+                      const float4* gin, float4* gout, float* tgrad, cudaStream_t st)
+{
+    PBF_AC_LAUNCH(k_ac_deltap, P, scenes, scene_of, table, CoopHits{list, list_len}, xl, auxd, gin, gout, tgrad);
+}
+
+void launch_ac_lambda(int G, const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const int2* table,
+                      const uint32_t* list, const uint32_t* list_len, const float4* xl, const float4* auxl,
+                      const float* rhol, float4* gout, cudaStream_t st)
+{
+    PBF_AC_LAUNCH(k_ac_lambda, P, scenes, scene_of, table, CoopHits{list, list_len}, xl, auxl, rhol, gout);
+}
+
+#undef PBF_AC_LAUNCH
 
 void launch_ad_predict(uint32_t n, float dt, const uint32_t* ids, const float4* gx, const float4* gv,
                        const float4* x0b, float4* posb, float4* velb, int sms, cudaStream_t st)

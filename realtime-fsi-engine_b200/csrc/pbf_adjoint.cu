@@ -2,19 +2,21 @@
 //
 // pbf_batch_forward_record runs one step (every substep, then vorticity)
 // exactly as pbf_batch_step does, saving the particle state at the start of
-// each substep.  pbf_batch_backward then walks the substeps in reverse: it
-// recomputes the substep from its checkpoint (predict, segmented sort, cell
-// table, reorder, processing order — the permutation is replayed, not
-// differentiated), re-runs the solver iterations recording (x*, lambda), the
-// lambda denominators and the raw dp of every iteration, and runs the
-// reverse kernels of k_adjoint.cu: vorticity (last substep), integrate,
-// (deltaP+apply, lambda) per iteration, predict.  Gradients are with respect
-// to the initial positions and velocities and each scene's SDF translation.
-// Both sequences are captured once into CUDA graphs.
+// each substep and, where memory allows, everything the reverse passes read of
+// it: the sort permutation and cell table (replayed, not differentiated), (x*,
+// lambda), the lambda denominators and the raw dp of every iteration and, for
+// small batches, every particle's hits.  pbf_batch_backward walks the substeps
+// in reverse with the kernels of k_adjoint.cu: vorticity (last substep),
+// integrate, (deltaP+apply, lambda) per iteration, predict.  Without the room,
+// or when a scene changed since the recording, it first runs each substep's
+// forward again from its checkpoint.  Gradients are with respect to the
+// initial positions and velocities and each scene's SDF translation.  Both
+// sequences are captured once into CUDA graphs.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 #include "../../include/pbf_b200.h"
 #include "pbf_batch.h"
@@ -52,11 +54,38 @@ static void afree(T*& p)
 
 void pbf_batch::ad_free()
 {
-    afree(cp_pos); afree(cp_vel); afree(xl); afree(auxl); afree(auxd); afree(rhol);
+    afree(cp_pos); afree(cp_vel); afree(ad_slab); afree(ad_sx0); afree(ad_om);
     afree(gxa); afree(gxb); afree(gv); afree(x0b); afree(pb); afree(vb); afree(pbs); afree(omb);
     afree(tpos); afree(tvel); afree(tgrad);
+    records.clear();
     ad_subs = ad_iters = 0;
     recorded = false;
+}
+
+// One record's arrays laid one after another from `base` (null: only counted);
+// returns its bytes.  `c` entries per array (a multiple of 64, pads included).
+static size_t lay_record(pbf_batch::Record& r, char* base, size_t c, uint32_t iters, size_t table, bool hits, bool order)
+{
+    size_t at = 0;
+    auto take = [&](auto*& p, size_t count) {
+        p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(base + at);
+        at += (count * sizeof(*p) + 255) / 256 * 256;
+    };
+    take(r.ids, c);
+    if (order) take(r.order, c);
+    take(r.table, table);
+    take(r.sv, c);
+    take(r.xf, c);
+    take(r.xl, c * iters);
+    take(r.auxl, c * iters);
+    take(r.auxd, c * iters);
+    take(r.rhol, c * iters);
+    if (hits) {
+        take(r.fsum, c);
+        take(r.list, c * (iters + 1) * kCoopList);
+        take(r.list_len, c * (iters + 1));
+    }
+    return at;
 }
 
 int pbf_batch::ad_alloc()
@@ -66,40 +95,127 @@ int pbf_batch::ad_alloc()
     ad_free();
     const size_t c = std::max<uint32_t>(n, 1u);
     int rc;
-    if ((rc = aalloc(cp_pos, c * S)) || (rc = aalloc(cp_vel, c * S)) || (rc = aalloc(xl, c * std::max(I, 1u))) ||
-        (rc = aalloc(auxl, c * std::max(I, 1u))) || (rc = aalloc(auxd, c * std::max(I, 1u))) ||
-        (rc = aalloc(rhol, c * std::max(I, 1u))) || (rc = aalloc(gxa, c)) || (rc = aalloc(gxb, c)) ||
+    if ((rc = aalloc(cp_pos, c * S)) || (rc = aalloc(cp_vel, c * S)) || (rc = aalloc(ad_sx0, c + kCoopPad)) ||
+        (rc = aalloc(ad_om, c)) || (rc = aalloc(gxa, c)) || (rc = aalloc(gxb, c)) ||
         (rc = aalloc(gv, c)) || (rc = aalloc(x0b, c)) || (rc = aalloc(pb, c)) || (rc = aalloc(vb, c)) ||
         (rc = aalloc(pbs, c)) || (rc = aalloc(omb, c)) || (rc = aalloc(tpos, c)) || (rc = aalloc(tvel, c)) ||
         (rc = aalloc(tgrad, 4 * scenes.size()))) {
         ad_free();
         return rc;
     }
+    // a record per substep when they take at most a quarter of the free memory
+    // (32,768 particles x 16 substeps x 4 iterations: 0.9 GB)
+    const bool hits = coop_lanes(n) != 0;
+    ad_stride = (c + kCoopPad + 63) / 64 * 64;
+    Record probe;
+    const size_t bytes = lay_record(probe, nullptr, ad_stride, I, table_size, hits, !hits);
+    size_t free_b = 0, total_b = 0;
+    ACK(cudaMemGetInfo(&free_b, &total_b));
+    ad_full = bytes * S <= free_b / 4;
+    const uint32_t R = ad_full ? S : 1u;
+    char* slab = nullptr;
+    if ((rc = aalloc(slab, bytes * R))) {
+        ad_free();
+        return rc;
+    }
+    ad_slab = slab;
+    records.resize(R);
+    for (uint32_t k = 0; k < R; ++k) lay_record(records[k], slab + bytes * k, ad_stride, I, table_size, hits, !hits);
     ad_subs = S;
     ad_iters = I;
     return PBF_OK;
 }
 
+// Substep `sub` from (src_pos, src_vel) to (dst_pos, dst_vel), as
+// substep_body runs it, with what the reverse passes read kept in r.
+int pbf_batch::record_substep(uint32_t sub, Record& r, const float4* src_pos, const float4* src_vel, float4* dst_pos,
+                              float4* dst_vel)
+{
+    const DevParams P = dev_params();
+    BatchLaunch L = launch;
+    L.sms = num_sms;
+    const int sms = num_sms, G = coop_lanes(n);
+    const uint32_t I = cfg.solver_iterations;
+    const bool last = sub + 1 == cfg.substep_iterations;
+    launch_b_predict(P, scenes_dev, scene_of, src_pos, src_vel, keys, sms, stream);
+    launch_radix_sort_into(n, key_bits, keys, ka, r.ids, kb, ib, hist, totals, stream);
+    ACK(cudaMemsetAsync(r.table, 0xFF, sizeof(int2) * (size_t)table_size, stream));
+    launch_build_table(n, ka, r.table, sms, stream);
+    const bool sorted = morton && !G;
+    float4* x = I ? sx[0] : r.xf;
+    launch_b_reorder(P, scenes_dev, scene_of, r.ids, src_pos, src_vel, x, r.sv, sx0, lod, sorted ? mcode : nullptr,
+                     mbits, sms, stream);
+    launches += 3 + 3 * ((key_bits + 7) / 8);
+    const uint32_t* ord = nullptr;
+    if (sorted) {
+        launch_radix_sort_into(n, order_bits, mcode, mka, r.order, mkb, mib, hist, totals, stream);
+        launches += 3 * ((order_bits + 7) / 8);
+        ord = r.order;
+    }
+    for (uint32_t it = 1; it <= I; ++it) {
+        const size_t at = (size_t)(it - 1) * ad_stride;
+        float4 *xl = r.xl + at, *out = it == I ? r.xf : sx[0];
+        if (G) {
+            uint32_t *list = r.list + at * kCoopList, *len = r.list_len + at;
+            launch_c_lambda(G, P, scenes_dev, scene_of, sx[0], xl, r.rhol + at, r.table, lod, it, nullptr, list, len,
+                            r.auxl + at, stream);
+            launch_c_deltap(G, P, scenes_dev, scene_of, xl, out, r.table, lod, it, nullptr, list, len, r.auxd + at,
+                            stream);
+        } else {
+            launch_ad_lambda_rec(P, scenes_dev, scene_of, ord, r.table, sx[0], xl, r.auxl + at, r.rhol + at, stream);
+            launch_ad_deltap_rec(P, scenes_dev, scene_of, ord, r.table, xl, out, r.auxd + at, stream);
+        }
+        launches += 2;
+    }
+    float4* x0 = sx0;
+    float4* om = somega;
+    if (last && cfg.enable_vorticity) {  // the vorticity pass and its reverse read these
+        ACK(cudaMemcpyAsync(ad_sx0, sx0, sizeof(float4) * n, cudaMemcpyDeviceToDevice, stream));
+        x0 = ad_sx0;
+        om = ad_om;
+    }
+    if (G)
+        launch_c_integrate(G, P, scenes_dev, scene_of, r.xf, r.sv, x0, om, r.ids, dst_pos, dst_vel, r.table, nullptr,
+                           r.list + (size_t)I * ad_stride * kCoopList, r.list_len + (size_t)I * ad_stride, r.fsum,
+                           stream);
+    else
+        launch_b_integrate(P, L, scenes_dev, scene_of, r.xf, r.sv, x0, om, r.ids, dst_pos, dst_vel, r.table, ord,
+                           stream);
+    ++launches;
+    return PBF_OK;
+}
+
 int pbf_batch::record_body()
 {
-    for (uint32_t sub = 0; sub < cfg.substep_iterations; ++sub) {
+    const DevParams P = dev_params();
+    BatchLaunch L = launch;
+    L.sms = num_sms;
+    const uint32_t S = cfg.substep_iterations;
+    const int G = coop_lanes(n);
+    for (uint32_t sub = 0; sub < S; ++sub) {
         ACK(cudaMemcpyAsync(cp_pos + (size_t)sub * n, pos, sizeof(float4) * n, cudaMemcpyDeviceToDevice, stream));
         ACK(cudaMemcpyAsync(cp_vel + (size_t)sub * n, vel, sizeof(float4) * n, cudaMemcpyDeviceToDevice, stream));
-        const int rc = substep_body(pos, vel, pos, vel);
+        const int rc = record_substep(sub, records[ad_full ? sub : 0], pos, vel, pos, vel);
         if (rc) return rc;
     }
-    if (cfg.enable_vorticity) vorticity_pass();
+    if (cfg.enable_vorticity) {
+        const Record& r = records[ad_full ? S - 1 : 0];
+        if (G)
+            launch_c_vorticity(G, P, scenes_dev, scene_of, ad_sx0, ad_om, r.ids, vel, r.table, nullptr, stream);
+        else
+            launch_b_vorticity(P, L, scenes_dev, scene_of, ad_sx0, ad_om, r.ids, vel, r.table, morton ? r.order : nullptr,
+                               stream);
+        ++launches;
+    }
     return PBF_OK;
 }
 
 // Inputs: pb, vb (adjoints of the recorded step's final state).  Outputs:
 // pb, vb (adjoints of its initial state), tgrad (of the SDF translations).
-int pbf_batch::backward_body()
+int pbf_batch::backward_body(bool recompute)
 {
     const DevParams P = dev_params();
-    BatchLaunch L = launch;
-    L.sms = num_sms;
-    const int sms = num_sms;
+    const int sms = num_sms, G = coop_lanes(n);
     const uint32_t S = cfg.substep_iterations, I = cfg.solver_iterations;
     const bool vort = cfg.enable_vorticity != 0;
     ACK(cudaMemsetAsync(tgrad, 0, sizeof(float) * 4 * scenes.size(), stream));
@@ -108,60 +224,47 @@ int pbf_batch::backward_body()
     for (int sub = (int)S - 1; sub >= 0; --sub) {
         const float4* src_pos = cp_pos + (size_t)sub * n;
         const float4* src_vel = cp_vel + (size_t)sub * n;
-        // replay the substep's sort, table and processing order
-        launch_b_predict(P, scenes_dev, scene_of, src_pos, src_vel, keys, sms, stream);
-        launch_radix_sort(n, key_bits, keys, ka, ia, kb, ib, hist, totals, &skeys, &ids, stream, &launches);
-        ACK(cudaMemsetAsync(table, 0xFF, sizeof(int2) * (size_t)table_size, stream));
-        launch_build_table(n, skeys, table, sms, stream);
-        launch_b_reorder(P, scenes_dev, scene_of, ids, src_pos, src_vel, sx[0], sv, sx0, lod,
-                         morton ? mcode : nullptr, mbits, sms, stream);
-        launches += 3;
-        order = nullptr;
-        if (morton) {
-            uint32_t* msorted = nullptr;
-            launch_radix_sort(n, order_bits, mcode, mka, mia, mkb, mib, hist, totals, &msorted, &order, stream,
-                              &launches);
+        Record& r = records[ad_full ? sub : 0];
+        if (recompute) {
+            const int rc = record_substep((uint32_t)sub, r, src_pos, src_vel, tpos, tvel);
+            if (rc) return rc;
         }
-        // recompute the iterations, recording what the reverse reads
-        for (uint32_t it = 1; it <= I; ++it) {
-            float4* xli = xl + (size_t)(it - 1) * n;
-            launch_ad_lambda_rec(P, scenes_dev, scene_of, order, table, sx[0], xli, auxl + (size_t)(it - 1) * n,
-                                 rhol + (size_t)(it - 1) * n, stream);
-            launch_ad_deltap_rec(P, scenes_dev, scene_of, order, table, xli, sx[0], auxd + (size_t)(it - 1) * n,
-                                 stream);
-            launches += 2;
-        }
+        const uint32_t* ord = morton && !G ? r.order : nullptr;
         const bool last = (sub == (int)S - 1) && vort;
         if (last) {
-            // committed state and omega of the last substep, for the vorticity reverse
-            if (const int G = coop_lanes(n))
-                launch_c_integrate(G, P, scenes_dev, scene_of, sx[0], sv, sx0, somega, ids, tpos, tvel, table, order,
-                                   stream);
-            else
-                launch_b_integrate(P, L, scenes_dev, scene_of, sx[0], sv, sx0, somega, ids, tpos, tvel, table, order,
-                                   stream);
-            launch_ad_vorticity(P, scenes_dev, scene_of, order, table, sx0, somega, ids, vb, pbs, omb, stream);
-            launches += 2;
+            launch_ad_vorticity(P, scenes_dev, scene_of, ord, r.table, ad_sx0, ad_om, r.ids, vb, pbs, omb, stream);
+            ++launches;
         }
         ACK(cudaMemsetAsync(gxa, 0, sizeof(float4) * n, stream));
         ACK(cudaMemsetAsync(gxb, 0, sizeof(float4) * n, stream));
         ACK(cudaMemsetAsync(gv, 0, sizeof(float4) * n, stream));
-        launch_ad_integrate(P, scenes_dev, scene_of, order, table, sx[0], sv, src_pos, ids, pb, vb,
-                            last ? pbs : nullptr, last ? omb : nullptr, somega, gxa, gv, x0b, tgrad, stream);
+        if (G)
+            launch_ac_integrate(G, P, scenes_dev, scene_of, r.table, r.list + (size_t)I * ad_stride * kCoopList,
+                                r.list_len + (size_t)I * ad_stride, r.fsum, r.xf, r.sv, src_pos, r.ids, pb, vb,
+                                last ? pbs : nullptr, last ? omb : nullptr, ad_om, gxa, gv, x0b, tgrad, stream);
+        else
+            launch_ad_integrate(P, scenes_dev, scene_of, ord, r.table, r.xf, r.sv, src_pos, r.ids, pb, vb,
+                                last ? pbs : nullptr, last ? omb : nullptr, ad_om, gxa, gv, x0b, tgrad, stream);
         ++launches;
         float4* a = gxa;
         float4* b = gxb;
         for (int it = (int)I; it >= 1; --it) {
-            const float4* xli = xl + (size_t)(it - 1) * n;
-            launch_ad_deltap(P, scenes_dev, scene_of, order, table, xli, auxd + (size_t)(it - 1) * n, a, b, tgrad,
-                             stream);
-            launch_ad_lambda(P, scenes_dev, scene_of, order, table, xli, auxl + (size_t)(it - 1) * n,
-                             rhol + (size_t)(it - 1) * n, b, stream);
+            const size_t at = (size_t)(it - 1) * ad_stride;
+            if (G) {
+                const uint32_t *list = r.list + at * kCoopList, *len = r.list_len + at;
+                launch_ac_deltap(G, P, scenes_dev, scene_of, r.table, list, len, r.xl + at, r.auxd + at, a, b, tgrad,
+                                 stream);
+                launch_ac_lambda(G, P, scenes_dev, scene_of, r.table, list, len, r.xl + at, r.auxl + at, r.rhol + at, b,
+                                 stream);
+            } else {
+                launch_ad_deltap(P, scenes_dev, scene_of, ord, r.table, r.xl + at, r.auxd + at, a, b, tgrad, stream);
+                launch_ad_lambda(P, scenes_dev, scene_of, ord, r.table, r.xl + at, r.auxl + at, r.rhol + at, b, stream);
+            }
             launches += 2;
             ACK(cudaMemsetAsync(a, 0, sizeof(float4) * n, stream));
             std::swap(a, b);
         }
-        launch_ad_predict(n, P.dt, ids, a, gv, x0b, pb, vb, sms, stream);
+        launch_ad_predict(n, P.dt, r.ids, a, gv, x0b, pb, vb, sms, stream);
         ++launches;
     }
     return PBF_OK;
@@ -254,6 +357,7 @@ extern "C" int pbf_batch_forward_record(pbf_batch* b)
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return set_error(PBF_ERR_CUDA, "kernel launch: %s", cudaGetErrorString(e));
     b->recorded = true;
+    b->recorded_gen = b->scenes_gen;
     return PBF_OK;
 }
 
@@ -269,7 +373,16 @@ extern "C" int pbf_batch_backward(pbf_batch* b, const void* gpos4, const void* g
     else ACK(cudaMemsetAsync(b->pb, 0, bytes, b->stream));
     if (gvel4) ACK(cudaMemcpyAsync(b->vb, gvel4, bytes, cudaMemcpyDefault, b->stream));
     else ACK(cudaMemsetAsync(b->vb, 0, bytes, b->stream));
-    rc = run_graph(b, b->bwd_graph, b->bwd_exec, b->bwd_launches, [&] { return b->backward_body(); });
+    // the records hold for the scenes they were made under
+    const bool recompute = !b->ad_full || b->recorded_gen != b->scenes_gen;
+    if (b->bwd_exec && b->bwd_recompute != recompute) {
+        cudaGraphExecDestroy(b->bwd_exec);
+        cudaGraphDestroy(b->bwd_graph);
+        b->bwd_exec = nullptr;
+        b->bwd_graph = nullptr;
+    }
+    b->bwd_recompute = recompute;
+    rc = run_graph(b, b->bwd_graph, b->bwd_exec, b->bwd_launches, [&] { return b->backward_body(recompute); });
     if (rc) return rc;
     if (out_gpos4) ACK(cudaMemcpyAsync(out_gpos4, b->pb, bytes, cudaMemcpyDefault, b->stream));
     if (out_gvel4) ACK(cudaMemcpyAsync(out_gvel4, b->vb, bytes, cudaMemcpyDefault, b->stream));

@@ -267,8 +267,9 @@ int pbf_batch::substep_body(const float4* src_pos, const float4* src_vel, float4
     for (uint32_t it = 1; it <= max_iter; ++it) {
         if (G) {
             launch_c_lambda(G, P, scenes_dev, scene_of, sx[0], sx[1], rho, table, lod, it, order, chits, chit_len,
-                            stream);
-            launch_c_deltap(G, P, scenes_dev, scene_of, sx[1], sx[0], table, lod, it, order, chits, chit_len, stream);
+                            nullptr, stream);
+            launch_c_deltap(G, P, scenes_dev, scene_of, sx[1], sx[0], table, lod, it, order, chits, chit_len,
+                            nullptr, stream);
         } else {
             launch_b_lambda(P, L, scenes_dev, scene_of, sx[0], sx[1], rho, table, lod, it, order, stream);
             launch_b_deltap(P, L, scenes_dev, scene_of, sx[1], sx[0], table, lod, it, order, stream);
@@ -277,7 +278,7 @@ int pbf_batch::substep_body(const float4* src_pos, const float4* src_vel, float4
     }
     if (G)
         launch_c_integrate(G, P, scenes_dev, scene_of, sx[0], sv, sx0, somega, ids, dst_pos, dst_vel, table, order,
-                           stream);
+                           nullptr, nullptr, nullptr, stream);
     else
         launch_b_integrate(P, L, scenes_dev, scene_of, sx[0], sv, sx0, somega, ids, dst_pos, dst_vel, table, order,
                            stream);

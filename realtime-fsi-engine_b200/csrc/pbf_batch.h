@@ -92,6 +92,19 @@ void launch_ad_deltap(const DevParams& P, const SceneDev* scenes, const uint16_t
 void launch_ad_lambda(const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const uint32_t* order,
                       const int2* table, const float4* xl, const float4* auxl, const float* rhol, float4* gout,
                       cudaStream_t st);
+// The reverse passes with a group of G lanes per particle, over the hits the
+// recording passes kept (list, list_len); fsum: the XSPH sums of the integrate pass.
+void launch_ac_integrate(int G, const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const int2* table,
+                         const uint32_t* list, const uint32_t* list_len, const float4* fsum, const float4* xs,
+                         const float4* sv, const float4* cp_pos, const uint32_t* ids, const float4* posb,
+                         const float4* velb, const float4* posb_s, const float4* omb, const float4* somega, float4* gx,
+                         float4* gv, float4* x0b, float* tgrad, cudaStream_t st);
+void launch_ac_deltap(int G, const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const int2* table,
+                      const uint32_t* list, const uint32_t* list_len, const float4* xl, const float4* auxd,
+                      const float4* gin, float4* gout, float* tgrad, cudaStream_t st);
+void launch_ac_lambda(int G, const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const int2* table,
+                      const uint32_t* list, const uint32_t* list_len, const float4* xl, const float4* auxl,
+                      const float* rhol, float4* gout, cudaStream_t st);
 void launch_ad_predict(uint32_t n, float dt, const uint32_t* ids, const float4* gx, const float4* gv,
                        const float4* x0b, float4* posb, float4* velb, int sms, cudaStream_t st);
 
@@ -178,13 +191,29 @@ struct pbf_batch {
     cudaGraphExec_t graph_exec = nullptr;
     uint64_t graph_launches = 0;
 
-    // adjoint (pbf_adjoint.cu): per-substep checkpoints of the recorded step,
-    // per-iteration recomputation buffers, adjoint accumulators
+    // adjoint (pbf_adjoint.cu): per-substep checkpoints of the recorded step
+    // and the forward of each substep as the reverse passes read it.  With room
+    // for it every substep has a record of its own, written by the recording
+    // forward; otherwise there is one, which the backward fills again from the
+    // substep's checkpoint.
+    struct Record {
+        uint32_t *ids = nullptr, *order = nullptr;  // sort permutation, processing order (null: sorted order)
+        int2* table = nullptr;
+        float4 *sv = nullptr, *xf = nullptr;        // v', x* after the last iteration (sorted)
+        float4* fsum = nullptr;                     // XSPH sums (groups of lanes only)
+        float4 *xl = nullptr, *auxl = nullptr, *auxd = nullptr;  // per iteration: (x*, lambda), (grad C, denominator), raw dp
+        float* rhol = nullptr;                      // per iteration: density
+        uint32_t *list = nullptr, *list_len = nullptr;  // per iteration, then integrate: hits (groups of lanes only)
+    };
+    std::vector<Record> records;
+    size_t ad_stride = 0;         // entries between the iterations' arrays of a record
+    void* ad_slab = nullptr;      // the records
     uint32_t ad_subs = 0, ad_iters = 0;
+    bool ad_full = false;         // a record per substep
     bool recorded = false;
+    uint64_t recorded_gen = 0;    // scenes_gen the records were made under
     float4 *cp_pos = nullptr, *cp_vel = nullptr;       // substeps x n, particle order
-    float4 *xl = nullptr, *auxl = nullptr, *auxd = nullptr;  // iterations x n, sorted
-    float* rhol = nullptr;                              // iterations x n
+    float4 *ad_sx0 = nullptr, *ad_om = nullptr;        // committed positions and omega of the last substep, sorted
     float4 *gxa = nullptr, *gxb = nullptr, *gv = nullptr, *x0b = nullptr;  // sorted
     float4 *pb = nullptr, *vb = nullptr;                // particle order
     float4 *pbs = nullptr, *omb = nullptr;              // sorted (vorticity reverse)
@@ -193,6 +222,7 @@ struct pbf_batch {
     cudaGraph_t rec_graph = nullptr, bwd_graph = nullptr;
     cudaGraphExec_t rec_exec = nullptr, bwd_exec = nullptr;
     uint64_t rec_launches = 0, bwd_launches = 0;
+    bool bwd_recompute = false;   // the captured backward fills the records again
 
     ~pbf_batch();
     pbf::DevParams dev_params() const;
@@ -210,6 +240,8 @@ struct pbf_batch {
     int substep_body(const float4* src_pos, const float4* src_vel, float4* dst_pos, float4* dst_vel);
     int ad_alloc();
     void ad_free();
+    int record_substep(uint32_t sub, Record& r, const float4* src_pos, const float4* src_vel, float4* dst_pos,
+                       float4* dst_vel);
     int record_body();
-    int backward_body();
+    int backward_body(bool recompute);
 };

@@ -725,7 +725,8 @@ int pbf_handle::stage(int st, uint32_t iter)
     case PBF_STAGE_LAMBDA:
         prof_begin(PBF_STAGE_LAMBDA);
         if (const int G = coop_lanes(n))
-            launch_c_lambda(G, P, nullptr, nullptr, sx[0], sx[1], rho, table, lod, iter, order, chits, chit_len, stream);
+            launch_c_lambda(G, P, nullptr, nullptr, sx[0], sx[1], rho, table, lod, iter, order, chits, chit_len, nullptr,
+                            stream);
         else
             launch_lambda_m(P, sx[0], sx[1], rho, table, lod, iter, order, stream);
         ++launches;
@@ -737,7 +738,7 @@ int pbf_handle::stage(int st, uint32_t iter)
         prof_begin(PBF_STAGE_DELTAP);
         if (const int G = coop_lanes(n))
             launch_c_deltap(G, P, nullptr, nullptr, sx[1], sx[0], table, lod, iter, order,
-                            chit_iter == (int)iter ? chits : nullptr, chit_len, stream);
+                            chit_iter == (int)iter ? chits : nullptr, chit_len, nullptr, stream);
         else
             launch_deltap_m(P, sx[1], sx[0], table, lod, iter, order, stream);
         ++launches;
@@ -748,7 +749,8 @@ int pbf_handle::stage(int st, uint32_t iter)
     case PBF_STAGE_INTEGRATE:
         prof_begin(PBF_STAGE_INTEGRATE);
         if (const int G = coop_lanes(n))
-            launch_c_integrate(G, P, nullptr, nullptr, sx[0], sv, sx0, somega, ids, pos, vel, table, order, stream);
+            launch_c_integrate(G, P, nullptr, nullptr, sx[0], sv, sx0, somega, ids, pos, vel, table, order, nullptr,
+                               nullptr, nullptr, stream);
         else
             launch_integrate_m(P, sx[0], sv, sx0, somega, ids, pos, vel, table, order, stream);
         ++launches;

@@ -43,16 +43,20 @@ constexpr int kCoopList = 64;
 // up to 8 candidates is loaded whole.
 constexpr int kCoopPad = 8;
 struct SceneDev;  // pbf_batch.h
-// scenes/scene_of: the scenes of a batch (null: one scene, constants in P)
+// scenes/scene_of: the scenes of a batch (null: one scene, constants in P).
+// What the adjoint reads is written where asked (null: not): lambda's (grad C,
+// denominator) to aux, the delta-p before its clamp to dp_out, and integrate's
+// hits and XSPH sum to list, list_len and fsum.
 void launch_c_lambda(int G, const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const float4* xin,
                      float4* xout, float* rho, const int2* table, const uint32_t* lod, uint32_t iter,
-                     const uint32_t* order, uint32_t* list, uint32_t* list_len, cudaStream_t st);
+                     const uint32_t* order, uint32_t* list, uint32_t* list_len, float4* aux, cudaStream_t st);
 void launch_c_deltap(int G, const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const float4* xin,
                      float4* xout, const int2* table, const uint32_t* lod, uint32_t iter, const uint32_t* order,
-                     const uint32_t* list, const uint32_t* list_len, cudaStream_t st);
+                     const uint32_t* list, const uint32_t* list_len, float4* dp_out, cudaStream_t st);
 void launch_c_integrate(int G, const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const float4* xs,
                         const float4* sv, float4* sx0, float4* somega, const uint32_t* ids, float4* pos, float4* vel,
-                        const int2* table, const uint32_t* order, cudaStream_t st);
+                        const int2* table, const uint32_t* order, uint32_t* list, uint32_t* list_len, float4* fsum,
+                        cudaStream_t st);
 void launch_c_vorticity(int G, const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of,
                         const float4* spos, const float4* somega, const uint32_t* ids, float4* vel, const int2* table,
                         const uint32_t* order, cudaStream_t st);
