@@ -16,6 +16,13 @@ constexpr int kCThreads = 128;
 // 32,768 particles at G = 8: 22.4 us; 6 blocks: 23.0, 10: 24.7, 12: 29.3).
 constexpr int kCBlocks = 8;
 
+// The passes over kept hits: loads of 4 chunks of G hits in flight, 8 resident
+// blocks (131,072 particles, delta-p / reverse delta-p / reverse lambda: 22.5 /
+// 31.6 / 24.2 us; 2 chunks 23.4 / 31.9 / 24.7, 8 chunks 22.1 / 34.8 / 24.4; 12
+// blocks of 2 chunks 23.3 / 38.0 / 24.0, 16 of 1 chunk 26.4 / 49.9 / 23.4: the
+// obstacle's reverse projection spills).
+constexpr int kReplayAhead = 4, kReplayBlocks = 8;
+
 template <int G>
 struct CoopShape {
     static constexpr int kBuckets = (27 + G - 1) / G;  // buckets whose ranges one lane reads
@@ -25,15 +32,25 @@ struct CoopShape {
     static constexpr int kRow = G + 4;                 // one term of the G hits of a chunk; rows start in different banks
 };
 
-// NT rows of pair terms and a row of ones.  Groups start G banks apart.
+// NT rows of the terms of a chunk of G hits and a row of ones.
+template <int G, int NT>
+constexpr int kCoopTerms = (NT + 1) * CoopShape<G>::kRow;
+
+// What a walk needs beside them.  Groups start G banks apart.
 template <int G, int NT>
 struct CoopMem {
     using S = CoopShape<G>;
-    static constexpr int kTerms = (NT + 1) * S::kRow;
-    static constexpr int kPad = ((G - kTerms - S::kHits - 2 * S::kRuns) % 32 + 32) % 32;
-    float term[kTerms];
+    static constexpr int kPad = ((G - kCoopTerms<G, NT> - S::kHits - 2 * S::kRuns) % 32 + 32) % 32;
+    float term[kCoopTerms<G, NT>];
     int2 run[S::kRuns];  // first candidate and candidates from there on in its bucket (a run takes up to 8)
     int hit[S::kHits + kPad];
+};
+
+// Terms alone, for the passes over kept hits.
+template <int G, int NT>
+struct CoopTermMem {
+    static constexpr int kPad = ((G - kCoopTerms<G, NT>) % 32 + 32) % 32;
+    float term[kCoopTerms<G, NT> + kPad];
 };
 
 // Hits of a particle in visiting order, kept from the lambda pass for the
@@ -41,19 +58,44 @@ struct CoopMem {
 constexpr uint32_t kNoHits = 0xFFFFFFFFu;
 
 // The particle's sums: lane gl of a group adds t[ra] * t[rb] (fused) over the
-// hits in order, row NT holding ones; pair(k, t) fills the terms of hit k.
-// Called by whole warps.
-template <int G, int NT, class Pair>
+// hits in order, row NT holding ones; load(k) reads hit k and pair(load(k), t)
+// fills its terms (none for k = self).  The loads of U chunks of G hits are
+// issued together.  Called by whole warps.
+template <int G, int NT, int U, class Load, class Pair>
 struct CoopSum {
-    using S = CoopShape<G>;
-    CoopMem<G, NT>& M;
-    int gl, ra, rb;
+    static constexpr int kRow = CoopShape<G>::kRow;
+    float* term;
+    int gl, self, ra, rb;
     float acc;
+    Load load;
     Pair pair;
-    __device__ __forceinline__ CoopSum(CoopMem<G, NT>& m, int lane_of_group, int a, int b, float init, Pair&& p)
-        : M(m), gl(lane_of_group), ra(a * S::kRow), rb(b * S::kRow), acc(init), pair(p)
+    __device__ __forceinline__ CoopSum(float* m, int lane_of_group, int s, int a, int b, float init, Load&& l, Pair&& p)
+        : term(m), gl(lane_of_group), self(s), ra(a * kRow), rb(b * kRow), acc(init), load(l), pair(p)
     {
-        M.term[NT * S::kRow + gl] = 1.0f;
+        term[NT * kRow + gl] = 1.0f;
+    }
+    // lane gl's hit k of a chunk (self: none); cnt hits in the chunk
+    template <class D>
+    __device__ __forceinline__ void chunk(int k, const D& d, int cnt)
+    {
+        float t[NT];
+#pragma unroll
+        for (int r = 0; r < NT; ++r) t[r] = 0.0f;
+        if (k != self) pair(d, t);
+#pragma unroll
+        for (int r = 0; r < NT; ++r) term[r * kRow + gl] = t[r];
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < G; q += 4) {
+            if (G > 8 && q >= cnt) break;
+            const float4 a = *reinterpret_cast<const float4*>(term + ra + q);
+            const float4 b = *reinterpret_cast<const float4*>(term + rb + q);
+            acc = __fmaf_rn(a.x, b.x, acc);
+            acc = __fmaf_rn(a.y, b.y, acc);
+            acc = __fmaf_rn(a.z, b.z, acc);
+            acc = __fmaf_rn(a.w, b.w, acc);
+        }
+        __syncwarp();
     }
     // cnt hits (per group), hit(i) = the i-th
     template <class HitAt>
@@ -61,28 +103,64 @@ struct CoopSum {
     {
         const int most = (int)__reduce_max_sync(0xffffffffu, (uint32_t)cnt);
 #pragma unroll 1
-        for (int h = 0; h < most; h += G) {
-            float t[NT];
+        for (int h = 0; h < most; h += U * G) {
+            int k[U];
 #pragma unroll
-            for (int r = 0; r < NT; ++r) t[r] = 0.0f;
-            if (h + gl < cnt) pair(hit(h + gl), t);
+            for (int u = 0; u < U; ++u) k[u] = h + u * G + gl < cnt ? hit(h + u * G + gl) : self;
+            decltype(load(0)) d[U];
 #pragma unroll
-            for (int r = 0; r < NT; ++r) M.term[r * S::kRow + gl] = t[r];
-            __syncwarp();
+            for (int u = 0; u < U; ++u) d[u] = load(k[u]);
 #pragma unroll
-            for (int q = 0; q < G; q += 4) {
-                if (G > 8 && h + q >= cnt) break;
-                const float4 a = *reinterpret_cast<const float4*>(M.term + ra + q);
-                const float4 b = *reinterpret_cast<const float4*>(M.term + rb + q);
-                acc = __fmaf_rn(a.x, b.x, acc);
-                acc = __fmaf_rn(a.y, b.y, acc);
-                acc = __fmaf_rn(a.z, b.z, acc);
-                acc = __fmaf_rn(a.w, b.w, acc);
+            for (int u = 0; u < U; ++u) {
+                if (u > 0 && h + u * G >= most) break;
+                chunk(k[u], d[u], cnt - h - u * G);
             }
-            __syncwarp();
         }
     }
     __device__ __forceinline__ float get(int k) const { return __shfl_sync(0xffffffffu, acc, k, G); }
+};
+
+// The walk of a particle whose hits were not kept, in a pass that otherwise
+// reads kept hits: each[k] for its buckets' candidates G at a time, in
+// visiting order (k = self where there is none).  Called by whole warps.
+template <int G, class Each>
+__device__ __forceinline__ void coop_plain_walk(const DevParams& P, const int2* __restrict__ table, uint32_t mask,
+                                                const float4* __restrict__ X, float4 xi, int self, bool on, Each&& each)
+{
+    const int gl = threadIdx.x & (G - 1);
+    const int cx = cell_coord(xi.x, P.h), cy = cell_coord(xi.y, P.h), cz = cell_coord(xi.z, P.h);
+#pragma unroll 1
+    for (int b = 0; b < 27; ++b) {
+        int2 se = make_int2(0, 0);
+        if (on) se = __ldg(table + grid_hash(cx + b % 3 - 1, cy + b / 3 % 3 - 1, cz + b / 9 - 1, mask));
+        const int len = se.x == -1 ? 0 : se.y - se.x;
+        const int most = (int)__reduce_max_sync(0xffffffffu, (uint32_t)len);
+#pragma unroll 1
+        for (int c = 0; c < most; c += G) {
+            int k = self;
+            if (c + gl < len) {
+                const float4 xj = __ldg(X + se.x + c + gl);
+                const float2 rxy = sub_f32x2(make_float2(xi.x, xi.y), make_float2(xj.x, xj.y));
+                const float rx = rxy.x, ry = rxy.y, rz = xi.z - xj.z;
+                if (rx * rx + ry * ry + rz * rz <= P.h2) k = se.x + c + gl;
+            }
+            each(k);
+        }
+    }
+}
+
+// One position per hit, and a second array's entry beside it.
+struct CoopLoad1 {
+    const float4* __restrict__ x;
+    __device__ __forceinline__ float4 operator()(int k) const { return __ldg(x + k); }
+};
+struct CoopTwo {
+    float4 x, v;
+};
+struct CoopLoad2 {
+    const float4* __restrict__ x;
+    const float4* __restrict__ v;
+    __device__ __forceinline__ CoopTwo operator()(int k) const { return CoopTwo{__ldg(x + k), __ldg(v + k)}; }
 };
 
 // The candidates of 32 / G rounds as one word: bit r * G + l of the group's

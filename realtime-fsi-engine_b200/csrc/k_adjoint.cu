@@ -3,12 +3,12 @@
 // The backward of one substep runs on the state the forward recorded for it
 // (recomputed from the substep's checkpoint): sorted slots, the cell table,
 // every iteration's (x*, lambda) with the lambda denominators and raw dp.
-// Each kernel is one thread per particle in the forward's processing order;
-// it recomputes what it needs of its own particle, accumulates its own
+// A group of lanes takes each particle: every lane recomputes what the pairs
+// need of it, takes a share of its pairs, accumulates the particle's own
 // adjoint in registers and scatters the neighbour's share of every pair term
-// with atomic adds (sm_90+ float4 atomics), walking the same 27 buckets with
-// the same multiplicity and order as the forward.  Discrete choices (neighbour
-// sets, wall/SDF contacts, clamps) are the forward's, replayed.
+// with atomic adds (sm_90+ float4 atomics).  The pairs are the forward's, with
+// the same multiplicity.  Discrete choices (neighbour sets, wall/SDF contacts,
+// clamps) are the forward's, replayed.
 //
 // Derivatives (r = x_i - x_j, q = |r|, W = poly6, grad W = r s(r^2)):
 //   dW/d(r^2)  = -3 K6 (h^2 - r^2)^2
@@ -18,14 +18,6 @@
 #include "pbf_batch.h"
 
 namespace pbf {
-
-constexpr int kAThreads = 128;
-// The reverse pair passes and the recording Δp are held to 8 resident blocks
-// (at most 64 registers).  Left to itself the compiler gave the Δp adjoint 56
-// registers and 1.2 KB of spills; at 8 blocks the backward of one step (16
-// substeps x 4 iterations) of 16 scenes of 32,768 particles takes 42.4 ms
-// instead of 46.0 (10 or 12 blocks: 44.1 / 45.2 ms; 4: 49.5).
-constexpr int kAdjBlocks = 8;
 
 __device__ __forceinline__ float poly6_d(const DevParams& P, float r2)
 {
@@ -147,105 +139,6 @@ __device__ __forceinline__ void add_t(float* tgrad, int k, float3 tb)
     if (tb.x != 0.0f) atomicAdd(tgrad + 4 * k + 0, tb.x);
     if (tb.y != 0.0f) atomicAdd(tgrad + 4 * k + 1, tb.y);
     if (tb.z != 0.0f) atomicAdd(tgrad + 4 * k + 2, tb.z);
-}
-
-#define AD_PROLOGUE                                                                                 \
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;                                            \
-    if (t >= (int)P.n) return;                                                                      \
-    const int s = order ? (int)__ldg(order + t) : t;                                                \
-    const int sid = (int)__ldg(scene_of + t);                                                       \
-    const SceneDev* SC = scenes + sid;                                                              \
-    const int2* tab = table + __ldg(&SC->table_off);                                                \
-    const uint32_t mask = __ldg(&SC->mask);
-
-// ---- recording forward passes -------------------------------------------------------------
-__global__ void __launch_bounds__(kAThreads) k_ad_lambda_rec(DevParams P, const SceneDev* __restrict__ scenes,
-                                                             const uint16_t* __restrict__ scene_of,
-                                                             const uint32_t* __restrict__ order,
-                                                             const int2* __restrict__ table,
-                                                             const float4* __restrict__ xin, float4* __restrict__ xl,
-                                                             float4* __restrict__ auxl, float* __restrict__ rhol)
-{
-    AD_PROLOGUE
-    float rho, den;
-    float3 g;
-    xl[s] = lambda_particle_x(P, tab, mask, xin, s, rho, g, den);
-    auxl[s] = make_float4(g.x, g.y, g.z, den);
-    rhol[s] = rho;
-}
-
-__global__ void __launch_bounds__(kAThreads, kAdjBlocks) k_ad_deltap_rec(DevParams P, const SceneDev* __restrict__ scenes,
-                                                             const uint16_t* __restrict__ scene_of,
-                                                             const uint32_t* __restrict__ order,
-                                                             const int2* __restrict__ table,
-                                                             const float4* __restrict__ xl, float4* __restrict__ xout,
-                                                             float4* __restrict__ auxd)
-{
-    AD_PROLOGUE
-    const SdfDev sdf = load_sdf(SC);
-    float3 dp;
-    xout[s] = deltap_particle_x(P, tab, mask, sdf, xl, s, dp);
-    auxd[s] = make_float4(dp.x, dp.y, dp.z, 0.0f);
-}
-
-// ---- CS_VorticityConfinement.glsl:133-167 reversed -----------------------------------------
-// velb (particle order) -> posb_s (sorted, committed positions) and omb
-// (sorted: xyz adjoint of omega_i, w adjoint of |omega_j| by scatter).
-__global__ void __launch_bounds__(kAThreads) k_ad_vorticity(DevParams P, const SceneDev* __restrict__ scenes,
-                                                            const uint16_t* __restrict__ scene_of,
-                                                            const uint32_t* __restrict__ order,
-                                                            const int2* __restrict__ table,
-                                                            const float4* __restrict__ spos,
-                                                            const float4* __restrict__ somega,
-                                                            const uint32_t* __restrict__ ids,
-                                                            const float4* __restrict__ velb,
-                                                            float4* __restrict__ posb_s, float4* __restrict__ omb)
-{
-    AD_PROLOGUE
-    const float4 xi = __ldg(spos + s);
-    float ex = 0.f, ey = 0.f, ez = 0.f;
-    auto hit = [&](float r2) { return r2 <= P.h2 && r2 >= 1e-10f; };
-    masked_walk(P, tab, mask, spos, xi.x, xi.y, xi.z, s, hit, [&](int k) {
-        const float4 xj = __ldg(spos + k);
-        const float rx = xi.x - xj.x, ry = xi.y - xj.y, rz = xi.z - xj.z;
-        const float r2 = rx * rx + ry * ry + rz * rz;
-        const float sc = spiky_scale(P, r2) * __ldg(&somega[k].w);
-        ex += rx * sc;
-        ey += ry * sc;
-        ez += rz * sc;
-    });
-    ex *= P.inv_rho0;
-    ey *= P.inv_rho0;
-    ez *= P.inv_rho0;
-    const float el = sqrtf(ex * ex + ey * ey + ez * ez);
-    if (el < 1e-6f) return;
-    const float3 N = make_float3(ex / el, ey / el, ez / el);
-    const float4 w = __ldg(somega + s);
-    const float4 vb4 = __ldg(velb + __ldg(ids + s));
-    const float k = P.vort_eps * P.dt;
-    const float3 yb = make_float3(k * vb4.x, k * vb4.y, k * vb4.z);
-    // y = N x w:  N_bar = w x y_bar,  w_bar = y_bar x N
-    const float3 Nb = make_float3(w.y * yb.z - w.z * yb.y, w.z * yb.x - w.x * yb.z, w.x * yb.y - w.y * yb.x);
-    const float3 wb = make_float3(yb.y * N.z - yb.z * N.y, yb.z * N.x - yb.x * N.z, yb.x * N.y - yb.y * N.x);
-    add_own(omb + s, wb, 0.0f);
-    const float nn = N.x * Nb.x + N.y * Nb.y + N.z * Nb.z;
-    const float ke = P.inv_rho0 / el;
-    const float3 eb = make_float3((Nb.x - N.x * nn) * ke, (Nb.y - N.y * nn) * ke, (Nb.z - N.z * nn) * ke);
-    float3 own = make_float3(0.f, 0.f, 0.f);
-    masked_walk(P, tab, mask, spos, xi.x, xi.y, xi.z, s, hit, [&](int k2) {
-        const float4 xj = __ldg(spos + k2);
-        const float rx = xi.x - xj.x, ry = xi.y - xj.y, rz = xi.z - xj.z;
-        const float r2 = rx * rx + ry * ry + rz * rz;
-        const float mag = __ldg(&somega[k2].w);
-        const float sg = spiky_scale(P, r2);
-        const float3 rb = grad_vjp(P, rx, ry, rz, r2, make_float3(mag * eb.x, mag * eb.y, mag * eb.z));
-        own.x += rb.x;
-        own.y += rb.y;
-        own.z += rb.z;
-        atomicAdd(posb_s + k2, make_float4(-rb.x, -rb.y, -rb.z, 0.0f));
-        atomicAdd(&omb[k2].w, sg * (rx * eb.x + ry * eb.y + rz * eb.z));
-    });
-    add_own(posb_s + s, own, 0.0f);
 }
 
 // ---- CS_Integrate.glsl:135-280 reversed -------------------------------------------------------
@@ -371,55 +264,6 @@ __device__ __forceinline__ void integrate_pair_adjoint(const DevParams& P, float
     }
 }
 
-// (posb, velb) particle order (+ posb_s sorted, omb sorted when the vorticity
-// pass was reversed) -> gx (adjoint of x*), gv (of v'), x0b, tgrad.
-__global__ void __launch_bounds__(kAThreads, kAdjBlocks) k_ad_integrate(
-    DevParams P, const SceneDev* __restrict__ scenes, const uint16_t* __restrict__ scene_of,
-    const uint32_t* __restrict__ order, const int2* __restrict__ table, const float4* __restrict__ xs,
-    const float4* __restrict__ sv, const float4* __restrict__ cp_pos, const uint32_t* __restrict__ ids,
-    const float4* __restrict__ posb, const float4* __restrict__ velb, const float4* __restrict__ posb_s,
-    const float4* __restrict__ omb, const float4* __restrict__ somega, float4* __restrict__ gx,
-    float4* __restrict__ gv, float4* __restrict__ x0b, float* __restrict__ tgrad)
-{
-    AD_PROLOGUE
-    const float4 x4 = __ldg(xs + s);
-    const float4 v0 = __ldg(sv + s);
-    const uint32_t id = __ldg(ids + s);
-    const float4 p0 = __ldg(cp_pos + id);
-    float fx = 0.f, fy = 0.f, fz = 0.f;
-    if (P.visc_on) {
-        masked_walk(P, tab, mask, xs, x4.x, x4.y, x4.z, s, [&](float r2) { return r2 <= P.h2; }, [&](int k) {
-            const float4 xj = __ldg(xs + k);
-            const float rx = x4.x - xj.x, ry = x4.y - xj.y, rz = x4.z - xj.z;
-            const float r2 = rx * rx + ry * ry + rz * rz;
-            const float4 vj = __ldg(sv + k);
-            const float w = poly6_in(P, r2) * P.inv_rho0;
-            fx += (vj.x - v0.x) * w;
-            fy += (vj.y - v0.y) * w;
-            fz += (vj.z - v0.z) * w;
-        });
-    }
-    float4 x0a;
-    const IntegrateAdjoint A = integrate_adjoint(P, SC, s, id, x4, p0, make_float3(fx, fy, fz), __ldg(posb + id),
-                                                 __ldg(velb + id), posb_s, omb, somega, x0a);
-    x0b[s] = x0a;
-    add_t(tgrad, sid, A.tb);
-    float3 own = A.own, vown = make_float3(0.f, 0.f, 0.f);
-    const bool curl = P.vort_on && omb;
-    if (P.visc_on || curl) {
-        masked_walk(P, tab, mask, xs, x4.x, x4.y, x4.z, s, [&](float r2) { return r2 <= P.h2; }, [&](int k) {
-            float3 ub, rb;
-            integrate_pair_adjoint(P, x4, v0, __ldg(xs + k), __ldg(sv + k), A.vfb, A.cb, curl, ub, rb);
-            own = make_float3(own.x + rb.x, own.y + rb.y, own.z + rb.z);
-            vown = make_float3(vown.x - ub.x, vown.y - ub.y, vown.z - ub.z);
-            atomicAdd(gx + k, make_float4(-rb.x, -rb.y, -rb.z, 0.0f));
-            atomicAdd(gv + k, make_float4(ub.x, ub.y, ub.z, 0.0f));
-        });
-    }
-    add_own(gx + s, own, 0.0f);
-    add_own(gv + s, vown, 0.0f);
-}
-
 // ---- CS_ComputeDeltaP.glsl:120-166 + CS_ApplyDeltaP.glsl:80-124 reversed --------------------
 // The per-particle part: from the adjoint xb of this iteration's output x*
 // (in) the adjoint of x* + dp (out), of the scaled sum (returned), and the SDF
@@ -470,36 +314,6 @@ __device__ __forceinline__ void deltap_pair_adjoint(const DevParams& P, float4 x
     }
 }
 
-// gin (adjoint of this iteration's output x*) -> gout.xyz (adjoint of the
-// input x*) and gout.w (adjoint of lambda), tgrad.
-__global__ void __launch_bounds__(kAThreads, kAdjBlocks) k_ad_deltap(DevParams P, const SceneDev* __restrict__ scenes,
-                                                         const uint16_t* __restrict__ scene_of,
-                                                         const uint32_t* __restrict__ order,
-                                                         const int2* __restrict__ table,
-                                                         const float4* __restrict__ xl,
-                                                         const float4* __restrict__ auxd,
-                                                         const float4* __restrict__ gin, float4* __restrict__ gout,
-                                                         float* __restrict__ tgrad)
-{
-    AD_PROLOGUE
-    const float4 xi = __ldg(xl + s);
-    const float4 g4 = gin[s];
-    float3 own = make_float3(g4.x, g4.y, g4.z), tb;
-    const float3 accb = deltap_adjoint(P, SC, xi, __ldg(auxd + s), own, tb);
-    add_t(tgrad, sid, tb);
-    float lown = 0.0f;
-    masked_walk(P, tab, mask, xl, xi.x, xi.y, xi.z, s, [&](float r2) { return r2 <= P.h2 && r2 >= 1e-10f; },
-                [&](int k) {
-                    float3 rb;
-                    float ga;
-                    deltap_pair_adjoint(P, xi, __ldg(xl + k), accb, rb, ga);
-                    lown += ga;
-                    own = make_float3(own.x + rb.x, own.y + rb.y, own.z + rb.z);
-                    atomicAdd(gout + k, make_float4(-rb.x, -rb.y, -rb.z, ga));
-                });
-    add_own(gout + s, own, lown);
-}
-
 // ---- CS_ComputeLambdas.glsl:108-162 reversed ----------------------------------------------------
 // The adjoints of a particle's sums from lambda's (lb): rhob of rho, gsb of
 // sum gradW, k2 of sum |gradW|^2.
@@ -540,69 +354,43 @@ __device__ __forceinline__ float3 lambda_pair_adjoint(const DevParams& P, float4
     return rb;
 }
 
-// gout.w (adjoint of lambda) -> gout.xyz
-__global__ void __launch_bounds__(kAThreads, kAdjBlocks) k_ad_lambda(DevParams P, const SceneDev* __restrict__ scenes,
-                                                         const uint16_t* __restrict__ scene_of,
-                                                         const uint32_t* __restrict__ order,
-                                                         const int2* __restrict__ table,
-                                                         const float4* __restrict__ xl,
-                                                         const float4* __restrict__ auxl,
-                                                         const float* __restrict__ rhol, float4* __restrict__ gout)
-{
-    AD_PROLOGUE
-    const float lb = gout[s].w;
-    if (lb == 0.0f) return;
-    const float4 xi = __ldg(xl + s);
-    const LambdaAdjoint A = lambda_adjoint(P, lb, __ldg(auxl + s), __ldg(rhol + s));
-    float3 own = make_float3(0.f, 0.f, 0.f);
-    masked_walk(P, tab, mask, xl, xi.x, xi.y, xi.z, s, [&](float r2) { return r2 <= P.h2; }, [&](int k) {
-        const float3 rb = lambda_pair_adjoint(P, xi, __ldg(xl + k), A);
-        own = make_float3(own.x + rb.x, own.y + rb.y, own.z + rb.z);
-        atomicAdd(gout + k, make_float4(-rb.x, -rb.y, -rb.z, 0.0f));
-    });
-    add_own(gout + s, own, 0.0f);
-}
-
-// ---- the same with a group of G lanes per particle (small batches) --------------------------------
+// ---- the passes: a group of G lanes per particle ------------------------------------------------
 // The pairs come from the hits the recording passes kept, one per lane; where
-// a particle had more than fit, its buckets are walked.  One thread walking
-// the buckets took 36 us a pass at 32,768 particles whatever the pass does.
+// a particle had more than fit, its buckets are walked.  (One thread per
+// particle walking the buckets again took 36 us for a reverse delta-p or
+// lambda pass of 32,768 particles and 182 us of 524,288; the groups take 12.4
+// and 8.2 us, 101 and 91 us.)
 struct CoopHits {
     const uint32_t* list;      // kCoopList slots per sorted slot
     const uint32_t* list_len;  // their number, kNoHits: walk
 };
 
-template <class F>
-struct CoopEach {  // coop_walk's hits one per lane, in no order
-    int gl, G;
-    F f;
-    template <class HitAt>
-    __device__ __forceinline__ void add(int cnt, HitAt&& hit)
-    {
-        for (int h = gl; h < cnt; h += G) f(hit(h));
-        __syncwarp();
-    }
-};
-
-// f(k) for every hit of particle s (itself left out), over the group's lanes
-template <int G, class F>
+// f(k, load(k)) for every hit of particle s (itself left out), over the
+// group's lanes in no order; the loads of a lane's next hits are issued together.
+template <int G, class Load, class F>
 __device__ __forceinline__ void coop_each(const DevParams& P, const int2* __restrict__ tab, uint32_t mask,
-                                          const float4* __restrict__ X, float4 xi, int s, bool on, CoopHits H,
-                                          CoopMem<G, 1>& M, F&& f)
+                                          const float4* __restrict__ X, float4 xi, int s, bool on, CoopHits H, Load load,
+                                          F&& f)
 {
+    constexpr int U = kReplayAhead;
     const int gl = threadIdx.x & (G - 1);
-    auto other = [&](int k) {
-        if (k != s) f(k);
-    };
     const uint32_t len = on ? __ldg(H.list_len + s) : 0u;
-    if (__any_sync(0xffffffffu, len == kNoHits)) {
-        CoopEach<decltype(other)> each{gl, G, other};
-        coop_walk<G, 1>(P, tab, mask, X, xi, len == kNoHits, M, each, [&](float r2) { return r2 <= P.h2; }, nullptr,
-                        nullptr);
-    }
-    if (len != kNoHits) {
-        const uint32_t* mine = H.list + (size_t)s * kCoopList;
-        for (uint32_t h = gl; h < len; h += G) other((int)__ldg(mine + h));
+    if (__any_sync(0xffffffffu, len == kNoHits))
+        coop_plain_walk<G>(P, tab, mask, X, xi, s, len == kNoHits, [&](int k) {
+            if (k != s) f(k, load(k));
+        });
+    const uint32_t* mine = H.list + (size_t)s * kCoopList;
+    const int cnt = len == kNoHits ? 0 : (int)len;
+    for (int h = gl; h < cnt; h += U * G) {
+        int k[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) k[u] = h + u * G < cnt ? (int)__ldg(mine + h + u * G) : s;
+        decltype(load(0)) d[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) d[u] = load(k[u]);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (k[u] != s) f(k[u], d[u]);
     }
     __syncwarp();
 }
@@ -621,7 +409,6 @@ __device__ __forceinline__ float3 group_sum(float3 v)
 }
 
 #define AD_COOP_PROLOGUE                                                                            \
-    __shared__ __align__(16) CoopMem<G, 1> mem[kCThreads / G];                                      \
     const CoopParticle cp = coop_particle<G>(P.n, nullptr);                                         \
     const int s = cp.s, gl = threadIdx.x & (G - 1);                                                 \
     const int sid = (int)__ldg(scene_of + s);                                                       \
@@ -630,7 +417,7 @@ __device__ __forceinline__ float3 group_sum(float3 v)
     const uint32_t mask = __ldg(&SC->mask);
 
 template <int G>
-__global__ void __launch_bounds__(kCThreads, kCBlocks) k_ac_integrate(
+__global__ void __launch_bounds__(kCThreads, kReplayBlocks) k_ac_integrate(
     DevParams P, const SceneDev* __restrict__ scenes, const uint16_t* __restrict__ scene_of,
     const int2* __restrict__ table, CoopHits H, const float4* __restrict__ fsum, const float4* __restrict__ xs,
     const float4* __restrict__ sv, const float4* __restrict__ cp_pos, const uint32_t* __restrict__ ids,
@@ -646,9 +433,10 @@ __global__ void __launch_bounds__(kCThreads, kCBlocks) k_ac_integrate(
                                                  __ldg(posb + id), __ldg(velb + id), posb_s, omb, somega, x0a);
     const bool curl = P.vort_on && omb;
     float3 own = make_float3(0.f, 0.f, 0.f), vown = make_float3(0.f, 0.f, 0.f);
-    coop_each<G>(P, tab, mask, xs, x4, s, cp.live && (P.visc_on || curl), H, mem[threadIdx.x / G], [&](int k) {
+    coop_each<G>(P, tab, mask, xs, x4, s, cp.live && (P.visc_on || curl), H,
+                 CoopLoad2{xs, sv}, [&](int k, CoopTwo j) {
         float3 ub, rb;
-        integrate_pair_adjoint(P, x4, v0, __ldg(xs + k), __ldg(sv + k), A.vfb, A.cb, curl, ub, rb);
+        integrate_pair_adjoint(P, x4, v0, j.x, j.v, A.vfb, A.cb, curl, ub, rb);
         own = make_float3(own.x + rb.x, own.y + rb.y, own.z + rb.z);
         vown = make_float3(vown.x - ub.x, vown.y - ub.y, vown.z - ub.z);
         atomicAdd(gx + k, make_float4(-rb.x, -rb.y, -rb.z, 0.0f));
@@ -664,7 +452,7 @@ __global__ void __launch_bounds__(kCThreads, kCBlocks) k_ac_integrate(
 }
 
 template <int G>
-__global__ void __launch_bounds__(kCThreads, kCBlocks) k_ac_deltap(
+__global__ void __launch_bounds__(kCThreads, kReplayBlocks) k_ac_deltap(
     DevParams P, const SceneDev* __restrict__ scenes, const uint16_t* __restrict__ scene_of,
     const int2* __restrict__ table, CoopHits H, const float4* __restrict__ xl, const float4* __restrict__ auxd,
     const float4* __restrict__ gin, float4* __restrict__ gout, float* __restrict__ tgrad)
@@ -676,8 +464,7 @@ __global__ void __launch_bounds__(kCThreads, kCBlocks) k_ac_deltap(
     const float3 accb = deltap_adjoint(P, SC, xi, __ldg(auxd + s), xb, tb);
     float3 own = make_float3(0.f, 0.f, 0.f);
     float lown = 0.0f;
-    coop_each<G>(P, tab, mask, xl, xi, s, cp.live, H, mem[threadIdx.x / G], [&](int k) {
-        const float4 xj = __ldg(xl + k);
+    coop_each<G>(P, tab, mask, xl, xi, s, cp.live, H, CoopLoad1{xl}, [&](int k, float4 xj) {
         const float rx = xi.x - xj.x, ry = xi.y - xj.y, rz = xi.z - xj.z;
         if (!(rx * rx + ry * ry + rz * rz >= 1e-10f)) return;
         float3 rb;
@@ -695,10 +482,10 @@ __global__ void __launch_bounds__(kCThreads, kCBlocks) k_ac_deltap(
 }
 
 template <int G>
-__global__ void __launch_bounds__(kCThreads, kCBlocks) k_ac_lambda(
+__global__ void __launch_bounds__(kCThreads, kReplayBlocks) k_ac_lambda(
     DevParams P, const SceneDev* __restrict__ scenes, const uint16_t* __restrict__ scene_of,
     const int2* __restrict__ table, CoopHits H, const float4* __restrict__ xl, const float4* __restrict__ auxl,
-    const float* __restrict__ rhol, float4* __restrict__ gout)
+    const float* __restrict__ rhol, float4* __restrict__ gout, float4* __restrict__ used)
 {
     AD_COOP_PROLOGUE
     (void)sid;
@@ -707,19 +494,102 @@ __global__ void __launch_bounds__(kCThreads, kCBlocks) k_ac_lambda(
     const float4 xi = __ldg(xl + s);
     const LambdaAdjoint A = lambda_adjoint(P, lb, __ldg(auxl + s), __ldg(rhol + s));
     float3 own = make_float3(0.f, 0.f, 0.f);
-    coop_each<G>(P, tab, mask, xl, xi, s, on, H, mem[threadIdx.x / G], [&](int k) {
-        const float3 rb = lambda_pair_adjoint(P, xi, __ldg(xl + k), A);
+    coop_each<G>(P, tab, mask, xl, xi, s, on, H, CoopLoad1{xl}, [&](int k, float4 xj) {
+        const float3 rb = lambda_pair_adjoint(P, xi, xj, A);
         own = make_float3(own.x + rb.x, own.y + rb.y, own.z + rb.z);
         atomicAdd(gout + k, make_float4(-rb.x, -rb.y, -rb.z, 0.0f));
     });
     own = group_sum<G>(own);
-    if (on && gl == 0) add_own(gout + s, own, 0.0f);
+    if (!cp.live || gl != 0) return;
+    if (on) add_own(gout + s, own, 0.0f);
+    // the adjoints that the reverse delta-p has read: the next one's output
+    used[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+// ---- CS_VorticityConfinement.glsl:133-167 reversed -----------------------------------------
+// velb (particle order) -> posb_s (sorted, committed positions) and omb
+// (sorted: xyz adjoint of omega_i, w adjoint of |omega_j| by scatter).  The
+// committed positions' hits are not kept (the pass runs once a step): the
+// group walks the buckets once for the confinement direction and once more for
+// the pairs.
+template <class F>
+struct EachHit {
+    int gl, G;
+    F f;
+    template <class HitAt>
+    __device__ __forceinline__ void add(int cnt, HitAt&& hit)
+    {
+        for (int h = gl; h < cnt; h += G) f(hit(h));
+        __syncwarp();
+    }
+};
+template <class F>
+__device__ __forceinline__ EachHit<F> each_hit(int gl, int G, F f)
+{
+    return EachHit<F>{gl, G, f};
+}
+
+template <int G>
+__global__ void __launch_bounds__(kCThreads, kCBlocks) k_ac_vorticity(
+    DevParams P, const SceneDev* __restrict__ scenes, const uint16_t* __restrict__ scene_of,
+    const int2* __restrict__ table, const float4* __restrict__ spos, const float4* __restrict__ somega,
+    const uint32_t* __restrict__ ids, const float4* __restrict__ velb, float4* __restrict__ posb_s,
+    float4* __restrict__ omb)
+{
+    AD_COOP_PROLOGUE
+    (void)sid;
+    __shared__ __align__(16) CoopMem<G, 1> mem[kCThreads / G];
+    CoopMem<G, 1>& M = mem[threadIdx.x / G];
+    const float4 xi = __ldg(spos + s);
+    auto hit = [&](float r2) { return r2 <= P.h2 && r2 >= 1e-10f; };
+    float3 e = make_float3(0.f, 0.f, 0.f);
+    auto direction = each_hit(gl, G, [&](int k) {
+        const float4 xj = __ldg(spos + k);
+        const float rx = xi.x - xj.x, ry = xi.y - xj.y, rz = xi.z - xj.z;
+        const float r2 = rx * rx + ry * ry + rz * rz;
+        const float sc = spiky_scale(P, r2) * __ldg(&somega[k].w);
+        e = make_float3(e.x + rx * sc, e.y + ry * sc, e.z + rz * sc);
+    });
+    coop_walk<G, 1>(P, tab, mask, spos, xi, cp.live, M, direction, hit, nullptr, nullptr);
+    e = group_sum<G>(e);
+    e = make_float3(e.x * P.inv_rho0, e.y * P.inv_rho0, e.z * P.inv_rho0);
+    const float el = sqrtf(e.x * e.x + e.y * e.y + e.z * e.z);
+    const bool on = cp.live && !(el < 1e-6f);
+    const float3 N = make_float3(e.x / el, e.y / el, e.z / el);
+    const float4 w = __ldg(somega + s);
+    const float4 vb4 = __ldg(velb + __ldg(ids + s));
+    const float k = P.vort_eps * P.dt;
+    const float3 yb = make_float3(k * vb4.x, k * vb4.y, k * vb4.z);
+    // y = N x w:  N_bar = w x y_bar,  w_bar = y_bar x N
+    const float3 Nb = make_float3(w.y * yb.z - w.z * yb.y, w.z * yb.x - w.x * yb.z, w.x * yb.y - w.y * yb.x);
+    const float3 wb = make_float3(yb.y * N.z - yb.z * N.y, yb.z * N.x - yb.x * N.z, yb.x * N.y - yb.y * N.x);
+    const float nn = N.x * Nb.x + N.y * Nb.y + N.z * Nb.z;
+    const float ke = P.inv_rho0 / el;
+    const float3 eb = make_float3((Nb.x - N.x * nn) * ke, (Nb.y - N.y * nn) * ke, (Nb.z - N.z * nn) * ke);
+    float3 own = make_float3(0.f, 0.f, 0.f);
+    auto pairs = each_hit(gl, G, [&](int k2) {
+        const float4 xj = __ldg(spos + k2);
+        const float rx = xi.x - xj.x, ry = xi.y - xj.y, rz = xi.z - xj.z;
+        const float r2 = rx * rx + ry * ry + rz * rz;
+        const float mag = __ldg(&somega[k2].w);
+        const float sg = spiky_scale(P, r2);
+        const float3 rb = grad_vjp(P, rx, ry, rz, r2, make_float3(mag * eb.x, mag * eb.y, mag * eb.z));
+        own = make_float3(own.x + rb.x, own.y + rb.y, own.z + rb.z);
+        atomicAdd(posb_s + k2, make_float4(-rb.x, -rb.y, -rb.z, 0.0f));
+        atomicAdd(&omb[k2].w, sg * (rx * eb.x + ry * eb.y + rz * eb.z));
+    });
+    coop_walk<G, 1>(P, tab, mask, spos, xi, on, M, pairs, hit, nullptr, nullptr);
+    own = group_sum<G>(own);
+    if (!on || gl != 0) return;
+    add_own(omb + s, wb, 0.0f);
+    add_own(posb_s + s, own, 0.0f);
 }
 
 // ---- CS_PredictAndHash.glsl:102,114 reversed (slot -> particle order) ----------------------------
-__global__ void k_ad_predict(uint32_t n, float dt, const uint32_t* __restrict__ ids, const float4* __restrict__ gx,
-                             const float4* __restrict__ gv, const float4* __restrict__ x0b,
-                             float4* __restrict__ posb, float4* __restrict__ velb)
+// gx and gv are left zero for the next substep's reverse passes.
+__global__ void k_ad_predict(uint32_t n, float dt, const uint32_t* __restrict__ ids, float4* __restrict__ gx,
+                             float4* __restrict__ gv, const float4* __restrict__ x0b, float4* __restrict__ posb,
+                             float4* __restrict__ velb)
 {
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += stride) {
@@ -727,62 +597,19 @@ __global__ void k_ad_predict(uint32_t n, float dt, const uint32_t* __restrict__ 
         const float4 a = gx[s], v = gv[s], b = x0b[s];
         velb[id] = make_float4(v.x + dt * a.x, v.y + dt * a.y, v.z + dt * a.z, 0.0f);
         posb[id] = make_float4(a.x + b.x, a.y + b.y, a.z + b.z, 0.0f);
+        gx[s] = gv[s] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
 }
 
 // ---- launchers ---------------------------------------------------------------------------
-static inline unsigned agrid(uint32_t n) { return (n + kAThreads - 1) / kAThreads; }
-
-void launch_ad_lambda_rec(const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const uint32_t* order,
-                          const int2* table, const float4* xin, float4* xl, float4* auxl, float* rhol, cudaStream_t st)
-{
-    k_ad_lambda_rec<<<agrid(P.n), kAThreads, 0, st>>>(P, scenes, scene_of, order, table, xin, xl, auxl, rhol);
-}
-
-void launch_ad_deltap_rec(const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const uint32_t* order,
-                          const int2* table, const float4* xl, float4* xout, float4* auxd, cudaStream_t st)
-{
-    k_ad_deltap_rec<<<agrid(P.n), kAThreads, 0, st>>>(P, scenes, scene_of, order, table, xl, xout, auxd);
-}
-
-void launch_ad_vorticity(const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const uint32_t* order,
-                         const int2* table, const float4* spos, const float4* somega, const uint32_t* ids,
-                         const float4* velb, float4* posb_s, float4* omb, cudaStream_t st)
-{
-    k_ad_vorticity<<<agrid(P.n), kAThreads, 0, st>>>(P, scenes, scene_of, order, table, spos, somega, ids, velb,
-                                                      posb_s, omb);
-}
-
-void launch_ad_integrate(const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const uint32_t* order,
-                         const int2* table, const float4* xs, const float4* sv, const float4* cp_pos,
-                         const uint32_t* ids, const float4* posb, const float4* velb, const float4* posb_s,
-                         const float4* omb, const float4* somega, float4* gx, float4* gv, float4* x0b, float* tgrad,
-                         cudaStream_t st)
-{
-    k_ad_integrate<<<agrid(P.n), kAThreads, 0, st>>>(P, scenes, scene_of, order, table, xs, sv, cp_pos, ids, posb,
-                                                      velb, posb_s, omb, somega, gx, gv, x0b, tgrad);
-}
-
-void launch_ad_deltap(const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const uint32_t* order,
-                      const int2* table, const float4* xl, const float4* auxd, const float4* gin, float4* gout,
-                      float* tgrad, cudaStream_t st)
-{
-    k_ad_deltap<<<agrid(P.n), kAThreads, 0, st>>>(P, scenes, scene_of, order, table, xl, auxd, gin, gout, tgrad);
-}
-
-void launch_ad_lambda(const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const uint32_t* order,
-                      const int2* table, const float4* xl, const float4* auxl, const float* rhol, float4* gout,
-                      cudaStream_t st)
-{
-    k_ad_lambda<<<agrid(P.n), kAThreads, 0, st>>>(P, scenes, scene_of, order, table, xl, auxl, rhol, gout);
-}
-
 #define PBF_AC_LAUNCH(KERNEL, ...)                                                                 \
     do {                                                                                          \
+        G = coop_replay_lanes(G, P.n);                                                            \
         const unsigned grid_ = (unsigned)(((uint64_t)P.n * (uint64_t)G + kCThreads - 1) / kCThreads); \
         if (G == 32) KERNEL<32><<<grid_, kCThreads, 0, st>>>(__VA_ARGS__);                        \
         else if (G == 16) KERNEL<16><<<grid_, kCThreads, 0, st>>>(__VA_ARGS__);                   \
-        else KERNEL<8><<<grid_, kCThreads, 0, st>>>(__VA_ARGS__);                                 \
+        else if (G == 8) KERNEL<8><<<grid_, kCThreads, 0, st>>>(__VA_ARGS__);                     \
+        else KERNEL<4><<<grid_, kCThreads, 0, st>>>(__VA_ARGS__);                                 \
     } while (0)
 
 void launch_ac_integrate(int G, const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const int2* table,
@@ -804,15 +631,27 @@ void launch_ac_deltap(int G, const DevParams& P, const SceneDev* scenes, const u
 
 void launch_ac_lambda(int G, const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const int2* table,
                       const uint32_t* list, const uint32_t* list_len, const float4* xl, const float4* auxl,
-                      const float* rhol, float4* gout, cudaStream_t st)
+                      const float* rhol, float4* gout, float4* used, cudaStream_t st)
 {
-    PBF_AC_LAUNCH(k_ac_lambda, P, scenes, scene_of, table, CoopHits{list, list_len}, xl, auxl, rhol, gout);
+    PBF_AC_LAUNCH(k_ac_lambda, P, scenes, scene_of, table, CoopHits{list, list_len}, xl, auxl, rhol, gout, used);
+}
+
+void launch_ac_vorticity(int G, const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const int2* table,
+                         const float4* spos, const float4* somega, const uint32_t* ids, const float4* velb,
+                         float4* posb_s, float4* omb, cudaStream_t st)
+{
+    const unsigned grid = (unsigned)(((uint64_t)P.n * (uint64_t)G + kCThreads - 1) / kCThreads);
+    if (G == 32)
+        k_ac_vorticity<32><<<grid, kCThreads, 0, st>>>(P, scenes, scene_of, table, spos, somega, ids, velb, posb_s, omb);
+    else if (G == 16)
+        k_ac_vorticity<16><<<grid, kCThreads, 0, st>>>(P, scenes, scene_of, table, spos, somega, ids, velb, posb_s, omb);
+    else
+        k_ac_vorticity<8><<<grid, kCThreads, 0, st>>>(P, scenes, scene_of, table, spos, somega, ids, velb, posb_s, omb);
 }
 
 #undef PBF_AC_LAUNCH
 
-void launch_ad_predict(uint32_t n, float dt, const uint32_t* ids, const float4* gx, const float4* gv,
-                       const float4* x0b, float4* posb, float4* velb, int sms, cudaStream_t st)
+void launch_ad_predict(uint32_t n, float dt, const uint32_t* ids, float4* gx, float4* gv, const float4* x0b, float4* posb, float4* velb, int sms, cudaStream_t st)
 {
     const uint32_t want = (n + 255u) / 256u, cap = (uint32_t)sms * 8u;
     k_ad_predict<<<want < 1 ? 1 : (want > cap ? cap : want), 256, 0, st>>>(n, dt, ids, gx, gv, x0b, posb, velb);

@@ -39,9 +39,7 @@ __global__ void __launch_bounds__(kCThreads, kCBlocks) k_c_lambda(DevParams P, c
         mask = __ldg(&S->mask);
     }
     const bool scorr = P.scorr && P.wq > 1e-12f;
-    auto pair = [&](int k, float(&t)[NT]) {
-        if (k == s) return;
-        const float4 xj = __ldg(xin + k);
+    auto pair = [&](float4 xj, float(&t)[NT]) {
         const float2 rxy = sub_f32x2(make_float2(xi.x, xi.y), make_float2(xj.x, xj.y));
         const float rx = rxy.x, ry = rxy.y, rz = xi.z - xj.z;
         const float r2 = rx * rx + ry * ry + rz * rz;
@@ -70,8 +68,8 @@ __global__ void __launch_bounds__(kCThreads, kCBlocks) k_c_lambda(DevParams P, c
     };
     // sums: rho, |gradW|^2, gradW xyz, (W / W(dq))^n gradW xyz
     CoopMem<G, NT>& M = mem[threadIdx.x / G];
-    CoopSum<G, NT, decltype(pair)> sum(M, gl, coop_row(0x43243210u, gl), coop_row(0x55566666u, gl),
-                                       gl == 0 ? P.w0_self : 0.0f, std::move(pair));
+    CoopSum<G, NT, 1, CoopLoad1, decltype(pair)> sum(M.term, gl, s, coop_row(0x43243210u, gl), coop_row(0x55566666u, gl),
+                                                  gl == 0 ? P.w0_self : 0.0f, CoopLoad1{xin}, std::move(pair));
     uint32_t len = kNoHits;
     coop_walk<G, NT>(P, table, mask, xin, xi, c.live && !skip, M, sum, [&](float r2) { return r2 <= P.h2; },
                      c.live && list ? list + (size_t)s * kCoopList : nullptr, &len);
@@ -93,7 +91,7 @@ __global__ void __launch_bounds__(kCThreads, kCBlocks) k_c_lambda(DevParams P, c
 }
 
 template <int G, bool B>
-__global__ void __launch_bounds__(kCThreads, kCBlocks) k_c_deltap(DevParams P, const SceneDev* __restrict__ scenes,
+__global__ void __launch_bounds__(kCThreads, kReplayBlocks) k_c_deltap(DevParams P, const SceneDev* __restrict__ scenes,
                                                         const uint16_t* __restrict__ scene_of,
                                                         const float4* __restrict__ xin, float4* __restrict__ xout,
                                                         const int2* __restrict__ table,
@@ -104,7 +102,7 @@ __global__ void __launch_bounds__(kCThreads, kCBlocks) k_c_deltap(DevParams P, c
                                                         float4* __restrict__ dp_out)
 {
     constexpr int NT = 4;
-    __shared__ __align__(16) CoopMem<G, NT> mem[kCThreads / G];
+    __shared__ __align__(16) CoopTermMem<G, NT> mem[kCThreads / G];
     const CoopParticle c = coop_particle<G>(P.n, order);
     const int gl = threadIdx.x & (G - 1), s = c.s;
     const float4 xi = __ldg(xin + s);
@@ -117,25 +115,25 @@ __global__ void __launch_bounds__(kCThreads, kCBlocks) k_c_deltap(DevParams P, c
         mask = __ldg(&S->mask);
     }
     const float4 b = __ldg(P.dpb + s);
-    auto pair = [&](int k, float(&t)[NT]) {
-        const float4 xj = __ldg(xin + k);
+    auto pair = [&](float4 xj, float(&t)[NT]) {
         const float2 rxy = sub_f32x2(make_float2(xi.x, xi.y), make_float2(xj.x, xj.y));
         const float rx = rxy.x, ry = rxy.y, rz = xi.z - xj.z;
         const float r2 = rx * rx + ry * ry + rz * rz;
-        if (k == s || !(r2 >= 1e-10f)) return;
+        if (!(r2 >= 1e-10f)) return;
         t[0] = rx;
         t[1] = ry;
         t[2] = rz;
         t[3] = spiky_scale(P, r2) * xj.w;
     };
     // sums: lambda_j gradW xyz, from the lambda pass's part on
-    CoopMem<G, NT>& M = mem[threadIdx.x / G];
-    CoopSum<G, NT, decltype(pair)> sum(M, gl, min(gl, 2), 3, gl == 0 ? b.x : gl == 1 ? b.y : b.z, std::move(pair));
+    CoopSum<G, NT, kReplayAhead, CoopLoad1, decltype(pair)> sum(mem[threadIdx.x / G].term, gl, s, min(gl, 2), 3,
+                                                                gl == 0 ? b.x : gl == 1 ? b.y : b.z, CoopLoad1{xin},
+                                                                std::move(pair));
     const bool on = c.live && !skip;
     const uint32_t len = on && list ? __ldg(list_len + s) : kNoHits;
     if (__any_sync(0xffffffffu, on && len == kNoHits))
-        coop_walk<G, NT>(P, table, mask, xin, xi, on && len == kNoHits, M, sum,
-                         [&](float r2) { return r2 <= P.h2 && r2 >= 1e-10f; }, nullptr, nullptr);
+        coop_plain_walk<G>(P, table, mask, xin, xi, s, on && len == kNoHits,
+                           [&](int k) { sum.chunk(k, __ldg(xin + k), G); });
     const uint32_t* mine = list + (size_t)s * kCoopList;
     sum.add(len == kNoHits ? 0 : (int)len, [&](int i) { return (int)__ldg(mine + i); });
     const float3 d = make_float3(sum.get(0), sum.get(1), sum.get(2));
@@ -178,10 +176,8 @@ __global__ void __launch_bounds__(kCThreads, kCBlocks) k_c_integrate(DevParams P
         table += __ldg(&S->table_off);
         mask = __ldg(&S->mask);
     }
-    auto pair = [&](int k, float(&t)[NT]) {
-        if (k == s) return;
-        const float4 xj = __ldg(xs + k);
-        const float4 vj = __ldg(sv + k);
+    auto pair = [&](CoopTwo j, float(&t)[NT]) {
+        const float4 xj = j.x, vj = j.v;
         const float2 rxy = sub_f32x2(make_float2(x4.x, x4.y), make_float2(xj.x, xj.y));
         const float rx = rxy.x, ry = rxy.y, rz = x4.z - xj.z;
         const float r2 = rx * rx + ry * ry + rz * rz;
@@ -202,8 +198,8 @@ __global__ void __launch_bounds__(kCThreads, kCBlocks) k_c_integrate(DevParams P
     };
     // sums: W u xyz, u x gradW xyz
     CoopMem<G, NT>& M = mem[threadIdx.x / G];
-    CoopSum<G, NT, decltype(pair)> sum(M, gl, coop_row(0x00654210u, gl), coop_row(0x77777333u, gl), 0.0f,
-                                       std::move(pair));
+    CoopSum<G, NT, 1, CoopLoad2, decltype(pair)> sum(M.term, gl, s, coop_row(0x00654210u, gl), coop_row(0x77777333u, gl), 0.0f,
+                                                  CoopLoad2{xs, sv}, std::move(pair));
     uint32_t len = kNoHits;
     coop_walk<G, NT>(P, table, mask, xs, x4, c.live && (P.visc_on || P.vort_on), M, sum,
                      [&](float r2) { return r2 <= P.h2; }, c.live && list ? list + (size_t)s * kCoopList : nullptr,
@@ -254,21 +250,20 @@ __global__ void __launch_bounds__(kCThreads, kCBlocks) k_c_vorticity(DevParams P
         table += __ldg(&S->table_off);
         mask = __ldg(&S->mask);
     }
-    auto pair = [&](int k, float(&t)[NT]) {
-        if (k == s) return;
-        const float4 xj = __ldg(spos + k);
-        const float m = __ldg(&somega[k].w);
+    auto pair = [&](CoopTwo j, float(&t)[NT]) {
+        const float4 xj = j.x;
         const float2 rxy = sub_f32x2(make_float2(xi.x, xi.y), make_float2(xj.x, xj.y));
         const float rx = rxy.x, ry = rxy.y, rz = xi.z - xj.z;
         const float r2 = rx * rx + ry * ry + rz * rz;
         t[0] = rx;
         t[1] = ry;
         t[2] = rz;
-        t[3] = spiky_scale(P, r2) * m;
+        t[3] = spiky_scale(P, r2) * j.v.w;
     };
     // sums: |omega_j| gradW xyz
     CoopMem<G, NT>& M = mem[threadIdx.x / G];
-    CoopSum<G, NT, decltype(pair)> sum(M, gl, min(gl, 2), 3, 0.0f, std::move(pair));
+    CoopSum<G, NT, 1, CoopLoad2, decltype(pair)> sum(M.term, gl, s, min(gl, 2), 3, 0.0f, CoopLoad2{spos, somega},
+                                                  std::move(pair));
     coop_walk<G, NT>(P, table, mask, spos, xi, c.live, M, sum, [&](float r2) { return r2 <= P.h2 && r2 >= 1e-10f; },
                      nullptr, nullptr);
     const float3 e = make_float3(sum.get(0), sum.get(1), sum.get(2));
@@ -297,6 +292,12 @@ int coop_lanes(uint32_t n)
     if (n <= 8192u) return 16;
     return n <= (1u << 18) ? 8 : 0;
 }
+
+// Passes over kept hits need no walk, and three or four sums: four lanes keep
+// more of the warp at work (131,072 particles: delta-p 22.5 us against 27.8
+// with 8 lanes, the reverse delta-p 31.6 against 34.4; 32,768: 8.2 against 10.0,
+// 12.6 against 12.9).
+int coop_replay_lanes(int G, uint32_t n) { return n > 16384u ? 4 : G; }
 
 static inline unsigned cgrid(uint32_t n, int G)
 {
@@ -327,6 +328,16 @@ void launch_c_deltap(int G, const DevParams& P, const SceneDev* scenes, const ui
                      float4* xout, const int2* table, const uint32_t* lod, uint32_t iter, const uint32_t* order,
                      const uint32_t* list, const uint32_t* list_len, float4* dp_out, cudaStream_t st)
 {
+    G = coop_replay_lanes(G, P.n);
+    if (G == 4) {
+        if (scenes)
+            k_c_deltap<4, true><<<cgrid(P.n, 4), kCThreads, 0, st>>>(P, scenes, scene_of, xin, xout, table, lod, iter,
+                                                                     order, list, list_len, dp_out);
+        else
+            k_c_deltap<4, false><<<cgrid(P.n, 4), kCThreads, 0, st>>>(P, scenes, scene_of, xin, xout, table, lod, iter,
+                                                                      order, list, list_len, dp_out);
+        return;
+    }
     PBF_COOP_LAUNCH(k_c_deltap, P, scenes, scene_of, xin, xout, table, lod, iter, order, list, list_len, dp_out);
 }
 

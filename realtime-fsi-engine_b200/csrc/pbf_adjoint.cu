@@ -4,8 +4,8 @@
 // exactly as pbf_batch_step does, saving the particle state at the start of
 // each substep and, where memory allows, everything the reverse passes read of
 // it: the sort permutation and cell table (replayed, not differentiated), (x*,
-// lambda), the lambda denominators and the raw dp of every iteration and, for
-// small batches, every particle's hits.  pbf_batch_backward walks the substeps
+// lambda), the lambda denominators, the raw dp and the particles' hits of every
+// iteration.  pbf_batch_backward walks the substeps
 // in reverse with the kernels of k_adjoint.cu: vorticity (last substep),
 // integrate, (deltaP+apply, lambda) per iteration, predict.  Without the room,
 // or when a scene changed since the recording, it first runs each substep's
@@ -62,9 +62,14 @@ void pbf_batch::ad_free()
     recorded = false;
 }
 
+// Lanes per particle of the recording and reverse passes: groups at any size
+// (524,288 particles in 16 scenes, per iteration: recording 322 us and reverse
+// 191, one thread per particle 278 and 361).
+int pbf_batch::ad_lanes() const { return std::max(coop_lanes(n), 8); }
+
 // One record's arrays laid one after another from `base` (null: only counted);
 // returns its bytes.  `c` entries per array (a multiple of 64, pads included).
-static size_t lay_record(pbf_batch::Record& r, char* base, size_t c, uint32_t iters, size_t table, bool hits, bool order)
+static size_t lay_record(pbf_batch::Record& r, char* base, size_t c, uint32_t iters, size_t table)
 {
     size_t at = 0;
     auto take = [&](auto*& p, size_t count) {
@@ -72,7 +77,6 @@ static size_t lay_record(pbf_batch::Record& r, char* base, size_t c, uint32_t it
         at += (count * sizeof(*p) + 255) / 256 * 256;
     };
     take(r.ids, c);
-    if (order) take(r.order, c);
     take(r.table, table);
     take(r.sv, c);
     take(r.xf, c);
@@ -80,11 +84,9 @@ static size_t lay_record(pbf_batch::Record& r, char* base, size_t c, uint32_t it
     take(r.auxl, c * iters);
     take(r.auxd, c * iters);
     take(r.rhol, c * iters);
-    if (hits) {
-        take(r.fsum, c);
-        take(r.list, c * (iters + 1) * kCoopList);
-        take(r.list_len, c * (iters + 1));
-    }
+    take(r.fsum, c);
+    take(r.list, c * (iters + 1) * kCoopList);
+    take(r.list_len, c * (iters + 1));
     return at;
 }
 
@@ -105,10 +107,9 @@ int pbf_batch::ad_alloc()
     }
     // a record per substep when they take at most a quarter of the free memory
     // (32,768 particles x 16 substeps x 4 iterations: 0.9 GB)
-    const bool hits = coop_lanes(n) != 0;
     ad_stride = (c + kCoopPad + 63) / 64 * 64;
     Record probe;
-    const size_t bytes = lay_record(probe, nullptr, ad_stride, I, table_size, hits, !hits);
+    const size_t bytes = lay_record(probe, nullptr, ad_stride, I, table_size);
     size_t free_b = 0, total_b = 0;
     ACK(cudaMemGetInfo(&free_b, &total_b));
     ad_full = bytes * S <= free_b / 4;
@@ -120,7 +121,7 @@ int pbf_batch::ad_alloc()
     }
     ad_slab = slab;
     records.resize(R);
-    for (uint32_t k = 0; k < R; ++k) lay_record(records[k], slab + bytes * k, ad_stride, I, table_size, hits, !hits);
+    for (uint32_t k = 0; k < R; ++k) lay_record(records[k], slab + bytes * k, ad_stride, I, table_size);
     ad_subs = S;
     ad_iters = I;
     return PBF_OK;
@@ -132,39 +133,24 @@ int pbf_batch::record_substep(uint32_t sub, Record& r, const float4* src_pos, co
                               float4* dst_vel)
 {
     const DevParams P = dev_params();
-    BatchLaunch L = launch;
-    L.sms = num_sms;
-    const int sms = num_sms, G = coop_lanes(n);
+    const int sms = num_sms, G = ad_lanes();
     const uint32_t I = cfg.solver_iterations;
     const bool last = sub + 1 == cfg.substep_iterations;
     launch_b_predict(P, scenes_dev, scene_of, src_pos, src_vel, keys, sms, stream);
     launch_radix_sort_into(n, key_bits, keys, ka, r.ids, kb, ib, hist, totals, stream);
     ACK(cudaMemsetAsync(r.table, 0xFF, sizeof(int2) * (size_t)table_size, stream));
     launch_build_table(n, ka, r.table, sms, stream);
-    const bool sorted = morton && !G;
-    float4* x = I ? sx[0] : r.xf;
-    launch_b_reorder(P, scenes_dev, scene_of, r.ids, src_pos, src_vel, x, r.sv, sx0, lod, sorted ? mcode : nullptr,
-                     mbits, sms, stream);
+    launch_b_reorder(P, scenes_dev, scene_of, r.ids, src_pos, src_vel, I ? sx[0] : r.xf, r.sv, sx0, lod, nullptr, mbits,
+                     sms, stream);
     launches += 3 + 3 * ((key_bits + 7) / 8);
-    const uint32_t* ord = nullptr;
-    if (sorted) {
-        launch_radix_sort_into(n, order_bits, mcode, mka, r.order, mkb, mib, hist, totals, stream);
-        launches += 3 * ((order_bits + 7) / 8);
-        ord = r.order;
-    }
     for (uint32_t it = 1; it <= I; ++it) {
         const size_t at = (size_t)(it - 1) * ad_stride;
-        float4 *xl = r.xl + at, *out = it == I ? r.xf : sx[0];
-        if (G) {
-            uint32_t *list = r.list + at * kCoopList, *len = r.list_len + at;
-            launch_c_lambda(G, P, scenes_dev, scene_of, sx[0], xl, r.rhol + at, r.table, lod, it, nullptr, list, len,
-                            r.auxl + at, stream);
-            launch_c_deltap(G, P, scenes_dev, scene_of, xl, out, r.table, lod, it, nullptr, list, len, r.auxd + at,
-                            stream);
-        } else {
-            launch_ad_lambda_rec(P, scenes_dev, scene_of, ord, r.table, sx[0], xl, r.auxl + at, r.rhol + at, stream);
-            launch_ad_deltap_rec(P, scenes_dev, scene_of, ord, r.table, xl, out, r.auxd + at, stream);
-        }
+        float4* xl = r.xl + at;
+        uint32_t *list = r.list + at * kCoopList, *len = r.list_len + at;
+        launch_c_lambda(G, P, scenes_dev, scene_of, sx[0], xl, r.rhol + at, r.table, lod, it, nullptr, list, len,
+                        r.auxl + at, stream);
+        launch_c_deltap(G, P, scenes_dev, scene_of, xl, it == I ? r.xf : sx[0], r.table, lod, it, nullptr, list, len,
+                        r.auxd + at, stream);
         launches += 2;
     }
     float4* x0 = sx0;
@@ -174,24 +160,15 @@ int pbf_batch::record_substep(uint32_t sub, Record& r, const float4* src_pos, co
         x0 = ad_sx0;
         om = ad_om;
     }
-    if (G)
-        launch_c_integrate(G, P, scenes_dev, scene_of, r.xf, r.sv, x0, om, r.ids, dst_pos, dst_vel, r.table, nullptr,
-                           r.list + (size_t)I * ad_stride * kCoopList, r.list_len + (size_t)I * ad_stride, r.fsum,
-                           stream);
-    else
-        launch_b_integrate(P, L, scenes_dev, scene_of, r.xf, r.sv, x0, om, r.ids, dst_pos, dst_vel, r.table, ord,
-                           stream);
+    launch_c_integrate(G, P, scenes_dev, scene_of, r.xf, r.sv, x0, om, r.ids, dst_pos, dst_vel, r.table, nullptr,
+                       r.list + (size_t)I * ad_stride * kCoopList, r.list_len + (size_t)I * ad_stride, r.fsum, stream);
     ++launches;
     return PBF_OK;
 }
 
 int pbf_batch::record_body()
 {
-    const DevParams P = dev_params();
-    BatchLaunch L = launch;
-    L.sms = num_sms;
     const uint32_t S = cfg.substep_iterations;
-    const int G = coop_lanes(n);
     for (uint32_t sub = 0; sub < S; ++sub) {
         ACK(cudaMemcpyAsync(cp_pos + (size_t)sub * n, pos, sizeof(float4) * n, cudaMemcpyDeviceToDevice, stream));
         ACK(cudaMemcpyAsync(cp_vel + (size_t)sub * n, vel, sizeof(float4) * n, cudaMemcpyDeviceToDevice, stream));
@@ -200,11 +177,8 @@ int pbf_batch::record_body()
     }
     if (cfg.enable_vorticity) {
         const Record& r = records[ad_full ? S - 1 : 0];
-        if (G)
-            launch_c_vorticity(G, P, scenes_dev, scene_of, ad_sx0, ad_om, r.ids, vel, r.table, nullptr, stream);
-        else
-            launch_b_vorticity(P, L, scenes_dev, scene_of, ad_sx0, ad_om, r.ids, vel, r.table, morton ? r.order : nullptr,
-                               stream);
+        launch_c_vorticity(ad_lanes(), dev_params(), scenes_dev, scene_of, ad_sx0, ad_om, r.ids, vel, r.table, nullptr,
+                           stream);
         ++launches;
     }
     return PBF_OK;
@@ -215,12 +189,17 @@ int pbf_batch::record_body()
 int pbf_batch::backward_body(bool recompute)
 {
     const DevParams P = dev_params();
-    const int sms = num_sms, G = coop_lanes(n);
+    const int sms = num_sms, G = ad_lanes();
     const uint32_t S = cfg.substep_iterations, I = cfg.solver_iterations;
     const bool vort = cfg.enable_vorticity != 0;
     ACK(cudaMemsetAsync(tgrad, 0, sizeof(float) * 4 * scenes.size(), stream));
     ACK(cudaMemsetAsync(pbs, 0, sizeof(float4) * n, stream));
     ACK(cudaMemsetAsync(omb, 0, sizeof(float4) * n, stream));
+    // accumulated with atomics; each pass that is through with one clears it
+    ACK(cudaMemsetAsync(gxa, 0, sizeof(float4) * n, stream));
+    ACK(cudaMemsetAsync(gxb, 0, sizeof(float4) * n, stream));
+    ACK(cudaMemsetAsync(gv, 0, sizeof(float4) * n, stream));
+    float4 *a = gxa, *b = gxb;
     for (int sub = (int)S - 1; sub >= 0; --sub) {
         const float4* src_pos = cp_pos + (size_t)sub * n;
         const float4* src_vel = cp_vel + (size_t)sub * n;
@@ -229,39 +208,22 @@ int pbf_batch::backward_body(bool recompute)
             const int rc = record_substep((uint32_t)sub, r, src_pos, src_vel, tpos, tvel);
             if (rc) return rc;
         }
-        const uint32_t* ord = morton && !G ? r.order : nullptr;
         const bool last = (sub == (int)S - 1) && vort;
         if (last) {
-            launch_ad_vorticity(P, scenes_dev, scene_of, ord, r.table, ad_sx0, ad_om, r.ids, vb, pbs, omb, stream);
+            launch_ac_vorticity(G, P, scenes_dev, scene_of, r.table, ad_sx0, ad_om, r.ids, vb, pbs, omb, stream);
             ++launches;
         }
-        ACK(cudaMemsetAsync(gxa, 0, sizeof(float4) * n, stream));
-        ACK(cudaMemsetAsync(gxb, 0, sizeof(float4) * n, stream));
-        ACK(cudaMemsetAsync(gv, 0, sizeof(float4) * n, stream));
-        if (G)
-            launch_ac_integrate(G, P, scenes_dev, scene_of, r.table, r.list + (size_t)I * ad_stride * kCoopList,
-                                r.list_len + (size_t)I * ad_stride, r.fsum, r.xf, r.sv, src_pos, r.ids, pb, vb,
-                                last ? pbs : nullptr, last ? omb : nullptr, ad_om, gxa, gv, x0b, tgrad, stream);
-        else
-            launch_ad_integrate(P, scenes_dev, scene_of, ord, r.table, r.xf, r.sv, src_pos, r.ids, pb, vb,
-                                last ? pbs : nullptr, last ? omb : nullptr, ad_om, gxa, gv, x0b, tgrad, stream);
+        launch_ac_integrate(G, P, scenes_dev, scene_of, r.table, r.list + (size_t)I * ad_stride * kCoopList,
+                            r.list_len + (size_t)I * ad_stride, r.fsum, r.xf, r.sv, src_pos, r.ids, pb, vb,
+                            last ? pbs : nullptr, last ? omb : nullptr, ad_om, a, gv, x0b, tgrad, stream);
         ++launches;
-        float4* a = gxa;
-        float4* b = gxb;
         for (int it = (int)I; it >= 1; --it) {
             const size_t at = (size_t)(it - 1) * ad_stride;
-            if (G) {
-                const uint32_t *list = r.list + at * kCoopList, *len = r.list_len + at;
-                launch_ac_deltap(G, P, scenes_dev, scene_of, r.table, list, len, r.xl + at, r.auxd + at, a, b, tgrad,
-                                 stream);
-                launch_ac_lambda(G, P, scenes_dev, scene_of, r.table, list, len, r.xl + at, r.auxl + at, r.rhol + at, b,
-                                 stream);
-            } else {
-                launch_ad_deltap(P, scenes_dev, scene_of, ord, r.table, r.xl + at, r.auxd + at, a, b, tgrad, stream);
-                launch_ad_lambda(P, scenes_dev, scene_of, ord, r.table, r.xl + at, r.auxl + at, r.rhol + at, b, stream);
-            }
+            const uint32_t *list = r.list + at * kCoopList, *len = r.list_len + at;
+            launch_ac_deltap(G, P, scenes_dev, scene_of, r.table, list, len, r.xl + at, r.auxd + at, a, b, tgrad, stream);
+            launch_ac_lambda(G, P, scenes_dev, scene_of, r.table, list, len, r.xl + at, r.auxl + at, r.rhol + at, b, a,
+                             stream);
             launches += 2;
-            ACK(cudaMemsetAsync(a, 0, sizeof(float4) * n, stream));
             std::swap(a, b);
         }
         launch_ad_predict(n, P.dt, r.ids, a, gv, x0b, pb, vb, sms, stream);

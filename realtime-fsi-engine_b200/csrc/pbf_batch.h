@@ -74,26 +74,11 @@ void launch_b_vorticity(const DevParams& P, const BatchLaunch& L, const SceneDev
 int batch_max_blocks_per_sm(int block);
 
 // ---- k_adjoint.cu ---------------------------------------------------------------------------
-void launch_ad_lambda_rec(const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const uint32_t* order,
-                          const int2* table, const float4* xin, float4* xl, float4* auxl, float* rhol, cudaStream_t st);
-void launch_ad_deltap_rec(const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const uint32_t* order,
-                          const int2* table, const float4* xl, float4* xout, float4* auxd, cudaStream_t st);
-void launch_ad_vorticity(const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const uint32_t* order,
-                         const int2* table, const float4* spos, const float4* somega, const uint32_t* ids,
-                         const float4* velb, float4* posb_s, float4* omb, cudaStream_t st);
-void launch_ad_integrate(const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const uint32_t* order,
-                         const int2* table, const float4* xs, const float4* sv, const float4* cp_pos,
-                         const uint32_t* ids, const float4* posb, const float4* velb, const float4* posb_s,
-                         const float4* omb, const float4* somega, float4* gx, float4* gv, float4* x0b, float* tgrad,
-                         cudaStream_t st);
-void launch_ad_deltap(const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const uint32_t* order,
-                      const int2* table, const float4* xl, const float4* auxd, const float4* gin, float4* gout,
-                      float* tgrad, cudaStream_t st);
-void launch_ad_lambda(const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const uint32_t* order,
-                      const int2* table, const float4* xl, const float4* auxl, const float* rhol, float4* gout,
-                      cudaStream_t st);
 // The reverse passes with a group of G lanes per particle, over the hits the
 // recording passes kept (list, list_len); fsum: the XSPH sums of the integrate pass.
+void launch_ac_vorticity(int G, const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const int2* table,
+                         const float4* spos, const float4* somega, const uint32_t* ids, const float4* velb,
+                         float4* posb_s, float4* omb, cudaStream_t st);
 void launch_ac_integrate(int G, const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const int2* table,
                          const uint32_t* list, const uint32_t* list_len, const float4* fsum, const float4* xs,
                          const float4* sv, const float4* cp_pos, const uint32_t* ids, const float4* posb,
@@ -104,9 +89,8 @@ void launch_ac_deltap(int G, const DevParams& P, const SceneDev* scenes, const u
                       const float4* gin, float4* gout, float* tgrad, cudaStream_t st);
 void launch_ac_lambda(int G, const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const int2* table,
                       const uint32_t* list, const uint32_t* list_len, const float4* xl, const float4* auxl,
-                      const float* rhol, float4* gout, cudaStream_t st);
-void launch_ad_predict(uint32_t n, float dt, const uint32_t* ids, const float4* gx, const float4* gv,
-                       const float4* x0b, float4* posb, float4* velb, int sms, cudaStream_t st);
+                      const float* rhol, float4* gout, float4* used, cudaStream_t st);
+void launch_ad_predict(uint32_t n, float dt, const uint32_t* ids, float4* gx, float4* gv, const float4* x0b, float4* posb, float4* velb, int sms, cudaStream_t st);
 
 }  // namespace pbf
 
@@ -197,13 +181,13 @@ struct pbf_batch {
     // forward; otherwise there is one, which the backward fills again from the
     // substep's checkpoint.
     struct Record {
-        uint32_t *ids = nullptr, *order = nullptr;  // sort permutation, processing order (null: sorted order)
+        uint32_t* ids = nullptr;                    // sort permutation
         int2* table = nullptr;
         float4 *sv = nullptr, *xf = nullptr;        // v', x* after the last iteration (sorted)
-        float4* fsum = nullptr;                     // XSPH sums (groups of lanes only)
+        float4* fsum = nullptr;                     // XSPH sums
         float4 *xl = nullptr, *auxl = nullptr, *auxd = nullptr;  // per iteration: (x*, lambda), (grad C, denominator), raw dp
         float* rhol = nullptr;                      // per iteration: density
-        uint32_t *list = nullptr, *list_len = nullptr;  // per iteration, then integrate: hits (groups of lanes only)
+        uint32_t *list = nullptr, *list_len = nullptr;  // per iteration, then integrate: hits (k_coop.cu)
     };
     std::vector<Record> records;
     size_t ad_stride = 0;         // entries between the iterations' arrays of a record
@@ -238,6 +222,7 @@ struct pbf_batch {
     int step();
     void vorticity_pass();
     int substep_body(const float4* src_pos, const float4* src_vel, float4* dst_pos, float4* dst_vel);
+    int ad_lanes() const;
     int ad_alloc();
     void ad_free();
     int record_substep(uint32_t sub, Record& r, const float4* src_pos, const float4* src_vel, float4* dst_pos,

@@ -36,6 +36,8 @@ void launch_vorticity_m(const DevParams& P, const float4* spos, const float4* so
 // Lanes per particle for a scene (or batch) of n particles; 0: one thread per
 // particle (k_masked.cu, k_batch.cu).
 int coop_lanes(uint32_t n);
+// ... and of the passes over kept hits, where the others take G.
+int coop_replay_lanes(int G, uint32_t n);
 // The hits of a lambda pass, kept for the delta-p pass of the same iteration:
 // kCoopList slots per sorted slot and their number (list, list_len; null: not kept).
 constexpr int kCoopList = 64;

@@ -250,3 +250,60 @@ def test_c4_gradient_at_the_accuracy_of_fp32_arithmetic(have_gpu):
     g, c = d[keep, 0], d[keep, 1]
     assert np.median(g) <= max(1e-3, 2 * np.median(c)), d
     assert g.max() <= max(1e-3, 2 * c.max()), d
+
+
+@pytest.mark.parametrize("nside", [8, 17, 21, 26])
+def test_group_widths_match_fp64(have_gpu, nside):
+    """Sizes on both sides of the lanes a particle gets (32, 16, 8, and 4 in
+    the passes over kept hits); the tolerance of the small cases above."""
+    cfg, _, pos, vel, grid, target = setup(nside=nside, subs=2, iters=2, scorr=False)
+    cfg.bounds_max[:] = [1.5, 1.5, 1.5]
+    Po = O.Params(_oracle_config(cfg))
+    b = make_batch(cfg, pos, vel, grid)
+    gp, gv, gt, _ = gpu_grads(b, pos, vel, target, np.zeros((1, 3)))
+    _, pT64 = loss(Po, pos, vel, grid, np.zeros(3), target)[:2]
+    gp0, gv0, gt0, _, _ = O.adjoint_step(Po, pos, vel, gpos=2 * (pT64 - target) / len(pos),
+                                         sdf=mk_sdf(grid, np.zeros(3)))
+    assert rel(gv, gv0) <= 1e-3 and rel(gp, gp0) <= 1e-3 and rel(gt[0], gt0) <= 1e-3
+
+
+def _oracle_config(cfg):
+    import ctypes as C
+    oc = O.FluidConfig()
+    C.memmove(C.byref(oc), C.byref(cfg), C.sizeof(oc))
+    return oc
+
+
+def test_more_hits_than_are_kept(have_gpu):
+    """A block at 0.55 of its spacing: about 200 hits a particle, so the
+    passes over kept hits walk the buckets instead."""
+    cfg, Po, pos, vel, grid, target = setup(nside=9, subs=1, iters=2, sdf=False, scorr=False)
+    mid = pos.mean(0)
+    pos = (mid + 0.55 * (pos - mid)).astype(np.float32).astype(np.float64)
+    b = make_batch(cfg, pos, vel, grid)
+    gp, gv, _, _ = gpu_grads(b, pos, vel, target, np.zeros((1, 3)))
+    _, pT64 = loss(Po, pos, vel, grid, np.zeros(3), target)[:2]
+    gp0, gv0, _, _, _ = O.adjoint_step(Po, pos, vel, gpos=2 * (pT64 - target) / len(pos))
+    assert rel(gv, gv0) <= 1e-3 and rel(gp, gp0) <= 1e-3
+
+
+def test_backward_after_a_scene_change_runs_the_forward_again(have_gpu):
+    """The same grid set again after the recording: the records are not used,
+    the gradient is the same up to the order of the atomic sums."""
+    cfg, Po, pos, vel, grid, target = setup(subs=3, iters=2, scorr=False)
+    dev = torch.device("cuda", 0)
+    n = len(pos)
+    g = torch.zeros((n, 4), device=dev)
+    g[:, :3] = torch.randn((n, 3), generator=torch.Generator().manual_seed(3)).to(dev)
+    got = []
+    for change in (False, True):
+        b = make_batch(cfg, pos, vel, grid)
+        b.forward_record()
+        if change:
+            b.set_sdf_grid(0, grid[0], grid[1], grid[2])
+        out = torch.empty((2, n, 4), device=dev)
+        torch.cuda.synchronize()
+        gt = b.backward(g.data_ptr(), g.data_ptr(), out[0].data_ptr(), out[1].data_ptr())
+        got.append((out.cpu().numpy().astype(np.float64), gt))
+    assert rel(got[1][0], got[0][0]) <= 1e-5
+    assert rel(got[1][1], got[0][1]) <= 1e-4
