@@ -182,10 +182,13 @@ struct MeshDev {
     float4* bmin;         // 2nf-1 (xyz)
     float4* bmax;         // 2nf-1
     int* leaf_face;       // nf: face index of leaf i (Morton order)
+    // what a search reads of a node or face in one go, written by the refit
+    float4* wide;         // 4 per internal node: left lo (w: left child), left hi, right lo (w: right child), right hi
+    float4* tri;          // 3 per leaf: A (w: face), B, C
     uint32_t* flags;      // nf-1 refit arrival counters
     const int* frontier;  // kMeshFrontier subtree roots that together cover the tree (-1: unused)
 };
-constexpr int kMeshFrontier = 32;  // one per lane of the grid kernel's warp
+constexpr int kMeshFrontier = 32;  // one per lane of a warp's search
 void launch_mesh_refit(MeshDev M, cudaStream_t st, uint64_t* launches);
 // Vertex (angle-weighted) and edge pseudo-normals from M.face_n (run after
 // launch_mesh_refit).  voff/vfc: per-vertex (face, corner) lists in face
@@ -193,14 +196,14 @@ void launch_mesh_refit(MeshDev M, cudaStream_t st, uint64_t* launches);
 // shared by exactly two faces, else -1.
 void launch_mesh_pseudo_normals(MeshDev M, const int* voff, const int2* vfc, const int* partner, float3* vert_n,
                                 float3* edge_n, cudaStream_t st, uint64_t* launches);
-void launch_mesh_grid_d(MeshDev M, int dx, int dy, int dz, const double* origin, double cell, float* out, int sms,
+void launch_mesh_grid_d(MeshDev M, int dx, int dy, int dz, const double* origin, double cell, float* out,
                         cudaStream_t st);
 void launch_morton(int nf, const int3* faces, const float3* verts, float3 lo, float3 inv_ext, uint32_t* codes,
                    cudaStream_t st);
-void launch_mesh_closest(MeshDev M, const float* pts3, uint32_t n, int* face, float* point3, cudaStream_t st);
+void launch_mesh_closest(MeshDev M, const float* pts3, uint32_t n, int* face, float* point3, int sms, cudaStream_t st);
 // Per-vertex force accumulation in 2^-32 fixed point (deterministic).
 void launch_vertex_forces(MeshDev M, const float4* cand, const uint32_t* count, uint32_t cap, float band,
-                          int use_vel, long long* acc3, int* contacts, cudaStream_t st);
+                          int use_vel, long long* acc3, int* contacts, int sms, cudaStream_t st);
 void launch_forces_to_float(int nv, const long long* acc3, float* out3, cudaStream_t st);
 // LBVH topology from sorted Morton codes (device).
 void launch_lbvh_topology(int nf, const uint32_t* sorted_codes, int2* child, int* parent, cudaStream_t st);

@@ -58,6 +58,7 @@ struct MeshHost {
     uint32_t *d_codes = nullptr, *d_ka = nullptr, *d_ia = nullptr, *d_kb = nullptr, *d_ib = nullptr;
     uint32_t *d_hist = nullptr, *d_tot = nullptr;
     int* d_frontier = nullptr;
+    float4 *d_wide = nullptr, *d_tri = nullptr;
 };
 
 struct D3 {
@@ -90,7 +91,7 @@ void free_mesh_host(MeshHost* m)
     dfree(m->d_faces); dfree(m->d_verts); dfree(m->d_face_n); dfree(m->d_edge_n); dfree(m->d_vert_n);
     dfree(m->d_child); dfree(m->d_parent); dfree(m->d_bmin); dfree(m->d_bmax); dfree(m->d_leaf_face);
     dfree(m->d_flags); dfree(m->d_codes); dfree(m->d_ka); dfree(m->d_ia); dfree(m->d_kb); dfree(m->d_ib);
-    dfree(m->d_hist); dfree(m->d_tot); dfree(m->d_frontier);
+    dfree(m->d_hist); dfree(m->d_tot); dfree(m->d_frontier); dfree(m->d_wide); dfree(m->d_tri);
     dfree(m->d_voff); dfree(m->d_vfc); dfree(m->d_partner);
     delete m;
 }
@@ -263,7 +264,7 @@ static int mesh_build_geometry(pbf_handle* h, const double* verts, double cell)
     const float of[3] = {(float)o[0], (float)o[1], (float)o[2]};
     int rc;
     if ((rc = h->upload_grid(nullptr, dims, of, (float)cell))) return rc;
-    launch_mesh_grid_d(M, dims[0], dims[1], dims[2], h->origin_d, cell, h->grid, h->num_sms, st);
+    launch_mesh_grid_d(M, dims[0], dims[1], dims[2], h->origin_d, cell, h->grid, st);
     launch_sdf_slab_min(h->grid, dims[0], dims[1], dims[2], h->slab_min, st);
     h->launches += 2;
     CK(cudaStreamSynchronize(st));
@@ -301,6 +302,7 @@ extern "C" int pbf_set_sdf_mesh(pbf_handle* h, const double* verts, int32_t nv, 
         (rc = dalloc(m->d_ka, nf)) || (rc = dalloc(m->d_ia, nf)) || (rc = dalloc(m->d_kb, nf)) ||
         (rc = dalloc(m->d_ib, nf)) || (rc = dalloc(m->d_hist, (size_t)256 * sort_num_tiles(nf))) ||
         (rc = dalloc(m->d_tot, 256)) || (rc = dalloc(m->d_frontier, (size_t)kMeshFrontier)) ||
+        (rc = dalloc(m->d_wide, 4 * std::max<size_t>(1, nf - 1))) || (rc = dalloc(m->d_tri, 3 * (size_t)nf)) ||
         (rc = dalloc(m->d_voff, (size_t)nv + 1)) || (rc = dalloc(m->d_vfc, 3 * (size_t)nf)) ||
         (rc = dalloc(m->d_partner, 3 * (size_t)nf)) || (rc = dalloc(h->force_acc, 3 * (size_t)nv)) ||
         (rc = dalloc(h->force_contacts, 1)) || (rc = dalloc(h->force_out, 3 * (size_t)nv))) {
@@ -328,6 +330,8 @@ extern "C" int pbf_set_sdf_mesh(pbf_handle* h, const double* verts, int32_t nv, 
     M.leaf_face = m->d_leaf_face;
     M.flags = m->d_flags;
     M.frontier = m->d_frontier;
+    M.wide = m->d_wide;
+    M.tri = m->d_tri;
     h->mesh = M;
     if ((rc = mesh_build_geometry(h, verts, cell))) {
         h->mesh_free();
@@ -364,7 +368,7 @@ extern "C" int pbf_update_mesh_vertices(pbf_handle* h, const double* verts, int3
     cudaStream_t st = h->stream;
     CK(cudaMemcpyAsync(m->d_verts, m->verts_f.data(), sizeof(float3) * nv, cudaMemcpyHostToDevice, st));
     launch_mesh_refit(h->mesh, st, &h->launches);
-    launch_mesh_grid_d(h->mesh, h->dims[0], h->dims[1], h->dims[2], h->origin_d, h->cell_d, h->grid, h->num_sms, st);
+    launch_mesh_grid_d(h->mesh, h->dims[0], h->dims[1], h->dims[2], h->origin_d, h->cell_d, h->grid, st);
     launch_sdf_slab_min(h->grid, h->dims[0], h->dims[1], h->dims[2], h->slab_min, st);
     h->launches += 2;
     // host verts_f is re-read by the copy above before the next call returns
@@ -400,7 +404,7 @@ extern "C" int pbf_closest_triangle(pbf_handle* h, const float* pts3, uint32_t n
         return rc;
     }
     cudaMemcpyAsync(dp, pts3, 12 * (size_t)n, cudaMemcpyHostToDevice, h->stream);
-    launch_mesh_closest(h->mesh, dp, n, df, dq, h->stream);
+    launch_mesh_closest(h->mesh, dp, n, df, dq, h->num_sms, h->stream);
     ++h->launches;
     cudaMemcpyAsync(out_face, df, 4 * (size_t)n, cudaMemcpyDeviceToHost, h->stream);
     cudaMemcpyAsync(out_point3, dq, 12 * (size_t)n, cudaMemcpyDeviceToHost, h->stream);
@@ -422,7 +426,8 @@ extern "C" int pbf_vertex_forces(pbf_handle* h, float band, int use_vel, float* 
     CK(cudaMemsetAsync(o->force_acc, 0, sizeof(long long) * 3 * (size_t)nv, st));
     CK(cudaMemsetAsync(o->force_contacts, 0, sizeof(int), st));
     if (h->contacts_valid && h->n > 0) {
-        launch_vertex_forces(o->mesh, h->cand, h->scalars, h->n, band, use_vel, o->force_acc, o->force_contacts, st);
+        launch_vertex_forces(o->mesh, h->cand, h->scalars, h->n, band, use_vel, o->force_acc, o->force_contacts,
+                             h->num_sms, st);
         ++h->launches;
     }
     launch_forces_to_float(nv, o->force_acc, o->force_out, st);
