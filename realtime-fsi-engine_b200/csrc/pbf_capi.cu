@@ -297,6 +297,25 @@ int pbf_handle::ensure_capacity(uint32_t need_n)
     return PBF_OK;
 }
 
+int pbf_handle::query_take(size_t bytes, char** p)
+{
+    if (bytes > query_cap) {
+        query_cap = 0;
+        if (const int rc = dalloc(query_buf, bytes)) return rc;
+        query_cap = bytes;
+    }
+    *p = query_buf;
+    return PBF_OK;
+}
+
+// Called when the call's work on the scratch has ended.
+void pbf_handle::query_done()
+{
+    if (query_cap <= kQueryKeep) return;
+    dfree(query_buf);
+    query_cap = 0;
+}
+
 void pbf_handle::invalidate_graph()
 {
     if (graph_exec) cudaGraphExecDestroy(graph_exec);
@@ -317,7 +336,7 @@ pbf_handle::~pbf_handle()
     for (cudaEvent_t e : event_pool) cudaEventDestroy(e);
     dfree(pos); dfree(vel); dfree(pred); dfree(aos); dfree(keys);
     dfree(mcode); dfree(mka); dfree(mia); dfree(mkb); dfree(mib); dfree(ka); dfree(ia); dfree(kb); dfree(ib);
-    dfree(sx[0]); dfree(sx[1]); dfree(sv); dfree(sx0); dfree(somega); dfree(dpb); dfree(rho); dfree(lod); dfree(chits); dfree(chit_len);
+    dfree(sx[0]); dfree(sx[1]); dfree(sv); dfree(sx0); dfree(somega); dfree(dpb); dfree(rho); dfree(lod); dfree(chits); dfree(chit_len); dfree(query_buf);
     dfree(hist); dfree(totals); dfree(table); dfree(cand); dfree(ct_counts); dfree(scalars);
     dfree(lx[0]); dfree(lx[1]); dfree(lxb); dfree(lv); dfree(lx0); dfree(lom); dfree(lrho);
     dfree(lid); dfree(lkey); dfree(inv); dfree(dkey_id);
@@ -1137,19 +1156,18 @@ extern "C" int pbf_sample_sdf(pbf_handle* h, const float* pts3, uint32_t n, floa
     if (!h->sdf_dev().enabled) return set_error(PBF_ERR_STATE, "no SDF attached");
     if (n == 0) return PBF_OK;
     if (!pts3 || !out_d) return set_error(PBF_ERR_INVALID, "null argument");
-    float *dp = nullptr, *dd = nullptr, *dg = nullptr;
-    int rc = PBF_OK;
-    if ((rc = dalloc(dp, 3 * (size_t)n)) || (rc = dalloc(dd, n)) || (out_g && (rc = dalloc(dg, 3 * (size_t)n)))) {
-        dfree(dp); dfree(dd); dfree(dg);
-        return rc;
-    }
+    std::lock_guard<std::mutex> lock(h->query_lock);
+    // points, distances, gradients
+    char* q = nullptr;
+    if (const int rc = h->query_take((out_g ? 28u : 16u) * (size_t)n, &q)) return rc;
+    float *dp = reinterpret_cast<float*>(q), *dd = dp + 3 * (size_t)n, *dg = out_g ? dd + n : nullptr;
     cudaMemcpyAsync(dp, pts3, 12 * (size_t)n, cudaMemcpyHostToDevice, h->stream);
     launch_sdf_sample(h->sdf_dev(), dp, n, dd, dg, h->stream);
     ++h->launches;
     cudaMemcpyAsync(out_d, dd, 4 * (size_t)n, cudaMemcpyDeviceToHost, h->stream);
     if (out_g) cudaMemcpyAsync(out_g, dg, 12 * (size_t)n, cudaMemcpyDeviceToHost, h->stream);
     const cudaError_t e = cudaStreamSynchronize(h->stream);
-    dfree(dp); dfree(dd); dfree(dg);
+    h->query_done();
     if (e != cudaSuccess) return set_error(PBF_ERR_CUDA, "sample_sdf: %s", cudaGetErrorString(e));
     return PBF_OK;
 }

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <mutex>
 #include <vector>
 
 #include "../../include/pbf_b200.h"
@@ -138,6 +139,17 @@ struct pbf_handle {
     int* force_contacts = nullptr;
     float* force_out = nullptr;
     void mesh_free();
+
+    // device scratch of the point queries (pbf_closest_triangle, pbf_sample_sdf):
+    // kept from call to call up to kQueryKeep bytes, as an allocation and its
+    // release take longer than the search (20,000 closest-triangle queries: 880
+    // us a call with three of each, 256 us with none)
+    static constexpr size_t kQueryKeep = 64u << 20;
+    char* query_buf = nullptr;
+    size_t query_cap = 0;
+    std::mutex query_lock;  // held by a query: several threads may ask one handle
+    int query_take(size_t bytes, char** p);
+    void query_done();
 
     // execution
     uint64_t launches = 0;

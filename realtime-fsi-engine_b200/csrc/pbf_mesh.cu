@@ -396,20 +396,19 @@ extern "C" int pbf_closest_triangle(pbf_handle* h, const float* pts3, uint32_t n
     if (!h->mesh_attached) return set_error(PBF_ERR_STATE, "no mesh attached");
     if (n == 0) return PBF_OK;
     if (!pts3 || !out_face || !out_point3) return set_error(PBF_ERR_INVALID, "null argument");
-    float *dp = nullptr, *dq = nullptr;
-    int* df = nullptr;
-    int rc;
-    if ((rc = dalloc(dp, 3 * (size_t)n)) || (rc = dalloc(dq, 3 * (size_t)n)) || (rc = dalloc(df, n))) {
-        dfree(dp); dfree(dq); dfree(df);
-        return rc;
-    }
+    std::lock_guard<std::mutex> lock(h->query_lock);
+    // points, nearest points, faces
+    char* q = nullptr;
+    if (const int rc = h->query_take(28 * (size_t)n, &q)) return rc;
+    float *dp = reinterpret_cast<float*>(q), *dq = dp + 3 * (size_t)n;
+    int* df = reinterpret_cast<int*>(dq + 3 * (size_t)n);
     cudaMemcpyAsync(dp, pts3, 12 * (size_t)n, cudaMemcpyHostToDevice, h->stream);
     launch_mesh_closest(h->mesh, dp, n, df, dq, h->num_sms, h->stream);
     ++h->launches;
     cudaMemcpyAsync(out_face, df, 4 * (size_t)n, cudaMemcpyDeviceToHost, h->stream);
     cudaMemcpyAsync(out_point3, dq, 12 * (size_t)n, cudaMemcpyDeviceToHost, h->stream);
     const cudaError_t e = cudaStreamSynchronize(h->stream);
-    dfree(dp); dfree(dq); dfree(df);
+    h->query_done();
     if (e != cudaSuccess) return set_error(PBF_ERR_CUDA, "closest_triangle: %s", cudaGetErrorString(e));
     return PBF_OK;
 }

@@ -99,3 +99,18 @@ def test_points_that_are_none(have_gpu):
     bad = np.array([[np.nan, 0, 0], [np.inf, 0, 0], [0, -np.inf, 0], [1e30, 0, 0]], np.float32)
     face, point = sdf.closest_many(bad)
     assert (face == -1).all() and (point == 0).all()
+
+
+def test_queries_of_several_threads(have_gpu):
+    """One SDF asked by four threads at once, with different numbers of points."""
+    from concurrent.futures import ThreadPoolExecutor
+    v, f = scenes.icosphere(3, 0.2, (0.8, 0.3, 0.5))
+    sdf = P.SDFBoundary()
+    sdf.buildFromMesh(v, f, 0.02)
+    pts = np.random.default_rng(5).uniform(0.2, 1.2, (6000, 3)).astype(np.float32)
+    face, point = sdf.closest_many(pts)
+    d = sdf.sample(pts)
+    with ThreadPoolExecutor(4) as ex:
+        for n, (a, b, c) in ex.map(lambda n: (n, (*sdf.closest_many(pts[:n]), sdf.sample(pts[:n]))),
+                                   [6000, 17, 3001, 1, 5999, 250] * 4):
+            assert np.array_equal(a, face[:n]) and np.array_equal(b, point[:n]) and np.array_equal(c, d[:n])
