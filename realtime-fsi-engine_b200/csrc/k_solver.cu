@@ -45,24 +45,11 @@ __global__ void __launch_bounds__(256) k_reorder(DevParams P, const uint32_t* __
         const uint32_t id = __ldg(ids + s);
         const float4 p = __ldg(pos + id);
         const float4 v = __ldg(vel + id);
-        float3 vp, xs;
-        predict_particle(P, p, v, vp, xs);
-        sx[s] = make_float4(xs.x, xs.y, xs.z, 0.0f);
-        sv[s] = make_float4(vp.x, vp.y, vp.z, v.w);
-        sx0[s] = p;
+        const float3 xs = reorder_particle(P, p, v, s, sx, sv, sx0, lod);
         if (mcode) {
             const uint32_t cx = (uint32_t)cell_coord(xs.x, P.h), cy = (uint32_t)cell_coord(xs.y, P.h),
                            cz = (uint32_t)cell_coord(xs.z, P.h);
             mcode[s] = (spread8(cz) << 2) | (spread8(cy) << 1) | spread8(cx);
-        }
-        if (P.apbf) {
-            const float dx = P.cam[0] - xs.x, dy = P.cam[1] - xs.y, dz = P.cam[2] - xs.z;
-            const float dist = sqrtf(dx * dx + dy * dy + dz * dz);
-            const float t = fminf(fmaxf(dist / P.lod_max_dist, 0.0f), 1.0f);
-            const float m = (float)P.max_lod * (1.0f - t) + (float)P.min_lod * t;
-            uint32_t l = (uint32_t)rintf(m);
-            l = min(max(l, P.min_lod), P.max_lod);
-            lod[s] = l;
         }
     }
 }

@@ -136,13 +136,19 @@ int pbf_batch::record_substep(uint32_t sub, Record& r, const float4* src_pos, co
     const int sms = num_sms, G = ad_lanes();
     const uint32_t I = cfg.solver_iterations;
     const bool last = sub + 1 == cfg.substep_iterations;
-    launch_b_predict(P, scenes_dev, scene_of, src_pos, src_vel, keys, sms, stream);
-    launch_radix_sort_into(n, key_bits, keys, ka, r.ids, kb, ib, hist, totals, stream);
-    ACK(cudaMemsetAsync(r.table, 0xFF, sizeof(int2) * (size_t)table_size, stream));
-    launch_build_table(n, ka, r.table, sms, stream);
-    launch_b_reorder(P, scenes_dev, scene_of, r.ids, src_pos, src_vel, I ? sx[0] : r.xf, r.sv, sx0, lod, nullptr, mbits,
-                     sms, stream);
-    launches += 3 + 3 * ((key_bits + 7) / 8);
+    float4* x = I ? sx[0] : r.xf;
+    if (bcnt) {
+        launch_bucket_sort(P, scenes_dev, scene_of, src_pos, src_vel, keys, mka, bcnt, table_size, r.table, mia, r.ids,
+                           nullptr, x, r.sv, sx0, lod, sms, stream, &launches);
+    } else {
+        launch_b_predict(P, scenes_dev, scene_of, src_pos, src_vel, keys, sms, stream);
+        launch_radix_sort_into(n, key_bits, keys, ka, r.ids, kb, ib, hist, totals, stream);
+        ACK(cudaMemsetAsync(r.table, 0xFF, sizeof(int2) * (size_t)table_size, stream));
+        launch_build_table(n, ka, r.table, sms, stream);
+        launch_b_reorder(P, scenes_dev, scene_of, r.ids, src_pos, src_vel, x, r.sv, sx0, lod, nullptr, mbits,
+                         sms, stream);
+        launches += 3 + 3 * ((key_bits + 7) / 8);
+    }
     for (uint32_t it = 1; it <= I; ++it) {
         const size_t at = (size_t)(it - 1) * ad_stride;
         float4* xl = r.xl + at;

@@ -76,7 +76,7 @@ pbf_batch::~pbf_batch()
     bfree(pos); bfree(vel); bfree(pred); bfree(aos); bfree(scene_of); bfree(scenes_dev);
     bfree(keys); bfree(ka); bfree(ia); bfree(kb); bfree(ib); bfree(hist); bfree(totals); bfree(table);
     bfree(mcode); bfree(mka); bfree(mia); bfree(mkb); bfree(mib);
-    bfree(sx[0]); bfree(sx[1]); bfree(sv); bfree(sx0); bfree(somega); bfree(dpb); bfree(rho); bfree(lod); bfree(chits); bfree(chit_len);
+    bfree(sx[0]); bfree(sx[1]); bfree(sv); bfree(sx0); bfree(somega); bfree(dpb); bfree(rho); bfree(lod); bfree(chits); bfree(chit_len); bfree(bcnt);
     bfree(save_pos); bfree(save_vel);
     dense_free();
     ad_free();
@@ -250,19 +250,26 @@ int pbf_batch::substep_body(const float4* src_pos, const float4* src_vel, float4
     L.sms = sms;
     const int G = coop_lanes(n);
     const uint32_t max_iter = derived.enable_apbf ? derived.max_lod : cfg.solver_iterations;
-    launch_b_predict(P, scenes_dev, scene_of, src_pos, src_vel, keys, sms, stream);
-    launch_radix_sort(n, key_bits, keys, ka, ia, kb, ib, hist, totals, &skeys, &ids, stream, &launches);
-    BCK(cudaMemsetAsync(table, 0xFF, sizeof(int2) * (size_t)table_size, stream));
-    launch_build_table(n, skeys, table, sms, stream);
-    const bool sorted = morton && !G;  // a group of lanes per particle needs no processing order
-    launch_b_reorder(P, scenes_dev, scene_of, ids, src_pos, src_vel, sx[0], sv, sx0, lod, sorted ? mcode : nullptr,
-                     mbits, sms, stream);
-    launches += 3;
     order = nullptr;
-    if (sorted) {
-        uint32_t* msorted = nullptr;
-        launch_radix_sort(n, order_bits, mcode, mka, mia, mkb, mib, hist, totals, &msorted, &order, stream,
-                          &launches);
+    if (bcnt) {
+        launch_bucket_sort(P, scenes_dev, scene_of, src_pos, src_vel, keys, mka, bcnt, table_size, table, mia, ia, ka,
+                           sx[0], sv, sx0, lod, sms, stream, &launches);
+        skeys = ka;
+        ids = ia;
+    } else {
+        launch_b_predict(P, scenes_dev, scene_of, src_pos, src_vel, keys, sms, stream);
+        launch_radix_sort(n, key_bits, keys, ka, ia, kb, ib, hist, totals, &skeys, &ids, stream, &launches);
+        BCK(cudaMemsetAsync(table, 0xFF, sizeof(int2) * (size_t)table_size, stream));
+        launch_build_table(n, skeys, table, sms, stream);
+        const bool sorted = morton && !G;  // a group of lanes per particle needs no processing order
+        launch_b_reorder(P, scenes_dev, scene_of, ids, src_pos, src_vel, sx[0], sv, sx0, lod, sorted ? mcode : nullptr,
+                         mbits, sms, stream);
+        launches += 3;
+        if (sorted) {
+            uint32_t* msorted = nullptr;
+            launch_radix_sort(n, order_bits, mcode, mka, mia, mkb, mib, hist, totals, &msorted, &order, stream,
+                              &launches);
+        }
     }
     for (uint32_t it = 1; it <= max_iter; ++it) {
         if (G) {
@@ -581,7 +588,8 @@ extern "C" int pbf_batch_create(const pbf_fluid_config* cfg, const pbf_scene_des
         (rc = balloc(b->mkb, c)) || (rc = balloc(b->mib, c)) || (rc = balloc(b->sx[0], c + kCoopPad)) ||
         (rc = balloc(b->sx[1], c + kCoopPad)) || (rc = balloc(b->sv, c)) || (rc = balloc(b->sx0, c + kCoopPad)) ||
         (rc = balloc(b->somega, c)) || (rc = balloc(b->dpb, c)) || (rc = balloc(b->rho, c)) || (rc = balloc(b->lod, c)) ||
-        (coop_lanes((uint32_t)c) && ((rc = balloc(b->chits, c * kCoopList)) || (rc = balloc(b->chit_len, c))))) {
+        (coop_lanes((uint32_t)c) && ((rc = balloc(b->chits, c * kCoopList)) || (rc = balloc(b->chit_len, c)))) ||
+        (bucket_sort_fits((uint32_t)c, b->table_size) && (rc = balloc(b->bcnt, bucket_scratch(b->table_size))))) {
         delete b;
         return rc;
     }
@@ -590,6 +598,7 @@ extern "C" int pbf_batch_create(const pbf_fluid_config* cfg, const pbf_scene_des
     cudaMemsetAsync(b->pred, 0, sizeof(float4) * c, b->stream);
     cudaMemsetAsync(b->somega, 0, sizeof(float4) * c, b->stream);
     cudaMemsetAsync(b->dpb, 0, sizeof(float4) * c, b->stream);
+    if (b->bcnt) cudaMemsetAsync(b->bcnt, 0, sizeof(uint32_t) * bucket_scratch(b->table_size), b->stream);
     if (total) cudaMemcpyAsync(b->scene_of, sid.data(), sizeof(uint16_t) * total, cudaMemcpyHostToDevice, b->stream);
     if ((rc = b->upload_scenes())) {
         delete b;

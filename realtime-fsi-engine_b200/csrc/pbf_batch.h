@@ -142,6 +142,7 @@ struct pbf_batch {
     float* rho = nullptr;
     uint32_t* lod = nullptr;
     uint32_t *chits = nullptr, *chit_len = nullptr;  // small batches: hits of a lambda pass (k_coop.cu)
+    uint32_t* bcnt = nullptr;                        // and scratch of their sort (k_bucket.cu)
     // autotuner state snapshot
     float4 *save_pos = nullptr, *save_vel = nullptr;
 

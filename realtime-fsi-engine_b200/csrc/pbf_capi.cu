@@ -288,6 +288,13 @@ int pbf_handle::ensure_capacity(uint32_t need_n)
         if ((rc = dalloc(chits, (size_t)need_n * kCoopList)) || (rc = dalloc(chit_len, need_n))) return rc;
         cap_chits = need_n;
     }
+    if (bucket_sort_fits(need_n, derived.hash_size) && derived.hash_size != cap_bcnt) {
+        cap_bcnt = 0;
+        const size_t words = bucket_scratch(derived.hash_size);
+        if ((rc = dalloc(bcnt, words))) return rc;
+        CK(cudaMemsetAsync(bcnt, 0, sizeof(uint32_t) * words, stream));
+        cap_bcnt = derived.hash_size;
+    }
     if (!totals && (rc = dalloc(totals, 256))) return rc;
     if (!scalars && (rc = dalloc(scalars, 8))) return rc;
     if (derived.hash_size != cap_h) {
@@ -312,7 +319,7 @@ int pbf_handle::query_take(size_t bytes, char** p)
 void pbf_handle::query_done()
 {
     if (query_cap <= kQueryKeep) return;
-    dfree(query_buf);
+    dfree(query_buf); dfree(bcnt);
     query_cap = 0;
 }
 
@@ -790,14 +797,33 @@ int pbf_handle::stage(int st, uint32_t iter)
     return PBF_OK;
 }
 
+// Predict, sort, table and reorder of a substep.  While passes are profiled
+// each is run and timed by itself.
+int pbf_handle::sort_stages()
+{
+    if (effective_mode() == 4 && bucket_sort_fits(n, derived.hash_size) && !profiling) {
+        dkey_valid = false;
+        launch_bucket_sort(dev_params(), nullptr, nullptr, pos, vel, keys, mka, bcnt, derived.hash_size, table, mia, ia, ka,
+                           sx[0], sv, sx0, lod, num_sms, stream, &launches);
+        skeys = ka;
+        ids = ia;
+        order = nullptr;
+        label_space = false;
+        chit_iter = 0;
+        last_x = 0;
+        return PBF_OK;
+    }
+    for (const int st : {PBF_STAGE_PREDICT, PBF_STAGE_SORT, PBF_STAGE_TABLE, PBF_STAGE_REORDER})
+        if (const int rc = stage(st, 0)) return rc;
+    return PBF_OK;
+}
+
 int pbf_handle::step_body()
 {
     int rc;
     const uint32_t max_iter = derived.enable_apbf ? derived.max_lod : cfg.solver_iterations;  // :455
     for (uint32_t s = 0; s < cfg.substep_iterations; ++s) {
-        if ((rc = stage(PBF_STAGE_PREDICT, 0)) || (rc = stage(PBF_STAGE_SORT, 0)) || (rc = stage(PBF_STAGE_TABLE, 0)) ||
-            (rc = stage(PBF_STAGE_REORDER, 0)))
-            return rc;
+        if ((rc = sort_stages())) return rc;
         for (uint32_t it = 1; it <= max_iter; ++it)
             if ((rc = stage(PBF_STAGE_LAMBDA, it)) || (rc = stage(PBF_STAGE_DELTAP, it))) return rc;
         if ((rc = stage(PBF_STAGE_INTEGRATE, 0))) return rc;

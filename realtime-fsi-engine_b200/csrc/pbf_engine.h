@@ -40,6 +40,8 @@ struct pbf_handle {
     uint32_t* hist = nullptr;
     uint32_t* totals = nullptr;
     int2* table = nullptr;
+    uint32_t* bcnt = nullptr;  // scratch of the small scenes' sort (k_bucket.cu), for cap_bcnt buckets
+    uint32_t cap_bcnt = 0;
     // spatial processing order of the neighbour passes (Morton order of the
     // predict-time cells); `order` points into one of the m* ping-pong pairs.
     // PBF_OPT_SPATIAL_ORDER: 4 hashed buckets in Morton thread order with
@@ -178,6 +180,7 @@ struct pbf_handle {
     void invalidate_graph();
     int upload_grid(const float* dist_host, const int32_t d[3], const float o[3], float c);
     int stage(int st, uint32_t iter);
+    int sort_stages();
     int step_body();
     int step();
     cudaEvent_t take_event();

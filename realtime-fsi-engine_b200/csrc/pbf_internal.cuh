@@ -106,6 +106,28 @@ __device__ __forceinline__ void predict_particle(const DevParams& P, float4 p, f
     xs = make_float3(__fmaf_rn(vx, P.dt, p.x), __fmaf_rn(vy, P.dt, p.y), __fmaf_rn(vz, P.dt, p.z));
 }
 
+// Particle (p, v) into sorted slot s: x* (lambda = 0, CS_PredictAndHash.glsl:121),
+// v' and x, plus the APBF level of CS_ComputeLOD.glsl:66-79; returns x*.
+__device__ __forceinline__ float3 reorder_particle(const DevParams& P, float4 p, float4 v, uint32_t s, float4* sx,
+                                                   float4* sv, float4* sx0, uint32_t* lod)
+{
+    float3 vp, xs;
+    predict_particle(P, p, v, vp, xs);
+    sx[s] = make_float4(xs.x, xs.y, xs.z, 0.0f);
+    sv[s] = make_float4(vp.x, vp.y, vp.z, v.w);
+    sx0[s] = p;
+    if (P.apbf) {
+        const float dx = P.cam[0] - xs.x, dy = P.cam[1] - xs.y, dz = P.cam[2] - xs.z;
+        const float dist = sqrtf(dx * dx + dy * dy + dz * dz);
+        const float t = fminf(fmaxf(dist / P.lod_max_dist, 0.0f), 1.0f);
+        const float m = (float)P.max_lod * (1.0f - t) + (float)P.min_lod * t;
+        uint32_t l = (uint32_t)rintf(m);
+        l = min(max(l, P.min_lod), P.max_lod);
+        lod[s] = l;
+    }
+    return xs;
+}
+
 // poly6 (CS_ComputeLambdas.glsl:74-81), valid for r2 <= h2.
 __device__ __forceinline__ float poly6_in(const DevParams& P, float r2)
 {

@@ -63,6 +63,18 @@ void launch_c_vorticity(int G, const DevParams& P, const SceneDev* scenes, const
                         const float4* spos, const float4* somega, const uint32_t* ids, float4* vel, const int2* table,
                         const uint32_t* order, cudaStream_t st);
 
+// ---- k_bucket.cu: predict, sort, table and reorder of a small scene in four launches ----
+constexpr uint32_t kBucketSortMax = 1u << 21;  // buckets
+bool bucket_sort_fits(uint32_t n, uint32_t buckets);
+size_t bucket_scratch(uint32_t buckets);  // words of scratch
+// Leaves keys, table, ids, skeys (may be null) and the sorted arrays as
+// predict, radix sort, table and reorder do.  arrival[n], ids_in[n]: scratch;
+// scratch[bucket_scratch(buckets)]: zero before the first call.
+void launch_bucket_sort(const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const float4* pos,
+                        const float4* vel, uint32_t* keys, uint32_t* arrival, uint32_t* scratch, uint32_t buckets,
+                        int2* table, uint32_t* ids_in, uint32_t* ids, uint32_t* skeys, float4* sx, float4* sv, float4* sx0,
+                        uint32_t* lod, int sms, cudaStream_t st, uint64_t* launches);
+
 // ---- k_dense.cu: x-runs of a dense cell window over relabelled data ----------
 constexpr int kDenseListWords = 16;
 // Label-space position/velocity arrays hold this many entries past the last

@@ -80,3 +80,35 @@ def test_coincident_particles(have_gpu):
     pos[1::2] = pos[::2]
     vel[1::2] = vel[::2]
     assert same(stepped(cfg, pos, vel, 4), stepped(cfg, pos, vel, 8))
+
+
+@pytest.mark.parametrize("n,hash_size", [(1, 1), (3, 2), (300, 1), (300, 4), (5000, 4096), (5000, 8192), (5000, 1 << 21),
+                                         (5000, 1 << 22), (70000, 1 << 17)])
+def test_sort_of_a_step_equals_the_stages(have_gpu, n, hash_size):
+    """A step's own sort (k_bucket.cu) leaves the keys, permutation and table
+    that the stages one by one leave, for tables of one bucket to more than it
+    takes, and the same state."""
+    cfg, pos, vel = moving_block(n, 0.02, 0.04, n, hash_size)
+    cfg.substep_iterations = 1
+    got = []
+    for stages in (False, True):
+        fl = P.PBFluids(cfg)
+        fl.set_option(1, 4)
+        fl.setParticles(P.make_particles(pos, vel))
+        for _ in range(2):
+            if stages:
+                for st in (P.STAGE_PREDICT, P.STAGE_SORT, P.STAGE_TABLE, P.STAGE_REORDER):
+                    fl.run_stage(st)
+                for it in range(1, cfg.solver_iterations + 1):
+                    fl.run_stage(P.STAGE_LAMBDA, it)
+                    fl.run_stage(P.STAGE_DELTAP, it)
+                fl.run_stage(P.STAGE_INTEGRATE)
+                fl.run_stage(P.STAGE_VORTICITY)
+            else:
+                fl.step()
+        fl.sync()
+        got.append([fl.read_buffer(P.BUF_KEYS, np.uint32, n), fl.read_buffer(P.BUF_SORTED_KEYS, np.uint32, n),
+                    fl.read_buffer(P.BUF_SORTED_IDS, np.uint32, n), fl.read_buffer(P.BUF_TABLE, np.int32, (hash_size, 2)),
+                    fl.read_buffer(P.BUF_XSTAR, np.float32, (n, 4)), fl.readbackParticles()])
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
