@@ -54,9 +54,8 @@ static void afree(T*& p)
 
 void pbf_batch::ad_free()
 {
-    afree(cp_pos); afree(cp_vel); afree(ad_slab); afree(ad_sx0); afree(ad_om);
-    afree(gxa); afree(gxb); afree(gv); afree(x0b); afree(pb); afree(vb); afree(pbs); afree(omb);
-    afree(tpos); afree(tvel); afree(tgrad);
+    afree(ad_slab);
+    ad_arrays.release();
     records.clear();
     ad_subs = ad_iters = 0;
     recorded = false;
@@ -97,14 +96,10 @@ int pbf_batch::ad_alloc()
     ad_free();
     const size_t c = std::max<uint32_t>(n, 1u);
     int rc;
-    if ((rc = aalloc(cp_pos, c * S)) || (rc = aalloc(cp_vel, c * S)) || (rc = aalloc(ad_sx0, c + kCoopPad)) ||
-        (rc = aalloc(ad_om, c)) || (rc = aalloc(gxa, c)) || (rc = aalloc(gxb, c)) ||
-        (rc = aalloc(gv, c)) || (rc = aalloc(x0b, c)) || (rc = aalloc(pb, c)) || (rc = aalloc(vb, c)) ||
-        (rc = aalloc(pbs, c)) || (rc = aalloc(omb, c)) || (rc = aalloc(tpos, c)) || (rc = aalloc(tvel, c)) ||
-        (rc = aalloc(tgrad, 4 * scenes.size()))) {
-        ad_free();
-        return rc;
-    }
+    ad_arrays.add(cp_pos, c * S).add(cp_vel, c * S).add(ad_sx0, c + kCoopPad).add(ad_om, c).add(gxa, c).add(gxb, c)
+        .add(gv, c).add(x0b, c).add(pb, c).add(vb, c).add(pbs, c).add(omb, c).add(tpos, c).add(tvel, c)
+        .add(tgrad, 4 * scenes.size());
+    if ((rc = ad_arrays.alloc())) return rc;
     // a record per substep when they take at most a quarter of the free memory
     // (32,768 particles x 16 substeps x 4 iterations: 0.9 GB)
     ad_stride = (c + kCoopPad + 63) / 64 * 64;

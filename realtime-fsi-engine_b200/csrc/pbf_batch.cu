@@ -73,10 +73,7 @@ pbf_batch::~pbf_batch()
         bfree(s.grid);
         bfree(s.slab_min);
     }
-    bfree(pos); bfree(vel); bfree(pred); bfree(aos); bfree(scene_of); bfree(scenes_dev);
-    bfree(keys); bfree(ka); bfree(ia); bfree(kb); bfree(ib); bfree(hist); bfree(totals); bfree(table);
-    bfree(mcode); bfree(mka); bfree(mia); bfree(mkb); bfree(mib);
-    bfree(sx[0]); bfree(sx[1]); bfree(sv); bfree(sx0); bfree(somega); bfree(dpb); bfree(rho); bfree(lod); bfree(chits); bfree(chit_len); bfree(bcnt);
+    particle_slab.release();
     bfree(save_pos); bfree(save_vel);
     dense_free();
     ad_free();
@@ -318,10 +315,8 @@ int pbf_batch::effective_mode() const
 
 void pbf_batch::dense_free()
 {
-    bfree(lx[0]); bfree(lx[1]); bfree(lxb); bfree(lv); bfree(lx0); bfree(lom); bfree(lrho);
-    bfree(lid); bfree(lkey); bfree(inv); bfree(dtable); bfree(druns); bfree(dclean); bfree(ddcol);
-    bfree(ddirty); bfree(dhcnt); bfree(dvmark); bfree(dslot_scene); bfree(dflag); bfree(dslot); bfree(dord); bfree(dcnt);
-    bfree(dbsum); bfree(dhm);
+    label_slab.release();
+    window_slab.release();
     dense_ready = false;
 }
 
@@ -337,17 +332,14 @@ int pbf_batch::dense_setup()
     int rc;
     const size_t c = std::max<uint32_t>(n, 1u), cp = c + kLabelPad, T = (size_t)dense_total;
     if (!lx[0]) {
-        if ((rc = balloc(lx[0], cp)) || (rc = balloc(lx[1], cp)) || (rc = balloc(lxb, c)) || (rc = balloc(lv, cp)) ||
-            (rc = balloc(lx0, cp)) || (rc = balloc(lom, cp)) || (rc = balloc(lrho, c)) || (rc = balloc(lid, c)) ||
-            (rc = balloc(lkey, c)) || (rc = balloc(inv, c)) || (rc = balloc(dslot, c)) || (rc = balloc(dord, c)) ||
-            (rc = balloc(dhm, c * kDenseListWords)) || (rc = balloc(dhcnt, c)) || (rc = balloc(dflag, 4))) {
-            dense_free();
-            return rc;
-        }
+        label_slab.add(lx[0], cp).add(lx[1], cp).add(lxb, c).add(lv, cp).add(lx0, cp).add(lom, cp).add(lrho, c).add(lid, c)
+            .add(lkey, c).add(inv, c).add(dslot, c).add(dord, c).add(dhm, c * kDenseListWords).add(dhcnt, c).add(dflag, 4);
+        if ((rc = label_slab.alloc())) return rc;
     }
-    if ((rc = balloc(dtable, T)) || (rc = balloc(druns, T)) || (rc = balloc(dclean, T)) || (rc = balloc(ddcol, T)) ||
-        (rc = balloc(ddirty, T)) || (rc = balloc(dvmark, T)) || (rc = balloc(dslot_scene, T)) || (rc = balloc(dcnt, T + 1)) ||
-        (rc = balloc(dbsum, order_scan_blocks((uint32_t)T)))) {
+    window_slab.release();
+    window_slab.add(dtable, T).add(druns, T).add(dclean, T).add(ddcol, T).add(ddirty, T).add(dvmark, T).add(dslot_scene, T)
+        .add(dcnt, T + 1).add(dbsum, order_scan_blocks((uint32_t)T));
+    if ((rc = window_slab.alloc())) {
         dense_free();
         return rc;
     }
@@ -579,17 +571,15 @@ extern "C" int pbf_batch_create(const pbf_fluid_config* cfg, const pbf_scene_des
     b->cfg.particle_count = b->n;
     pbf_derive_params(&b->cfg, 0.0f, &b->derived);
     const size_t c = std::max<uint32_t>(b->n, 1u);
-    if ((rc = balloc(b->pos, c)) || (rc = balloc(b->vel, c)) || (rc = balloc(b->pred, c)) ||
-        (rc = balloc(b->aos, 3 * c)) || (rc = balloc(b->scene_of, c)) || (rc = balloc(b->scenes_dev, num_scenes)) ||
-        (rc = balloc(b->keys, c)) || (rc = balloc(b->ka, c)) || (rc = balloc(b->ia, c)) || (rc = balloc(b->kb, c)) ||
-        (rc = balloc(b->ib, c)) || (rc = balloc(b->hist, (size_t)256 * sort_num_tiles((uint32_t)c))) ||
-        (rc = balloc(b->totals, 256)) || (rc = balloc(b->table, std::max<uint32_t>(b->table_size, 1u))) ||
-        (rc = balloc(b->mcode, c)) || (rc = balloc(b->mka, c)) || (rc = balloc(b->mia, c)) ||
-        (rc = balloc(b->mkb, c)) || (rc = balloc(b->mib, c)) || (rc = balloc(b->sx[0], c + kCoopPad)) ||
-        (rc = balloc(b->sx[1], c + kCoopPad)) || (rc = balloc(b->sv, c)) || (rc = balloc(b->sx0, c + kCoopPad)) ||
-        (rc = balloc(b->somega, c)) || (rc = balloc(b->dpb, c)) || (rc = balloc(b->rho, c)) || (rc = balloc(b->lod, c)) ||
-        (coop_lanes((uint32_t)c) && ((rc = balloc(b->chits, c * kCoopList)) || (rc = balloc(b->chit_len, c)))) ||
-        (bucket_sort_fits((uint32_t)c, b->table_size) && (rc = balloc(b->bcnt, bucket_scratch(b->table_size))))) {
+    b->particle_slab.add(b->pos, c).add(b->vel, c).add(b->pred, c).add(b->aos, 3 * c).add(b->scene_of, c)
+        .add(b->scenes_dev, num_scenes).add(b->keys, c).add(b->ka, c).add(b->ia, c).add(b->kb, c).add(b->ib, c)
+        .add(b->hist, (size_t)256 * sort_num_tiles((uint32_t)c)).add(b->totals, 256)
+        .add(b->table, std::max<uint32_t>(b->table_size, 1u)).add(b->mcode, c).add(b->mka, c).add(b->mia, c).add(b->mkb, c)
+        .add(b->mib, c).add(b->sx[0], c + kCoopPad).add(b->sx[1], c + kCoopPad).add(b->sv, c).add(b->sx0, c + kCoopPad)
+        .add(b->somega, c).add(b->dpb, c).add(b->rho, c).add(b->lod, c);
+    if (coop_lanes((uint32_t)c)) b->particle_slab.add(b->chits, c * kCoopList).add(b->chit_len, c);
+    if (bucket_sort_fits((uint32_t)c, b->table_size)) b->particle_slab.add(b->bcnt, bucket_scratch(b->table_size));
+    if ((rc = b->particle_slab.alloc())) {
         delete b;
         return rc;
     }

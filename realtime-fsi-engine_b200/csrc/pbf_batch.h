@@ -7,6 +7,7 @@
 
 #include "../../include/pbf_b200.h"
 #include "pbf_kernels.h"
+#include "pbf_slab.h"
 
 namespace pbf {
 
@@ -122,6 +123,10 @@ struct pbf_batch {
     uint32_t key_bits = 1;     // bits of the offset hash keys
     uint32_t mbits = 8;        // Morton bits per axis
     uint32_t order_bits = 24;  // bits of the scene-prefixed Morton keys
+
+    // owners of the arrays below: per particle; mode 8's per particle and per
+    // window slot; the adjoint's
+    pbf::Slab particle_slab, label_slab, window_slab, ad_arrays;
 
     // particle order
     float4 *pos = nullptr, *vel = nullptr, *pred = nullptr, *aos = nullptr;

@@ -273,19 +273,20 @@ int pbf_handle::ensure_capacity(uint32_t need_n)
     int rc = PBF_OK;
     if (need_n > cap_n) {
         const size_t c = need_n;
-        if ((rc = dalloc(pos, c)) || (rc = dalloc(vel, c)) || (rc = dalloc(pred, c)) || (rc = dalloc(aos, 3 * c)) ||
-            (rc = dalloc(keys, c)) || (rc = dalloc(ka, c)) || (rc = dalloc(mcode, c)) || (rc = dalloc(mka, c)) ||
-            (rc = dalloc(mia, c)) || (rc = dalloc(mkb, c)) || (rc = dalloc(mib, c)) || (rc = dalloc(ia, c)) || (rc = dalloc(kb, c)) || (rc = dalloc(ib, c)) || (rc = dalloc(sx[0], c + kCoopPad)) ||
-            (rc = dalloc(sx[1], c + kCoopPad)) || (rc = dalloc(sv, c)) || (rc = dalloc(sx0, c + kCoopPad)) || (rc = dalloc(somega, c)) || (rc = dalloc(dpb, c)) ||
-            (rc = dalloc(rho, c)) || (rc = dalloc(lod, c)) || (rc = dalloc(cand, 2 * c)) ||
-            (rc = dalloc(ct_counts, (size_t)contact_num_blocks(need_n) + 1)))
-            return rc;
-        if ((rc = dalloc(hist, (size_t)256 * sort_num_tiles(need_n)))) return rc;
+        cap_n = 0;
+        particle_slab.release();
+        particle_slab.add(pos, c).add(vel, c).add(pred, c).add(aos, 3 * c).add(keys, c).add(ka, c).add(ia, c).add(kb, c)
+            .add(ib, c).add(mcode, c).add(mka, c).add(mia, c).add(mkb, c).add(mib, c).add(sx[0], c + kCoopPad)
+            .add(sx[1], c + kCoopPad).add(sv, c).add(sx0, c + kCoopPad).add(somega, c).add(dpb, c).add(rho, c).add(lod, c)
+            .add(cand, 2 * c).add(ct_counts, (size_t)contact_num_blocks(need_n) + 1)
+            .add(hist, (size_t)256 * sort_num_tiles(need_n));
+        if ((rc = particle_slab.alloc())) return rc;
         cap_n = need_n;
     }
     if (coop_lanes(need_n) && need_n > cap_chits) {
         cap_chits = 0;
-        if ((rc = dalloc(chits, (size_t)need_n * kCoopList)) || (rc = dalloc(chit_len, need_n))) return rc;
+        hit_slab.release();
+        if ((rc = hit_slab.add(chits, (size_t)need_n * kCoopList).add(chit_len, need_n).alloc())) return rc;
         cap_chits = need_n;
     }
     if (bucket_sort_fits(need_n, derived.hash_size) && derived.hash_size != cap_bcnt) {
@@ -319,7 +320,7 @@ int pbf_handle::query_take(size_t bytes, char** p)
 void pbf_handle::query_done()
 {
     if (query_cap <= kQueryKeep) return;
-    dfree(query_buf); dfree(bcnt);
+    dfree(query_buf);
     query_cap = 0;
 }
 
@@ -341,14 +342,12 @@ pbf_handle::~pbf_handle()
         cudaEventDestroy(r.b);
     }
     for (cudaEvent_t e : event_pool) cudaEventDestroy(e);
-    dfree(pos); dfree(vel); dfree(pred); dfree(aos); dfree(keys);
-    dfree(mcode); dfree(mka); dfree(mia); dfree(mkb); dfree(mib); dfree(ka); dfree(ia); dfree(kb); dfree(ib);
-    dfree(sx[0]); dfree(sx[1]); dfree(sv); dfree(sx0); dfree(somega); dfree(dpb); dfree(rho); dfree(lod); dfree(chits); dfree(chit_len); dfree(query_buf);
-    dfree(hist); dfree(totals); dfree(table); dfree(cand); dfree(ct_counts); dfree(scalars);
-    dfree(lx[0]); dfree(lx[1]); dfree(lxb); dfree(lv); dfree(lx0); dfree(lom); dfree(lrho);
-    dfree(lid); dfree(lkey); dfree(inv); dfree(dkey_id);
-    dfree(dtable); dfree(druns); dfree(dclean); dfree(ddcol); dfree(ddirty); dfree(dflag);
-    dfree(dslot); dfree(dord); dfree(dcnt); dfree(dbsum); dfree(dhm); dfree(dhcnt); dfree(dvmark);
+    particle_slab.release();
+    hit_slab.release();
+    label_slab.release();
+    order_slab.release();
+    window_slab.release();
+    dfree(query_buf); dfree(bcnt); dfree(totals); dfree(table); dfree(scalars); dfree(dflag);
     dfree(grid); dfree(slab_min);
     mesh_free();
     if (stream) cudaStreamDestroy(stream);
@@ -434,10 +433,11 @@ int pbf_handle::ensure_label_capacity()
     if (cap_label_n < n || !inv) {
         // (kLabelPad entries past the last label: a run's last chunk loads them and masks them out)
         const size_t c = std::max<uint32_t>(n, 1u), cp = c + kLabelPad;
-        if ((rc = dalloc(lx[0], cp)) || (rc = dalloc(lx[1], cp)) || (rc = dalloc(lxb, c)) || (rc = dalloc(lv, cp)) ||
-            (rc = dalloc(lx0, cp)) || (rc = dalloc(lom, cp)) || (rc = dalloc(lrho, c)) || (rc = dalloc(lid, c)) ||
-            (rc = dalloc(lkey, c)) || (rc = dalloc(inv, c)) || (rc = dalloc(dkey_id, c)))
-            return rc;
+        cap_label_n = 0;
+        label_slab.release();
+        label_slab.add(lx[0], cp).add(lx[1], cp).add(lxb, c).add(lv, cp).add(lx0, cp).add(lom, cp).add(lrho, c).add(lid, c)
+            .add(lkey, c).add(inv, c).add(dkey_id, c);
+        if ((rc = label_slab.alloc())) return rc;
         dkey_valid = false;
         cap_label_n = (uint32_t)c;
     }
@@ -513,9 +513,9 @@ int pbf_handle::ensure_dense()
     if (cap_ord_n < n || !dord) {
         if (capturing) return set_error(PBF_ERR_INVALID, "particle count grew during graph capture");
         const size_t c = std::max<uint32_t>(n, 1u);
-        if ((rc = dalloc(dslot, c)) || (rc = dalloc(dord, c)) || (rc = dalloc(dhm, c * kDenseListWords)) ||
-            (rc = dalloc(dhcnt, c)))
-            return rc;
+        cap_ord_n = 0;
+        order_slab.release();
+        if ((rc = order_slab.add(dslot, c).add(dord, c).add(dhm, c * kDenseListWords).add(dhcnt, c).alloc())) return rc;
         cap_ord_n = (uint32_t)c;
     }
     int g0[3];
@@ -527,11 +527,12 @@ int pbf_handle::ensure_dense()
     if (same) return PBF_OK;
     if (capturing) return set_error(PBF_ERR_INVALID, "dense cell window changed during graph capture");
     if (slots > cap_slots || !dtable) {
-        if ((rc = dalloc(dtable, slots + 1)) || (rc = dalloc(druns, slots)) || (rc = dalloc(dcnt, slots + 1)) ||
-            (rc = dalloc(dbsum, order_scan_blocks((uint32_t)slots))) || (rc = dalloc(dclean, slots)) ||
-            (rc = dalloc(ddcol, slots)) ||
-            (rc = dalloc(ddirty, slots)) || (rc = dalloc(dvmark, slots)))
-            return rc;
+        cap_slots = 0;
+        window_slab.release();
+        window_slab.add(dtable, slots + 1).add(druns, slots).add(dcnt, slots + 1)
+            .add(dbsum, order_scan_blocks((uint32_t)slots)).add(dclean, slots).add(ddcol, slots).add(ddirty, slots)
+            .add(dvmark, slots);
+        if ((rc = window_slab.alloc())) return rc;
         cap_slots = slots;
     }
     if (!dflag && (rc = dalloc(dflag, 4))) return rc;

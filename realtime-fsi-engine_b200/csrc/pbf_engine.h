@@ -8,6 +8,7 @@
 
 #include "../../include/pbf_b200.h"
 #include "pbf_kernels.h"
+#include "pbf_slab.h"
 
 namespace pbf {
 int set_error(int code, const char* fmt, ...);
@@ -26,6 +27,10 @@ struct pbf_handle {
     float camera[3] = {0, 0, 0};
 
     uint32_t n = 0, cap_n = 0, cap_h = 0;
+
+    // owners of the arrays below: per particle; the small scenes' hits; mode 8's
+    // labels, thread orders and window
+    pbf::Slab particle_slab, hit_slab, label_slab, order_slab, window_slab;
 
     // particle order
     float4* pos = nullptr;

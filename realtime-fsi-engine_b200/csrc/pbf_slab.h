@@ -1,0 +1,64 @@
+// pbf_slab.h — device arrays that live and go together, in one allocation.
+//
+// An allocation of 2 MB or more takes 0.32 ms on a B200 whatever its size, and
+// its release as much: the 25 arrays of a scene of 262,144 particles took 6.1
+// ms one by one, 1.5 ms together.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <vector>
+
+#include "../../include/pbf_b200.h"
+
+namespace pbf {
+int set_error(int code, const char* fmt, ...);
+
+class Slab {
+public:
+    Slab() = default;
+    Slab(const Slab&) = delete;
+    Slab& operator=(const Slab&) = delete;
+    ~Slab() { release(); }
+
+    // Lists an array for the next alloc(); p is null until then.
+    template <class T>
+    Slab& add(T*& p, size_t count)
+    {
+        p = nullptr;
+        items_.push_back({reinterpret_cast<void**>(&p), bytes_});
+        bytes_ += (count * sizeof(T) + 255) / 256 * 256;
+        return *this;
+    }
+    // The listed arrays, 256-byte aligned.  The listed pointers must outlive the slab.
+    int alloc()
+    {
+        const cudaError_t e = cudaMalloc(&base_, bytes_ ? bytes_ : 256);
+        if (e != cudaSuccess) {
+            base_ = nullptr;
+            const int rc = set_error(PBF_ERR_ALLOC, "cudaMalloc(%zu B): %s", bytes_, cudaGetErrorString(e));
+            release();
+            return rc;
+        }
+        for (const Item& i : items_) *i.p = static_cast<char*>(base_) + i.at;
+        return PBF_OK;
+    }
+    void release()
+    {
+        if (base_) cudaFree(base_);
+        base_ = nullptr;
+        for (const Item& i : items_) *i.p = nullptr;
+        items_.clear();
+        bytes_ = 0;
+    }
+
+private:
+    struct Item {
+        void** p;
+        size_t at;
+    };
+    std::vector<Item> items_;
+    size_t bytes_ = 0;
+    void* base_ = nullptr;
+};
+}  // namespace pbf
