@@ -47,6 +47,10 @@ public:
     void updateColumns(const SymCsc& A, const std::vector<int>& changed);
     // Solve A^B x = b in place.
     void solveInPlace(std::vector<double>& b) const;
+    // Three right-hand sides at once, each with solveInPlace's operations in
+    // its order; the backward solve's chain of dependent subtractions runs
+    // once for the three.
+    void solveInPlace(std::vector<double>& x, std::vector<double>& y, std::vector<double>& z) const;
 
     int size() const { return n_; }
     bool ok() const { return ok_; }
@@ -63,8 +67,15 @@ private:
     std::vector<double> work_;         // dense accumulator of the current row
     std::vector<int> stack_, visit_;   // row-pattern scratch and visit stamps
     int stamp_ = 0;
+    // Rows of a column of L come in runs of consecutive indices (the bandwidth-
+    // reducing order fills them): column j's are runs_[rp_[j]] .. runs_[rp_[j+1]-1].
+    struct Run {
+        int row, at, len;              // first row, its place in li_/lx_, rows
+    };
+    std::vector<int> rp_;
+    std::vector<Run> runs_;
+    std::vector<int> cursor_;          // per column: the run its last computed row lies in
 
-    int slot(int col, int row) const;  // position of L(row, col) in li_/lx_
     void column(const SymCsc& A, int k);
 };
 

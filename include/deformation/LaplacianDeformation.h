@@ -132,7 +132,7 @@ private:
     void buildNormalSystem();
     std::vector<int> constrainedSorted() const;
     void targets(std::vector<double>& tx, std::vector<double>& ty, std::vector<double>& tz) const;
-    void solveAxisIncremental(const std::vector<double>& b, const std::vector<double>& t,
+    void rhsIncremental(const std::vector<double>& b, const std::vector<double>& t,
                               std::vector<double>& x) const;
     void precomputeLocal();
     void solveLocal();

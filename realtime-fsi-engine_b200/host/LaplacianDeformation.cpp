@@ -342,9 +342,7 @@ void LaplacianDeformation::solveLocal()
         ry[P.handleLocal[c]] += t[1];
         rz[P.handleLocal[c]] += t[2];
     }
-    P.factor.solveInPlace(rx);
-    P.factor.solveInPlace(ry);
-    P.factor.solveInPlace(rz);
+    P.factor.solveInPlace(rx, ry, rz);
     for (int i = 0; i < ni; ++i) mesh_.points[P.interior[i]] = {rx[i], ry[i], rz[i]};
 }
 
@@ -395,10 +393,11 @@ void LaplacianDeformation::targets(std::vector<double>& tx, std::vector<double>&
     for (size_t i = 0; i < controlIndices_.size(); ++i) set(controlIndices_[i], controlTargets_[i]);
 }
 
-void LaplacianDeformation::solveAxisIncremental(const std::vector<double>& b, const std::vector<double>& t,
-                                                std::vector<double>& x) const
+// Right-hand side of one axis in the factor's order: free rows b - A_IC t_C,
+// constrained rows their targets.
+void LaplacianDeformation::rhsIncremental(const std::vector<double>& b, const std::vector<double>& t,
+                                          std::vector<double>& rp) const
 {
-    // free rows: b - A_IC t_C; constrained rows: their targets
     std::vector<double> rhs = b;
     for (int k = 0; k < n_; ++k) {
         if (!mask_[k]) continue;
@@ -406,11 +405,8 @@ void LaplacianDeformation::solveAxisIncremental(const std::vector<double>& b, co
     }
     for (int k = 0; k < n_; ++k)
         if (mask_[k]) rhs[k] = t[k];
-    std::vector<double> rp(n_);
+    rp.resize(n_);
     for (int i = 0; i < n_; ++i) rp[i] = rhs[perm_[i]];
-    inc_.solveInPlace(rp);
-    x.assign(n_, 0.0);
-    for (int i = 0; i < n_; ++i) x[perm_[i]] = rp[i];
 }
 
 double LaplacianDeformation::verifyIncremental()
@@ -452,8 +448,10 @@ double LaplacianDeformation::verifyIncremental()
         for (int j = k + 1; j < n_; ++j) s -= M[(size_t)k * n_ + j] * y[j];
         y[k] = s / M[(size_t)k * n_ + k];
     }
-    std::vector<double> xi;
-    solveAxisIncremental(bx_, tx, xi);
+    std::vector<double> rp, xi(n_);
+    rhsIncremental(bx_, tx, rp);
+    inc_.solveInPlace(rp);
+    for (int i = 0; i < n_; ++i) xi[perm_[i]] = rp[i];
     double m = 0.0;
     for (int i = 0; i < n_; ++i) m = std::max(m, std::fabs(xi[i] - y[i]));
     return m;
@@ -527,10 +525,11 @@ void LaplacianDeformation::solve()
         if (!incReady_) return;
         std::vector<double> tx, ty, tz, x, y, z;
         targets(tx, ty, tz);
-        solveAxisIncremental(bx_, tx, x);
-        solveAxisIncremental(by_, ty, y);
-        solveAxisIncremental(bz_, tz, z);
-        for (int i = 0; i < n_; ++i) mesh_.points[i] = {x[i], y[i], z[i]};
+        rhsIncremental(bx_, tx, x);
+        rhsIncremental(by_, ty, y);
+        rhsIncremental(bz_, tz, z);
+        inc_.solveInPlace(x, y, z);
+        for (int i = 0; i < n_; ++i) mesh_.points[perm_[i]] = {x[i], y[i], z[i]};
         return;
     }
     if (!softReady_) return;
@@ -550,9 +549,7 @@ void LaplacianDeformation::solve()
     for (size_t i = 0; i < anchors_.size(); ++i) add(anchors_[i], anchorPos_[i]);
     if (controlIndex_ >= 0) add(controlIndex_, controlTarget_);
     for (size_t i = 0; i < controlIndices_.size(); ++i) add(controlIndices_[i], controlTargets_[i]);
-    softFactor_.solveInPlace(rx);
-    softFactor_.solveInPlace(ry);
-    softFactor_.solveInPlace(rz);
+    softFactor_.solveInPlace(rx, ry, rz);
     for (int i = 0; i < n_; ++i) mesh_.points[i] = {rx[i], ry[i], rz[i]};
 }
 
