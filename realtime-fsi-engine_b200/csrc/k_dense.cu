@@ -56,6 +56,8 @@
 //     recorded (same positions, same runs, same hits), and the vorticity pass
 //     those of the integrate pass, except near particles the walls or the
 //     SDF moved there;
+//   * one scene's particles with rows on the buckets go first, in groups of
+//     lanes, so that their longer walks end before the others';
 //   * x/y arithmetic in packed f32x2 instructions, each lane rounded as the
 //     scalar operation.
 // One kernel serves one scene (B = false, constants read from the kernel
@@ -69,7 +71,7 @@
 
 namespace pbf {
 
-constexpr int kDThreads = 128;
+constexpr int kDThreads = kDensePassThreads;
 // The nine rows (dz, dy) of a cell's neighbourhood, bit (dz + 1) * 3 + (dy + 1).
 constexpr uint32_t kAllRows = 0x1FFu;
 
@@ -193,17 +195,90 @@ __global__ void __launch_bounds__(256) k_d_keys_gather(uint32_t n, const uint32_
         dkey[s] = __ldg(dkey_id + __ldg(ids + s));
 }
 
+// Global slot of the cell of x (cells outside the window: the extra slot D.total).
+__device__ __forceinline__ uint32_t current_slot(const DevParams& P, const DenseArgs& D, float4 x)
+{
+    const uint32_t ux = (uint32_t)cell_coord(x.x, P.h) - (uint32_t)D.gx0;
+    const uint32_t uy = (uint32_t)cell_coord(x.y, P.h) - (uint32_t)D.gy0;
+    const uint32_t uz = (uint32_t)cell_coord(x.z, P.h) - (uint32_t)D.gz0;
+    return (ux < D.nx && uy < D.ny && uz < D.nz) ? D.slot0 + (uz * D.ny + uy) * D.nx + ux : D.total;
+}
+
+// ---- the particles that walk buckets, first -----------------------------------------------
+// A particle with rows on the buckets takes up to twice as long as its
+// neighbours, and its warp with it.  They are few (the cells along the box's
+// near-zero edges, mostly), and the order of the threads leaves some of them
+// to the end of the launch, where they ran on alone: with 262,144 particles
+// the last quarter of a lambda launch's 110 us had fewer than 100 warps in
+// flight.  So the order lists them: its entry has kListed set, its thread
+// leaves the particle alone, and the launch's first `list_blocks` blocks take
+// the listed ones, kListLanes lanes each (GroupWalk), consecutive warps of them
+// on different blocks.  A full list leaves the rest where they are.
+// One scene only: a batch has too many of them (dense_list_blocks).
+// Lambda / delta-p of 262,144 particles (3,100 listed) 108 / 84 -> 90 / 63 us,
+// of 602,263 (4,000 listed) 173 / 93 -> 150 / 83 us; a step of 4,194,304 (8,900
+// listed) 8.83 -> 8.77 ms.  One lane per listed particle made the list's warps
+// the longest themselves (the 262,144-particle step 2.47 ms, against 2.22
+// without a list and 1.85 so); 4 lanes 2.15, 16 lanes 1.93.
+constexpr uint32_t kListed = 0x80000000u;
+constexpr int kListLanes = 32 / kDenseListPerWarp;  // lanes of a listed particle
+
+// The order entry of label t, and its list entry when it walks buckets.  Every
+// lane that holds a label calls it.
+__device__ __forceinline__ uint32_t list_bucket_walker(const DenseArgs& D, uint32_t t, bool buckets)
+{
+    const uint32_t am = __activemask(), m = __ballot_sync(am, buckets);
+    if (!m) return t;
+    const int lane = threadIdx.x & 31, lead = __ffs(m) - 1;
+    uint32_t at = 0;
+    if (lane == lead) at = atomicAdd(D.list, (uint32_t)__popc(m));
+    at = __shfl_sync(am, at, lead) + (uint32_t)__popc(m & ((1u << lane) - 1u));
+    if (!buckets || at >= dense_list_room(D.list_blocks)) return t;
+    D.list[1u + at] = t;
+    return t | kListed;
+}
+
+// What a thread of a pass works on.
+struct PassLabel {
+    bool live;    // it has a label
+    bool listed;  // with the kListLanes lanes of its group, which walk together
+    bool first;   // and is the one that writes
+    int t;
+};
+template <bool B>
+__device__ __forceinline__ PassLabel pass_label(const DenseArgs& D, uint32_t n)
+{
+    if constexpr (B) {
+        const uint32_t i = blockIdx.x * kDThreads + threadIdx.x;
+        const bool live = i < n;
+        return {live, false, live, !live ? 0 : D.order ? (int)__ldg(D.order + i) : (int)i};
+    }
+    if (blockIdx.x < D.list_blocks) {
+        const uint32_t warp = (threadIdx.x >> 5) * D.list_blocks + blockIdx.x, lane = threadIdx.x & 31u;
+        const uint32_t at = warp * kDenseListPerWarp + lane / kListLanes;
+        if (!D.order || at >= min(__ldg(D.list), dense_list_room(D.list_blocks))) return {false, false, false, 0};
+        return {true, true, lane % kListLanes == 0, (int)__ldg(D.list + 1u + at)};
+    }
+    const uint32_t i = (blockIdx.x - D.list_blocks) * kDThreads + threadIdx.x;
+    if (i >= n) return {false, false, false, 0};
+    const uint32_t o = D.order ? __ldg(D.order + i) : i;
+    if (o & kListed) return {false, false, false, 0};
+    return {true, false, true, (int)o};
+}
+
 // Label t = hash-sorted index order[t]: its x* (also the predict-time copy),
 // predicted velocity, substep-start position, id and key, gathered from the
 // particle state (the predict pass's arithmetic again), and inv[order[t]] = t.
-__global__ void __launch_bounds__(256) k_d_permute(DevParams P, const uint32_t* __restrict__ order,
+// Also the first iteration's thread order: the labels themselves, with those
+// that walk buckets listed (BucketList).
+__global__ void __launch_bounds__(256) k_d_permute(DevParams P, DenseArgs D, const uint32_t* __restrict__ order,
                                                    const uint32_t* __restrict__ ids,
                                                    const uint32_t* __restrict__ skeys,
                                                    const float4* __restrict__ pos, const float4* __restrict__ vel,
                                                    float4* __restrict__ lx, float4* __restrict__ lxb,
                                                    float4* __restrict__ lv, float4* __restrict__ lx0,
                                                    uint32_t* __restrict__ lid, uint32_t* __restrict__ lkey,
-                                                   uint32_t* __restrict__ inv)
+                                                   uint32_t* __restrict__ inv, uint32_t* __restrict__ thread_order)
 {
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < P.n; t += stride) {
@@ -221,6 +296,10 @@ __global__ void __launch_bounds__(256) k_d_permute(DevParams P, const uint32_t* 
         lid[t] = id;
         lkey[t] = __ldg(skeys + s);
         inv[s] = t;
+        if (D.list_blocks) {
+            const uint32_t g = current_slot(P, D, x);
+            thread_order[t] = list_bucket_walker(D, t, g == D.total || __ldg(D.clean + g) != 0);
+        }
     }
 }
 
@@ -602,6 +681,78 @@ struct MixedWalk {
     }
 };
 
+// The mixed walk by the kListLanes lanes of a listed particle: each tests one
+// candidate of a chunk, all run the body for the chunk's hits (the same loads,
+// the same sums in every lane), so a bucket of up to kListLanes candidates
+// takes one test instead of kListLanes.
+struct GroupWalk {
+    const DevParams& P;
+    const int2* __restrict__ runs;
+    const int2* __restrict__ htable;
+    const uint32_t* __restrict__ inv;
+    const float4* __restrict__ X;
+    float4 xi;
+    int self;
+    int s0;
+    int nx, nxy;
+    uint32_t rows;
+    template <class Map, class Hit, class Body>
+    __device__ __forceinline__ void range(int lo, int hi, Map&& map, Hit&& hit, Body&& body) const
+    {
+        const int lane = threadIdx.x & 31, gl = lane & (kListLanes - 1), base = lane & ~(kListLanes - 1);
+        const uint32_t group = ((1u << kListLanes) - 1u) << base;
+#pragma unroll 1
+        for (int k0 = lo; k0 < hi; k0 += kListLanes) {
+            int j = self;
+            bool h = false;
+            if (k0 + gl < hi) {
+                j = map(k0 + gl);
+                const float4 xj = __ldg(X + j);
+                const float2 rxy = sub_f32x2(make_float2(xi.x, xi.y), make_float2(xj.x, xj.y));
+                const float rx = rxy.x, ry = rxy.y, rz = xi.z - xj.z;
+                h = hit(rx * rx + ry * ry + rz * rz) && j != self;
+            }
+            uint32_t m = __ballot_sync(group, h) >> base;
+            while (m) {
+                const int c = __ffs(m) - 1;
+                m &= m - 1u;
+                body(__shfl_sync(group, j, c, kListLanes));
+            }
+        }
+    }
+    template <class Hit, class Body>
+    __device__ __forceinline__ void operator()(Hit&& hit, Body&& body) const
+    {
+        const int cx = cell_coord(xi.x, P.h), cy = cell_coord(xi.y, P.h), cz = cell_coord(xi.z, P.h);
+#pragma unroll 1
+        for (int dz = -1; dz <= 1; ++dz) {
+            const uint32_t hz = (uint32_t)(cz + dz) * kP3;
+#pragma unroll 1
+            for (int dy = -1; dy <= 1; ++dy) {
+                // the row's candidates: its run, or its three buckets one after the other
+                const bool buckets = (rows >> ((dz + 1) * 3 + (dy + 1))) & 1u;
+                int2 r0, r1 = make_int2(0, 0), r2 = make_int2(0, 0);
+                if (buckets) {
+                    const uint32_t hyz = hz ^ ((uint32_t)(cy + dy) * kP2);
+                    r0 = __ldg(htable + ((((uint32_t)(cx - 1) * kP1) ^ hyz) & P.mask));
+                    r1 = __ldg(htable + ((((uint32_t)cx * kP1) ^ hyz) & P.mask));
+                    r2 = __ldg(htable + ((((uint32_t)(cx + 1) * kP1) ^ hyz) & P.mask));
+                } else {
+                    r0 = __ldg(runs + s0 + dz * nxy + dy * nx);
+                }
+                // (an empty bucket is (-1, -1))
+                const int n0 = r0.y - r0.x, n1 = n0 + r1.y - r1.x, all = n1 + r2.y - r2.x;
+                range(0, all,
+                      [&](int k) {
+                          const int c = k < n0 ? r0.x + k : k < n1 ? r1.x + k - n0 : r2.x + k - n1;
+                          return buckets ? (int)__ldg(inv + c) : c;
+                      },
+                      hit, body);
+            }
+        }
+    }
+};
+
 // Window slot of the particle's current cell when its neighbourhood lies in
 // the window interior (else -1); dense_rows adds the rows that (b) and (c)
 // send to the buckets.
@@ -630,6 +781,12 @@ __device__ __forceinline__ MixedWalk mixed_walk(const DevParams& P, const DenseA
     return MixedWalk{P, D.runs, D.htable, D.inv, X, xi, t, s0, (int)D.nx, (int)(D.nx * D.ny), rows};
 }
 
+__device__ __forceinline__ GroupWalk group_walk(const DevParams& P, const DenseArgs& D, const float4* X, float4 xi,
+                                                int t, int s0, uint32_t rows)
+{
+    return GroupWalk{P, D.runs, D.htable, D.inv, X, xi, t, s0, (int)D.nx, (int)(D.nx * D.ny), rows};
+}
+
 __device__ __forceinline__ void count_bucket_walk(const DenseArgs& D)
 {
     const uint32_t am = __activemask();
@@ -640,10 +797,16 @@ __device__ __forceinline__ void count_bucket_walk(const DenseArgs& D)
 // row, else with the mixed walk (the rows they rule out through the buckets).
 template <class Core>
 __device__ __forceinline__ void with_dense_walker(const DevParams& P, const DenseArgs& D, const float4* X, float4 xi,
-                                                  int t, Core&& core)
+                                                  const PassLabel& L, Core&& core)
 {
+    const int t = L.t;
     uint32_t rows;
     const int s0 = dense_rows(P, D, xi, rows);
+    if (L.listed) {
+        if (L.first) count_bucket_walk(D);
+        core(group_walk(P, D, X, xi, t, s0, rows));
+        return;
+    }
     if (rows == 0) {
         core(RunWalk{D.runs, X, xi, t, s0, (int)D.nx, (int)(D.nx * D.ny)});
         return;
@@ -783,15 +946,6 @@ __device__ __forceinline__ void slot_run(uint32_t s, uint32_t lane, uint32_t& he
 
 constexpr uint32_t kNoSlot = 0xffffffffu;
 
-// Global slot of the cell of x (cells outside the window: the extra slot D.total).
-__device__ __forceinline__ uint32_t current_slot(const DevParams& P, const DenseArgs& D, float4 x)
-{
-    const uint32_t ux = (uint32_t)cell_coord(x.x, P.h) - (uint32_t)D.gx0;
-    const uint32_t uy = (uint32_t)cell_coord(x.y, P.h) - (uint32_t)D.gy0;
-    const uint32_t uz = (uint32_t)cell_coord(x.z, P.h) - (uint32_t)D.gz0;
-    return (ux < D.nx && uy < D.ny && uz < D.nz) ? D.slot0 + (uz * D.ny + uy) * D.nx + ux : D.total;
-}
-
 // slot of the current cell
 template <bool B>
 __global__ void __launch_bounds__(256) k_d_cslot(DevParams P0, DenseArgs D0, const float4* __restrict__ X,
@@ -867,8 +1021,11 @@ __global__ void __launch_bounds__(1024) k_d_scan_blocks(uint32_t* __restrict__ c
     if (threadIdx.x == 1023) block_sums[blockIdx.x] = warp_sums[31];
 }
 
-__global__ void __launch_bounds__(1024) k_d_scan_sums(uint32_t* __restrict__ block_sums, uint32_t nb)
+// (and the bucket walkers' list emptied for the placement that follows)
+__global__ void __launch_bounds__(1024) k_d_scan_sums(uint32_t* __restrict__ block_sums, uint32_t nb,
+                                                      uint32_t* __restrict__ list)
 {
+    if (list && threadIdx.x == 0) *list = 0;
     __shared__ uint32_t warp_sums[32];
     const uint32_t chunk = (nb + 1023u) / 1024u;
     const uint32_t begin = threadIdx.x * chunk, end = min(begin + chunk, nb);
@@ -901,7 +1058,7 @@ __global__ void __launch_bounds__(1024) k_d_scan_sums(uint32_t* __restrict__ blo
     }
 }
 
-__global__ void __launch_bounds__(256) k_d_place(uint32_t n, const uint32_t* __restrict__ slot_of,
+__global__ void __launch_bounds__(256) k_d_place(DenseArgs D, uint32_t n, const uint32_t* __restrict__ slot_of,
                                                  uint32_t* __restrict__ start, const uint32_t* __restrict__ block_offs,
                                                  uint32_t* __restrict__ order)
 {
@@ -913,7 +1070,11 @@ __global__ void __launch_bounds__(256) k_d_place(uint32_t n, const uint32_t* __r
     uint32_t b = 0;
     if (lane == head && s != kNoSlot) b = atomicAdd(start + s, len);
     b = __shfl_sync(0xffffffffu, b, head);
-    if (s != kNoSlot) order[__ldg(block_offs + s / kScanItems) + b + (lane - head)] = t;
+    if (s == kNoSlot) return;
+    uint32_t o = t;
+    if (D.list_blocks)
+        o = list_bucket_walker(D, t, s == D.total || __ldg(D.clean + s) != 0 || D.dirty[s] != 0);
+    order[__ldg(block_offs + s / kScanItems) + b + (lane - head)] = o;
 }
 
 // ---- relabelling of one scene by counting -----------------------------------------------
@@ -968,9 +1129,9 @@ template <bool B>
 __global__ void __launch_bounds__(kDThreads, 10) k_d_lambda(DevParams P0, DenseArgs D0, const float4* __restrict__ lx_in,
                                                             float4* __restrict__ lx_out, float* __restrict__ lrho)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (int)P0.n) return;
-    const int t = D0.order ? (int)__ldg(D0.order + i) : i;
+    const PassLabel L = pass_label<B>(D0, P0.n);
+    if (!L.live) return;
+    const int t = L.t;
     with_scene<B>(P0, D0, t, [&](const DevParams& P, const DenseArgs& D) {
         const float4 xi = __ldg(lx_in + t);
         float rho, den;
@@ -979,7 +1140,12 @@ __global__ void __launch_bounds__(kDThreads, 10) k_d_lambda(DevParams P0, DenseA
         uint32_t rows;
         const int s0 = dense_rows(P, D, xi, rows);
         float3 b;
-        if (rows == 0) {
+        if (L.listed) {
+            if (L.first) count_bucket_walk(D);
+            out = lambda_core(P, GSrc{lx_in}, xi, group_walk(P, D, lx_in, xi, t, s0, rows), rho, g, den, b);
+            if (!L.first) return;
+            D.hcnt[t] = kNoList;
+        } else if (rows == 0) {
             int q = 0;
             out = lambda_core(P, GSrc{lx_in}, xi,
                               RunWalkRec{D.runs, lx_in, xi, t, s0, (int)D.nx, (int)(D.nx * D.ny), D.hm, P.n, &q}, rho, g,
@@ -1004,12 +1170,11 @@ template <bool B>
 __global__ void __launch_bounds__(kDThreads, 16) k_d_deltap(DevParams P0, DenseArgs D0, const float4* __restrict__ lx_in,
                                                             float4* __restrict__ lx_out)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool live = i < (int)P0.n;
-    const int t = live ? (D0.order ? (int)__ldg(D0.order + i) : i) : 0;
+    const PassLabel L = pass_label<B>(D0, P0.n);
+    const int t = L.t;
     with_scene<B>(P0, D0, t, [&](const DevParams& P, const DenseArgs& D) {
         float4 out = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (live) {
+        if (L.live) {
             const float4 xi = __ldg(lx_in + t);
             const float4 b4 = __ldg(P.dpb + t);
             const float3 b = make_float3(b4.x, b4.y, b4.z);
@@ -1021,13 +1186,15 @@ __global__ void __launch_bounds__(kDThreads, 16) k_d_deltap(DevParams P0, DenseA
                                   RunWalkList{D.runs, lx_in, xi, t, s0, (int)D.nx, (int)(D.nx * D.ny), D.hm, P.n}, dp,
                                   b);
             } else {
-                with_dense_walker(P, D, lx_in, xi, t,
+                with_dense_walker(P, D, lx_in, xi, L,
                                   [&](auto&& walk) { out = deltap_core(P, P.sdf, GSrc{lx_in}, xi, walk, dp, b); });
             }
-            lx_out[t] = out;
-            check_drift(P, D, out, t);
+            if (L.first) {
+                lx_out[t] = out;
+                check_drift(P, D, out, t);
+            }
         }
-        if (D.rec_cnt) record_slot(P, D, out, t, live);
+        if (D.rec_cnt) record_slot(P, D, out, t, L.first);
     });
 }
 
@@ -1038,12 +1205,11 @@ __global__ void __launch_bounds__(kDThreads, 10) k_d_integrate(DevParams P0, Den
                                                            const uint32_t* __restrict__ lid, float4* __restrict__ pos,
                                                            float4* __restrict__ vel)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool live = i < (int)P0.n;
-    const int t = live ? (D0.order ? (int)__ldg(D0.order + i) : i) : 0;
+    const PassLabel L = pass_label<B>(D0, P0.n);
+    const int t = L.t;
     with_scene<B>(P0, D0, t, [&](const DevParams& P, const DenseArgs& D) {
         float4 xo = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (live) {
+        if (L.live) {
             const float4 x4 = __ldg(lx + t);
             const float4 v0 = __ldg(lv + t);
             float4 vo, om;
@@ -1058,7 +1224,11 @@ __global__ void __launch_bounds__(kDThreads, 10) k_d_integrate(DevParams P0, Den
                 // cells whose runs hold it
                 uint32_t rows;
                 const int s0 = dense_rows(P, D, x4, rows);
-                if (rows == 0) {
+                if (L.listed) {
+                    if (L.first) count_bucket_walk(D);
+                    core(group_walk(P, D, lx, x4, t, s0, rows));
+                    if (L.first) D.hcnt[t] = kNoList;
+                } else if (rows == 0) {
                     int q = 0;
                     core(RunWalkRec{D.runs, lx, x4, t, s0, (int)D.nx, (int)(D.nx * D.ny), D.hm, P.n, &q});
                     D.hcnt[t] = q <= kListChunks ? (uint8_t)q : kNoList;
@@ -1067,23 +1237,25 @@ __global__ void __launch_bounds__(kDThreads, 10) k_d_integrate(DevParams P0, Den
                     core(mixed_walk(P, D, lx, x4, t, s0, rows));
                     D.hcnt[t] = kNoList;
                 }
-                if (xo.x != x4.x || xo.y != x4.y || xo.z != x4.z) {
+                if (L.first && (xo.x != x4.x || xo.y != x4.y || xo.z != x4.z)) {
                     D.hcnt[t] = kNoList;
                     mark_moved(P, D, t);
                 }
             } else {
-                with_dense_walker(P, D, lx, x4, t, core);
+                with_dense_walker(P, D, lx, x4, L, core);
             }
-            if (P.vort_on) lom[t] = om;
-            const uint32_t id = __ldg(lid + t);
-            pos[id] = xo;
-            vel[id] = vo;
-            // (the committed position carries |omega| in w for the vorticity
-            // pass, which then reads a neighbour's position and |omega| in one load)
-            lx0[t] = P.vort_on ? make_float4(xo.x, xo.y, xo.z, om.w) : xo;
-            check_drift(P, D, xo, t);
+            if (L.first) {
+                if (P.vort_on) lom[t] = om;
+                const uint32_t id = __ldg(lid + t);
+                pos[id] = xo;
+                vel[id] = vo;
+                // (the committed position carries |omega| in w for the vorticity
+                // pass, which then reads a neighbour's position and |omega| in one load)
+                lx0[t] = P.vort_on ? make_float4(xo.x, xo.y, xo.z, om.w) : xo;
+                check_drift(P, D, xo, t);
+            }
         }
-        if (D.rec_cnt) record_slot(P, D, xo, t, live);
+        if (D.rec_cnt) record_slot(P, D, xo, t, L.first);
     });
 }
 
@@ -1092,9 +1264,9 @@ __global__ void __launch_bounds__(kDThreads, 12) k_d_vorticity(DevParams P0, Den
                                                            const float4* __restrict__ lom,
                                                            const uint32_t* __restrict__ lid, float4* __restrict__ vel)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (int)P0.n) return;
-    const int t = D0.order ? (int)__ldg(D0.order + i) : i;
+    const PassLabel L = pass_label<B>(D0, P0.n);
+    if (!L.live) return;
+    const int t = L.t;
     with_scene<B>(P0, D0, t, [&](const DevParams& P, const DenseArgs& D) {
         const float4 xi = __ldg(lx0 + t);
         float3 dv;
@@ -1107,8 +1279,8 @@ __global__ void __launch_bounds__(kDThreads, 12) k_d_vorticity(DevParams P0, Den
             // integrate walked this particle's runs over the same positions
             core(RunWalkList{D.runs, lx0, xi, t, s0, (int)D.nx, (int)(D.nx * D.ny), D.hm, P.n});
         else
-            with_dense_walker(P, D, lx0, xi, t, core);
-        if (!any) return;
+            with_dense_walker(P, D, lx0, xi, L, core);
+        if (!any || !L.first) return;
         const uint32_t id = __ldg(lid + t);
         float4 v = vel[id];
         v.x += dv.x;
@@ -1119,7 +1291,8 @@ __global__ void __launch_bounds__(kDThreads, 12) k_d_vorticity(DevParams P0, Den
 }
 
 // ---- launchers ------------------------------------------------------------------------------
-static inline unsigned dgrid(uint32_t n) { return (n + kDThreads - 1) / kDThreads; }
+// the list's blocks, then the order's
+static inline unsigned dgrid(const DenseArgs& D, uint32_t n) { return D.list_blocks + (n + kDThreads - 1) / kDThreads; }
 static inline unsigned capped_grid(uint32_t n, uint32_t threads, int sms, uint32_t per_sm)
 {
     const uint32_t want = (n + threads - 1u) / threads, cap = (uint32_t)sms * per_sm;
@@ -1153,12 +1326,12 @@ void launch_d_keys_gather(uint32_t n, const uint32_t* ids, const uint32_t* dkey_
     k_d_keys_gather<<<capped_grid(n, 256, sms, 8), 256, 0, st>>>(n, ids, dkey_id, dkey);
 }
 
-void launch_d_permute(const DevParams& P, const uint32_t* order, const uint32_t* ids, const uint32_t* skeys,
+void launch_d_permute(const DevParams& P, const DenseArgs& D, const uint32_t* order, const uint32_t* ids, const uint32_t* skeys,
                       const float4* pos, const float4* vel, float4* lx, float4* lxb, float4* lv, float4* lx0,
-                      uint32_t* lid, uint32_t* lkey, uint32_t* inv, int sms, cudaStream_t st)
+                      uint32_t* lid, uint32_t* lkey, uint32_t* inv, uint32_t* thread_order, int sms, cudaStream_t st)
 {
-    k_d_permute<<<capped_grid(P.n, 256, sms, 8), 256, 0, st>>>(P, order, ids, skeys, pos, vel, lx, lxb, lv, lx0, lid,
-                                                               lkey, inv);
+    k_d_permute<<<capped_grid(P.n, 256, sms, 8), 256, 0, st>>>(P, D, order, ids, skeys, pos, vel, lx, lxb, lv, lx0, lid,
+                                                               lkey, inv, thread_order);
 }
 
 void launch_d_clean(const DenseArgs& D, uint32_t mask, uint16_t* clean, uint32_t* unclean, int sms, cudaStream_t st)
@@ -1187,12 +1360,12 @@ void launch_d_order(const DevParams& P, const DenseArgs& D, const float4* X, uin
     const unsigned g = (P.n + 255u) / 256u;
     PBF_DENSE_LAUNCH(k_d_cslot, g, 256, P, D, X, slot_of, cnt);
     k_d_scan_blocks<<<nb, 1024, 0, st>>>(cnt, m, block_sums);
-    k_d_scan_sums<<<1, 1024, 0, st>>>(block_sums, nb);
-    k_d_place<<<g, 256, 0, st>>>(P.n, slot_of, cnt, block_sums, order);
+    k_d_scan_sums<<<1, 1024, 0, st>>>(block_sums, nb, D.list);
+    k_d_place<<<g, 256, 0, st>>>(D, P.n, slot_of, cnt, block_sums, order);
     *launches += 4;
 }
 
-void launch_d_relabel(uint32_t n, uint32_t slots, const uint32_t* dkey, const uint32_t* skeys, uint32_t* cnt,
+void launch_d_relabel(const DenseArgs& D, uint32_t n, uint32_t slots, const uint32_t* dkey, const uint32_t* skeys, uint32_t* cnt,
                       uint32_t* block_sums, uint32_t* overflow_count, uint32_t* order, uint32_t* sorted_keys, int sms,
                       cudaStream_t st, uint64_t* launches)
 {
@@ -1202,7 +1375,7 @@ void launch_d_relabel(uint32_t n, uint32_t slots, const uint32_t* dkey, const ui
     cudaMemsetAsync(overflow_count, 0, sizeof(uint32_t), st);
     k_d_relabel_count<<<(n + 255u) / 256u, 256, 0, st>>>(n, dkey, cnt);
     k_d_scan_blocks<<<nb, 1024, 0, st>>>(cnt, m, block_sums);
-    k_d_scan_sums<<<1, 1024, 0, st>>>(block_sums, nb);
+    k_d_scan_sums<<<1, 1024, 0, st>>>(block_sums, nb, D.list);
     k_d_relabel_place<<<capped_grid(n, 256, sms, 8), 256, 0, st>>>(n, dkey, skeys, cnt, block_sums, slots,
                                                                   overflow_count, order, sorted_keys);
     *launches += 4;
@@ -1215,20 +1388,20 @@ void launch_d_order_recorded(const DevParams& P, const DenseArgs& D, const uint3
     const uint32_t nb = order_scan_blocks(D.total);
     const unsigned g = (P.n + 255u) / 256u;
     k_d_scan_blocks<<<nb, 1024, 0, st>>>(cnt, m, block_sums);
-    k_d_scan_sums<<<1, 1024, 0, st>>>(block_sums, nb);
-    k_d_place<<<g, 256, 0, st>>>(P.n, slot_of, cnt, block_sums, order);
+    k_d_scan_sums<<<1, 1024, 0, st>>>(block_sums, nb, D.list);
+    k_d_place<<<g, 256, 0, st>>>(D, P.n, slot_of, cnt, block_sums, order);
     *launches += 3;
 }
 
 void launch_d_lambda(const DevParams& P, const DenseArgs& D, const float4* lx_in, float4* lx_out, float* lrho,
                      cudaStream_t st)
 {
-    PBF_DENSE_LAUNCH(k_d_lambda, dgrid(P.n), kDThreads, P, D, lx_in, lx_out, lrho);
+    PBF_DENSE_LAUNCH(k_d_lambda, dgrid(D, P.n), kDThreads, P, D, lx_in, lx_out, lrho);
 }
 
 void launch_d_deltap(const DevParams& P, const DenseArgs& D, const float4* lx_in, float4* lx_out, cudaStream_t st)
 {
-    PBF_DENSE_LAUNCH(k_d_deltap, dgrid(P.n), kDThreads, P, D, lx_in, lx_out);
+    PBF_DENSE_LAUNCH(k_d_deltap, dgrid(D, P.n), kDThreads, P, D, lx_in, lx_out);
 }
 
 void launch_d_integrate(const DevParams& P, const DenseArgs& D, const float4* lx, const float4* lv, float4* lx0,
@@ -1237,21 +1410,21 @@ void launch_d_integrate(const DevParams& P, const DenseArgs& D, const float4* lx
     // R: record hit masks for the vorticity pass
     if (D.rec_list) {
         if (D.scenes)
-            k_d_integrate<true, true><<<dgrid(P.n), kDThreads, 0, st>>>(P, D, lx, lv, lx0, lom, lid, pos, vel);
+            k_d_integrate<true, true><<<dgrid(D, P.n), kDThreads, 0, st>>>(P, D, lx, lv, lx0, lom, lid, pos, vel);
         else
-            k_d_integrate<false, true><<<dgrid(P.n), kDThreads, 0, st>>>(P, D, lx, lv, lx0, lom, lid, pos, vel);
+            k_d_integrate<false, true><<<dgrid(D, P.n), kDThreads, 0, st>>>(P, D, lx, lv, lx0, lom, lid, pos, vel);
     } else {
         if (D.scenes)
-            k_d_integrate<true, false><<<dgrid(P.n), kDThreads, 0, st>>>(P, D, lx, lv, lx0, lom, lid, pos, vel);
+            k_d_integrate<true, false><<<dgrid(D, P.n), kDThreads, 0, st>>>(P, D, lx, lv, lx0, lom, lid, pos, vel);
         else
-            k_d_integrate<false, false><<<dgrid(P.n), kDThreads, 0, st>>>(P, D, lx, lv, lx0, lom, lid, pos, vel);
+            k_d_integrate<false, false><<<dgrid(D, P.n), kDThreads, 0, st>>>(P, D, lx, lv, lx0, lom, lid, pos, vel);
     }
 }
 
 void launch_d_vorticity(const DevParams& P, const DenseArgs& D, const float4* lx0, const float4* lom,
                         const uint32_t* lid, float4* vel, cudaStream_t st)
 {
-    PBF_DENSE_LAUNCH(k_d_vorticity, dgrid(P.n), kDThreads, P, D, lx0, lom, lid, vel);
+    PBF_DENSE_LAUNCH(k_d_vorticity, dgrid(D, P.n), kDThreads, P, D, lx0, lom, lid, vel);
 }
 
 #undef PBF_DENSE_LAUNCH

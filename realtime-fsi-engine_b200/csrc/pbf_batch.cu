@@ -422,7 +422,7 @@ int pbf_batch::dense_step_body()
         uint32_t *msorted = nullptr, *lorder = nullptr;
         launch_radix_sort(n, slot_bits, mcode, mka, mia, mkb, mib, hist, totals, &msorted, &lorder, stream,
                           &launches);
-        launch_d_permute(P, lorder, ids, skeys, pos, vel, lx[0], lxb, lv, lx0, lid, lkey, inv, sms, stream);
+        launch_d_permute(P, D, lorder, ids, skeys, pos, vel, lx[0], lxb, lv, lx0, lid, lkey, inv, nullptr, sms, stream);
         BCK(cudaMemsetAsync(dtable, 0xFF, sizeof(int2) * (size_t)T, stream));
         launch_build_table(n, msorted, dtable, sms, stream);
         launch_d_runs(D, dtable, druns, sms, stream);

@@ -473,6 +473,8 @@ DenseArgs pbf_handle::dense_args() const
     D.table = dtable;
     D.runs = druns;
     D.order = nullptr;
+    D.list = dlist;
+    D.list_blocks = dense_list_blocks(num_sms, dwin_unclean, (uint64_t)dwin_n[0] * dwin_n[1] * dwin_n[2]);
     D.hm = dhm;
     D.hcnt = dhcnt;
     D.use_list = 0;
@@ -515,7 +517,8 @@ int pbf_handle::ensure_dense()
         const size_t c = std::max<uint32_t>(n, 1u);
         cap_ord_n = 0;
         order_slab.release();
-        if ((rc = order_slab.add(dslot, c).add(dord, c).add(dhm, c * kDenseListWords).add(dhcnt, c).alloc())) return rc;
+        if ((rc = order_slab.add(dslot, c).add(dord, c).add(dhm, c * kDenseListWords).add(dhcnt, c)
+                      .add(dlist, 1 + dense_list_room(dense_list_max(num_sms))).alloc())) return rc;
         cap_ord_n = (uint32_t)c;
     }
     int g0[3];
@@ -611,13 +614,15 @@ int pbf_handle::stage(int st, uint32_t iter)
             if (iter >= 2) {
                 order_by(lx[0]);
                 dord_iter = (int)iter;
+            } else if (dord_iter == 1) {
+                D.order = dord;  // of the reorder stage
             }
             launch_d_lambda(P, D, lx[0], lx[1], lrho, stream);
             dlist_iter = (int)iter;
             last_x = 1;
             break;
         case PBF_STAGE_DELTAP:
-            if (iter >= 2 && dord_iter == (int)iter) D.order = dord;
+            if (dord_iter && dord_iter == std::max((int)iter, 1)) D.order = dord;
             D.use_list = dlist_iter == (int)iter ? 1 : 0;
             dlist_iter = 0;
             if (const int rc = record_next()) return rc;
@@ -708,7 +713,7 @@ int pbf_handle::stage(int st, uint32_t iter)
                 // buffers; each particle scans the part of its bucket before it, so
                 // the buckets must stay short
                 order = mia;
-                launch_d_relabel(n, (uint32_t)slots, mcode, skeys, dcnt, dbsum, dflag + 3, order, msorted, sms,
+                launch_d_relabel(D, n, (uint32_t)slots, mcode, skeys, dcnt, dbsum, dflag + 3, order, msorted, sms,
                                  stream, &launches);
             } else {
                 // a hash table far smaller than the particle count: a stable radix
@@ -717,8 +722,9 @@ int pbf_handle::stage(int st, uint32_t iter)
                 while ((1ull << bits) <= slots) ++bits;
                 launch_radix_sort(n, bits, mcode, mka, mia, mkb, mib, hist, totals, &msorted, &order, stream,
                                   &launches);
+                CK(cudaMemsetAsync(dlist, 0, sizeof(uint32_t), stream));
             }
-            launch_d_permute(P, order, ids, skeys, pos, vel, lx[0], lxb, lv, lx0, lid, lkey, inv, sms, stream);
+            launch_d_permute(P, D, order, ids, skeys, pos, vel, lx[0], lxb, lv, lx0, lid, lkey, inv, dord, sms, stream);
             ++launches;
             // (slot `slots` holds the overflow's labels)
             CK(cudaMemsetAsync(dtable, 0xFF, sizeof(int2) * (slots + 1), stream));
@@ -726,7 +732,7 @@ int pbf_handle::stage(int st, uint32_t iter)
             launch_d_runs(dense_args(), dtable, druns, sms, stream);
             launches += 2;
             CK(cudaMemsetAsync(ddirty, 0, sizeof(uint32_t) * slots, stream));
-            dord_iter = 0;
+            dord_iter = D.list_blocks ? 1 : 0;
             dlist_iter = 0;
             dvlist_ready = false;
             dslot_fresh = false;

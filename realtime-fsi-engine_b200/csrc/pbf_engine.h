@@ -68,8 +68,8 @@ struct pbf_handle {
     uint8_t* ddcol = nullptr;    // per window slot: distance to the nearest other cell of its bucket
     uint32_t* ddirty = nullptr;  // per window slot: rows through which a moved particle is within reach (per substep)
     uint32_t* dflag = nullptr;   // [0] drift-bound crossings, [1] bucket walks, [2] unclean slots, [3] overflow labels
-    // thread order of the passes after particles have moved (labels by current cell)
-    uint32_t *dslot = nullptr, *dord = nullptr, *dcnt = nullptr, *dbsum = nullptr;
+    // thread order of the passes (labels by current cell) and its list of bucket walkers
+    uint32_t *dslot = nullptr, *dord = nullptr, *dlist = nullptr, *dcnt = nullptr, *dbsum = nullptr;
     uint32_t cap_ord_n = 0;
     int dord_iter = 0;           // solver iteration the order was computed for (0: none)
     bool dslot_fresh = false;    // dslot/dcnt hold the slots of the latest positions (recorded by a pass)

@@ -76,7 +76,25 @@ void launch_bucket_sort(const DevParams& P, const SceneDev* scenes, const uint16
                         uint32_t* lod, int sms, cudaStream_t st, uint64_t* launches);
 
 // ---- k_dense.cu: x-runs of a dense cell window over relabelled data ----------
+constexpr int kDensePassThreads = 128;
 constexpr int kDenseListWords = 16;
+// The list of bucket walkers (DenseArgs::list): particles per warp, entries
+// that so many blocks take, and the blocks for a window of `slots` cells with
+// `unclean` inner ones whose neighbourhood a hash collision touches.  None
+// when those are more than 1 in 100: eight lanes a particle cost more work than
+// the mixed walk, which a short tail repays and a long list does not (shares
+// of 0.14 - 0.56 %, one scene of 131,072 - 4,194,304 particles: steps 0.6 - 17 %
+// shorter; 1.3 %, tried in batches of 8 - 64 scenes: 2 - 6 % longer).
+constexpr uint32_t kDenseListPerWarp = 4;
+__host__ __device__ inline uint32_t dense_list_room(uint32_t blocks)
+{
+    return blocks * (kDensePassThreads / 32) * kDenseListPerWarp;
+}
+inline uint32_t dense_list_max(int sms) { return 4u * (uint32_t)sms; }
+inline uint32_t dense_list_blocks(int sms, uint64_t unclean, uint64_t slots)
+{
+    return unclean * 100u <= slots ? dense_list_max(sms) : 0u;
+}
 // Label-space position/velocity arrays hold this many entries past the last
 // label, so a run's last chunk of candidates may load past the run's end.
 constexpr int kLabelPad = 32;
@@ -91,7 +109,9 @@ constexpr int kDenseMargin = 6;
 struct DenseArgs {
     const int2* table;     // per window slot: label range of its particles, (-1, -1) when empty
     const int2* runs;      // per window slot: label range of slots s-1 .. s+1 of its row
-    const uint32_t* order; // pass thread i takes label order[i] (null: label i)
+    const uint32_t* order; // pass thread i takes label order[i] (null: label i), unless it is marked as listed
+    uint32_t* list;        // one scene (null in a batch): [0] how many listed, [1 ...] the listed labels (those that walk buckets)
+    uint32_t list_blocks;  // a pass's first blocks, which take them: room for list_blocks * kDensePassThreads
     uint32_t* hm;          // lambda hit masks for the delta-p of the same iteration (kDenseListWords x n)
     uint8_t* hcnt;         // per label: chunks recorded, 0xFF = none
     int use_list;          // delta-p: the lambda pass of this iteration recorded hm/hcnt
@@ -127,9 +147,12 @@ void launch_d_predict_hash(const DevParams& P, const DenseArgs& D, const float4*
                            uint32_t* keys, uint32_t* dkey_id, int sms, cudaStream_t st);
 void launch_d_keys_gather(uint32_t n, const uint32_t* ids, const uint32_t* dkey_id, uint32_t* dkey, int sms,
                           cudaStream_t st);
-void launch_d_permute(const DevParams& P, const uint32_t* order, const uint32_t* ids, const uint32_t* skeys,
-                      const float4* pos, const float4* vel, float4* lx, float4* lxb, float4* lv, float4* lx0,
-                      uint32_t* lid, uint32_t* lkey, uint32_t* inv, int sms, cudaStream_t st);
+// thread_order[n]: the first iteration's order, where the bucket walkers are
+// listed (D.list empty on entry).
+void launch_d_permute(const DevParams& P, const DenseArgs& D, const uint32_t* order, const uint32_t* ids,
+                      const uint32_t* skeys, const float4* pos, const float4* vel, float4* lx, float4* lxb, float4* lv,
+                      float4* lx0, uint32_t* lid, uint32_t* lkey, uint32_t* inv, uint32_t* thread_order, int sms,
+                      cudaStream_t st);
 void launch_d_clean(const DenseArgs& D, uint32_t mask, uint16_t* clean, uint32_t* unclean, int sms, cudaStream_t st);
 void launch_d_dcol(const DenseArgs& D, uint32_t mask, uint8_t* dcol, int sms, cudaStream_t st);
 void launch_d_runs(const DenseArgs& D, const int2* cells, int2* runs, int sms, cudaStream_t st);
@@ -143,7 +166,8 @@ void launch_d_order(const DevParams& P, const DenseArgs& D, const float4* X, uin
 // = hash-sorted index of label t and sorted_keys[t] its key, as a stable sort
 // by key orders them (the overflow slot's entries in any order).  Scratch:
 // cnt[slots + 1], block_sums[order_scan_blocks(slots)], one overflow counter.
-void launch_d_relabel(uint32_t n, uint32_t slots, const uint32_t* dkey, const uint32_t* skeys, uint32_t* cnt,
+// Empties D.list, as the orders above and below do.
+void launch_d_relabel(const DenseArgs& D, uint32_t n, uint32_t slots, const uint32_t* dkey, const uint32_t* skeys, uint32_t* cnt,
                       uint32_t* block_sums, uint32_t* overflow_count, uint32_t* order, uint32_t* sorted_keys, int sms,
                       cudaStream_t st, uint64_t* launches);
 // The same order from slots and counts a pass recorded (DenseArgs::rec_slot / rec_cnt).

@@ -112,3 +112,22 @@ def test_sort_of_a_step_equals_the_stages(have_gpu, n, hash_size):
                     fl.read_buffer(P.BUF_XSTAR, np.float32, (n, 4)), fl.readbackParticles()])
     for a, b in zip(*got):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [1, 15, 17, 600, 25000])
+@pytest.mark.parametrize("fast", [False, True])
+def test_bucket_walkers_of_a_dense_window(have_gpu, n, fast):
+    """Particles along the box's near-zero edges, whose cells meet exact hash
+    collisions: all of them walk buckets, in a large window of clean cells (one
+    group of lanes each), up to more than the list of a launch holds; `fast`
+    ones leave the window in between."""
+    rng = np.random.default_rng(n)
+    h, box = 0.04, 3.0
+    pos = rng.uniform(0.0, 1.0, (n, 3)) * [2 * h, 2 * h, box]
+    turn = rng.integers(0, 3, n)
+    pos = np.stack([np.take_along_axis(pos, ((k + turn) % 3)[:, None], 1)[:, 0] for k in range(3)], 1).astype(np.float32)
+    vel = rng.normal(size=(n, 3)).astype(np.float32)
+    if fast:
+        vel[::3] *= 200.0
+    cfg = scenes.base_config(h, h / 2, (box, box, box), 2, 3, 1.0 / 60.0, n, 1 << 16)
+    assert same(stepped(cfg, pos, vel, 4), stepped(cfg, pos, vel, 8))
