@@ -360,16 +360,36 @@ __global__ void __launch_bounds__(128) k_d_clean(DenseArgs D0, uint32_t mask0, u
 }
 
 // Label range of the x-run centred on each window slot: slots s - 1, s, s + 1
-// of one row, (-1, -1) entries being empty cells; (0, 0) when all three are
-// empty and at the row ends (never walked: a walked cell is interior).
-template <bool B>
-__global__ void __launch_bounds__(256) k_d_runs(DenseArgs D0, const int2* __restrict__ cells, int2* __restrict__ runs)
+// of one row; empty when all three are empty and at the row ends (never
+// walked: a walked cell is interior).  Slot g's labels are first(g) ..
+// first(g + 1) - 1.  Also clears the substep's dirty rows and crossings.
+constexpr uint32_t kScanItems = kDenseScanItems;
+
+__global__ void __launch_bounds__(256) k_d_runs(DenseArgs D, const uint32_t* __restrict__ start,
+                                                const uint32_t* __restrict__ block_offs, int2* __restrict__ runs)
+{
+    if (blockIdx.x == 0 && threadIdx.x == 0) D.flag[0] = 0;
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < D.total; g += stride) {
+        const uint32_t ux = g % D.nx;
+        const auto first = [&](uint32_t q) { return __ldg(block_offs + q / kScanItems) + __ldg(start + q); };
+        int2 r = make_int2(0, 0);
+        if (ux >= 1 && ux + 1 < D.nx) r = make_int2((int)first(g - 1), (int)first(g + 2));
+        runs[g] = r;
+        D.dirty[g] = 0;
+    }
+}
+
+// The same for a batch from its table of label ranges, (-1, -1) entries being
+// empty cells.
+__global__ void __launch_bounds__(256) k_d_runs_batch(DenseArgs D0, const int2* __restrict__ cells,
+                                                      int2* __restrict__ runs)
 {
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < D0.total; g += stride) {
         DenseArgs D = D0;
         uint32_t mask = 0;
-        const uint32_t ux = window_of_slot<B>(D, mask, g) % D.nx;
+        const uint32_t ux = window_of_slot<true>(D, mask, g) % D.nx;
         int2 r = make_int2(0, 0);
         if (ux >= 1 && ux + 1 < D.nx) {
             const int2 e0 = __ldg(cells + g - 1), e1 = __ldg(cells + g), e2 = __ldg(cells + g + 1);
@@ -930,8 +950,6 @@ __global__ void k_d_unpermute1(uint32_t n, const uint32_t* __restrict__ inv, con
 // scan, place); the pass's thread i then takes label order[i].  The order only
 // changes which thread computes which particle, never a result, so the place
 // step may use atomics in any order.
-constexpr uint32_t kScanItems = 4096;  // counters per block of the slot scan
-
 // Runs of equal slots among the lanes of a warp (lanes hold consecutive
 // labels, mostly of one cell): the lane that heads this lane's run and the
 // run's length.
@@ -980,8 +998,34 @@ __device__ __forceinline__ void record_slot(const DevParams& P, const DenseArgs&
     if (lane == head && s != kNoSlot) atomicAdd(D.rec_cnt + s, len);
 }
 
-// exclusive scan of cnt[0 .. m) in place: per block of kScanItems, then the
-// block sums, then the block offsets
+__device__ __forceinline__ uint32_t block_scan(uint32_t local, uint32_t* warp_sums)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t incl = local;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+    }
+    if (lane == 31) warp_sums[warp] = incl;
+    __syncthreads();
+    if (warp == 0) {
+        uint32_t w = warp_sums[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += u;
+        }
+        warp_sums[lane] = w;
+    }
+    __syncthreads();
+    return incl - local + (warp ? warp_sums[warp - 1] : 0u);
+}
+
+// Exclusive scan of cnt[0 .. m) in place within blocks of kScanItems, their sums
+// to block_sums.  (Scanning into a second array and clearing the counts on the
+// way took 51 us for 5 million counters against 16, and the scan of the sums in
+// the last block's hands 78 us.)
 __global__ void __launch_bounds__(1024) k_d_scan_blocks(uint32_t* __restrict__ cnt, uint32_t m,
                                                         uint32_t* __restrict__ block_sums)
 {
@@ -993,26 +1037,7 @@ __global__ void __launch_bounds__(1024) k_d_scan_blocks(uint32_t* __restrict__ c
         v[k] = base + k < m ? cnt[base + k] : 0u;
         local += v[k];
     }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t incl = local;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += u;
-    }
-    if (lane == 31) warp_sums[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t w = warp_sums[lane];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t u = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += u;
-        }
-        warp_sums[lane] = w;
-    }
-    __syncthreads();
-    uint32_t run = incl - local + (warp ? warp_sums[warp - 1] : 0u);
+    uint32_t run = block_scan(local, warp_sums);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         if (base + k < m) cnt[base + k] = run;
@@ -1021,40 +1046,26 @@ __global__ void __launch_bounds__(1024) k_d_scan_blocks(uint32_t* __restrict__ c
     if (threadIdx.x == 1023) block_sums[blockIdx.x] = warp_sums[31];
 }
 
-// (and the bucket walkers' list emptied for the placement that follows)
+// block_sums[0 .. nb) to their exclusive scan; the bucket walkers' list and the
+// overflow counter (both may be null) emptied for the placement that follows.
 __global__ void __launch_bounds__(1024) k_d_scan_sums(uint32_t* __restrict__ block_sums, uint32_t nb,
-                                                      uint32_t* __restrict__ list)
+                                                      uint32_t* __restrict__ list,
+                                                      uint32_t* __restrict__ overflow_count)
 {
-    if (list && threadIdx.x == 0) *list = 0;
     __shared__ uint32_t warp_sums[32];
     const uint32_t chunk = (nb + 1023u) / 1024u;
     const uint32_t begin = threadIdx.x * chunk, end = min(begin + chunk, nb);
     uint32_t local = 0;
     for (uint32_t i = begin; i < end; ++i) local += block_sums[i];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t incl = local;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += u;
-    }
-    if (lane == 31) warp_sums[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t w = warp_sums[lane];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t u = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += u;
-        }
-        warp_sums[lane] = w;
-    }
-    __syncthreads();
-    uint32_t run = incl - local + (warp ? warp_sums[warp - 1] : 0u);
+    uint32_t off = block_scan(local, warp_sums);
     for (uint32_t i = begin; i < end; ++i) {
-        const uint32_t v = block_sums[i];
-        block_sums[i] = run;
-        run += v;
+        const uint32_t c = block_sums[i];
+        block_sums[i] = off;
+        off += c;
+    }
+    if (threadIdx.x == 0) {
+        if (list) *list = 0;
+        if (overflow_count) *overflow_count = 0;
     }
 }
 
@@ -1067,14 +1078,22 @@ __global__ void __launch_bounds__(256) k_d_place(DenseArgs D, uint32_t n, const 
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t head, len;
     slot_run(s, lane, head, len);
-    uint32_t b = 0;
-    if (lane == head && s != kNoSlot) b = atomicAdd(start + s, len);
+    uint32_t b = 0, offs = 0;
+    bool buckets = false;
+    if (lane == head && s != kNoSlot) {
+        b = atomicAdd(start + s, len);
+        offs = __ldg(block_offs + s / kScanItems);
+        // (no crossing has marked a row dirty while flag[0] is 0)
+        if (D.list_blocks) buckets = s == D.total || __ldg(D.clean + s) != 0 || (D.flag[0] && D.dirty[s] != 0);
+        b += offs;
+    }
     b = __shfl_sync(0xffffffffu, b, head);
-    if (s == kNoSlot) return;
     uint32_t o = t;
-    if (D.list_blocks)
-        o = list_bucket_walker(D, t, s == D.total || __ldg(D.clean + s) != 0 || D.dirty[s] != 0);
-    order[__ldg(block_offs + s / kScanItems) + b + (lane - head)] = o;
+    if (D.list_blocks) {
+        const uint32_t listed = __ballot_sync(0xffffffffu, buckets);
+        if (listed) o = list_bucket_walker(D, t, (listed >> head) & 1u);
+    }
+    if (s != kNoSlot) order[b + (lane - head)] = o;
 }
 
 // ---- relabelling of one scene by counting -----------------------------------------------
@@ -1102,7 +1121,7 @@ __global__ void __launch_bounds__(256) k_d_relabel_place(uint32_t n, const uint3
                                                          const uint32_t* __restrict__ start,
                                                          const uint32_t* __restrict__ block_offs, uint32_t overflow,
                                                          uint32_t* __restrict__ overflow_count,
-                                                         uint32_t* __restrict__ order, uint32_t* __restrict__ sorted_keys)
+                                                         uint32_t* __restrict__ order)
 {
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += stride) {
@@ -1117,7 +1136,6 @@ __global__ void __launch_bounds__(256) k_d_relabel_place(uint32_t n, const uint3
         }
         const uint32_t t = __ldg(block_offs + k / kScanItems) + __ldg(start + k) + r;
         order[t] = s;
-        sorted_keys[t] = k;
     }
 }
 
@@ -1129,6 +1147,11 @@ template <bool B>
 __global__ void __launch_bounds__(kDThreads, 10) k_d_lambda(DevParams P0, DenseArgs D0, const float4* __restrict__ lx_in,
                                                             float4* __restrict__ lx_out, float* __restrict__ lrho)
 {
+    // the slot counts the delta-p pass of this iteration adds to (its
+    // clearing launch saved: the stores are not waited for)
+    if (D0.clear_cnt)
+        for (uint32_t g = blockIdx.x * kDThreads + threadIdx.x; g <= D0.total; g += gridDim.x * kDThreads)
+            D0.clear_cnt[g] = 0;
     const PassLabel L = pass_label<B>(D0, P0.n);
     if (!L.live) return;
     const int t = L.t;
@@ -1339,9 +1362,15 @@ void launch_d_clean(const DenseArgs& D, uint32_t mask, uint16_t* clean, uint32_t
     PBF_DENSE_LAUNCH(k_d_clean, capped_grid(D.total, 128, sms, 16), 128, D, mask, clean, unclean);
 }
 
-void launch_d_runs(const DenseArgs& D, const int2* cells, int2* runs, int sms, cudaStream_t st)
+void launch_d_runs(const DenseArgs& D, const uint32_t* start, const uint32_t* block_sums, int2* runs, int sms,
+                   cudaStream_t st)
 {
-    PBF_DENSE_LAUNCH(k_d_runs, capped_grid(D.total, 256, sms, 8), 256, D, cells, runs);
+    k_d_runs<<<capped_grid(D.total, 256, sms, 8), 256, 0, st>>>(D, start, block_sums, runs);
+}
+
+void launch_d_runs_batch(const DenseArgs& D, const int2* cells, int2* runs, int sms, cudaStream_t st)
+{
+    k_d_runs_batch<<<capped_grid(D.total, 256, sms, 8), 256, 0, st>>>(D, cells, runs);
 }
 
 void launch_d_dcol(const DenseArgs& D, uint32_t mask, uint8_t* dcol, int sms, cudaStream_t st)
@@ -1351,45 +1380,43 @@ void launch_d_dcol(const DenseArgs& D, uint32_t mask, uint8_t* dcol, int sms, cu
 
 uint32_t order_scan_blocks(uint32_t slots) { return (slots + 1u + kScanItems - 1u) / kScanItems; }
 
+static void launch_d_scan(const DenseArgs& D, uint32_t m, uint32_t* cnt, uint32_t* block_sums, uint32_t* overflow_count,
+                          cudaStream_t st)
+{
+    const uint32_t nb = order_scan_blocks(m - 1u);
+    k_d_scan_blocks<<<nb, 1024, 0, st>>>(cnt, m, block_sums);
+    k_d_scan_sums<<<1, 1024, 0, st>>>(block_sums, nb, D.list, overflow_count);
+}
+
 void launch_d_order(const DevParams& P, const DenseArgs& D, const float4* X, uint32_t* slot_of, uint32_t* cnt,
                     uint32_t* block_sums, uint32_t* order, cudaStream_t st, uint64_t* launches)
 {
-    const uint32_t m = D.total + 1u;  // slots + the outside slot
-    const uint32_t nb = order_scan_blocks(D.total);
-    cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * m, st);
-    const unsigned g = (P.n + 255u) / 256u;
-    PBF_DENSE_LAUNCH(k_d_cslot, g, 256, P, D, X, slot_of, cnt);
-    k_d_scan_blocks<<<nb, 1024, 0, st>>>(cnt, m, block_sums);
-    k_d_scan_sums<<<1, 1024, 0, st>>>(block_sums, nb, D.list);
-    k_d_place<<<g, 256, 0, st>>>(D, P.n, slot_of, cnt, block_sums, order);
-    *launches += 4;
+    cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * (D.total + 1u), st);
+    PBF_DENSE_LAUNCH(k_d_cslot, (P.n + 255u) / 256u, 256, P, D, X, slot_of, cnt);
+    ++*launches;
+    launch_d_order_recorded(P, D, slot_of, cnt, block_sums, order, st, launches);
 }
 
-void launch_d_relabel(const DenseArgs& D, uint32_t n, uint32_t slots, const uint32_t* dkey, const uint32_t* skeys, uint32_t* cnt,
-                      uint32_t* block_sums, uint32_t* overflow_count, uint32_t* order, uint32_t* sorted_keys, int sms,
+void launch_d_relabel(const DenseArgs& D, uint32_t n, uint32_t slots, const uint32_t* dkey, const uint32_t* skeys,
+                      uint32_t* cnt, uint32_t* block_sums, uint32_t* overflow_count, uint32_t* order, int sms,
                       cudaStream_t st, uint64_t* launches)
 {
     const uint32_t m = slots + 1u;  // window slots + the overflow slot
-    const uint32_t nb = order_scan_blocks(slots);
     cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * m, st);
-    cudaMemsetAsync(overflow_count, 0, sizeof(uint32_t), st);
     k_d_relabel_count<<<(n + 255u) / 256u, 256, 0, st>>>(n, dkey, cnt);
-    k_d_scan_blocks<<<nb, 1024, 0, st>>>(cnt, m, block_sums);
-    k_d_scan_sums<<<1, 1024, 0, st>>>(block_sums, nb, D.list);
+    launch_d_scan(D, m, cnt, block_sums, overflow_count, st);
+    *launches += 3;
+    if (!order) return;
     k_d_relabel_place<<<capped_grid(n, 256, sms, 8), 256, 0, st>>>(n, dkey, skeys, cnt, block_sums, slots,
-                                                                  overflow_count, order, sorted_keys);
-    *launches += 4;
+                                                                  overflow_count, order);
+    ++*launches;
 }
 
 void launch_d_order_recorded(const DevParams& P, const DenseArgs& D, const uint32_t* slot_of, uint32_t* cnt,
                              uint32_t* block_sums, uint32_t* order, cudaStream_t st, uint64_t* launches)
 {
-    const uint32_t m = D.total + 1u;
-    const uint32_t nb = order_scan_blocks(D.total);
-    const unsigned g = (P.n + 255u) / 256u;
-    k_d_scan_blocks<<<nb, 1024, 0, st>>>(cnt, m, block_sums);
-    k_d_scan_sums<<<1, 1024, 0, st>>>(block_sums, nb, D.list);
-    k_d_place<<<g, 256, 0, st>>>(D, P.n, slot_of, cnt, block_sums, order);
+    launch_d_scan(D, D.total + 1u, cnt, block_sums, nullptr, st);  // slots + the outside slot
+    k_d_place<<<(P.n + 255u) / 256u, 256, 0, st>>>(D, P.n, slot_of, cnt, block_sums, order);
     *launches += 3;
 }
 

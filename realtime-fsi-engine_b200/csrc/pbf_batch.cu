@@ -365,7 +365,6 @@ DenseArgs pbf_batch::dense_args() const
 {
     DenseArgs D;
     std::memset(&D, 0, sizeof(D));
-    D.table = dtable;
     D.runs = druns;
     D.hm = dhm;
     D.hcnt = dhcnt;
@@ -400,11 +399,9 @@ int pbf_batch::dense_step_body()
     const uint32_t iters = cfg.solver_iterations;
     const bool vort = cfg.enable_vorticity;
     DenseArgs D = dense_args();
-    auto record = [&]() -> int {
-        BCK(cudaMemsetAsync(dcnt, 0, sizeof(uint32_t) * ((size_t)T + 1), stream));
+    auto record = [&]() {
         D.rec_slot = dslot;
         D.rec_cnt = dcnt;
-        return PBF_OK;
     };
     auto order_recorded = [&]() {
         launch_d_order_recorded(P, D, dslot, dcnt, dbsum, dord, stream, &launches);
@@ -425,7 +422,7 @@ int pbf_batch::dense_step_body()
         launch_d_permute(P, D, lorder, ids, skeys, pos, vel, lx[0], lxb, lv, lx0, lid, lkey, inv, nullptr, sms, stream);
         BCK(cudaMemsetAsync(dtable, 0xFF, sizeof(int2) * (size_t)T, stream));
         launch_build_table(n, msorted, dtable, sms, stream);
-        launch_d_runs(D, dtable, druns, sms, stream);
+        launch_d_runs_batch(D, dtable, druns, sms, stream);
         BCK(cudaMemsetAsync(ddirty, 0, sizeof(uint32_t) * (size_t)T, stream));
         BCK(cudaMemsetAsync(dflag, 0, sizeof(uint32_t), stream));
         launches += 3;
@@ -434,9 +431,10 @@ int pbf_batch::dense_step_body()
             D.rec_cnt = nullptr;
             D.use_list = 0;
             if (it >= 2) order_recorded();
+            D.clear_cnt = dcnt;
             launch_d_lambda(P, D, lx[0], lx[1], lrho, stream);
             D.use_list = 1;
-            if (const int rc = record()) return rc;
+            record();
             launch_d_deltap(P, D, lx[1], lx[0], stream);
             launches += 2;
         }
@@ -445,7 +443,8 @@ int pbf_batch::dense_step_body()
         D.use_list = 0;
         order_recorded();
         if (last && vort) {
-            if (const int rc = record()) return rc;
+            BCK(cudaMemsetAsync(dcnt, 0, sizeof(uint32_t) * ((size_t)T + 1), stream));
+            record();
             // hit masks for the vorticity pass
             BCK(cudaMemsetAsync(dvmark, 0, (size_t)T, stream));
             D.rec_list = 1;

@@ -470,10 +470,10 @@ bool pbf_handle::dense_window(int g0[3], uint32_t nd[3]) const
 DenseArgs pbf_handle::dense_args() const
 {
     DenseArgs D;
-    D.table = dtable;
     D.runs = druns;
     D.order = nullptr;
     D.list = dlist;
+    D.clear_cnt = nullptr;
     D.list_blocks = dense_list_blocks(num_sms, dwin_unclean, (uint64_t)dwin_n[0] * dwin_n[1] * dwin_n[2]);
     D.hm = dhm;
     D.hcnt = dhcnt;
@@ -529,10 +529,10 @@ int pbf_handle::ensure_dense()
                       std::equal(nd, nd + 3, dwin_n);
     if (same) return PBF_OK;
     if (capturing) return set_error(PBF_ERR_INVALID, "dense cell window changed during graph capture");
-    if (slots > cap_slots || !dtable) {
+    if (slots > cap_slots || !druns) {
         cap_slots = 0;
         window_slab.release();
-        window_slab.add(dtable, slots + 1).add(druns, slots).add(dcnt, slots + 1)
+        window_slab.add(druns, slots).add(dcnt, slots + 1)
             .add(dbsum, order_scan_blocks((uint32_t)slots)).add(dclean, slots).add(ddcol, slots).add(ddirty, slots)
             .add(dvmark, slots);
         if ((rc = window_slab.alloc())) return rc;
@@ -599,11 +599,13 @@ int pbf_handle::stage(int st, uint32_t iter)
             else
                 launch_d_order(P, D, X, dslot, dcnt, dbsum, dord, stream, &launches);
             dslot_fresh = false;
+            dcnt_clear = false;
             D.order = dord;
         };
         const size_t slots = (size_t)dwin_n[0] * dwin_n[1] * dwin_n[2];
         auto record_next = [&]() -> int {
-            CK(cudaMemsetAsync(dcnt, 0, sizeof(uint32_t) * (slots + 1), stream));
+            if (!dcnt_clear) CK(cudaMemsetAsync(dcnt, 0, sizeof(uint32_t) * (slots + 1), stream));
+            dcnt_clear = false;
             D.rec_slot = dslot;
             D.rec_cnt = dcnt;
             dslot_fresh = true;
@@ -617,7 +619,10 @@ int pbf_handle::stage(int st, uint32_t iter)
             } else if (dord_iter == 1) {
                 D.order = dord;  // of the reorder stage
             }
+            // (recorded slots that no order took, by stages out of turn, stay)
+            D.clear_cnt = dslot_fresh ? nullptr : dcnt;
             launch_d_lambda(P, D, lx[0], lx[1], lrho, stream);
+            dcnt_clear = !dslot_fresh;
             dlist_iter = (int)iter;
             last_x = 1;
             break;
@@ -707,36 +712,32 @@ int pbf_handle::stage(int st, uint32_t iter)
                 launch_d_keys_pred(P, D, ids, pos, vel, mcode, sms, stream);
             ++launches;
             const uint64_t slots = (uint64_t)dwin_n[0] * dwin_n[1] * dwin_n[2];
-            uint32_t* msorted = mka;
+            dcnt_clear = false;
             if ((uint64_t)derived.hash_size * 64u >= n) {
                 // labels by counting (launch_d_relabel), into the relabelling's sort
                 // buffers; each particle scans the part of its bucket before it, so
                 // the buckets must stay short
                 order = mia;
-                launch_d_relabel(D, n, (uint32_t)slots, mcode, skeys, dcnt, dbsum, dflag + 3, order, msorted, sms,
+                launch_d_relabel(D, n, (uint32_t)slots, mcode, skeys, dcnt, dbsum, dflag + 3, order, sms,
                                  stream, &launches);
             } else {
                 // a hash table far smaller than the particle count: a stable radix
                 // sort of the keys (the overflow key `slots` included)
                 uint32_t bits = 1;
                 while ((1ull << bits) <= slots) ++bits;
+                uint32_t* msorted = nullptr;
                 launch_radix_sort(n, bits, mcode, mka, mia, mkb, mib, hist, totals, &msorted, &order, stream,
                                   &launches);
-                CK(cudaMemsetAsync(dlist, 0, sizeof(uint32_t), stream));
+                launch_d_relabel(D, n, (uint32_t)slots, mcode, skeys, dcnt, dbsum, nullptr, nullptr, sms, stream,
+                                 &launches);
             }
             launch_d_permute(P, D, order, ids, skeys, pos, vel, lx[0], lxb, lv, lx0, lid, lkey, inv, dord, sms, stream);
-            ++launches;
-            // (slot `slots` holds the overflow's labels)
-            CK(cudaMemsetAsync(dtable, 0xFF, sizeof(int2) * (slots + 1), stream));
-            launch_build_table(n, msorted, dtable, sms, stream);
-            launch_d_runs(dense_args(), dtable, druns, sms, stream);
+            launch_d_runs(D, dcnt, dbsum, druns, sms, stream);
             launches += 2;
-            CK(cudaMemsetAsync(ddirty, 0, sizeof(uint32_t) * slots, stream));
             dord_iter = D.list_blocks ? 1 : 0;
             dlist_iter = 0;
             dvlist_ready = false;
             dslot_fresh = false;
-            CK(cudaMemsetAsync(dflag, 0, sizeof(uint32_t), stream));
             label_space = true;
             last_x = 0;
             prof_end(PBF_STAGE_REORDER);

@@ -62,7 +62,6 @@ struct pbf_handle {
     bool label_space = false;    // the current substep's state lives in the label arrays
     uint32_t cap_label_n = 0;
     // mode 8: runs of a dense cell window
-    int2* dtable = nullptr;      // per window slot: label range
     int2* druns = nullptr;       // per window slot: label range of its x-run (slots s-1 .. s+1)
     uint16_t* dclean = nullptr;  // per window slot: rows whose buckets a hash collision near the cell affects
     uint8_t* ddcol = nullptr;    // per window slot: distance to the nearest other cell of its bucket
@@ -72,6 +71,7 @@ struct pbf_handle {
     uint32_t *dslot = nullptr, *dord = nullptr, *dlist = nullptr, *dcnt = nullptr, *dbsum = nullptr;
     uint32_t cap_ord_n = 0;
     int dord_iter = 0;           // solver iteration the order was computed for (0: none)
+    bool dcnt_clear = false;     // dcnt is zero (the lambda pass cleared it)
     bool dslot_fresh = false;    // dslot/dcnt hold the slots of the latest positions (recorded by a pass)
     // lambda hit masks replayed by the delta-p pass of the same iteration
     uint32_t* dhm = nullptr;

@@ -77,6 +77,7 @@ void launch_bucket_sort(const DevParams& P, const SceneDev* scenes, const uint16
 
 // ---- k_dense.cu: x-runs of a dense cell window over relabelled data ----------
 constexpr int kDensePassThreads = 128;
+constexpr uint32_t kDenseScanItems = 4096;  // counters per block of the slot scan
 constexpr int kDenseListWords = 16;
 // The list of bucket walkers (DenseArgs::list): particles per warp, entries
 // that so many blocks take, and the blocks for a window of `slots` cells with
@@ -107,7 +108,6 @@ constexpr int kDenseMargin = 6;
 // cells).  The window fields below describe one window; the passes of a batch
 // replace them, the hash mask, walls and SDF with the scene of each label.
 struct DenseArgs {
-    const int2* table;     // per window slot: label range of its particles, (-1, -1) when empty
     const int2* runs;      // per window slot: label range of slots s-1 .. s+1 of its row
     const uint32_t* order; // pass thread i takes label order[i] (null: label i), unless it is marked as listed
     uint32_t* list;        // one scene (null in a batch): [0] how many listed, [1 ...] the listed labels (those that walk buckets)
@@ -118,7 +118,8 @@ struct DenseArgs {
     int rec_list;          // integrate: record hm/hcnt for the vorticity pass (positions it leaves in place)
     uint8_t* vmark;        // per window slot: a query there sees a particle integrate moved (no replay)
     uint32_t* rec_slot;    // delta-p / integrate (may be null): current slot of each output position
-    uint32_t* rec_cnt;     //   and per-slot counts (zeroed by the caller), for the next pass's order
+    uint32_t* rec_cnt;     //   and per-slot counts (zeroed before), for the next pass's order
+    uint32_t* clear_cnt;   // lambda (may be null): the counts it zeroes for the delta-p pass
     const uint16_t* clean; // per window slot: rows (bit (dz+1)*3+(dy+1)) whose buckets a hash collision near the cell
                            //   affects; 0 = none, 0x1FF at the window's edge
     const uint8_t* dcol;   // per window slot: Chebyshev distance to the nearest other cell of its bucket
@@ -155,7 +156,11 @@ void launch_d_permute(const DevParams& P, const DenseArgs& D, const uint32_t* or
                       cudaStream_t st);
 void launch_d_clean(const DenseArgs& D, uint32_t mask, uint16_t* clean, uint32_t* unclean, int sms, cudaStream_t st);
 void launch_d_dcol(const DenseArgs& D, uint32_t mask, uint8_t* dcol, int sms, cudaStream_t st);
-void launch_d_runs(const DenseArgs& D, const int2* cells, int2* runs, int sms, cudaStream_t st);
+// The runs of one scene from the relabelling's scan (cnt, block_sums), and
+// the substep's dirty rows and crossings cleared; of a batch from its cell table.
+void launch_d_runs(const DenseArgs& D, const uint32_t* cnt, const uint32_t* block_sums, int2* runs, int sms,
+                   cudaStream_t st);
+void launch_d_runs_batch(const DenseArgs& D, const int2* cells, int2* runs, int sms, cudaStream_t st);
 // Labels bucketed by the window slot of their current cell (X) into order[n].
 // Scratch: slot_of[n], cnt[slots + 1], block_sums[order_scan_blocks(slots)].
 uint32_t order_scan_blocks(uint32_t slots);
@@ -163,12 +168,12 @@ void launch_d_order(const DevParams& P, const DenseArgs& D, const float4* X, uin
                     uint32_t* block_sums, uint32_t* order, cudaStream_t st, uint64_t* launches);
 // One scene's relabelling: for the hash-sorted sequence of slot keys dkey[n]
 // (window slots, `slots` for the overflow) with hash keys skeys[n], order[t]
-// = hash-sorted index of label t and sorted_keys[t] its key, as a stable sort
-// by key orders them (the overflow slot's entries in any order).  Scratch:
-// cnt[slots + 1], block_sums[order_scan_blocks(slots)], one overflow counter.
-// Empties D.list, as the orders above and below do.
-void launch_d_relabel(const DenseArgs& D, uint32_t n, uint32_t slots, const uint32_t* dkey, const uint32_t* skeys, uint32_t* cnt,
-                      uint32_t* block_sums, uint32_t* overflow_count, uint32_t* order, uint32_t* sorted_keys, int sms,
+// = hash-sorted index of label t, as a stable sort by key orders them (the overflow slot's entries in any order).  Scratch:
+// cnt, block_sums as above (left holding the labels' starts: slot g's first
+// label is cnt[g] + block_sums[g / kDenseScanItems]), one overflow counter.
+// Empties D.list, as the orders do.  order = null: the counting scan alone.
+void launch_d_relabel(const DenseArgs& D, uint32_t n, uint32_t slots, const uint32_t* dkey, const uint32_t* skeys,
+                      uint32_t* cnt, uint32_t* block_sums, uint32_t* overflow_count, uint32_t* order, int sms,
                       cudaStream_t st, uint64_t* launches);
 // The same order from slots and counts a pass recorded (DenseArgs::rec_slot / rec_cnt).
 void launch_d_order_recorded(const DevParams& P, const DenseArgs& D, const uint32_t* slot_of, uint32_t* cnt,
