@@ -67,6 +67,7 @@
 #include "masked_body.cuh"
 #include "pbf_batch.h"
 #include "pbf_kernels.h"
+#include <algorithm>
 #include <type_traits>
 
 namespace pbf {
@@ -266,40 +267,40 @@ __device__ __forceinline__ PassLabel pass_label(const DenseArgs& D, uint32_t n)
     return {true, false, true, (int)o};
 }
 
-// Label t = hash-sorted index order[t]: its x* (also the predict-time copy),
-// predicted velocity, substep-start position, id and key, gathered from the
-// particle state (the predict pass's arithmetic again), and inv[order[t]] = t.
-// Also the first iteration's thread order: the labels themselves, with those
-// that walk buckets listed (BucketList).
+// Label t = hash-sorted index s, particle id at (p, v): its x* (also the
+// predict-time copy), predicted velocity, substep-start position and id, and
+// inv[s] = t.  Also its entry of the first iteration's thread order, the labels
+// themselves, with those that walk buckets listed.
+__device__ __forceinline__ void write_label(const DevParams& P, const DenseArgs& D, const DenseLabels& L, uint32_t t,
+                                            uint32_t s, uint32_t id, float4 p, float4 v)
+{
+    float3 vp, xs;
+    predict_particle(P, p, v, vp, xs);
+    const float4 x = make_float4(xs.x, xs.y, xs.z, 0.0f);
+    L.x[t] = x;
+    L.xb[t] = x;
+    L.v[t] = make_float4(vp.x, vp.y, vp.z, v.w);
+    L.x0[t] = p;
+    L.id[t] = id;
+    L.inv[s] = t;
+    if (D.list_blocks) {
+        const uint32_t g = current_slot(P, D, x);
+        L.thread_order[t] = list_bucket_walker(D, t, g == D.total || __ldg(D.clean + g) != 0);
+    }
+}
+
+// The labels in the order of a sort: label t is hash-sorted index order[t],
+// gathered from the particle state (the predict pass's arithmetic again).
 __global__ void __launch_bounds__(256) k_d_permute(DevParams P, DenseArgs D, const uint32_t* __restrict__ order,
                                                    const uint32_t* __restrict__ ids,
-                                                   const uint32_t* __restrict__ skeys,
                                                    const float4* __restrict__ pos, const float4* __restrict__ vel,
-                                                   float4* __restrict__ lx, float4* __restrict__ lxb,
-                                                   float4* __restrict__ lv, float4* __restrict__ lx0,
-                                                   uint32_t* __restrict__ lid, uint32_t* __restrict__ lkey,
-                                                   uint32_t* __restrict__ inv, uint32_t* __restrict__ thread_order)
+                                                   DenseLabels L)
 {
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < P.n; t += stride) {
         const uint32_t s = __ldg(order + t);
         const uint32_t id = __ldg(ids + s);
-        const float4 p = __ldg(pos + id);
-        const float4 v = __ldg(vel + id);
-        float3 vp, xs;
-        predict_particle(P, p, v, vp, xs);
-        const float4 x = make_float4(xs.x, xs.y, xs.z, 0.0f);
-        lx[t] = x;
-        lxb[t] = x;
-        lv[t] = make_float4(vp.x, vp.y, vp.z, v.w);
-        lx0[t] = p;
-        lid[t] = id;
-        lkey[t] = __ldg(skeys + s);
-        inv[s] = t;
-        if (D.list_blocks) {
-            const uint32_t g = current_slot(P, D, x);
-            thread_order[t] = list_bucket_walker(D, t, g == D.total || __ldg(D.clean + g) != 0);
-        }
+        write_label(P, D, L, t, s, id, __ldg(pos + id), __ldg(vel + id));
     }
 }
 
@@ -365,16 +366,26 @@ __global__ void __launch_bounds__(128) k_d_clean(DenseArgs D0, uint32_t mask0, u
 // first(g + 1) - 1.  Also clears the substep's dirty rows and crossings.
 constexpr uint32_t kScanItems = kDenseScanItems;
 
-__global__ void __launch_bounds__(256) k_d_runs(DenseArgs D, const uint32_t* __restrict__ start,
-                                                const uint32_t* __restrict__ block_offs, int2* __restrict__ runs)
+// Starts left by a counting scan: entry `base` + g begins at first(g).
+struct SlotScan {
+    const uint32_t* __restrict__ start;
+    const uint32_t* __restrict__ block_offs;
+    uint32_t base, before;  // entries ahead of these, and what they counted
+    __device__ __forceinline__ uint32_t first(uint32_t g) const
+    {
+        return __ldg(block_offs + (base + g) / kScanItems) + __ldg(start + base + g) - before;
+    }
+};
+
+// (scan: the slots' starts less the entries before them)
+__global__ void __launch_bounds__(256) k_d_runs(DenseArgs D, SlotScan scan, int2* __restrict__ runs)
 {
     if (blockIdx.x == 0 && threadIdx.x == 0) D.flag[0] = 0;
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < D.total; g += stride) {
         const uint32_t ux = g % D.nx;
-        const auto first = [&](uint32_t q) { return __ldg(block_offs + q / kScanItems) + __ldg(start + q); };
         int2 r = make_int2(0, 0);
-        if (ux >= 1 && ux + 1 < D.nx) r = make_int2((int)first(g - 1), (int)first(g + 2));
+        if (ux >= 1 && ux + 1 < D.nx) r = make_int2((int)scan.first(g - 1), (int)scan.first(g + 2));
         runs[g] = r;
         D.dirty[g] = 0;
     }
@@ -1139,6 +1150,75 @@ __global__ void __launch_bounds__(256) k_d_relabel_place(uint32_t n, const uint3
     }
 }
 
+// ---- one scene's predict, hash sort, cell table and relabelling ----------------------------
+// As k_bucket.cu sorts a small scene: count, scan, place in order of arrival,
+// rank by id within the bucket; the buckets' and the window slots' counts are
+// scanned as one array.  A particle's label is its slot's start plus the
+// smaller ids of its slot, all of them in its bucket (the overflow slot's
+// particles take any order, as in the relabelling above).  Seven launches
+// and one gather of the state, where predict, a radix sort of nine launches,
+// the table, the relabelling and the gather took 19.
+// cnt: buckets (to a multiple of four), then slots and the overflow slot.
+__global__ void __launch_bounds__(256) k_d_sort_count(DevParams P, DenseArgs D, const float4* __restrict__ pos,
+                                                      const float4* __restrict__ vel, uint32_t slot_base,
+                                                      uint32_t* __restrict__ keys, uint32_t* __restrict__ dkey_id,
+                                                      uint32_t* __restrict__ arrival, uint32_t* __restrict__ cnt)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= P.n) return;
+    float3 vp, xs;
+    predict_particle(P, __ldg(pos + i), __ldg(vel + i), vp, xs);
+    const int cx = cell_coord(xs.x, P.h), cy = cell_coord(xs.y, P.h), cz = cell_coord(xs.z, P.h);
+    const uint32_t k = grid_hash(cx, cy, cz, P.mask), w = scene_key(D, cx, cy, cz);
+    keys[i] = k;
+    dkey_id[i] = w;
+    arrival[i] = atomicAdd(cnt + k, 1u);
+    atomicAdd(cnt + slot_base + w, 1u);
+}
+
+// The cell table, the buckets' particles (id, slot) in order of arrival, and the
+// sorted keys (every place of a bucket has its key).
+__global__ void __launch_bounds__(256) k_d_sort_place(uint32_t n, uint32_t buckets, SlotScan bucket,
+                                                      const uint32_t* __restrict__ keys,
+                                                      const uint32_t* __restrict__ dkey_id,
+                                                      const uint32_t* __restrict__ arrival, int2* __restrict__ table,
+                                                      uint2* __restrict__ arrived, uint32_t* __restrict__ skeys)
+{
+    const uint32_t stride = gridDim.x * blockDim.x, first = blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint32_t i = first; i < n; i += stride) {
+        const uint32_t k = __ldg(keys + i), q = bucket.first(k) + __ldg(arrival + i);
+        arrived[q] = make_uint2(i, __ldg(dkey_id + i));
+        skeys[q] = k;
+    }
+    for (uint32_t k = first; k < buckets; k += stride) {
+        const int b = (int)bucket.first(k), e = (int)bucket.first(k + 1u);
+        table[k] = b < e ? make_int2(b, e) : make_int2(-1, -1);
+    }
+}
+
+__global__ void __launch_bounds__(256) k_d_sort_rank(DevParams P, DenseArgs D, SlotScan slot,
+                                                     const uint2* __restrict__ arrived,
+                                                     const uint32_t* __restrict__ skeys, const int2* __restrict__ table,
+                                                     const float4* __restrict__ pos, const float4* __restrict__ vel,
+                                                     uint32_t* __restrict__ overflow_count, uint32_t* __restrict__ ids,
+                                                     DenseLabels L)
+{
+    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= P.n) return;
+    const uint2 me = __ldg(arrived + q);
+    const float4 p = __ldg(pos + me.x), v = __ldg(vel + me.x);
+    const int2 se = __ldg(table + __ldg(skeys + q));
+    uint32_t s = (uint32_t)se.x, r = 0;
+    for (int x = se.x; x < se.y; ++x) {
+        const uint2 o = __ldg(arrived + x);
+        s += o.x < me.x ? 1u : 0u;
+        r += o.x < me.x && o.y == me.y ? 1u : 0u;
+    }
+    if (me.y == D.total) r = atomicAdd(overflow_count, 1u);
+    ids[s] = me.x;
+    write_label(P, D, L, slot.first(me.y) + r, s, me.x, p, v);
+}
+
 // 10 resident blocks (48 registers, 8 bytes spilled): with the s_corr sum of
 // the delta-p pass in its pair body, 12 blocks (40 registers, 132 bytes
 // spilled) took 1.225 ms per 4M launch against 1.165.  The pass also writes
@@ -1349,12 +1429,10 @@ void launch_d_keys_gather(uint32_t n, const uint32_t* ids, const uint32_t* dkey_
     k_d_keys_gather<<<capped_grid(n, 256, sms, 8), 256, 0, st>>>(n, ids, dkey_id, dkey);
 }
 
-void launch_d_permute(const DevParams& P, const DenseArgs& D, const uint32_t* order, const uint32_t* ids, const uint32_t* skeys,
-                      const float4* pos, const float4* vel, float4* lx, float4* lxb, float4* lv, float4* lx0,
-                      uint32_t* lid, uint32_t* lkey, uint32_t* inv, uint32_t* thread_order, int sms, cudaStream_t st)
+void launch_d_permute(const DevParams& P, const DenseArgs& D, const uint32_t* order, const uint32_t* ids,
+                      const float4* pos, const float4* vel, const DenseLabels& L, int sms, cudaStream_t st)
 {
-    k_d_permute<<<capped_grid(P.n, 256, sms, 8), 256, 0, st>>>(P, D, order, ids, skeys, pos, vel, lx, lxb, lv, lx0, lid,
-                                                               lkey, inv, thread_order);
+    k_d_permute<<<capped_grid(P.n, 256, sms, 8), 256, 0, st>>>(P, D, order, ids, pos, vel, L);
 }
 
 void launch_d_clean(const DenseArgs& D, uint32_t mask, uint16_t* clean, uint32_t* unclean, int sms, cudaStream_t st)
@@ -1362,10 +1440,10 @@ void launch_d_clean(const DenseArgs& D, uint32_t mask, uint16_t* clean, uint32_t
     PBF_DENSE_LAUNCH(k_d_clean, capped_grid(D.total, 128, sms, 16), 128, D, mask, clean, unclean);
 }
 
-void launch_d_runs(const DenseArgs& D, const uint32_t* start, const uint32_t* block_sums, int2* runs, int sms,
+void launch_d_runs(const DenseArgs& D, const uint32_t* cnt, const uint32_t* block_sums, int2* runs, int sms,
                    cudaStream_t st)
 {
-    k_d_runs<<<capped_grid(D.total, 256, sms, 8), 256, 0, st>>>(D, start, block_sums, runs);
+    k_d_runs<<<capped_grid(D.total, 256, sms, 8), 256, 0, st>>>(D, SlotScan{cnt, block_sums, 0, 0}, runs);
 }
 
 void launch_d_runs_batch(const DenseArgs& D, const int2* cells, int2* runs, int sms, cudaStream_t st)
@@ -1418,6 +1496,28 @@ void launch_d_order_recorded(const DevParams& P, const DenseArgs& D, const uint3
     launch_d_scan(D, D.total + 1u, cnt, block_sums, nullptr, st);  // slots + the outside slot
     k_d_place<<<(P.n + 255u) / 256u, 256, 0, st>>>(D, P.n, slot_of, cnt, block_sums, order);
     *launches += 3;
+}
+
+static uint32_t dense_sort_base(uint32_t buckets) { return (buckets + 3u) / 4u * 4u; }
+size_t dense_sort_counts(uint32_t buckets, uint32_t slots) { return (size_t)dense_sort_base(buckets) + slots + 1u; }
+size_t dense_sort_sums(uint32_t buckets, uint32_t slots) { return order_scan_blocks(dense_sort_base(buckets) + slots); }
+
+void launch_d_sort(const DevParams& P, const DenseArgs& D, const float4* pos, const float4* vel, uint32_t buckets,
+                   uint32_t* keys, uint32_t* dkey_id, uint32_t* arrival, uint32_t* cnt, uint32_t* block_sums,
+                   uint32_t* overflow_count, uint2* arrived, int2* table, uint32_t* ids, uint32_t* skeys,
+                   const DenseLabels& L, int2* runs, int sms, cudaStream_t st, uint64_t* launches)
+{
+    const uint32_t base = dense_sort_base(buckets), m = base + D.total + 1u;
+    const unsigned g = (P.n + 255u) / 256u;
+    cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * m, st);
+    k_d_sort_count<<<g, 256, 0, st>>>(P, D, pos, vel, base, keys, dkey_id, arrival, cnt);
+    launch_d_scan(D, m, cnt, block_sums, overflow_count, st);
+    k_d_sort_place<<<capped_grid(std::max(P.n, buckets), 256, sms, 8), 256, 0, st>>>(
+        P.n, buckets, SlotScan{cnt, block_sums, 0, 0}, keys, dkey_id, arrival, table, arrived, skeys);
+    const SlotScan slot{cnt, block_sums, base, P.n};
+    k_d_sort_rank<<<g, 256, 0, st>>>(P, D, slot, arrived, skeys, table, pos, vel, overflow_count, ids, L);
+    k_d_runs<<<capped_grid(D.total, 256, sms, 8), 256, 0, st>>>(D, slot, runs);
+    *launches += 6;
 }
 
 void launch_d_lambda(const DevParams& P, const DenseArgs& D, const float4* lx_in, float4* lx_out, float* lrho,

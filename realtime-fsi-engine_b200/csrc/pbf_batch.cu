@@ -333,7 +333,7 @@ int pbf_batch::dense_setup()
     const size_t c = std::max<uint32_t>(n, 1u), cp = c + kLabelPad, T = (size_t)dense_total;
     if (!lx[0]) {
         label_slab.add(lx[0], cp).add(lx[1], cp).add(lxb, c).add(lv, cp).add(lx0, cp).add(lom, cp).add(lrho, c).add(lid, c)
-            .add(lkey, c).add(inv, c).add(dslot, c).add(dord, c).add(dhm, c * kDenseListWords).add(dhcnt, c).add(dflag, 4);
+            .add(inv, c).add(dslot, c).add(dord, c).add(dhm, c * kDenseListWords).add(dhcnt, c).add(dflag, 4);
         if ((rc = label_slab.alloc())) return rc;
     }
     window_slab.release();
@@ -419,7 +419,7 @@ int pbf_batch::dense_step_body()
         uint32_t *msorted = nullptr, *lorder = nullptr;
         launch_radix_sort(n, slot_bits, mcode, mka, mia, mkb, mib, hist, totals, &msorted, &lorder, stream,
                           &launches);
-        launch_d_permute(P, D, lorder, ids, skeys, pos, vel, lx[0], lxb, lv, lx0, lid, lkey, inv, nullptr, sms, stream);
+        launch_d_permute(P, D, lorder, ids, pos, vel, DenseLabels{lx[0], lxb, lv, lx0, lid, inv, nullptr}, sms, stream);
         BCK(cudaMemsetAsync(dtable, 0xFF, sizeof(int2) * (size_t)T, stream));
         launch_build_table(n, msorted, dtable, sms, stream);
         launch_d_runs_batch(D, dtable, druns, sms, stream);

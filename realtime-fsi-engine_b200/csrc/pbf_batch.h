@@ -166,7 +166,7 @@ struct pbf_batch {
     bool dense_ready = false;     // the clean/dcol tables below match `win` and the hash masks
     float4 *lx[2] = {nullptr, nullptr}, *lxb = nullptr, *lv = nullptr, *lx0 = nullptr, *lom = nullptr;
     float* lrho = nullptr;
-    uint32_t *lid = nullptr, *lkey = nullptr, *inv = nullptr;
+    uint32_t *lid = nullptr, *inv = nullptr;
     int2 *dtable = nullptr, *druns = nullptr;
     uint16_t* dclean = nullptr;
     uint32_t* ddirty = nullptr;

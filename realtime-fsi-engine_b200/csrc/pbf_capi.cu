@@ -347,6 +347,7 @@ pbf_handle::~pbf_handle()
     label_slab.release();
     order_slab.release();
     window_slab.release();
+    sort_slab.release();
     dfree(query_buf); dfree(bcnt); dfree(totals); dfree(table); dfree(scalars); dfree(dflag);
     dfree(grid); dfree(slab_min);
     mesh_free();
@@ -436,7 +437,7 @@ int pbf_handle::ensure_label_capacity()
         cap_label_n = 0;
         label_slab.release();
         label_slab.add(lx[0], cp).add(lx[1], cp).add(lxb, c).add(lv, cp).add(lx0, cp).add(lom, cp).add(lrho, c).add(lid, c)
-            .add(lkey, c).add(inv, c).add(dkey_id, c);
+            .add(inv, c).add(dkey_id, c);
         if ((rc = label_slab.alloc())) return rc;
         dkey_valid = false;
         cap_label_n = (uint32_t)c;
@@ -525,6 +526,15 @@ int pbf_handle::ensure_dense()
     uint32_t nd[3];
     if (!dense_window(g0, nd)) return set_error(PBF_ERR_INVALID, "dense cell window larger than 2^26 cells");
     const size_t slots = (size_t)nd[0] * nd[1] * nd[2];
+    const size_t counts = dense_sort_counts(derived.hash_size, (uint32_t)slots);
+    if (n <= kDenseSortMax && counts > cap_dsort) {
+        if (capturing) return set_error(PBF_ERR_INVALID, "dense cell window changed during graph capture");
+        cap_dsort = 0;
+        sort_slab.release();
+        sort_slab.add(dsort, counts).add(dsort_sums, dense_sort_sums(derived.hash_size, (uint32_t)slots));
+        if ((rc = sort_slab.alloc())) return rc;
+        cap_dsort = counts;
+    }
     const bool same = dwin_ready && dwin_mask == derived.hash_size - 1 && std::equal(g0, g0 + 3, dwin_g0) &&
                       std::equal(nd, nd + 3, dwin_n);
     if (same) return PBF_OK;
@@ -550,6 +560,20 @@ int pbf_handle::ensure_dense()
     CK(cudaStreamSynchronize(stream));
     dwin_ready = true;
     return PBF_OK;
+}
+
+DenseLabels pbf_handle::dense_labels() const { return {lx[0], lxb, lv, lx0, lid, inv, dord}; }
+
+// The state of a substep whose labels have just been written.
+void pbf_handle::dense_begin(const DenseArgs& D)
+{
+    dord_iter = D.list_blocks ? 1 : 0;
+    dlist_iter = 0;
+    dvlist_ready = false;
+    dslot_fresh = false;
+    dcnt_clear = false;
+    label_space = true;
+    last_x = 0;
 }
 
 // Sorted-order buffers are kept in label order in mode 8: gather the one asked
@@ -712,8 +736,7 @@ int pbf_handle::stage(int st, uint32_t iter)
                 launch_d_keys_pred(P, D, ids, pos, vel, mcode, sms, stream);
             ++launches;
             const uint64_t slots = (uint64_t)dwin_n[0] * dwin_n[1] * dwin_n[2];
-            dcnt_clear = false;
-            if ((uint64_t)derived.hash_size * 64u >= n) {
+            if (short_buckets()) {
                 // labels by counting (launch_d_relabel), into the relabelling's sort
                 // buffers; each particle scans the part of its bucket before it, so
                 // the buckets must stay short
@@ -731,15 +754,10 @@ int pbf_handle::stage(int st, uint32_t iter)
                 launch_d_relabel(D, n, (uint32_t)slots, mcode, skeys, dcnt, dbsum, nullptr, nullptr, sms, stream,
                                  &launches);
             }
-            launch_d_permute(P, D, order, ids, skeys, pos, vel, lx[0], lxb, lv, lx0, lid, lkey, inv, dord, sms, stream);
+            launch_d_permute(P, D, order, ids, pos, vel, dense_labels(), sms, stream);
             launch_d_runs(D, dcnt, dbsum, druns, sms, stream);
             launches += 2;
-            dord_iter = D.list_blocks ? 1 : 0;
-            dlist_iter = 0;
-            dvlist_ready = false;
-            dslot_fresh = false;
-            label_space = true;
-            last_x = 0;
+            dense_begin(D);
             prof_end(PBF_STAGE_REORDER);
             break;
         }
@@ -819,6 +837,19 @@ int pbf_handle::sort_stages()
         label_space = false;
         chit_iter = 0;
         last_x = 0;
+        return PBF_OK;
+    }
+    if (effective_mode() == 8 && n <= kDenseSortMax && short_buckets() && !profiling) {
+        if (const int rc = ensure_dense()) return rc;
+        const DenseArgs D = dense_args();
+        dkey_valid = false;
+        order = nullptr;
+        // (the scratch of the particles in order of arrival: the lambda pass's output)
+        launch_d_sort(dev_params(), D, pos, vel, derived.hash_size, keys, dkey_id, mka, dsort, dsort_sums, dflag + 3,
+                      reinterpret_cast<uint2*>(lx[1]), table, ia, ka, dense_labels(), druns, num_sms, stream, &launches);
+        skeys = ka;
+        ids = ia;
+        dense_begin(D);
         return PBF_OK;
     }
     for (const int st : {PBF_STAGE_PREDICT, PBF_STAGE_SORT, PBF_STAGE_TABLE, PBF_STAGE_REORDER})

@@ -29,8 +29,8 @@ struct pbf_handle {
     uint32_t n = 0, cap_n = 0, cap_h = 0;
 
     // owners of the arrays below: per particle; the small scenes' hits; mode 8's
-    // labels, thread orders and window
-    pbf::Slab particle_slab, hit_slab, label_slab, order_slab, window_slab;
+    // labels, thread orders, window and sort
+    pbf::Slab particle_slab, hit_slab, label_slab, order_slab, window_slab, sort_slab;
 
     // particle order
     float4* pos = nullptr;
@@ -58,7 +58,7 @@ struct pbf_handle {
     // mode 8: the per-particle arrays relabelled by window slot
     float4 *lx[2] = {nullptr, nullptr}, *lxb = nullptr, *lv = nullptr, *lx0 = nullptr, *lom = nullptr;
     float* lrho = nullptr;
-    uint32_t *lid = nullptr, *lkey = nullptr, *inv = nullptr;
+    uint32_t *lid = nullptr, *inv = nullptr;
     bool label_space = false;    // the current substep's state lives in the label arrays
     uint32_t cap_label_n = 0;
     // mode 8: runs of a dense cell window
@@ -97,6 +97,14 @@ struct pbf_handle {
     bool dense_window(int g0[3], uint32_t nd[3]) const;
     int ensure_dense();
     pbf::DenseArgs dense_args() const;
+    pbf::DenseLabels dense_labels() const;
+    void dense_begin(const pbf::DenseArgs& D);
+    // Buckets short enough that a particle may read its own whole (the sort and
+    // the relabelling by counting).
+    bool short_buckets() const { return (uint64_t)derived.hash_size * 64u >= n; }
+    // counts of mode 8's sort (launch_d_sort)
+    uint32_t *dsort = nullptr, *dsort_sums = nullptr;
+    size_t cap_dsort = 0;
     int effective_mode() const;
     int ensure_label_capacity();
     int unpermute_for_read(int which);

@@ -148,12 +148,32 @@ void launch_d_predict_hash(const DevParams& P, const DenseArgs& D, const float4*
                            uint32_t* keys, uint32_t* dkey_id, int sms, cudaStream_t st);
 void launch_d_keys_gather(uint32_t n, const uint32_t* ids, const uint32_t* dkey_id, uint32_t* dkey, int sms,
                           cudaStream_t st);
-// thread_order[n]: the first iteration's order, where the bucket walkers are
-// listed (D.list empty on entry).
+// The label-order arrays, and the hash-sorted index -> label map.
+struct DenseLabels {
+    float4 *x, *xb, *v, *x0;  // x* (twice), predicted velocity, substep-start position
+    uint32_t *id, *inv;
+    uint32_t* thread_order;   // one scene: the first iteration's order, where bucket walkers are listed (D.list
+                              //   empty on entry)
+};
 void launch_d_permute(const DevParams& P, const DenseArgs& D, const uint32_t* order, const uint32_t* ids,
-                      const uint32_t* skeys, const float4* pos, const float4* vel, float4* lx, float4* lxb, float4* lv,
-                      float4* lx0, uint32_t* lid, uint32_t* lkey, uint32_t* inv, uint32_t* thread_order, int sms,
-                      cudaStream_t st);
+                      const float4* pos, const float4* vel, const DenseLabels& L, int sms, cudaStream_t st);
+// One scene's substep from the particle state to the runs: what predict, hash
+// sort, table, relabelling, launch_d_permute and launch_d_runs leave, to the
+// bit (the overflow slot's labels in any order).  A particle reads its whole
+// bucket, so the buckets must stay short.  Up to kDenseSortMax particles: they
+// are written in bucket order, to labels a cell apart, which costs little
+// while they stay in L2 (step of 262,144 particles 1813 -> 1752 us, 602,263
+// 1362 -> 1317, 983,040 2339 -> 2311; but of 1,966,080 4273 -> 4290 and of
+// 4,194,304 8.70 -> 8.86 ms, the write alone 321 us where the gather in label
+// order takes 105).  Scratch: arrival[n], arrived[n], cnt[dense_sort_counts],
+// block_sums[dense_sort_sums].
+constexpr uint32_t kDenseSortMax = 1u << 20;
+size_t dense_sort_counts(uint32_t buckets, uint32_t slots);
+size_t dense_sort_sums(uint32_t buckets, uint32_t slots);
+void launch_d_sort(const DevParams& P, const DenseArgs& D, const float4* pos, const float4* vel, uint32_t buckets,
+                   uint32_t* keys, uint32_t* dkey_id, uint32_t* arrival, uint32_t* cnt, uint32_t* block_sums,
+                   uint32_t* overflow_count, uint2* arrived, int2* table, uint32_t* ids, uint32_t* skeys,
+                   const DenseLabels& L, int2* runs, int sms, cudaStream_t st, uint64_t* launches);
 void launch_d_clean(const DenseArgs& D, uint32_t mask, uint16_t* clean, uint32_t* unclean, int sms, cudaStream_t st);
 void launch_d_dcol(const DenseArgs& D, uint32_t mask, uint8_t* dcol, int sms, cudaStream_t st);
 // The runs of one scene from the relabelling's scan (cnt, block_sums), and

@@ -131,3 +131,35 @@ def test_bucket_walkers_of_a_dense_window(have_gpu, n, fast):
         vel[::3] *= 200.0
     cfg = scenes.base_config(h, h / 2, (box, box, box), 2, 3, 1.0 / 60.0, n, 1 << 16)
     assert same(stepped(cfg, pos, vel, 4), stepped(cfg, pos, vel, 8))
+
+
+@pytest.mark.parametrize("n,hash_size", [(1, 1), (3, 2), (200, 4), (255, 8), (5000, 128), (5000, 1 << 14), (70001, 1 << 17),
+                                         (1 << 20, 1 << 18), ((1 << 20) + 1, 1 << 18)])
+def test_sort_of_a_dense_step_equals_the_stages(have_gpu, n, hash_size):
+    """The same for dense windows (k_d_sort_*), up to one particle more than it
+    takes, with cells outside the window."""
+    cfg, pos, vel = moving_block(n, 0.02, 0.04, n, hash_size)
+    vel[::7] *= 100.0
+    cfg.substep_iterations = 1
+    got = []
+    for stages in (False, True):
+        fl = P.PBFluids(cfg)
+        fl.set_option(1, 8)
+        fl.setParticles(P.make_particles(pos, vel))
+        for _ in range(2):
+            if stages:
+                for st in (P.STAGE_PREDICT, P.STAGE_SORT, P.STAGE_TABLE, P.STAGE_REORDER):
+                    fl.run_stage(st)
+                for it in range(1, cfg.solver_iterations + 1):
+                    fl.run_stage(P.STAGE_LAMBDA, it)
+                    fl.run_stage(P.STAGE_DELTAP, it)
+                fl.run_stage(P.STAGE_INTEGRATE)
+                fl.run_stage(P.STAGE_VORTICITY)
+            else:
+                fl.step()
+        fl.sync()
+        got.append([fl.read_buffer(P.BUF_KEYS, np.uint32, n), fl.read_buffer(P.BUF_SORTED_KEYS, np.uint32, n),
+                    fl.read_buffer(P.BUF_SORTED_IDS, np.uint32, n), fl.read_buffer(P.BUF_TABLE, np.int32, (hash_size, 2)),
+                    fl.read_buffer(P.BUF_XSTAR, np.float32, (n, 4)), fl.readbackParticles()])
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
