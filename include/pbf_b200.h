@@ -313,10 +313,11 @@ int pbf_set_use_graph(pbf_handle* h, int on);
  *                          particle within reach has moved 0.9 h since the
  *                          predict near a colliding cell; the hashed buckets
  *                          elsewhere.  Same pairs, same order as the buckets.
- *                          -1 (default): mode 8 from 2^19 particles, or from
- *                          3 * 2^16 when the window has at most 8 cells per
- *                          particle, mode 4 below (where mode 8's relabelling
- *                          launches cost more than its walk saves); APBF and
+ *                          -1 (default): mode 8 from 2^19 particles, above
+ *                          2^18 when the window has at most 64 cells per
+ *                          particle, from 3 * 2^16 when it has at most 16, else
+ *                          mode 4 (where mode 8's launches and window cost
+ *                          more than its walk saves); APBF and
  *                          windows over 2^26 cells run mode 4.  Modes 4 and 8 give
  *                          bit-identical results (same pairs, order and pair
  *                          arithmetic).  Other values: PBF_ERR_INVALID. */

@@ -410,12 +410,13 @@ int pbf_handle::prof_collect()
 // Mode 8 (dense-window runs) needs label arrays without APBF's per-particle
 // skips and a dense window of the box within 2^26 cells; otherwise the
 // handle runs mode 4 (hashed buckets).  Automatic choice (the default,
-// pass_mode < 0): mode 8 from 2^19 particles, and from 3 * 2^16 where the
-// window has at most 8 cells per particle (its per-substep tables are cleared
-// and scanned whole).  Below, its relabelling launches cost more than its walk
-// saves over mode 4's groups of lanes (k_coop.cu): one step of 151,250
-// particles 1401 us in mode 4 and 1710 in mode 8, 180,000 1653 and 1802,
-// 262,144 2335 and 2202.
+// pass_mode < 0): mode 8 from 2^19 particles, from 2^18 where the window has at
+// most 64 cells per particle and from 3 * 2^16 where it has at most 16 (its
+// per-substep tables are cleared and scanned whole, 44 us a step and million
+// cells).  Below, its launches cost more than its walk saves over mode 4's groups
+// of lanes (k_coop.cu), which end at 2^18.  Steps in mode 4 / mode 8, us:
+// 132,651 particles 1144 / 1276, 195,112 1637 / 1463 (5.9 cells a particle 1496,
+// 22.9 1642), 262,144 2164 / 1709 (17.1: 1898), 373,248 4320 / 2154 (12.0: 2334).
 int pbf_handle::effective_mode() const
 {
     if (pass_mode >= 0 && pass_mode != 8) return pass_mode;
@@ -424,7 +425,7 @@ int pbf_handle::effective_mode() const
     int g0[3];
     uint32_t nd[3];
     if (!dense_window(g0, nd)) return 4;
-    const bool roomy = (uint64_t)nd[0] * nd[1] * nd[2] > 8ull * n;
+    const bool roomy = (uint64_t)nd[0] * nd[1] * nd[2] > (n > (1u << 18) ? 64ull : 16ull) * n;
     return automatic && n < (1u << 19) && roomy ? 4 : 8;
 }
 
