@@ -522,13 +522,95 @@ __device__ __forceinline__ void label_range(const float4* __restrict__ X, float4
             if (ds < (uint32_t)C) mg &= ~(1u << ds);
             const int left = hi - kb;
             if (left < C) mg &= (1u << left) - 1u;
-            rec(mg);
             m |= mg << (g * C);
         }
+        rec(m);
         while (m) {
             const int c = __ffs(m) - 1;
             m &= m - 1u;
             body(k0 + c);
+        }
+    }
+}
+
+// Hits of up to W blocks of 32 consecutive labels, oldest block first, for one
+// drain: a warp runs the pair body as many times as its busiest lane has hits
+// in the W blocks together, which is less than the sum of the busiest lanes of
+// each (a lane has some 4 hits in a block, the busiest of 32 lanes 8 to 9).
+// For the passes that replay masks, whose issue slots these iterations fill: W =
+// 3 (the rows of a plane), 4M particles: delta-p 492 -> 474 us (W = 2: 483, 4:
+// 502, 5: 548), vorticity 568 -> 543.  Not for the passes that test candidates,
+// which wait on L1: lambda 1050 -> 1092, integrate 1290 -> 1476.
+template <int W>
+struct HitBlocks {
+    uint32_t m[W];
+    int k[W];
+    int room = W;  // the same in every lane of the walk
+    __device__ __forceinline__ HitBlocks()
+    {
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+            m[w] = 0;
+            k[w] = 0;
+        }
+    }
+    // the lane's next block (mask 0: none), from label `first`
+    template <class Body>
+    __device__ __forceinline__ void add(uint32_t mask, int first, Body&& body)
+    {
+        if (mask) {
+#pragma unroll
+            for (int w = 0; w + 1 < W; ++w) {
+                m[w] = m[w + 1];
+                k[w] = k[w + 1];
+            }
+            m[W - 1] = mask;
+            k[W - 1] = first;
+        }
+        if (--room == 0) drain(body);
+    }
+    template <class Body>
+    __device__ __forceinline__ void drain(Body&& body)
+    {
+#pragma unroll
+        for (int w = 0; w + 1 < W; ++w) shift();
+        while (m[0]) {
+            const int j = k[0] + __ffs(m[0]) - 1;
+            m[0] &= m[0] - 1u;
+            shift();
+            body(j);
+        }
+        room = W;
+    }
+
+private:
+    __device__ __forceinline__ void shift()
+    {
+        if (m[0] == 0) {
+#pragma unroll
+            for (int w = 0; w + 1 < W; ++w) {
+                m[w] = m[w + 1];
+                k[w] = k[w + 1];
+            }
+            m[W - 1] = 0;
+        }
+    }
+};
+
+// Blocks of 32 candidates each of the nine runs: block(first, end, has) for
+// the lanes' blocks of a row in turn, as often as the longest run among them
+// asks (has = this lane has such a block).
+template <class Block>
+__device__ __forceinline__ void each_block(const int2* __restrict__ runs, int s0, int nx, int nxy, Block&& block)
+{
+#pragma unroll 1
+    for (int dz = -1; dz <= 1; ++dz) {
+#pragma unroll 1
+        for (int dy = -1; dy <= 1; ++dy) {
+            const int2 r = __ldg(runs + s0 + dz * nxy + dy * nx);
+            const int longest = (int)__reduce_max_sync(__activemask(), (uint32_t)(r.y - r.x));
+#pragma unroll 1
+            for (int b = 0; b < longest; b += 32) block(r.x + b, r.y);
         }
     }
 }
@@ -540,6 +622,7 @@ struct InvMap {
 
 // Candidates per hit mask in a run (a run holds about 24).
 constexpr int kRunChunk = 16;
+constexpr int kDrainBlocks = 3;
 static_assert(kRunChunk <= kLabelPad, "a run's last chunk stays inside the padded label arrays");
 
 // The 9 x-runs of a particle whose cell satisfies (a), (b) and (c).
@@ -566,15 +649,13 @@ struct RunWalk {
 
 // Hit masks a lambda pass records for the delta-p pass of the same
 // iteration, which reads the same positions and so walks the same runs in the
-// same chunks and finds the same hits: word w of label t at hm[w * n + t], two
-// 16-bit chunk masks per word in walk order; the chunk count in cnt[t], or
-// kNoList when the particle walked the buckets or had more than kListChunks
-// chunks.  The delta-p pass then tests only the recorded hits (for its own
-// r >= 1e-10 condition) instead of every candidate.
+// same blocks and finds the same hits: word w of label t at hm[w * n + t], one
+// block's mask per word in walk order; the block count in cnt[t], or kNoList
+// when the particle walked the buckets or had more than kListWords blocks.  The
+// delta-p pass then tests only the recorded hits (for its own r >= 1e-10
+// condition) instead of every candidate.
 constexpr int kListWords = kDenseListWords;
-constexpr int kListChunks = 2 * kListWords;
 constexpr uint8_t kNoList = 0xFF;
-static_assert(kRunChunk == 16, "two chunk masks per list word");
 
 struct RunWalkRec {
     const int2* __restrict__ runs;
@@ -585,30 +666,23 @@ struct RunWalkRec {
     int nx, nxy;
     uint32_t* __restrict__ hm;
     uint32_t n;
-    int* chunks;
+    int* blocks;
     template <class Hit, class Body>
     __device__ __forceinline__ void operator()(Hit&& hit, Body&& body) const
     {
         int q = 0;
-        uint32_t word = 0;
 #pragma unroll 1
         for (int dz = -1; dz <= 1; ++dz) {
 #pragma unroll 1
             for (int dy = -1; dy <= 1; ++dy) {
                 const int2 r = __ldg(runs + s0 + dz * nxy + dy * nx);
                 label_range<kRunChunk>(X, xi, self, r.x, r.y, hit, body, [&](uint32_t m) {
-                    if (q < kListChunks) {
-                        if (q & 1)
-                            hm[(size_t)(q >> 1) * n + self] = word | (m << 16);
-                        else
-                            word = m;
-                    }
+                    if (q < kListWords) hm[(size_t)q * n + self] = m;
                     ++q;
                 });
             }
         }
-        if (q <= kListChunks && (q & 1)) hm[(size_t)(q >> 1) * n + self] = word;
-        *chunks = q;
+        *blocks = q;
     }
 };
 
@@ -621,50 +695,27 @@ struct RunWalkList {
     int nx, nxy;
     const uint32_t* __restrict__ hm;
     uint32_t n;
-    __device__ __forceinline__ uint32_t chunk_mask(int q) const
-    {
-        const uint32_t w = __ldg(hm + (size_t)(q >> 1) * n + self);
-        return (q & 1) ? (w >> 16) : (w & 0xFFFFu);
-    }
-    // Two consecutive chunks of a run (32 consecutive candidates) are drained
-    // as one 32-bit mask: a warp then runs the pair body as many times as its
-    // busiest lane has hits among 32 candidates rather than 16 twice over.
     template <class Hit, class Body>
     __device__ __forceinline__ void operator()(Hit&& hit, Body&& body) const
     {
+        (void)hit;
+        const auto replay = [&](int k) {
+            const float4 xj = __ldg(X + k);
+            // (the pair body repeats this subtraction; the two merge)
+            const float2 rxy = sub_f32x2(make_float2(xi.x, xi.y), make_float2(xj.x, xj.y));
+            const float rx = rxy.x, ry = rxy.y, rz = xi.z - xj.z;
+            // a recorded hit passed r^2 <= h^2 with these positions and this
+            // arithmetic; of the replaying passes' test (r^2 <= h^2 and
+            // r^2 >= 1e-10, delta-p and vorticity alike) the lower bound remains
+            if (rx * rx + ry * ry + rz * rz >= 1e-10f) body(k);
+        };
         int q = 0;
-#pragma unroll 1
-        for (int dz = -1; dz <= 1; ++dz) {
-#pragma unroll 1
-            for (int dy = -1; dy <= 1; ++dy) {
-                const int2 r = __ldg(runs + s0 + dz * nxy + dy * nx);
-#pragma unroll 1
-                for (int k0 = r.x; k0 < r.y; k0 += 2 * kRunChunk) {
-                    uint32_t m;
-                    if ((q & 1) == 0 && k0 + kRunChunk < r.y) {
-                        m = __ldg(hm + (size_t)(q >> 1) * n + self);  // both halves belong to this run
-                        q += 2;
-                    } else {
-                        m = chunk_mask(q++);
-                        if (k0 + kRunChunk < r.y) m |= chunk_mask(q++) << 16;
-                    }
-                    while (m) {
-                        const int c = __ffs(m) - 1;
-                        m &= m - 1u;
-                        const int k = k0 + c;
-                        const float4 xj = __ldg(X + k);
-                        // (the pair body repeats this subtraction; the two merge)
-                        const float2 rxy = sub_f32x2(make_float2(xi.x, xi.y), make_float2(xj.x, xj.y));
-                        const float rx = rxy.x, ry = rxy.y, rz = xi.z - xj.z;
-                        // a recorded hit passed r^2 <= h^2 with these positions and this
-                        // arithmetic; of the replaying passes' test (r^2 <= h^2 and
-                        // r^2 >= 1e-10, delta-p and vorticity alike) the lower bound remains
-                        (void)hit;
-                        if (rx * rx + ry * ry + rz * rz >= 1e-10f) body(k);
-                    }
-                }
-            }
-        }
+        HitBlocks<kDrainBlocks> hits;
+        each_block(runs, s0, nx, nxy, [&](int k, int end) {
+            const uint32_t m = k < end ? __ldg(hm + (size_t)q++ * n + self) : 0u;
+            hits.add(m, k, replay);
+        });
+        hits.drain(replay);
     }
 };
 
@@ -1253,7 +1304,7 @@ __global__ void __launch_bounds__(kDThreads, 10) k_d_lambda(DevParams P0, DenseA
             out = lambda_core(P, GSrc{lx_in}, xi,
                               RunWalkRec{D.runs, lx_in, xi, t, s0, (int)D.nx, (int)(D.nx * D.ny), D.hm, P.n, &q}, rho, g,
                               den, b);
-            D.hcnt[t] = q <= kListChunks ? (uint8_t)q : kNoList;
+            D.hcnt[t] = q <= kListWords ? (uint8_t)q : kNoList;
         } else {
             count_bucket_walk(D);
             out = lambda_core(P, GSrc{lx_in}, xi, mixed_walk(P, D, lx_in, xi, t, s0, rows), rho, g, den, b);
@@ -1268,7 +1319,7 @@ __global__ void __launch_bounds__(kDThreads, 10) k_d_lambda(DevParams P0, DenseA
 // 16 resident blocks (32 registers, spills on the SDF projection's path): the
 // replay's pair bodies, which load and scale only lambda_j, wait on their
 // neighbour loads, and the extra warps hide more of that than the spills cost
-// (12 blocks: 0.758 ms per 4M launch, 16: 0.731).
+// (4M launch, 16 blocks 474 us, 12 blocks 512).
 template <bool B>
 __global__ void __launch_bounds__(kDThreads, 16) k_d_deltap(DevParams P0, DenseArgs D0, const float4* __restrict__ lx_in,
                                                             float4* __restrict__ lx_out)
@@ -1334,7 +1385,7 @@ __global__ void __launch_bounds__(kDThreads, 10) k_d_integrate(DevParams P0, Den
                 } else if (rows == 0) {
                     int q = 0;
                     core(RunWalkRec{D.runs, lx, x4, t, s0, (int)D.nx, (int)(D.nx * D.ny), D.hm, P.n, &q});
-                    D.hcnt[t] = q <= kListChunks ? (uint8_t)q : kNoList;
+                    D.hcnt[t] = q <= kListWords ? (uint8_t)q : kNoList;
                 } else {
                     count_bucket_walk(D);
                     core(mixed_walk(P, D, lx, x4, t, s0, rows));
@@ -1362,8 +1413,10 @@ __global__ void __launch_bounds__(kDThreads, 10) k_d_integrate(DevParams P0, Den
     });
 }
 
+// 14 resident blocks (32 registers; 4,194,304 particles: 499 us, 12 blocks 543),
+// for the scenes of a batch 12 (2.2 million: 437 us, 14 blocks 448: more spills).
 template <bool B>
-__global__ void __launch_bounds__(kDThreads, 12) k_d_vorticity(DevParams P0, DenseArgs D0, const float4* __restrict__ lx0,
+__global__ void __launch_bounds__(kDThreads, B ? 12 : 14) k_d_vorticity(DevParams P0, DenseArgs D0, const float4* __restrict__ lx0,
                                                            const float4* __restrict__ lom,
                                                            const uint32_t* __restrict__ lid, float4* __restrict__ vel)
 {

@@ -78,7 +78,7 @@ void launch_bucket_sort(const DevParams& P, const SceneDev* scenes, const uint16
 // ---- k_dense.cu: x-runs of a dense cell window over relabelled data ----------
 constexpr int kDensePassThreads = 128;
 constexpr uint32_t kDenseScanItems = 4096;  // counters per block of the slot scan
-constexpr int kDenseListWords = 16;
+constexpr int kDenseListWords = 20;
 // The list of bucket walkers (DenseArgs::list): particles per warp, entries
 // that so many blocks take, and the blocks for a window of `slots` cells with
 // `unclean` inner ones whose neighbourhood a hash collision touches.  None
