@@ -4,9 +4,8 @@
 // The scene's box plus a margin of cells on each side is a dense window.
 // After the hash sort of a substep, every particle is relabelled by the
 // window slot of its predict-time cell (z, then y, then x; cells outside the
-// window go to one overflow slot after it for one scene, wrap into the
-// scene's window in a batch) and the per-particle arrays are gathered into
-// that label order.  The three x-adjacent cells of a row are then one contiguous
+// window go to one overflow slot after it) and the per-particle arrays are
+// gathered into that label order.  The three x-adjacent cells of a row are then one contiguous
 // label range, so a particle walks 9 runs of about 24 candidates instead of
 // 27 buckets of about 8 (the reference, CS_ComputeLambdas.glsl:126-150).
 //
@@ -24,8 +23,7 @@
 // is more than 2h - 0.9h from c's box, so out of range; by (b) no other
 // colliding cell is nearer.  So the in-range candidates of bucket hash(N) are
 // N's own, in id order (the stable sort), and the run walk sees N's particles
-// in the same order; particles of other cells wrapped into N's slot (a
-// batch) are far and fail r <= h.  Within a run the cells come x - 1, x, x + 1, the
+// in the same order.  Within a run the cells come x - 1, x, x + 1, the
 // reference's innermost loop.
 //
 // (b) and (c) hold or fail row by row: the argument above is about the three
@@ -132,21 +130,16 @@ __device__ __forceinline__ uint32_t wrap_axis(int c, int g0, uint32_t n)
     return (uint32_t)r;
 }
 
-__device__ __forceinline__ uint32_t dense_key(const DenseArgs& D, int cx, int cy, int cz)
-{
-    return D.slot0 +
-           (wrap_axis(cz, D.gz0, D.nz) * D.ny + wrap_axis(cy, D.gy0, D.ny)) * D.nx + wrap_axis(cx, D.gx0, D.nx);
-}
-
-// One scene's relabelling key of a cell: its window slot, or D.total (the
-// overflow slot, after every window slot) for a cell outside the window.
-// Runs never reach the overflow slot's labels; the bucket walk reaches them
-// through the hash-slot -> label map like any other.
+// A scene's relabelling key of a cell: its window slot, or the overflow slot
+// after them for a cell outside the window (one scene: D.total).  Runs never
+// reach the overflow slot's labels; the bucket walk reaches them through the
+// hash-slot -> label map like any other.
+__device__ __forceinline__ uint32_t overflow_slot(const DenseArgs& D) { return D.slot0 + D.nx * D.ny * D.nz; }
 __device__ __forceinline__ uint32_t scene_key(const DenseArgs& D, int cx, int cy, int cz)
 {
     const uint32_t ux = (uint32_t)cx - (uint32_t)D.gx0, uy = (uint32_t)cy - (uint32_t)D.gy0,
                    uz = (uint32_t)cz - (uint32_t)D.gz0;
-    return (ux < D.nx && uy < D.ny && uz < D.nz) ? (uz * D.ny + uy) * D.nx + ux : D.total;
+    return (ux < D.nx && uy < D.ny && uz < D.nz) ? D.slot0 + (uz * D.ny + uy) * D.nx + ux : overflow_slot(D);
 }
 
 // Window slot of each hash-sorted particle's predict-time cell, x* re-derived
@@ -163,7 +156,7 @@ __global__ void __launch_bounds__(256) k_d_keys_pred(DevParams P0, DenseArgs D0,
         predict_particle(P0, __ldg(pos + id), __ldg(vel + id), vp, xs);
         with_scene<B>(P0, D0, (int)s, [&](const DevParams& P, const DenseArgs& D) {
             const int cx = cell_coord(xs.x, P.h), cy = cell_coord(xs.y, P.h), cz = cell_coord(xs.z, P.h);
-            dkey[s] = B ? dense_key(D, cx, cy, cz) : scene_key(D, cx, cy, cz);
+            dkey[s] = scene_key(D, cx, cy, cz);
         });
     }
 }
@@ -378,37 +371,19 @@ struct SlotScan {
 };
 
 // (scan: the slots' starts less the entries before them)
-__global__ void __launch_bounds__(256) k_d_runs(DenseArgs D, SlotScan scan, int2* __restrict__ runs)
+template <bool B>
+__global__ void __launch_bounds__(256) k_d_runs(DenseArgs D0, SlotScan scan, int2* __restrict__ runs)
 {
-    if (blockIdx.x == 0 && threadIdx.x == 0) D.flag[0] = 0;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < D.total; g += stride) {
-        const uint32_t ux = g % D.nx;
-        int2 r = make_int2(0, 0);
-        if (ux >= 1 && ux + 1 < D.nx) r = make_int2((int)scan.first(g - 1), (int)scan.first(g + 2));
-        runs[g] = r;
-        D.dirty[g] = 0;
-    }
-}
-
-// The same for a batch from its table of label ranges, (-1, -1) entries being
-// empty cells.
-__global__ void __launch_bounds__(256) k_d_runs_batch(DenseArgs D0, const int2* __restrict__ cells,
-                                                      int2* __restrict__ runs)
-{
+    if (blockIdx.x == 0 && threadIdx.x == 0) D0.flag[0] = 0;
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < D0.total; g += stride) {
         DenseArgs D = D0;
         uint32_t mask = 0;
-        const uint32_t ux = window_of_slot<true>(D, mask, g) % D.nx;
+        const uint32_t ux = window_of_slot<B>(D, mask, g) % D.nx;
         int2 r = make_int2(0, 0);
-        if (ux >= 1 && ux + 1 < D.nx) {
-            const int2 e0 = __ldg(cells + g - 1), e1 = __ldg(cells + g), e2 = __ldg(cells + g + 1);
-            const int hi = max(max(e0.y, e1.y), e2.y);
-            // as unsigned, an empty cell's start (-1) is the largest
-            if (hi >= 0) r = make_int2((int)min(min((uint32_t)e0.x, (uint32_t)e1.x), (uint32_t)e2.x), hi);
-        }
+        if (ux >= 1 && ux + 1 < D.nx) r = make_int2((int)scan.first(g - 1), (int)scan.first(g + 2));
         runs[g] = r;
+        D.dirty[g] = 0;
     }
 }
 
@@ -1201,30 +1176,47 @@ __global__ void __launch_bounds__(256) k_d_relabel_place(uint32_t n, const uint3
     }
 }
 
-// ---- one scene's predict, hash sort, cell table and relabelling ----------------------------
+// ---- predict, hash sort, cell table and relabelling ----------------------------------------
 // As k_bucket.cu sorts a small scene: count, scan, place in order of arrival,
 // rank by id within the bucket; the buckets' and the window slots' counts are
 // scanned as one array.  A particle's label is its slot's start plus the
 // smaller ids of its slot, all of them in its bucket (the overflow slot's
 // particles take any order, as in the relabelling above).  Seven launches
 // and one gather of the state, where predict, a radix sort of nine launches,
-// the table, the relabelling and the gather took 19.
-// cnt: buckets (to a multiple of four), then slots and the overflow slot.
-__global__ void __launch_bounds__(256) k_d_sort_count(DevParams P, DenseArgs D, const float4* __restrict__ pos,
+// the table, the relabelling and the gather took 19 (in a batch two radix sorts,
+// 28: 64 scenes of 2.2 million particles 11.36 -> 11.20 ms a step, 8 scenes of
+// 325,433 2650 -> 2507 us).
+// cnt: buckets (to a multiple of four), then slots, a scene's overflow slot the
+// last of its own.  dkey_id: the slot, kOverflow set on an overflow slot, where
+// outside[] is the particle's order of arrival.
+constexpr uint32_t kOverflow = 0x80000000u;
+template <bool B>
+__global__ void __launch_bounds__(256) k_d_sort_count(DevParams P0, DenseArgs D0, const float4* __restrict__ pos,
                                                       const float4* __restrict__ vel, uint32_t slot_base,
                                                       uint32_t* __restrict__ keys, uint32_t* __restrict__ dkey_id,
-                                                      uint32_t* __restrict__ arrival, uint32_t* __restrict__ cnt)
+                                                      uint32_t* __restrict__ arrival, uint32_t* __restrict__ outside,
+                                                      uint32_t* __restrict__ cnt)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.n) return;
+    if (i >= P0.n) return;
     float3 vp, xs;
-    predict_particle(P, __ldg(pos + i), __ldg(vel + i), vp, xs);
-    const int cx = cell_coord(xs.x, P.h), cy = cell_coord(xs.y, P.h), cz = cell_coord(xs.z, P.h);
-    const uint32_t k = grid_hash(cx, cy, cz, P.mask), w = scene_key(D, cx, cy, cz);
-    keys[i] = k;
-    dkey_id[i] = w;
-    arrival[i] = atomicAdd(cnt + k, 1u);
-    atomicAdd(cnt + slot_base + w, 1u);
+    predict_particle(P0, __ldg(pos + i), __ldg(vel + i), vp, xs);
+    uint32_t off = 0;
+    if constexpr (B) off = __ldg(&D0.scenes[__ldg(D0.scene_of + i)].table_off);
+    with_scene<B>(P0, D0, (int)i, [&](const DevParams& P, const DenseArgs& D) {
+        const int cx = cell_coord(xs.x, P.h), cy = cell_coord(xs.y, P.h), cz = cell_coord(xs.z, P.h);
+        const uint32_t k = off + grid_hash(cx, cy, cz, P.mask);
+        uint32_t w = scene_key(D, cx, cy, cz);
+        keys[i] = k;
+        arrival[i] = atomicAdd(cnt + k, 1u);
+        if (w == overflow_slot(D)) {
+            outside[i] = atomicAdd(cnt + slot_base + w, 1u);
+            w |= kOverflow;
+        } else {
+            atomicAdd(cnt + slot_base + w, 1u);
+        }
+        dkey_id[i] = w;
+    });
 }
 
 // The cell table, the buckets' particles (id, slot) in order of arrival, and the
@@ -1251,7 +1243,7 @@ __global__ void __launch_bounds__(256) k_d_sort_rank(DevParams P, DenseArgs D, S
                                                      const uint2* __restrict__ arrived,
                                                      const uint32_t* __restrict__ skeys, const int2* __restrict__ table,
                                                      const float4* __restrict__ pos, const float4* __restrict__ vel,
-                                                     uint32_t* __restrict__ overflow_count, uint32_t* __restrict__ ids,
+                                                     const uint32_t* __restrict__ outside, uint32_t* __restrict__ ids,
                                                      DenseLabels L)
 {
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1265,9 +1257,9 @@ __global__ void __launch_bounds__(256) k_d_sort_rank(DevParams P, DenseArgs D, S
         s += o.x < me.x ? 1u : 0u;
         r += o.x < me.x && o.y == me.y ? 1u : 0u;
     }
-    if (me.y == D.total) r = atomicAdd(overflow_count, 1u);
+    if (me.y & kOverflow) r = __ldg(outside + me.x);
     ids[s] = me.x;
-    write_label(P, D, L, slot.first(me.y) + r, s, me.x, p, v);
+    write_label(P, D, L, slot.first(me.y & ~kOverflow) + r, s, me.x, p, v);
 }
 
 // 10 resident blocks (48 registers, 8 bytes spilled): with the s_corr sum of
@@ -1498,12 +1490,8 @@ void launch_d_clean(const DenseArgs& D, uint32_t mask, uint16_t* clean, uint32_t
 void launch_d_runs(const DenseArgs& D, const uint32_t* cnt, const uint32_t* block_sums, int2* runs, int sms,
                    cudaStream_t st)
 {
-    k_d_runs<<<capped_grid(D.total, 256, sms, 8), 256, 0, st>>>(D, SlotScan{cnt, block_sums, 0, 0}, runs);
-}
-
-void launch_d_runs_batch(const DenseArgs& D, const int2* cells, int2* runs, int sms, cudaStream_t st)
-{
-    k_d_runs_batch<<<capped_grid(D.total, 256, sms, 8), 256, 0, st>>>(D, cells, runs);
+    const SlotScan scan{cnt, block_sums, 0, 0};
+    PBF_DENSE_LAUNCH(k_d_runs, capped_grid(D.total, 256, sms, 8), 256, D, scan, runs);
 }
 
 void launch_d_dcol(const DenseArgs& D, uint32_t mask, uint8_t* dcol, int sms, cudaStream_t st)
@@ -1558,20 +1546,20 @@ size_t dense_sort_counts(uint32_t buckets, uint32_t slots) { return (size_t)dens
 size_t dense_sort_sums(uint32_t buckets, uint32_t slots) { return order_scan_blocks(dense_sort_base(buckets) + slots); }
 
 void launch_d_sort(const DevParams& P, const DenseArgs& D, const float4* pos, const float4* vel, uint32_t buckets,
-                   uint32_t* keys, uint32_t* dkey_id, uint32_t* arrival, uint32_t* cnt, uint32_t* block_sums,
-                   uint32_t* overflow_count, uint2* arrived, int2* table, uint32_t* ids, uint32_t* skeys,
+                   uint32_t* keys, uint32_t* dkey_id, uint32_t* arrival, uint32_t* outside, uint32_t* cnt,
+                   uint32_t* block_sums, uint2* arrived, int2* table, uint32_t* ids, uint32_t* skeys,
                    const DenseLabels& L, int2* runs, int sms, cudaStream_t st, uint64_t* launches)
 {
     const uint32_t base = dense_sort_base(buckets), m = base + D.total + 1u;
     const unsigned g = (P.n + 255u) / 256u;
     cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * m, st);
-    k_d_sort_count<<<g, 256, 0, st>>>(P, D, pos, vel, base, keys, dkey_id, arrival, cnt);
-    launch_d_scan(D, m, cnt, block_sums, overflow_count, st);
+    PBF_DENSE_LAUNCH(k_d_sort_count, g, 256, P, D, pos, vel, base, keys, dkey_id, arrival, outside, cnt);
+    launch_d_scan(D, m, cnt, block_sums, nullptr, st);
     k_d_sort_place<<<capped_grid(std::max(P.n, buckets), 256, sms, 8), 256, 0, st>>>(
         P.n, buckets, SlotScan{cnt, block_sums, 0, 0}, keys, dkey_id, arrival, table, arrived, skeys);
     const SlotScan slot{cnt, block_sums, base, P.n};
-    k_d_sort_rank<<<g, 256, 0, st>>>(P, D, slot, arrived, skeys, table, pos, vel, overflow_count, ids, L);
-    k_d_runs<<<capped_grid(D.total, 256, sms, 8), 256, 0, st>>>(D, slot, runs);
+    k_d_sort_rank<<<g, 256, 0, st>>>(P, D, slot, arrived, skeys, table, pos, vel, outside, ids, L);
+    PBF_DENSE_LAUNCH(k_d_runs, capped_grid(D.total, 256, sms, 8), 256, D, slot, runs);
     *launches += 6;
 }
 

@@ -199,7 +199,8 @@ int pbf_batch::upload_scenes()
             d.win_n[a] = ok ? (uint32_t)((int)hi - (int)lo + 1 + 2 * kDenseMargin) : 1u;
             cells *= d.win_n[a];
         }
-        d.slot0 = (uint32_t)std::min<uint64_t>(total, 0xFFFFFFFFull);
+        // (behind the earlier windows and an overflow slot of each)
+        d.slot0 = (uint32_t)std::min<uint64_t>(total + k, 0xFFFFFFFFull);
         total = std::min<uint64_t>(total + cells, 1ull << 40);
         for (int a = 0; a < 3; ++a) {
             w[7 * k + a] = d.win_g0[a];
@@ -330,15 +331,22 @@ int pbf_batch::dense_setup()
                          (unsigned long long)dense_total);
     if (capturing) return set_error(PBF_ERR_STATE, "dense windows changed during graph capture");
     int rc;
-    const size_t c = std::max<uint32_t>(n, 1u), cp = c + kLabelPad, T = (size_t)dense_total;
+    const size_t c = std::max<uint32_t>(n, 1u), cp = c + kLabelPad, T = dense_slots();
     if (!lx[0]) {
         label_slab.add(lx[0], cp).add(lx[1], cp).add(lxb, c).add(lv, cp).add(lx0, cp).add(lom, cp).add(lrho, c).add(lid, c)
             .add(inv, c).add(dslot, c).add(dord, c).add(dhm, c * kDenseListWords).add(dhcnt, c).add(dflag, 4);
         if ((rc = label_slab.alloc())) return rc;
     }
     window_slab.release();
-    window_slab.add(dtable, T).add(druns, T).add(dclean, T).add(ddcol, T).add(ddirty, T).add(dvmark, T).add(dslot_scene, T)
+    window_slab.add(druns, T).add(dclean, T).add(ddcol, T).add(ddirty, T).add(dvmark, T).add(dslot_scene, T)
         .add(dcnt, T + 1).add(dbsum, order_scan_blocks((uint32_t)T));
+    dense_count = n > 0;
+    for (const auto& s : scenes)
+        dense_count = dense_count && s.desc.num_particles <= kDenseSortMax &&
+                      (uint64_t)s.desc.hash_size * 64u >= s.desc.num_particles;
+    if (dense_count)
+        window_slab.add(dsort, dense_sort_counts(table_size, (uint32_t)T))
+            .add(dsort_sums, dense_sort_sums(table_size, (uint32_t)T));
     if ((rc = window_slab.alloc())) {
         dense_free();
         return rc;
@@ -347,7 +355,7 @@ int pbf_batch::dense_setup()
     for (size_t k = 0; k < scenes.size(); ++k) {
         const size_t b0 = (size_t)(uint32_t)win[7 * k + 6];
         const size_t cells = (size_t)win[7 * k + 3] * (size_t)win[7 * k + 4] * (size_t)win[7 * k + 5];
-        std::fill(ss.begin() + b0, ss.begin() + b0 + cells, (uint16_t)k);
+        std::fill(ss.begin() + b0, ss.begin() + b0 + cells + 1, (uint16_t)k);
     }
     BCK(cudaMemcpyAsync(dslot_scene, ss.data(), sizeof(uint16_t) * T, cudaMemcpyHostToDevice, stream));
     BCK(cudaMemsetAsync(dflag, 0, sizeof(uint32_t) * 4, stream));
@@ -378,7 +386,7 @@ DenseArgs pbf_batch::dense_args() const
     D.flag = dflag;
     const float b = 0.9f * derived.h;
     D.drift2 = b * b;
-    D.total = (uint32_t)dense_total;
+    D.total = (uint32_t)dense_slots();
     D.scenes = scenes_dev;
     D.scene_of = scene_of;
     D.slot_scene = dslot_scene;
@@ -394,7 +402,7 @@ int pbf_batch::dense_step_body()
 {
     const DevParams P = dev_params();
     const int sms = num_sms;
-    const uint32_t T = (uint32_t)dense_total;
+    const uint32_t T = (uint32_t)dense_slots();
     const uint32_t slot_bits = std::max<uint32_t>(ceil_log2(T), 1u);
     const uint32_t iters = cfg.solver_iterations;
     const bool vort = cfg.enable_vorticity;
@@ -409,23 +417,28 @@ int pbf_batch::dense_step_body()
     };
     for (uint32_t sub = 0; sub < cfg.substep_iterations; ++sub) {
         const bool last = sub + 1 == cfg.substep_iterations;
-        launch_b_predict(P, scenes_dev, scene_of, pos, vel, keys, sms, stream);
-        launch_radix_sort(n, key_bits, keys, ka, ia, kb, ib, hist, totals, &skeys, &ids, stream, &launches);
-        BCK(cudaMemsetAsync(table, 0xFF, sizeof(int2) * (size_t)table_size, stream));
-        launch_build_table(n, skeys, table, sms, stream);
         D = dense_args();
-        launch_d_keys_pred(P, D, ids, pos, vel, mcode, sms, stream);
-        launches += 3;
-        uint32_t *msorted = nullptr, *lorder = nullptr;
-        launch_radix_sort(n, slot_bits, mcode, mka, mia, mkb, mib, hist, totals, &msorted, &lorder, stream,
-                          &launches);
-        launch_d_permute(P, D, lorder, ids, pos, vel, DenseLabels{lx[0], lxb, lv, lx0, lid, inv, nullptr}, sms, stream);
-        BCK(cudaMemsetAsync(dtable, 0xFF, sizeof(int2) * (size_t)T, stream));
-        launch_build_table(n, msorted, dtable, sms, stream);
-        launch_d_runs_batch(D, dtable, druns, sms, stream);
-        BCK(cudaMemsetAsync(ddirty, 0, sizeof(uint32_t) * (size_t)T, stream));
-        BCK(cudaMemsetAsync(dflag, 0, sizeof(uint32_t), stream));
-        launches += 3;
+        const DenseLabels L{lx[0], lxb, lv, lx0, lid, inv, nullptr};
+        if (dense_count) {
+            // (scratch of the particles in order of arrival: the lambda pass's output)
+            launch_d_sort(P, D, pos, vel, table_size, keys, mcode, mka, mkb, dsort, dsort_sums,
+                          reinterpret_cast<uint2*>(lx[1]), table, ia, ka, L, druns, sms, stream, &launches);
+            ids = ia;
+            skeys = ka;
+        } else {
+            launch_b_predict(P, scenes_dev, scene_of, pos, vel, keys, sms, stream);
+            launch_radix_sort(n, key_bits, keys, ka, ia, kb, ib, hist, totals, &skeys, &ids, stream, &launches);
+            BCK(cudaMemsetAsync(table, 0xFF, sizeof(int2) * (size_t)table_size, stream));
+            launch_build_table(n, skeys, table, sms, stream);
+            launch_d_keys_pred(P, D, ids, pos, vel, mcode, sms, stream);
+            uint32_t *msorted = nullptr, *lorder = nullptr;
+            launch_radix_sort(n, slot_bits, mcode, mka, mia, mkb, mib, hist, totals, &msorted, &lorder, stream,
+                              &launches);
+            launch_d_relabel(D, n, T, mcode, skeys, dcnt, dbsum, nullptr, nullptr, sms, stream, &launches);
+            launch_d_permute(P, D, lorder, ids, pos, vel, L, sms, stream);
+            launch_d_runs(D, dcnt, dbsum, druns, sms, stream);
+            launches += 5;
+        }
         for (uint32_t it = 1; it <= iters; ++it) {
             D.rec_slot = nullptr;
             D.rec_cnt = nullptr;

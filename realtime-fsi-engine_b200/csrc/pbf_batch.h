@@ -162,12 +162,15 @@ struct pbf_batch {
     // window at global slots [SceneDev::slot0, + its cells); labels sorted by
     // (global slot of the predict-time cell, hash-sorted index), scene-contiguous
     std::vector<int> win;         // per scene: g0[3], n[3], slot0 (7 ints), as uploaded
-    uint64_t dense_total = 0;     // slots of all windows
+    uint64_t dense_total = 0;     // cells of all windows
+    size_t dense_slots() const { return (size_t)dense_total + scenes.size(); }  // and an overflow slot per scene
+    bool dense_count = false;     // sort by counting (launch_d_sort): no scene too large, no bucket too long
+    uint32_t *dsort = nullptr, *dsort_sums = nullptr;
     bool dense_ready = false;     // the clean/dcol tables below match `win` and the hash masks
     float4 *lx[2] = {nullptr, nullptr}, *lxb = nullptr, *lv = nullptr, *lx0 = nullptr, *lom = nullptr;
     float* lrho = nullptr;
     uint32_t *lid = nullptr, *inv = nullptr;
-    int2 *dtable = nullptr, *druns = nullptr;
+    int2* druns = nullptr;
     uint16_t* dclean = nullptr;
     uint32_t* ddirty = nullptr;
     uint8_t *ddcol = nullptr, *dhcnt = nullptr, *dvmark = nullptr;

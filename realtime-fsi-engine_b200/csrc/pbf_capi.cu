@@ -846,7 +846,7 @@ int pbf_handle::sort_stages()
         dkey_valid = false;
         order = nullptr;
         // (the scratch of the particles in order of arrival: the lambda pass's output)
-        launch_d_sort(dev_params(), D, pos, vel, derived.hash_size, keys, dkey_id, mka, dsort, dsort_sums, dflag + 3,
+        launch_d_sort(dev_params(), D, pos, vel, derived.hash_size, keys, dkey_id, mka, mcode, dsort, dsort_sums,
                       reinterpret_cast<uint2*>(lx[1]), table, ia, ka, dense_labels(), druns, num_sms, stream, &launches);
         skeys = ka;
         ids = ia;

@@ -157,7 +157,7 @@ struct DenseLabels {
 };
 void launch_d_permute(const DevParams& P, const DenseArgs& D, const uint32_t* order, const uint32_t* ids,
                       const float4* pos, const float4* vel, const DenseLabels& L, int sms, cudaStream_t st);
-// One scene's substep from the particle state to the runs: what predict, hash
+// A substep from the particle state to the runs (one scene or a batch): what predict, hash
 // sort, table, relabelling, launch_d_permute and launch_d_runs leave, to the
 // bit (the overflow slot's labels in any order).  A particle reads its whole
 // bucket, so the buckets must stay short.  Up to kDenseSortMax particles: they
@@ -165,22 +165,21 @@ void launch_d_permute(const DevParams& P, const DenseArgs& D, const uint32_t* or
 // while they stay in L2 (step of 262,144 particles 1813 -> 1752 us, 602,263
 // 1362 -> 1317, 983,040 2339 -> 2311; but of 1,966,080 4273 -> 4290 and of
 // 4,194,304 8.70 -> 8.86 ms, the write alone 321 us where the gather in label
-// order takes 105).  Scratch: arrival[n], arrived[n], cnt[dense_sort_counts],
-// block_sums[dense_sort_sums].
+// order takes 105).  Scratch: dkey_id, arrival, outside, arrived[n],
+// cnt[dense_sort_counts], block_sums[dense_sort_sums].
 constexpr uint32_t kDenseSortMax = 1u << 20;
 size_t dense_sort_counts(uint32_t buckets, uint32_t slots);
 size_t dense_sort_sums(uint32_t buckets, uint32_t slots);
 void launch_d_sort(const DevParams& P, const DenseArgs& D, const float4* pos, const float4* vel, uint32_t buckets,
-                   uint32_t* keys, uint32_t* dkey_id, uint32_t* arrival, uint32_t* cnt, uint32_t* block_sums,
-                   uint32_t* overflow_count, uint2* arrived, int2* table, uint32_t* ids, uint32_t* skeys,
+                   uint32_t* keys, uint32_t* dkey_id, uint32_t* arrival, uint32_t* outside, uint32_t* cnt,
+                   uint32_t* block_sums, uint2* arrived, int2* table, uint32_t* ids, uint32_t* skeys,
                    const DenseLabels& L, int2* runs, int sms, cudaStream_t st, uint64_t* launches);
 void launch_d_clean(const DenseArgs& D, uint32_t mask, uint16_t* clean, uint32_t* unclean, int sms, cudaStream_t st);
 void launch_d_dcol(const DenseArgs& D, uint32_t mask, uint8_t* dcol, int sms, cudaStream_t st);
-// The runs of one scene from the relabelling's scan (cnt, block_sums), and
-// the substep's dirty rows and crossings cleared; of a batch from its cell table.
+// The runs from a relabelling's scan (cnt, block_sums), and the substep's dirty
+// rows and crossings cleared.
 void launch_d_runs(const DenseArgs& D, const uint32_t* cnt, const uint32_t* block_sums, int2* runs, int sms,
                    cudaStream_t st);
-void launch_d_runs_batch(const DenseArgs& D, const int2* cells, int2* runs, int sms, cudaStream_t st);
 // Labels bucketed by the window slot of their current cell (X) into order[n].
 // Scratch: slot_of[n], cnt[slots + 1], block_sums[order_scan_blocks(slots)].
 uint32_t order_scan_blocks(uint32_t slots);

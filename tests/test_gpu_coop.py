@@ -163,3 +163,23 @@ def test_sort_of_a_dense_step_equals_the_stages(have_gpu, n, hash_size):
                     fl.read_buffer(P.BUF_XSTAR, np.float32, (n, 4)), fl.readbackParticles()])
     for a, b in zip(*got):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("hash_size", [16, 128, 1 << 14])
+def test_sort_of_a_dense_batch(have_gpu, hash_size):
+    """A batch's sort by counting, and by radix where a scene's buckets are too
+    long for it, with particles that leave their scene's window."""
+    from pbf_b200 import batch as PB
+    cfg, sc = scenes.c3(5, 4, [5000, 1, 300, 8000])
+    for k, s in enumerate(sc):
+        s["hash_size"] = hash_size
+        s["vel"] = np.array(s["vel"], np.float32)
+        s["vel"][k::5] += np.float32(60.0)
+    out = []
+    for mode in (4, 8):
+        b = PB.make_batch(cfg, sc)
+        b.set_option(P.BOPT_NEIGHBOUR_MODE, mode)
+        for _ in range(2):
+            b.step()
+        out.append(b.read_particles())
+    assert same(*out)
