@@ -68,7 +68,7 @@ def parse():
     ap.add_argument("--no-extras", action="store_true",
                     help="c2 only: skip the short C3 batch and C4 adjoint runs attached to the line")
     ap.add_argument("--mode", type=int, default=-1, choices=[-1, 4, 8],
-                    help="neighbour passes: -1 automatic (default: 8 from 2^19 particles, else 4), 4 hashed "
+                    help="neighbour passes: -1 automatic (default: 8 from 3 * 2^16 particles, else 4), 4 hashed "
                          "buckets in Morton thread order with per-bucket hit masks, 8 x-runs of a dense cell window")
     ap.add_argument("--sample", type=int, nargs=3, default=None, metavar=("NX", "NY", "NZ"),
                     help="smaller lattice of the same scene (profiling captures only)")
@@ -347,7 +347,7 @@ def run_b200(args, dist):
     torch.cuda.synchronize(dev)
     clocks = Clocks(dev)
     l0 = fl.kernel_launches()
-    mode = args.mode if args.mode >= 0 else (8 if n >= (1 << 19) else 4)
+    mode = args.mode if args.mode >= 0 else (8 if n >= (3 << 16) else 4)
     ws0 = fl.list_stats() if mode == 8 else None
     e0.record(stream)
     for _ in range(args.steps):
