@@ -1349,10 +1349,12 @@ __global__ void __launch_bounds__(kDThreads, 16) k_d_deltap(DevParams P0, DenseA
     });
 }
 
-// 10 resident blocks (9: no faster), for the scenes of a batch 9 (56 registers
-// for its constants: batch of 64 scenes 907 / 831 -> 893 / 811 us, 8 blocks 926 / 838).
+// 9 resident blocks (56 registers): 10 spill on the bucket walks' path, which a
+// collapsed block's edges take (983,040 particles after 40 steps 386 -> 362 us,
+// 4,194,304 over 30 steps 1406 -> 1376; fresh blocks alike; batch of 64 scenes
+// 907 / 831 -> 893 / 811); 8: batch 926 / 838, 11: 439 us.
 template <bool B, bool R>
-__global__ void __launch_bounds__(kDThreads, B ? 9 : 10) k_d_integrate(DevParams P0, DenseArgs D0, const float4* __restrict__ lx,
+__global__ void __launch_bounds__(kDThreads, 9) k_d_integrate(DevParams P0, DenseArgs D0, const float4* __restrict__ lx,
                                                            const float4* __restrict__ lv, float4* __restrict__ lx0,
                                                            float4* __restrict__ lom,
                                                            const uint32_t* __restrict__ lid, float4* __restrict__ pos,
@@ -1412,10 +1414,12 @@ __global__ void __launch_bounds__(kDThreads, B ? 9 : 10) k_d_integrate(DevParams
     });
 }
 
-// 14 resident blocks (32 registers; 4,194,304 particles: 499 us, 12 blocks 543),
-// for the scenes of a batch 12 (2.2 million: 437 us, 14 blocks 448: more spills).
-template <bool B>
-__global__ void __launch_bounds__(kDThreads, B ? 12 : 14) k_d_vorticity(DevParams P0, DenseArgs D0, const float4* __restrict__ lx0,
+// 12 resident blocks (40 registers): after 40 steps of a dam break of 262,144
+// particles 121 us (14 blocks, 32 registers: 129), of 983,040 249 (260), of
+// 2,097,152 479 (486), batch of 2.2 million fresh 437 (448).  14 in one scene of
+// more than 2^21: 4,194,304 fresh 499 (12 blocks: 543), over 30 steps 817 (824).
+template <bool B, int Blocks>
+__global__ void __launch_bounds__(kDThreads, Blocks) k_d_vorticity(DevParams P0, DenseArgs D0, const float4* __restrict__ lx0,
                                                            const float4* __restrict__ lom,
                                                            const uint32_t* __restrict__ lid, float4* __restrict__ vel)
 {
@@ -1599,7 +1603,12 @@ void launch_d_integrate(const DevParams& P, const DenseArgs& D, const float4* lx
 void launch_d_vorticity(const DevParams& P, const DenseArgs& D, const float4* lx0, const float4* lom,
                         const uint32_t* lid, float4* vel, cudaStream_t st)
 {
-    PBF_DENSE_LAUNCH(k_d_vorticity, dgrid(D, P.n), kDThreads, P, D, lx0, lom, lid, vel);
+    if (D.scenes)
+        k_d_vorticity<true, 12><<<dgrid(D, P.n), kDThreads, 0, st>>>(P, D, lx0, lom, lid, vel);
+    else if (P.n <= (1u << 21))
+        k_d_vorticity<false, 12><<<dgrid(D, P.n), kDThreads, 0, st>>>(P, D, lx0, lom, lid, vel);
+    else
+        k_d_vorticity<false, 14><<<dgrid(D, P.n), kDThreads, 0, st>>>(P, D, lx0, lom, lid, vel);
 }
 
 #undef PBF_DENSE_LAUNCH

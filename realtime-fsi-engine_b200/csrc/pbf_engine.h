@@ -50,8 +50,8 @@ struct pbf_handle {
     // spatial processing order of the neighbour passes (Morton order of the
     // predict-time cells); `order` points into one of the m* ping-pong pairs.
     // PBF_OPT_SPATIAL_ORDER: 4 hashed buckets in Morton thread order with
-    // per-bucket hit masks, 8 x-runs of the dense cell window; -1 (default): 8
-    // from 2^19 particles, 4 below
+    // per-bucket hit masks, 8 x-runs of the dense cell window; -1 (default): by
+    // size and window (effective_mode)
     int pass_mode = -1;
     uint32_t *mcode = nullptr, *mka = nullptr, *mia = nullptr, *mkb = nullptr, *mib = nullptr;
     uint32_t* order = nullptr;
