@@ -136,11 +136,10 @@ __device__ __forceinline__ float centre_d2(float3 p, float4 lo, float4 hi)
     return x * x + y * y + z * z;
 }
 
-// Squared distance to the face reached by taking the nearer child from
-// `root` (by box distance, then by box centre when P lies in both boxes, as
-// it does inside a closed mesh): an upper bound of the subtree's nearest
-// distance.
-__device__ float first_leaf_d2(const MeshDev& M, float3 P, int root)
+// The leaf reached by taking the nearer child from `root` (by box distance,
+// then by box centre when P lies in both boxes, as it does inside a closed
+// mesh): its face's distance is an upper bound of the subtree's nearest.
+__device__ int first_leaf(const MeshDev& M, float3 P, int root)
 {
     const int n_int = M.nf - 1;
     int node = root;
@@ -150,7 +149,7 @@ __device__ float first_leaf_d2(const MeshDev& M, float3 P, int root)
         const bool left = dl != dr ? dl < dr : centre_d2(P, w.l0, w.l1) <= centre_d2(P, w.r0, w.r1);
         node = left ? w.left() : w.right();
     }
-    return leaf_hit(M, P, node - n_int).d2;
+    return node;
 }
 
 // Position of `node` in the visiting order of one near-first walk
@@ -180,10 +179,16 @@ __device__ unsigned long long visit_rank(const MeshDev& M, float3 P, int node)
 // one thread per query took 1516 us for 20,000 queries against 5,120 faces, a
 // warp takes 159.
 // The bound is right from the start (the nearest of 32 faces, one greedy
-// descent per frontier subtree), so few nodes are opened in vain.
-// A box distance and a face distance round differently: a node is passed over
-// only when its box is farther than the bound by more than that.
-constexpr float kBoxSlack = 1.0f + 4e-6f;
+// descent per frontier subtree), so few nodes are opened in vain, and the face
+// that gave it is the nearest if no other is found.
+// A face's nearest point is rounded at the size of its coordinates and so can
+// lie outside the face's box by that much, whatever its distance; a box
+// distance itself rounds in proportion.  A node is passed over only when its
+// box is farther than the bound d2 by more than both.  With r = 1e-6 of the
+// largest coordinate (8 units in its last place), (d + r)^2 <= d2 (1 + e) +
+// r^2 (1 + 1 / e) for any e; e = 1e-5 here (a square root a round, for the
+// exact sum: 1 % of the time of 20,000 searches).
+constexpr float kBoxSlack = 1.0f + 1.4e-5f, kPointSlack = 1.0001e-7f;
 constexpr int kWarpNodes = 320;  // waiting inner nodes (a balanced tree of 2^14 faces needs at most 32 * 9)
 struct WarpNodes {
     int2 node[kWarpNodes];  // node, box distance
@@ -208,23 +213,27 @@ __device__ Hit warp_closest(const MeshDev& M, float3 P, WarpNodes& W, int& leaf)
     const int lane = threadIdx.x & 31, n_int = M.nf - 1;
     const uint32_t below = (1u << lane) - 1u;
     const int root = M.frontier[lane];
-    // distances are non-negative: their bits compare as they do
-    float bound;
-    if (leaf >= 0)
-        bound = leaf_hit(M, P, leaf - n_int).d2;
-    else
-        bound = __uint_as_float(__reduce_min_sync(
-            all, root >= 0 ? __float_as_uint(first_leaf_d2(M, P, root)) : 0x7F7FFFFFu));
+    // the bound, and the leaf whose face gave it
+    const int first = leaf >= 0 ? leaf : root >= 0 ? first_leaf(M, P, root) : -1;
     leaf = -1;
     Hit best;
-    best.d2 = bound;
+    best.d2 = first >= 0 ? leaf_hit(M, P, first - n_int).d2 : 3.0e38f;
     best.p = make_float3(0.f, 0.f, 0.f);
     best.feature = 0;
     best.face = -1;
     int best_node = -1, ni = 0, nl = 0;
+    // distances are non-negative: their bits compare as they do
+    float bound = __uint_as_float(__reduce_min_sync(all, __float_as_uint(best.d2)));
     if (!(bound < 3.0e38f)) return best;  // no face is near enough to be found (or P is not a point)
+    const int seed = best.d2 == bound ? first : -1;
+    best.d2 = bound;
+    const float4 m0 = __ldg(M.bmin), m1 = __ldg(M.bmax);  // the mesh's box
+    const float size = fmaxf(fmaxf(fmaxf(fabsf(m0.x), fabsf(m1.x)), fmaxf(fabsf(m0.y), fabsf(m1.y))),
+                             fmaxf(fabsf(m0.z), fabsf(m1.z)));
+    const float slack = kPointSlack * size * size;
+    float limit = __fmaf_rn(bound, kBoxSlack, slack);
     auto push = [&](int node, float d2, bool on) {
-        on = on && d2 <= bound * kBoxSlack;  // (a face at exactly the bound may come first in the walk)
+        on = on && d2 <= limit;  // (a face at exactly the bound may come first in the walk)
         const bool inner = node < n_int;
         const uint32_t bi = __ballot_sync(all, on && inner), bl = __ballot_sync(all, on && !inner);
         if (on) {
@@ -248,7 +257,7 @@ __device__ Hit warp_closest(const MeshDev& M, float3 P, WarpNodes& W, int& leaf)
             nl -= c;
             if (lane < c) {
                 const int2 e = W.leaf[nl + lane];
-                if (__int_as_float(e.y) <= bound * kBoxSlack)
+                if (__int_as_float(e.y) <= limit)
                     keep_nearer(M, P, best, best_node, leaf_hit(M, P, e.x - n_int), e.x);
             }
         } else {
@@ -257,7 +266,7 @@ __device__ Hit warp_closest(const MeshDev& M, float3 P, WarpNodes& W, int& leaf)
             const bool room = ni + c <= kWarpNodes;
             ni -= c;
             const int2 e = lane < c ? W.node[ni + lane] : make_int2(0, 0);
-            bool on = lane < c && __int_as_float(e.y) <= bound * kBoxSlack;
+            bool on = lane < c && __int_as_float(e.y) <= limit;
             __syncwarp();
             if (room) {
                 const WideNode w = wide_node(M, on ? e.x : 0);  // (an inner node waits: there is a node 0)
@@ -265,14 +274,19 @@ __device__ Hit warp_closest(const MeshDev& M, float3 P, WarpNodes& W, int& leaf)
                 push(w.right(), box_d2(P, w.r0, w.r1), on);
             } else if (on) {
                 // a very deep tree: each lane walks its subtree alone
-                const Hit h = subtree_closest(M, P, e.x, bound * kBoxSlack);
+                const Hit h = subtree_closest(M, P, e.x, limit);
                 keep_nearer(M, P, best, best_node, h, e.x);
             }
         }
         bound = __uint_as_float(__reduce_min_sync(all, __float_as_uint(best.d2)));
+        limit = __fmaf_rn(bound, kBoxSlack, slack);
         __syncwarp();
     }
     // the lanes' nearest, ties as above
+    if (!__any_sync(all, best.face >= 0 && best.d2 == bound) && seed >= 0) {
+        best = leaf_hit(M, P, seed - n_int);
+        best_node = seed;
+    }
     const bool mine = best.face >= 0 && best.d2 == bound;
     uint32_t win = __ballot_sync(all, mine);
     if (__popc(win) > 1) {
