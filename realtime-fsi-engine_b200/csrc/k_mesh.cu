@@ -213,19 +213,26 @@ __device__ Hit warp_closest(const MeshDev& M, float3 P, WarpNodes& W, int& leaf)
     const int lane = threadIdx.x & 31, n_int = M.nf - 1;
     const uint32_t below = (1u << lane) - 1u;
     const int root = M.frontier[lane];
-    // the bound, and the leaf whose face gave it
-    const int first = leaf >= 0 ? leaf : root >= 0 ? first_leaf(M, P, root) : -1;
-    leaf = -1;
     Hit best;
-    best.d2 = first >= 0 ? leaf_hit(M, P, first - n_int).d2 : 3.0e38f;
     best.p = make_float3(0.f, 0.f, 0.f);
     best.feature = 0;
     best.face = -1;
     int best_node = -1, ni = 0, nl = 0;
+    // the bound, and the leaf whose face gave it (a collapsed face's distance
+    // can be no number: none is known from it)
+    constexpr float kNone = 3.0e38f;
+    int first = leaf;
+    float d2 = first >= 0 ? leaf_hit(M, P, first - n_int).d2 : kNone;
+    if (!(d2 < kNone)) {
+        first = root >= 0 ? first_leaf(M, P, root) : -1;
+        if (first >= 0) d2 = leaf_hit(M, P, first - n_int).d2;
+    }
+    best.d2 = d2 < kNone ? d2 : kNone;
+    leaf = -1;
     // distances are non-negative: their bits compare as they do
     float bound = __uint_as_float(__reduce_min_sync(all, __float_as_uint(best.d2)));
-    if (!(bound < 3.0e38f)) return best;  // no face is near enough to be found (or P is not a point)
-    const int seed = best.d2 == bound ? first : -1;
+    if (!(bound < kNone) && isnan(P.x + P.y + P.z)) return best;  // not a point
+    const int seed = best.d2 == bound && bound < kNone ? first : -1;
     best.d2 = bound;
     const float4 m0 = __ldg(M.bmin), m1 = __ldg(M.bmax);  // the mesh's box
     const float size = fmaxf(fmaxf(fmaxf(fabsf(m0.x), fabsf(m1.x)), fmaxf(fabsf(m0.y), fabsf(m1.y))),
