@@ -569,7 +569,7 @@ DenseLabels pbf_handle::dense_labels() const { return {lx[0], lxb, lv, lx0, lid,
 void pbf_handle::dense_begin(const DenseArgs& D)
 {
     dord_iter = D.list_blocks ? 1 : 0;
-    dlist_iter = 0;
+    forget_hits();
     dvlist_ready = false;
     dslot_fresh = false;
     dcnt_clear = false;
@@ -648,13 +648,13 @@ int pbf_handle::stage(int st, uint32_t iter)
             D.clear_cnt = dslot_fresh ? nullptr : dcnt;
             launch_d_lambda(P, D, lx[0], lx[1], lrho, stream);
             dcnt_clear = !dslot_fresh;
-            dlist_iter = (int)iter;
+            dlist_iter = iter;
             last_x = 1;
             break;
         case PBF_STAGE_DELTAP:
             if (dord_iter && dord_iter == std::max((int)iter, 1)) D.order = dord;
-            D.use_list = dlist_iter == (int)iter ? 1 : 0;
-            dlist_iter = 0;
+            D.use_list = dlist_iter == iter ? 1 : 0;
+            forget_hits();
             if (const int rc = record_next()) return rc;
             launch_d_deltap(P, D, lx[1], lx[0], stream);
             last_x = 0;
@@ -662,7 +662,7 @@ int pbf_handle::stage(int st, uint32_t iter)
         case PBF_STAGE_INTEGRATE:
             order_by(lx[0]);
             dord_iter = 0;
-            dlist_iter = 0;
+            forget_hits();
             if (P.vort_on) {
                 if (const int rc = record_next()) return rc;
                 // hit masks for the vorticity pass
@@ -714,6 +714,7 @@ int pbf_handle::stage(int st, uint32_t iter)
         CK(cudaMemsetAsync(table, 0xFF, sizeof(int2) * (size_t)derived.hash_size, stream));
         launch_build_table(n, skeys, table, sms, stream);
         ++launches;
+        forget_hits();
         prof_end(PBF_STAGE_TABLE);
         break;
     case PBF_STAGE_REORDER:
@@ -771,7 +772,7 @@ int pbf_handle::stage(int st, uint32_t iter)
             launch_radix_sort(n, 24, mcode, mka, mia, mkb, mib, hist, totals, &msorted, &order, stream, &launches);
         }
         label_space = false;
-        chit_iter = 0;
+        forget_hits();
         last_x = 0;
         prof_end(PBF_STAGE_REORDER);
         break;
@@ -783,7 +784,7 @@ int pbf_handle::stage(int st, uint32_t iter)
         else
             launch_lambda_m(P, sx[0], sx[1], rho, table, lod, iter, order, stream);
         ++launches;
-        chit_iter = (int)iter;
+        chit_iter = iter;
         last_x = 1;
         prof_end(PBF_STAGE_LAMBDA);
         break;
@@ -791,11 +792,11 @@ int pbf_handle::stage(int st, uint32_t iter)
         prof_begin(PBF_STAGE_DELTAP);
         if (const int G = coop_lanes(n))
             launch_c_deltap(G, P, nullptr, nullptr, sx[1], sx[0], table, lod, iter, order,
-                            chit_iter == (int)iter ? chits : nullptr, chit_len, nullptr, stream);
+                            chit_iter == iter ? chits : nullptr, chit_len, nullptr, stream);
         else
             launch_deltap_m(P, sx[1], sx[0], table, lod, iter, order, stream);
         ++launches;
-        chit_iter = 0;
+        forget_hits();
         last_x = 0;
         prof_end(PBF_STAGE_DELTAP);
         break;
@@ -836,7 +837,7 @@ int pbf_handle::sort_stages()
         ids = ia;
         order = nullptr;
         label_space = false;
-        chit_iter = 0;
+        forget_hits();
         last_x = 0;
         return PBF_OK;
     }
@@ -962,6 +963,7 @@ extern "C" int pbf_set_params(pbf_handle* h, const pbf_fluid_config* cfg)
     h->cfg.particle_count = h->n ? h->n : cfg->particle_count;
     pbf_derive_params(&h->cfg, h->collision_padding, &h->derived);
     h->invalidate_graph();
+    h->forget_hits();
     if (h->n && (rc = h->ensure_capacity(h->n))) return rc;
     return PBF_OK;
 }
@@ -1028,6 +1030,7 @@ extern "C" int pbf_set_particles(pbf_handle* h, const pbf_particle* ps, uint32_t
     h->invalidate_graph();
     h->n = n;
     h->label_space = false;
+    h->forget_hits();
     h->cfg.particle_count = n;  // PBFluids.cpp:117-118
     pbf_derive_params(&h->cfg, h->collision_padding, &h->derived);
     h->contact_count_host = 0;
@@ -1092,6 +1095,7 @@ extern "C" int pbf_set_particles_device(pbf_handle* h, const void* pos4, const v
         h->invalidate_graph();
         h->n = n;
         h->label_space = false;
+        h->forget_hits();
         h->cfg.particle_count = n;
         pbf_derive_params(&h->cfg, h->collision_padding, &h->derived);
         if (n) {
@@ -1435,6 +1439,7 @@ extern "C" int pbf_set_option(pbf_handle* h, int option, int value)
             return set_error(PBF_ERR_INVALID, "neighbour mode %d: -1 (automatic), 4 or 8", value);
         h->pass_mode = value;
         h->label_space = false;
+        h->forget_hits();
         break;
     default: return set_error(PBF_ERR_INVALID, "unknown option %d", option);
     }

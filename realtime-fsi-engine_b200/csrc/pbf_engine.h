@@ -76,7 +76,8 @@ struct pbf_handle {
     // lambda hit masks replayed by the delta-p pass of the same iteration
     uint32_t* dhm = nullptr;
     uint8_t* dhcnt = nullptr;
-    int dlist_iter = 0;          // solver iteration whose lambda recorded them (0: none)
+    static constexpr int64_t kNoIter = -1;  // (no uint32_t, which a stage's iteration may be any of)
+    int64_t dlist_iter = kNoIter;  // solver iteration whose lambda recorded them
     uint8_t* dvmark = nullptr;   // per window slot: integrate moved a particle its runs hold
     bool dvlist_ready = false;   // dhm/dhcnt hold the integrate pass's masks for the vorticity pass
     size_t cap_slots = 0;
@@ -120,7 +121,9 @@ struct pbf_handle {
     // small scenes: the hits of the latest lambda pass (k_coop.cu)
     uint32_t *chits = nullptr, *chit_len = nullptr;
     uint32_t cap_chits = 0;
-    int chit_iter = 0;  // solver iteration that recorded them (0: none)
+    int64_t chit_iter = kNoIter;  // solver iteration that recorded them
+    // Positions, table or radius are no longer those the hits were found with.
+    void forget_hits() { chit_iter = dlist_iter = kNoIter; }
     // contacts
     float4* cand = nullptr;
     uint32_t* ct_counts = nullptr;
