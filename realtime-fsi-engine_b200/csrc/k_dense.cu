@@ -53,7 +53,7 @@
 //   * the delta-p pass replays the hit masks its iteration's lambda pass
 //     recorded (same positions, same runs, same hits), and the vorticity pass
 //     those of the integrate pass, except near particles the walls or the
-//     SDF moved there;
+//     SDF moved there and in cells whose rows that made dirty;
 //   * one scene's particles with rows on the buckets go first, in groups of
 //     lanes, so that their longer walks end before the others';
 //   * x/y arithmetic in packed f32x2 instructions, each lane rounded as the
@@ -1434,7 +1434,9 @@ __global__ void __launch_bounds__(kDThreads, Blocks) k_d_vorticity(DevParams P0,
             any = vorticity_core(P, GSrc{lx0}, GMagX{lx0}, xi, [&] { return __ldg(lom + t); }, walk, dv);
         };
         const int s0 = D.use_list && __ldg(D.hcnt + t) != kNoList ? interior_slot(P, D, xi) : -1;
-        if (s0 >= 0 && !D.vmark[s0])
+        // (integrate may have brought a particle into reach through a row's
+        // buckets alone: the row is then dirty; none is while flag[0] is 0)
+        if (s0 >= 0 && !D.vmark[s0] && !(D.flag[0] && D.dirty[s0]))
             // integrate walked this particle's runs over the same positions
             core(RunWalkList{D.runs, lx0, xi, t, s0, (int)D.nx, (int)(D.nx * D.ny), D.hm, P.n});
         else
