@@ -519,10 +519,12 @@ int pbf_spawn_particles(const pbf_fluid_config* cfg, pbf_particle* out, uint32_t
  * sort permutation and every discrete choice (neighbour sets, wall and SDF
  * contacts, clamps) are replayed from the recorded forward, not
  * differentiated.  Per-substep checkpoints of (x, v) are kept and, when a
- * quarter of the free device memory holds it (1.7 KB per particle and substep
+ * quarter of the free device memory holds it (1.6 KB per particle and substep
  * at 4 iterations), each substep's forward; otherwise, or when a scene changed
- * since, the backward recomputes each substep from its checkpoint.  APBF must
- * be off.
+ * since, the backward recomputes each substep from its checkpoint, in 1.6 KB
+ * per particle, or 0.2 KB (slower) where that is more than half of the free
+ * memory.  What is held is chosen and allocated by the first
+ * pbf_batch_forward_record and kept until pbf_batch_destroy.  APBF must be off.
  *
  * State arrays are n float4 (x, pad) / (v, pad) in the concatenated particle
  * order; pointers may be device or host memory (unified addressing). */

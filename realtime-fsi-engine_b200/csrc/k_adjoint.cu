@@ -356,7 +356,8 @@ __device__ __forceinline__ float3 lambda_pair_adjoint(const DevParams& P, float4
 
 // ---- the passes: a group of G lanes per particle ------------------------------------------------
 // The pairs come from the hits the recording passes kept, one per lane; where
-// a particle had more than fit, its buckets are walked.  (One thread per
+// a particle had more than fit, its buckets are walked, and where none are kept
+// (W) all are, by the forward's own walk.  (One thread per
 // particle walking the buckets again took 36 us for a reverse delta-p or
 // lambda pass of 32,768 particles and 182 us of 524,288; the groups take 12.4
 // and 8.2 us, 101 and 91 us.)
@@ -365,15 +366,41 @@ struct CoopHits {
     const uint32_t* list_len;  // their number, kNoHits: walk
 };
 
+template <class F>
+struct EachHit {
+    int gl, G;
+    F f;
+    template <class HitAt>
+    __device__ __forceinline__ void add(int cnt, HitAt&& hit)
+    {
+        for (int h = gl; h < cnt; h += G) f(hit(h));
+        __syncwarp();
+    }
+};
+template <class F>
+__device__ __forceinline__ EachHit<F> each_hit(int gl, int G, F f)
+{
+    return EachHit<F>{gl, G, f};
+}
+
 // f(k, load(k)) for every hit of particle s (itself left out), over the
 // group's lanes in no order; the loads of a lane's next hits are issued together.
-template <int G, class Load, class F>
+template <int G, bool W, class Load, class F>
 __device__ __forceinline__ void coop_each(const DevParams& P, const int2* __restrict__ tab, uint32_t mask,
                                           const float4* __restrict__ X, float4 xi, int s, bool on, CoopHits H, Load load,
                                           F&& f)
 {
     constexpr int U = kReplayAhead;
     const int gl = threadIdx.x & (G - 1);
+    if constexpr (W) {
+        __shared__ __align__(16) CoopMem<G, 1> mem[kCThreads / G];
+        auto each = each_hit(gl, G, [&](int k) {
+            if (k != s) f(k, load(k));
+        });
+        coop_walk<G, 1>(P, tab, mask, X, xi, on, mem[threadIdx.x / G], each, [&](float r2) { return r2 <= P.h2; }, nullptr,
+                        nullptr);
+        return;
+    }
     const uint32_t len = on ? __ldg(H.list_len + s) : 0u;
     if (__any_sync(0xffffffffu, len == kNoHits))
         coop_plain_walk<G>(P, tab, mask, X, xi, s, len == kNoHits, [&](int k) {
@@ -416,7 +443,7 @@ __device__ __forceinline__ float3 group_sum(float3 v)
     const int2* tab = table + __ldg(&SC->table_off);                                                \
     const uint32_t mask = __ldg(&SC->mask);
 
-template <int G>
+template <int G, bool W>
 __global__ void __launch_bounds__(kCThreads, kReplayBlocks) k_ac_integrate(
     DevParams P, const SceneDev* __restrict__ scenes, const uint16_t* __restrict__ scene_of,
     const int2* __restrict__ table, CoopHits H, const float4* __restrict__ fsum, const float4* __restrict__ xs,
@@ -433,7 +460,7 @@ __global__ void __launch_bounds__(kCThreads, kReplayBlocks) k_ac_integrate(
                                                  __ldg(posb + id), __ldg(velb + id), posb_s, omb, somega, x0a);
     const bool curl = P.vort_on && omb;
     float3 own = make_float3(0.f, 0.f, 0.f), vown = make_float3(0.f, 0.f, 0.f);
-    coop_each<G>(P, tab, mask, xs, x4, s, cp.live && (P.visc_on || curl), H,
+    coop_each<G, W>(P, tab, mask, xs, x4, s, cp.live && (P.visc_on || curl), H,
                  CoopLoad2{xs, sv}, [&](int k, CoopTwo j) {
         float3 ub, rb;
         integrate_pair_adjoint(P, x4, v0, j.x, j.v, A.vfb, A.cb, curl, ub, rb);
@@ -451,7 +478,7 @@ __global__ void __launch_bounds__(kCThreads, kReplayBlocks) k_ac_integrate(
     add_own(gv + s, vown, 0.0f);
 }
 
-template <int G>
+template <int G, bool W>
 __global__ void __launch_bounds__(kCThreads, kReplayBlocks) k_ac_deltap(
     DevParams P, const SceneDev* __restrict__ scenes, const uint16_t* __restrict__ scene_of,
     const int2* __restrict__ table, CoopHits H, const float4* __restrict__ xl, const float4* __restrict__ auxd,
@@ -464,7 +491,7 @@ __global__ void __launch_bounds__(kCThreads, kReplayBlocks) k_ac_deltap(
     const float3 accb = deltap_adjoint(P, SC, xi, __ldg(auxd + s), xb, tb);
     float3 own = make_float3(0.f, 0.f, 0.f);
     float lown = 0.0f;
-    coop_each<G>(P, tab, mask, xl, xi, s, cp.live, H, CoopLoad1{xl}, [&](int k, float4 xj) {
+    coop_each<G, W>(P, tab, mask, xl, xi, s, cp.live, H, CoopLoad1{xl}, [&](int k, float4 xj) {
         const float rx = xi.x - xj.x, ry = xi.y - xj.y, rz = xi.z - xj.z;
         if (!(rx * rx + ry * ry + rz * rz >= 1e-10f)) return;
         float3 rb;
@@ -481,7 +508,7 @@ __global__ void __launch_bounds__(kCThreads, kReplayBlocks) k_ac_deltap(
     add_own(gout + s, make_float3(own.x + xb.x, own.y + xb.y, own.z + xb.z), lown);
 }
 
-template <int G>
+template <int G, bool W>
 __global__ void __launch_bounds__(kCThreads, kReplayBlocks) k_ac_lambda(
     DevParams P, const SceneDev* __restrict__ scenes, const uint16_t* __restrict__ scene_of,
     const int2* __restrict__ table, CoopHits H, const float4* __restrict__ xl, const float4* __restrict__ auxl,
@@ -494,7 +521,7 @@ __global__ void __launch_bounds__(kCThreads, kReplayBlocks) k_ac_lambda(
     const float4 xi = __ldg(xl + s);
     const LambdaAdjoint A = lambda_adjoint(P, lb, __ldg(auxl + s), __ldg(rhol + s));
     float3 own = make_float3(0.f, 0.f, 0.f);
-    coop_each<G>(P, tab, mask, xl, xi, s, on, H, CoopLoad1{xl}, [&](int k, float4 xj) {
+    coop_each<G, W>(P, tab, mask, xl, xi, s, on, H, CoopLoad1{xl}, [&](int k, float4 xj) {
         const float3 rb = lambda_pair_adjoint(P, xi, xj, A);
         own = make_float3(own.x + rb.x, own.y + rb.y, own.z + rb.z);
         atomicAdd(gout + k, make_float4(-rb.x, -rb.y, -rb.z, 0.0f));
@@ -512,23 +539,6 @@ __global__ void __launch_bounds__(kCThreads, kReplayBlocks) k_ac_lambda(
 // committed positions' hits are not kept (the pass runs once a step): the
 // group walks the buckets once for the confinement direction and once more for
 // the pairs.
-template <class F>
-struct EachHit {
-    int gl, G;
-    F f;
-    template <class HitAt>
-    __device__ __forceinline__ void add(int cnt, HitAt&& hit)
-    {
-        for (int h = gl; h < cnt; h += G) f(hit(h));
-        __syncwarp();
-    }
-};
-template <class F>
-__device__ __forceinline__ EachHit<F> each_hit(int gl, int G, F f)
-{
-    return EachHit<F>{gl, G, f};
-}
-
 template <int G>
 __global__ void __launch_bounds__(kCThreads, kCBlocks) k_ac_vorticity(
     DevParams P, const SceneDev* __restrict__ scenes, const uint16_t* __restrict__ scene_of,
@@ -604,12 +614,13 @@ __global__ void k_ad_predict(uint32_t n, float dt, const uint32_t* __restrict__ 
 // ---- launchers ---------------------------------------------------------------------------
 #define PBF_AC_LAUNCH(KERNEL, ...)                                                                 \
     do {                                                                                          \
-        G = coop_replay_lanes(G, P.n);                                                            \
+        G = list ? coop_replay_lanes(G, P.n) : 8;                                                 \
         const unsigned grid_ = (unsigned)(((uint64_t)P.n * (uint64_t)G + kCThreads - 1) / kCThreads); \
-        if (G == 32) KERNEL<32><<<grid_, kCThreads, 0, st>>>(__VA_ARGS__);                        \
-        else if (G == 16) KERNEL<16><<<grid_, kCThreads, 0, st>>>(__VA_ARGS__);                   \
-        else if (G == 8) KERNEL<8><<<grid_, kCThreads, 0, st>>>(__VA_ARGS__);                     \
-        else KERNEL<4><<<grid_, kCThreads, 0, st>>>(__VA_ARGS__);                                 \
+        if (!list) KERNEL<8, true><<<grid_, kCThreads, 0, st>>>(__VA_ARGS__);                     \
+        else if (G == 32) KERNEL<32, false><<<grid_, kCThreads, 0, st>>>(__VA_ARGS__);            \
+        else if (G == 16) KERNEL<16, false><<<grid_, kCThreads, 0, st>>>(__VA_ARGS__);            \
+        else if (G == 8) KERNEL<8, false><<<grid_, kCThreads, 0, st>>>(__VA_ARGS__);              \
+        else KERNEL<4, false><<<grid_, kCThreads, 0, st>>>(__VA_ARGS__);                          \
     } while (0)
 
 void launch_ac_integrate(int G, const DevParams& P, const SceneDev* scenes, const uint16_t* scene_of, const int2* table,

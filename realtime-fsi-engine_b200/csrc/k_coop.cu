@@ -11,6 +11,8 @@
 // sequential ones: the lanes' pair terms go through shared memory and one
 // lane per sum adds them in visiting order with the roundings of the
 // one-thread bodies (masked_body.cuh), so every result has their bits.
+#include <type_traits>
+
 #include "coop_walk.cuh"
 #include "pbf_batch.h"
 
@@ -90,7 +92,8 @@ __global__ void __launch_bounds__(kCThreads, kCBlocks) k_c_lambda(DevParams P, c
     if (aux) aux[s] = make_float4(gc.x, gc.y, gc.z, den);
 }
 
-template <int G, bool B>
+// W: no hits are kept for any particle
+template <int G, bool B, bool W = false>
 __global__ void __launch_bounds__(kCThreads, kReplayBlocks) k_c_deltap(DevParams P, const SceneDev* __restrict__ scenes,
                                                         const uint16_t* __restrict__ scene_of,
                                                         const float4* __restrict__ xin, float4* __restrict__ xout,
@@ -102,7 +105,7 @@ __global__ void __launch_bounds__(kCThreads, kReplayBlocks) k_c_deltap(DevParams
                                                         float4* __restrict__ dp_out)
 {
     constexpr int NT = 4;
-    __shared__ __align__(16) CoopTermMem<G, NT> mem[kCThreads / G];
+    __shared__ __align__(16) std::conditional_t<W, CoopMem<G, NT>, CoopTermMem<G, NT>> mem[kCThreads / G];
     const CoopParticle c = coop_particle<G>(P.n, order);
     const int gl = threadIdx.x & (G - 1), s = c.s;
     const float4 xi = __ldg(xin + s);
@@ -126,16 +129,21 @@ __global__ void __launch_bounds__(kCThreads, kReplayBlocks) k_c_deltap(DevParams
         t[3] = spiky_scale(P, r2) * xj.w;
     };
     // sums: lambda_j gradW xyz, from the lambda pass's part on
-    CoopSum<G, NT, kReplayAhead, CoopLoad1, decltype(pair)> sum(mem[threadIdx.x / G].term, gl, s, min(gl, 2), 3,
-                                                                gl == 0 ? b.x : gl == 1 ? b.y : b.z, CoopLoad1{xin},
-                                                                std::move(pair));
+    CoopSum<G, NT, W ? 1 : kReplayAhead, CoopLoad1, decltype(pair)> sum(
+        mem[threadIdx.x / G].term, gl, s, min(gl, 2), 3, gl == 0 ? b.x : gl == 1 ? b.y : b.z, CoopLoad1{xin},
+        std::move(pair));
     const bool on = c.live && !skip;
-    const uint32_t len = on && list ? __ldg(list_len + s) : kNoHits;
-    if (__any_sync(0xffffffffu, on && len == kNoHits))
-        coop_plain_walk<G>(P, table, mask, xin, xi, s, on && len == kNoHits,
-                           [&](int k) { sum.chunk(k, __ldg(xin + k), G); });
-    const uint32_t* mine = list + (size_t)s * kCoopList;
-    sum.add(len == kNoHits ? 0 : (int)len, [&](int i) { return (int)__ldg(mine + i); });
+    if constexpr (W) {
+        coop_walk<G, NT>(P, table, mask, xin, xi, on, mem[threadIdx.x / G], sum, [&](float r2) { return r2 <= P.h2; },
+                         nullptr, nullptr);
+    } else {
+        const uint32_t len = on && list ? __ldg(list_len + s) : kNoHits;
+        if (__any_sync(0xffffffffu, on && len == kNoHits))
+            coop_plain_walk<G>(P, table, mask, xin, xi, s, on && len == kNoHits,
+                               [&](int k) { sum.chunk(k, __ldg(xin + k), G); });
+        const uint32_t* mine = list + (size_t)s * kCoopList;
+        sum.add(len == kNoHits ? 0 : (int)len, [&](int i) { return (int)__ldg(mine + i); });
+    }
     const float3 d = make_float3(sum.get(0), sum.get(1), sum.get(2));
     if (!c.live || gl != 0) return;
     if (skip) {
@@ -207,10 +215,8 @@ __global__ void __launch_bounds__(kCThreads, kCBlocks) k_c_integrate(DevParams P
     const float3 f = make_float3(sum.get(0), sum.get(1), sum.get(2));
     const float3 cu = make_float3(sum.get(3), sum.get(4), sum.get(5));
     if (!c.live || gl != 0) return;
-    if (list) {
-        list_len[s] = len;
-        fsum[s] = make_float4(f.x, f.y, f.z, 0.f);
-    }
+    if (list) list_len[s] = len;
+    if (fsum) fsum[s] = make_float4(f.x, f.y, f.z, 0.f);
     float4 xo, vo, om;
     if constexpr (B) {
         float bmin[3], bmax[3];
@@ -329,6 +335,11 @@ void launch_c_deltap(int G, const DevParams& P, const SceneDev* scenes, const ui
                      const uint32_t* list, const uint32_t* list_len, float4* dp_out, cudaStream_t st)
 {
     G = coop_replay_lanes(G, P.n);
+    if (scenes && !list) {  // an adjoint's record without hits
+        k_c_deltap<8, true, true><<<cgrid(P.n, 8), kCThreads, 0, st>>>(P, scenes, scene_of, xin, xout, table, lod, iter,
+                                                                       order, list, list_len, dp_out);
+        return;
+    }
     if (G == 4) {
         if (scenes)
             k_c_deltap<4, true><<<cgrid(P.n, 4), kCThreads, 0, st>>>(P, scenes, scene_of, xin, xout, table, lod, iter,

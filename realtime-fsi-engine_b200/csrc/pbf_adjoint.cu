@@ -9,7 +9,8 @@
 // in reverse with the kernels of k_adjoint.cu: vorticity (last substep),
 // integrate, (deltaP+apply, lambda) per iteration, predict.  Without the room,
 // or when a scene changed since the recording, it first runs each substep's
-// forward again from its checkpoint.  Gradients are with respect to the
+// forward again from its checkpoint, and with room for no hits either its
+// passes walk the buckets again.  Gradients are with respect to the
 // initial positions and velocities and each scene's SDF translation.  Both
 // sequences are captured once into CUDA graphs.
 #include <cuda_runtime.h>
@@ -57,6 +58,7 @@ void pbf_batch::ad_free()
     afree(ad_slab);
     ad_arrays.release();
     records.clear();
+    ad_sx0 = ad_om = nullptr;
     ad_subs = ad_iters = 0;
     recorded = false;
 }
@@ -68,55 +70,82 @@ int pbf_batch::ad_lanes() const { return std::max(coop_lanes(n), 8); }
 
 // One record's arrays laid one after another from `base` (null: only counted);
 // returns its bytes.  `c` entries per array (a multiple of 64, pads included).
-static size_t lay_record(pbf_batch::Record& r, char* base, size_t c, uint32_t iters, size_t table)
+// Without hits (and so recomputed before each use) it holds what the
+// iterations leave; the rest stays in the batch's own arrays of a substep (fsum
+// in the lambda pass's part of delta-p, which an integrate pass does not read).
+static size_t lay_record(pbf_batch& b, pbf_batch::Record& r, char* base, size_t c, uint32_t iters, bool hits)
 {
     size_t at = 0;
     auto take = [&](auto*& p, size_t count) {
         p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(base + at);
         at += (count * sizeof(*p) + 255) / 256 * 256;
     };
-    take(r.ids, c);
-    take(r.table, table);
-    take(r.sv, c);
-    take(r.xf, c);
     take(r.xl, c * iters);
     take(r.auxl, c * iters);
     take(r.auxd, c * iters);
     take(r.rhol, c * iters);
-    take(r.fsum, c);
-    take(r.list, c * (iters + 1) * kCoopList);
-    take(r.list_len, c * (iters + 1));
+    if (hits) {
+        take(r.ids, c);
+        take(r.table, b.table_size);
+        take(r.sv, c);
+        take(r.xf, c);
+        take(r.fsum, c);
+        take(r.list, c * (iters + 1) * kCoopList);
+        take(r.list_len, c * (iters + 1));
+    } else {
+        r.ids = b.ia;
+        r.table = b.table;
+        r.sv = b.sv;
+        r.xf = b.sx[0];
+        r.fsum = b.dpb;
+        r.list = r.list_len = nullptr;
+    }
     return at;
 }
 
 int pbf_batch::ad_alloc()
 {
     const uint32_t S = cfg.substep_iterations, I = cfg.solver_iterations;
-    if (S == ad_subs && I == ad_iters && cp_pos) return PBF_OK;
+    if (ad_subs == S && ad_iters == I && cp_pos) return PBF_OK;
     ad_free();
     const size_t c = std::max<uint32_t>(n, 1u);
     int rc;
-    ad_arrays.add(cp_pos, c * S).add(cp_vel, c * S).add(ad_sx0, c + kCoopPad).add(ad_om, c).add(gxa, c).add(gxb, c)
-        .add(gv, c).add(x0b, c).add(pb, c).add(vb, c).add(pbs, c).add(omb, c).add(tpos, c).add(tvel, c)
-        .add(tgrad, 4 * scenes.size());
+    ad_arrays.add(cp_pos, c * S).add(cp_vel, c * S).add(gxa, c).add(gxb, c).add(gv, c).add(x0b, c).add(pb, c).add(vb, c)
+        .add(pbs, c).add(omb, c).add(tpos, c).add(tvel, c).add(tgrad, 4 * scenes.size());
     if ((rc = ad_arrays.alloc())) return rc;
-    // a record per substep when they take at most a quarter of the free memory
-    // (32,768 particles x 16 substeps x 4 iterations: 0.9 GB)
+    // A record per substep when they take at most a quarter of the free memory
+    // (32,768 particles x 16 substeps x 4 iterations: 0.9 GB), else one when it
+    // takes at most half (1.6 KB a particle), else one without hits (0.2 KB: no
+    // more than the checkpoints and adjoints cannot do without, so that a batch
+    // that fits at all can be differentiated).  Step and backward of 524,288
+    // particles x 16 substeps: 43 ms holding 13.3 GB, 67 ms 1.4 GB, 98 ms 0.7 GB.
     ad_stride = (c + kCoopPad + 63) / 64 * 64;
-    Record probe;
-    const size_t bytes = lay_record(probe, nullptr, ad_stride, I, table_size);
+    const size_t tail = 2 * sizeof(float4) * ad_stride;  // ad_sx0, ad_om
     size_t free_b = 0, total_b = 0;
     ACK(cudaMemGetInfo(&free_b, &total_b));
-    ad_full = bytes * S <= free_b / 4;
-    const uint32_t R = ad_full ? S : 1u;
-    char* slab = nullptr;
-    if ((rc = aalloc(slab, bytes * R))) {
-        ad_free();
-        return rc;
+    for (int kind = 0; kind < 3; ++kind) {
+        const bool hits = kind < 2;
+        const uint32_t R = kind == 0 ? S : 1u;
+        Record probe;
+        const size_t bytes = lay_record(*this, probe, nullptr, ad_stride, I, hits);
+        if (hits && bytes * R + tail > free_b / (kind == 0 ? 4 : 2)) continue;
+        char* slab = nullptr;
+        if ((rc = aalloc(slab, bytes * R + (hits ? tail : 0)))) {
+            if (hits) {
+                cudaGetLastError();  // a smaller record is tried
+                continue;
+            }
+            ad_free();
+            return rc;
+        }
+        ad_slab = slab;
+        ad_full = kind == 0;
+        records.resize(R);
+        for (uint32_t k = 0; k < R; ++k) lay_record(*this, records[k], slab + bytes * k, ad_stride, I, hits);
+        ad_sx0 = hits ? reinterpret_cast<float4*>(slab + bytes * R) : sx0;
+        ad_om = hits ? ad_sx0 + ad_stride : somega;
+        break;
     }
-    ad_slab = slab;
-    records.resize(R);
-    for (uint32_t k = 0; k < R; ++k) lay_record(records[k], slab + bytes * k, ad_stride, I, table_size);
     ad_subs = S;
     ad_iters = I;
     return PBF_OK;
@@ -147,7 +176,7 @@ int pbf_batch::record_substep(uint32_t sub, Record& r, const float4* src_pos, co
     for (uint32_t it = 1; it <= I; ++it) {
         const size_t at = (size_t)(it - 1) * ad_stride;
         float4* xl = r.xl + at;
-        uint32_t *list = r.list + at * kCoopList, *len = r.list_len + at;
+        uint32_t *list = r.hits(at), *len = r.hit_count(at);
         launch_c_lambda(G, P, scenes_dev, scene_of, sx[0], xl, r.rhol + at, r.table, lod, it, nullptr, list, len,
                         r.auxl + at, stream);
         launch_c_deltap(G, P, scenes_dev, scene_of, xl, it == I ? r.xf : sx[0], r.table, lod, it, nullptr, list, len,
@@ -157,12 +186,12 @@ int pbf_batch::record_substep(uint32_t sub, Record& r, const float4* src_pos, co
     float4* x0 = sx0;
     float4* om = somega;
     if (last && cfg.enable_vorticity) {  // the vorticity pass and its reverse read these
-        ACK(cudaMemcpyAsync(ad_sx0, sx0, sizeof(float4) * n, cudaMemcpyDeviceToDevice, stream));
+        if (ad_sx0 != sx0) ACK(cudaMemcpyAsync(ad_sx0, sx0, sizeof(float4) * n, cudaMemcpyDeviceToDevice, stream));
         x0 = ad_sx0;
         om = ad_om;
     }
     launch_c_integrate(G, P, scenes_dev, scene_of, r.xf, r.sv, x0, om, r.ids, dst_pos, dst_vel, r.table, nullptr,
-                       r.list + (size_t)I * ad_stride * kCoopList, r.list_len + (size_t)I * ad_stride, r.fsum, stream);
+                       r.hits((size_t)I * ad_stride), r.hit_count((size_t)I * ad_stride), r.fsum, stream);
     ++launches;
     return PBF_OK;
 }
@@ -173,11 +202,14 @@ int pbf_batch::record_body()
     for (uint32_t sub = 0; sub < S; ++sub) {
         ACK(cudaMemcpyAsync(cp_pos + (size_t)sub * n, pos, sizeof(float4) * n, cudaMemcpyDeviceToDevice, stream));
         ACK(cudaMemcpyAsync(cp_vel + (size_t)sub * n, vel, sizeof(float4) * n, cudaMemcpyDeviceToDevice, stream));
-        const int rc = record_substep(sub, records[ad_full ? sub : 0], pos, vel, pos, vel);
+        // (a record that the backward fills is not written here)
+        const int rc = ad_full ? record_substep(sub, records[sub], pos, vel, pos, vel) : substep_body(pos, vel, pos, vel);
         if (rc) return rc;
     }
-    if (cfg.enable_vorticity) {
-        const Record& r = records[ad_full ? S - 1 : 0];
+    if (cfg.enable_vorticity && !ad_full) {
+        vorticity_pass();
+    } else if (cfg.enable_vorticity) {
+        const Record& r = records[S - 1];
         launch_c_vorticity(ad_lanes(), dev_params(), scenes_dev, scene_of, ad_sx0, ad_om, r.ids, vel, r.table, nullptr,
                            stream);
         ++launches;
@@ -214,13 +246,13 @@ int pbf_batch::backward_body(bool recompute)
             launch_ac_vorticity(G, P, scenes_dev, scene_of, r.table, ad_sx0, ad_om, r.ids, vb, pbs, omb, stream);
             ++launches;
         }
-        launch_ac_integrate(G, P, scenes_dev, scene_of, r.table, r.list + (size_t)I * ad_stride * kCoopList,
-                            r.list_len + (size_t)I * ad_stride, r.fsum, r.xf, r.sv, src_pos, r.ids, pb, vb,
+        launch_ac_integrate(G, P, scenes_dev, scene_of, r.table, r.hits((size_t)I * ad_stride),
+                            r.hit_count((size_t)I * ad_stride), r.fsum, r.xf, r.sv, src_pos, r.ids, pb, vb,
                             last ? pbs : nullptr, last ? omb : nullptr, ad_om, a, gv, x0b, tgrad, stream);
         ++launches;
         for (int it = (int)I; it >= 1; --it) {
             const size_t at = (size_t)(it - 1) * ad_stride;
-            const uint32_t *list = r.list + at * kCoopList, *len = r.list_len + at;
+            const uint32_t *list = r.hits(at), *len = r.hit_count(at);
             launch_ac_deltap(G, P, scenes_dev, scene_of, r.table, list, len, r.xl + at, r.auxd + at, a, b, tgrad, stream);
             launch_ac_lambda(G, P, scenes_dev, scene_of, r.table, list, len, r.xl + at, r.auxl + at, r.rhol + at, b, a,
                              stream);

@@ -187,8 +187,8 @@ struct pbf_batch {
     // adjoint (pbf_adjoint.cu): per-substep checkpoints of the recorded step
     // and the forward of each substep as the reverse passes read it.  With room
     // for it every substep has a record of its own, written by the recording
-    // forward; otherwise there is one, which the backward fills again from the
-    // substep's checkpoint.
+    // forward; otherwise there is one, which the backward fills from the
+    // substep's checkpoint, with little room one without hits.
     struct Record {
         uint32_t* ids = nullptr;                    // sort permutation
         int2* table = nullptr;
@@ -196,7 +196,9 @@ struct pbf_batch {
         float4* fsum = nullptr;                     // XSPH sums
         float4 *xl = nullptr, *auxl = nullptr, *auxd = nullptr;  // per iteration: (x*, lambda), (grad C, denominator), raw dp
         float* rhol = nullptr;                      // per iteration: density
-        uint32_t *list = nullptr, *list_len = nullptr;  // per iteration, then integrate: hits (k_coop.cu)
+        uint32_t *list = nullptr, *list_len = nullptr;  // per iteration, then integrate: hits (k_coop.cu), or null
+        uint32_t* hits(size_t at) const { return list ? list + at * pbf::kCoopList : nullptr; }
+        uint32_t* hit_count(size_t at) const { return list ? list_len + at : nullptr; }
     };
     std::vector<Record> records;
     size_t ad_stride = 0;         // entries between the iterations' arrays of a record
