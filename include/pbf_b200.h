@@ -423,7 +423,9 @@ typedef struct pbf_batch_tuning {
  * the fastest and restores the particle state that the trials advanced.  The
  * candidates: block x order x persistence in neighbour mode 4, and mode 8 when
  * the windows fit, as PBF_BOPT_NEIGHBOUR_MODE allows (-1: both; the pick then
- * decides the automatic mode).  `results` (may be null) receives up to
+ * decides the automatic mode).  Up to 2^18 particles, where the shapes change
+ * nothing, mode 4 is timed once: its candidates share that time, and the pick
+ * has the settings that were there.  `results` (may be null) receives up to
  * `max_results` timed candidates, `*num_results` their count; `*best` the pick. */
 int pbf_batch_autotune(pbf_batch* b, uint32_t trial_steps, pbf_batch_tuning* best, pbf_batch_tuning* results,
                        uint32_t max_results, uint32_t* num_results);

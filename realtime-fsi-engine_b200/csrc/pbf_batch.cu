@@ -825,7 +825,7 @@ extern "C" int pbf_batch_get_option(const pbf_batch* b, int option, int* value)
 }
 
 // Autotuner: every candidate (neighbour mode 8 when the windows fit; block x
-// order x persistence in mode 4) is timed with CUDA events over `trial_steps`
+// order x persistence in mode 4, one of them where they shape nothing) is timed with CUDA events over `trial_steps`
 // graph replays after one warm-up replay (which also captures the graph); the
 // particle state is saved before and restored after, so tuning leaves the
 // simulation where it was.
@@ -877,20 +877,28 @@ extern "C" int pbf_batch_autotune(pbf_batch* b, uint32_t trial_steps, pbf_batch_
         }
     }
     b->neighbour_mode = 4;
+    // groups of lanes take the same passes whatever the shape: one timing for
+    // all of them, and the shape set before is kept
+    const bool shaped = !coop_lanes(b->n);
+    float any_ms = 0.0f;
+    if (!shaped && !rc && mode_was != 8 && !(rc = time_steps(&any_ms)) && any_ms < pick.ms_per_step)
+        pick = {b->launch.block, b->morton, b->launch.blocks_per_sm, any_ms, 4};
     for (int order = 0; order <= 1 && !rc && mode_was != 8; ++order) {
         for (int bi = 0; bi < 3 && !rc; ++bi) {
             const int occ = batch_max_blocks_per_sm(blocks[bi]);
             const int bps_list[2] = {0, occ};
             for (int pi = 0; pi < 2 && !rc; ++pi) {
-                b->launch.block = blocks[bi];
-                b->morton = order;
-                b->launch.blocks_per_sm = bps_list[pi];
-                float ms = 0.0f;
-                if ((rc = time_steps(&ms))) break;
+                float ms = any_ms;
+                if (shaped) {
+                    b->launch.block = blocks[bi];
+                    b->morton = order;
+                    b->launch.blocks_per_sm = bps_list[pi];
+                    if ((rc = time_steps(&ms))) break;
+                }
                 const pbf_batch_tuning r{blocks[bi], order, bps_list[pi], ms, 4};
                 if (results && count < max_results) results[count] = r;
                 ++count;
-                if (r.ms_per_step < pick.ms_per_step) pick = r;
+                if (shaped && r.ms_per_step < pick.ms_per_step) pick = r;
             }
         }
     }
