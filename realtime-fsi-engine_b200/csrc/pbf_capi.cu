@@ -185,6 +185,7 @@ static int dalloc(T*& p, size_t count)
     cudaError_t e = cudaMalloc((void**)&p, count * sizeof(T));
     if (e != cudaSuccess) {
         p = nullptr;
+        cudaGetLastError();  // (else the next launch's check reports it again)
         return set_error(PBF_ERR_ALLOC, "cudaMalloc(%zu B): %s", count * sizeof(T), cudaGetErrorString(e));
     }
     return PBF_OK;
@@ -268,6 +269,8 @@ SdfDev pbf_handle::sdf_dev() const
     return S;
 }
 
+// Device arrays for need_n particles and the current parameters; a later call
+// makes what an earlier one could not.
 int pbf_handle::ensure_capacity(uint32_t need_n)
 {
     int rc = PBF_OK;
@@ -299,6 +302,7 @@ int pbf_handle::ensure_capacity(uint32_t need_n)
     if (!totals && (rc = dalloc(totals, 256))) return rc;
     if (!scalars && (rc = dalloc(scalars, 8))) return rc;
     if (derived.hash_size != cap_h) {
+        cap_h = 0;
         if ((rc = dalloc(table, derived.hash_size))) return rc;
         cap_h = derived.hash_size;
     }
@@ -540,6 +544,7 @@ int pbf_handle::ensure_dense()
                       std::equal(nd, nd + 3, dwin_n);
     if (same) return PBF_OK;
     if (capturing) return set_error(PBF_ERR_INVALID, "dense cell window changed during graph capture");
+    dwin_ready = false;
     if (slots > cap_slots || !druns) {
         cap_slots = 0;
         window_slab.release();
@@ -876,6 +881,7 @@ int pbf_handle::step_body()
 int pbf_handle::step()
 {
     if (n == 0) return PBF_OK;  // PBFluids.cpp:325
+    if (const int rc = ensure_capacity(n)) return rc;
     if (effective_mode() == 8) {
         const int rc = ensure_dense();  // allocation and slot flags before any capture
         if (rc) return rc;
@@ -1037,7 +1043,10 @@ extern "C" int pbf_set_particles(pbf_handle* h, const pbf_particle* ps, uint32_t
     h->contacts_valid = false;
     if (n == 0) return PBF_OK;
     int rc = h->ensure_capacity(n);
-    if (rc) return rc;
+    if (rc) {
+        h->n = h->cfg.particle_count = 0;  // no particles, rather than as many without their arrays
+        return rc;
+    }
     // one copy of the Particle array, split into the engine's arrays on the GPU
     CK(cudaMemcpyAsync(h->aos, ps, sizeof(pbf_particle) * (size_t)n, cudaMemcpyHostToDevice, h->stream));
     launch_unpack_particles(n, h->aos, h->pos, h->pred, h->vel, h->num_sms, h->stream);
@@ -1100,7 +1109,10 @@ extern "C" int pbf_set_particles_device(pbf_handle* h, const void* pos4, const v
         pbf_derive_params(&h->cfg, h->collision_padding, &h->derived);
         if (n) {
             int rc = h->ensure_capacity(n);
-            if (rc) return rc;
+            if (rc) {
+                h->n = h->cfg.particle_count = 0;
+                return rc;
+            }
             CK(cudaMemsetAsync(h->pred, 0, sizeof(float4) * n, h->stream));
             CK(cudaMemsetAsync(h->dpb, 0, sizeof(float4) * n, h->stream));
         }
@@ -1282,8 +1294,10 @@ extern "C" int pbf_run_stage(pbf_handle* h, int stage, uint32_t iter)
 {
     CHECK_HANDLE(h);
     if (h->n == 0) return set_error(PBF_ERR_STATE, "no particles");
+    int rc = h->ensure_capacity(h->n);
+    if (rc) return rc;
     if (stage > PBF_STAGE_SORT && !h->ids) return set_error(PBF_ERR_STATE, "stage %d before sort", stage);
-    int rc = h->stage(stage, iter);
+    rc = h->stage(stage, iter);
     if (rc) return rc;
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return set_error(PBF_ERR_CUDA, "stage %d: %s", stage, cudaGetErrorString(e));

@@ -36,6 +36,7 @@ public:
         const cudaError_t e = cudaMalloc(&base_, bytes_ ? bytes_ : 256);
         if (e != cudaSuccess) {
             base_ = nullptr;
+            cudaGetLastError();  // (else the next launch's check reports it again)
             const int rc = set_error(PBF_ERR_ALLOC, "cudaMalloc(%zu B): %s", bytes_, cudaGetErrorString(e));
             release();
             return rc;
