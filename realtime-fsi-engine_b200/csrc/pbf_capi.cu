@@ -277,6 +277,7 @@ int pbf_handle::ensure_capacity(uint32_t need_n)
     if (need_n > cap_n) {
         const size_t c = need_n;
         cap_n = 0;
+        ids = skeys = order = nullptr;  // in the arrays that go
         particle_slab.release();
         particle_slab.add(pos, c).add(vel, c).add(pred, c).add(aos, 3 * c).add(keys, c).add(ka, c).add(ia, c).add(kb, c)
             .add(ib, c).add(mcode, c).add(mka, c).add(mia, c).add(mkb, c).add(mib, c).add(sx[0], c + kCoopPad)
@@ -304,6 +305,8 @@ int pbf_handle::ensure_capacity(uint32_t need_n)
     if (derived.hash_size != cap_h) {
         cap_h = 0;
         if ((rc = dalloc(table, derived.hash_size))) return rc;
+        // (no cell holds anything until a table stage has run)
+        CK(cudaMemsetAsync(table, 0xFF, sizeof(int2) * (size_t)derived.hash_size, stream));
         cap_h = derived.hash_size;
     }
     return PBF_OK;
