@@ -41,6 +41,7 @@ static int aalloc(T*& p, size_t count)
     cudaError_t e = cudaMalloc((void**)&p, count * sizeof(T));
     if (e != cudaSuccess) {
         p = nullptr;
+        cudaGetLastError();  // (else the next launch's check reports it again)
         return set_error(PBF_ERR_ALLOC, "cudaMalloc(%zu B): %s", count * sizeof(T), cudaGetErrorString(e));
     }
     return PBF_OK;
@@ -131,10 +132,7 @@ int pbf_batch::ad_alloc()
         if (hits && bytes * R + tail > free_b / (kind == 0 ? 4 : 2)) continue;
         char* slab = nullptr;
         if ((rc = aalloc(slab, bytes * R + (hits ? tail : 0)))) {
-            if (hits) {
-                cudaGetLastError();  // a smaller record is tried
-                continue;
-            }
+            if (hits) continue;
             ad_free();
             return rc;
         }

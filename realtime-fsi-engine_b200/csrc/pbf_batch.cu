@@ -45,6 +45,7 @@ static int balloc(T*& p, size_t count)
     cudaError_t e = cudaMalloc((void**)&p, count * sizeof(T));
     if (e != cudaSuccess) {
         p = nullptr;
+        cudaGetLastError();  // (else the next launch's check reports it again)
         return set_error(PBF_ERR_ALLOC, "cudaMalloc(%zu B): %s", count * sizeof(T), cudaGetErrorString(e));
     }
     return PBF_OK;
@@ -703,10 +704,13 @@ extern "C" int pbf_batch_set_sdf_grid(pbf_batch* b, uint32_t scene, const float*
     pbf_batch::Scene& s = b->scenes[scene];
     const size_t total = (size_t)dims[0] * dims[1] * dims[2];
     const size_t have = (size_t)s.dims[0] * s.dims[1] * s.dims[2];
-    int rc;
-    if (!s.grid || total != have) {
-        if ((rc = balloc(s.grid, total))) return rc;
+    int rc = PBF_OK;
+    if ((!s.grid || total != have) && s.sdf_on) {
+        // the scene has no obstacle while its grid is another's size or gone
+        s.sdf_on = false;
+        if ((rc = b->upload_scenes())) return rc;
     }
+    if ((!s.grid || total != have) && (rc = balloc(s.grid, total))) return rc;
     if (!s.slab_min && (rc = balloc(s.slab_min, 6))) return rc;
     for (int a = 0; a < 3; ++a) {
         s.dims[a] = dims[a];

@@ -1161,10 +1161,13 @@ int pbf_handle::upload_grid(const float* dist_host, const int32_t d[3], const fl
 {
     const size_t total = (size_t)d[0] * d[1] * d[2];
     int rc;
-    if (total != grid_elems) {
+    if (total != grid_elems || !grid) {
+        // (captured steps, of attached scenes too, hold the grid that goes)
+        grid_elems = 0;
+        ++grid_generation;
+        invalidate_graph();
         if ((rc = dalloc(grid, total))) return rc;
         grid_elems = total;
-        ++grid_generation;
     }
     if (!slab_min && (rc = dalloc(slab_min, 6))) return rc;
     for (int a = 0; a < 3; ++a) {

@@ -80,6 +80,7 @@ int dalloc(T*& p, size_t n)
     const cudaError_t e = cudaMalloc((void**)&p, n * sizeof(T));
     if (e != cudaSuccess) {
         p = nullptr;
+        cudaGetLastError();  // (else the next launch's check reports it again)
         return set_error(PBF_ERR_ALLOC, "cudaMalloc(%zu B): %s", n * sizeof(T), cudaGetErrorString(e));
     }
     return PBF_OK;
