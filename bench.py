@@ -68,7 +68,8 @@ def parse():
     ap.add_argument("--no-extras", action="store_true",
                     help="c2 only: skip the short C3 batch and C4 adjoint runs attached to the line")
     ap.add_argument("--mode", type=int, default=-1, choices=[-1, 4, 8],
-                    help="neighbour passes: -1 automatic (default: 8 from 3 * 2^16 particles, else 4), 4 hashed "
+                    help="neighbour passes: -1 automatic (default: 8 from 3 * 2^16 particles unless the window is "
+                         "large for them, else 4), 4 hashed "
                          "buckets in Morton thread order with per-bucket hit masks, 8 x-runs of a dense cell window")
     ap.add_argument("--sample", type=int, nargs=3, default=None, metavar=("NX", "NY", "NZ"),
                     help="smaller lattice of the same scene (profiling captures only)")
@@ -313,6 +314,21 @@ def run_reference(args):
     print(json.dumps(line), flush=True)
 
 
+def neighbour_mode(asked, n, d):
+    """The neighbour mode a scene of n particles with derived parameters d runs
+    in (pbf_handle::effective_mode): asked if it is 4, else 8 where the dense
+    window (the walls' box in cells, 6 more on each side) has at most 2^26 cells
+    and, for the automatic choice, as few per particle as the engine wants."""
+    if asked == 4 or d.enable_apbf or n >= 1 << 27 or (asked < 0 and n < 3 << 16):
+        return 4
+    lo, hi = (np.floor(np.float32(b)[:3] / np.float32(d.h)).astype(np.float64) for b in (d.bounds_min, d.bounds_max))
+    cells = float(np.prod(hi - lo + 13.0))
+    if not cells <= 1 << 26 or (hi < lo).any():
+        return 4
+    roomy = cells > (64 if n > 1 << 18 else 16) * n
+    return 4 if asked < 0 and n < 1 << 19 and roomy else 8
+
+
 # ---- GPU arm ------------------------------------------------------------------------------------------
 def run_b200(args, dist):
     import torch
@@ -347,7 +363,7 @@ def run_b200(args, dist):
     torch.cuda.synchronize(dev)
     clocks = Clocks(dev)
     l0 = fl.kernel_launches()
-    mode = args.mode if args.mode >= 0 else (8 if n >= (3 << 16) else 4)
+    mode = neighbour_mode(args.mode, n, fl.derived())
     ws0 = fl.list_stats() if mode == 8 else None
     e0.record(stream)
     for _ in range(args.steps):
