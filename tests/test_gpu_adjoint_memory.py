@@ -47,6 +47,7 @@ def test_gradients_at_every_size_of_record(have_gpu, nside, copies):
             got, held = run(b, pos, vel, target, offs)
         finally:
             del hog
+            torch.cuda.empty_cache()
         assert held <= most + 96 * MB
         assert rel(got[0], first[0]) <= 1e-5 and rel(got[1], first[1]) <= 1e-5 and rel(got[2], first[2]) <= 1e-4
         assert np.array_equal(got[3], first[3])

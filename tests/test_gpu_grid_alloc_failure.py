@@ -25,10 +25,12 @@ def refused(call, handle, *head):
     grid = np.empty(DIMS, np.float32)
     torch.cuda.synchronize()
     hog = torch.empty(torch.cuda.mem_get_info()[0] - (512 << 20), dtype=torch.uint8, device="cuda")
-    rc = call(handle, *head, grid.ctypes.data_as(C.c_void_p), (C.c_int32 * 3)(*DIMS), (C.c_float * 3)(0, 0, 0), C.c_float(0.1))
-    del hog
-    torch.cuda.empty_cache()
-    return rc
+    try:
+        return call(handle, *head, grid.ctypes.data_as(C.c_void_p), (C.c_int32 * 3)(*DIMS), (C.c_float * 3)(0, 0, 0),
+                    C.c_float(0.1))
+    finally:
+        del hog
+        torch.cuda.empty_cache()
 
 
 @pytest.mark.parametrize("graph", [False, True])
