@@ -287,6 +287,9 @@ int pbf_sort_keys_noalloc(const uint32_t* keys_dev, uint32_t n, uint32_t key_bit
 /* ---- timing ------------------------------------------------------------- */
 /* When on, every pass of pbf_step records CUDA events on the handle's stream
  * and accumulates per-pass device time (read with pbf_read_pass_times).
+ * Predict, sort, table and reorder are then launched one by one; up to 2^20
+ * particles a step without profiling takes them together (the same results in
+ * fewer launches), so their slots say what the stages cost, not the step.
  * Pass slots follow enum pbf_stage (index = stage); slot 0 = whole steps. */
 #define PBF_NUM_PASS_SLOTS 12
 int pbf_set_profiling(pbf_handle* h, int on);

@@ -311,7 +311,9 @@ int pbf_batch::effective_mode() const
     if (tuned_mode) return tuned_mode;
     // mode 8 where mode 4 leaves its groups of lanes (k_coop.cu: 146,319
     // particles in 40 scenes 1219 us a step against 2069 in mode 8, 162,133 in 14
-    // scenes 1396 against 1954) and the windows have at most 8 cells per particle
+    // scenes 1396 against 1954).  Below 2^19 particles the windows may have at most
+    // 8 cells per particle; in batches of 2^18 to 2^19 that limit is not measured
+    // (one scene of that size gains in mode 8 up to 64, pbf_handle::effective_mode)
     return dense_fits() && n > (1u << 18) && (n >= (1u << 19) || dense_total <= 8ull * n) ? 8 : 4;
 }
 

@@ -111,7 +111,7 @@ struct DenseArgs {
     const int2* runs;      // per window slot: label range of slots s-1 .. s+1 of its row
     const uint32_t* order; // pass thread i takes label order[i] (null: label i), unless it is marked as listed
     uint32_t* list;        // one scene (null in a batch): [0] how many listed, [1 ...] the listed labels (those that walk buckets)
-    uint32_t list_blocks;  // a pass's first blocks, which take them: room for list_blocks * kDensePassThreads
+    uint32_t list_blocks;  // a pass's first blocks, which take them: room for dense_list_room(list_blocks)
     uint32_t* hm;          // lambda hit masks for the delta-p of the same iteration (kDenseListWords x n)
     uint8_t* hcnt;         // per label: chunks recorded, 0xFF = none
     int use_list;          // delta-p: the lambda pass of this iteration recorded hm/hcnt

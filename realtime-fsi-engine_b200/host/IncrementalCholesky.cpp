@@ -25,7 +25,8 @@ namespace pbfdrop {
 // column in 1.12 runs for a sphere of 2,562 vertices), so a run is one loop
 // over consecutive memory where a walk over li_ gathered and scattered: the
 // factorization with 585 handles 21 -> 4.8 ms, three axes' solve 2.9 -> 0.9 ms
-// (one core), a frame with 262,144 particles 11.0 -> 3.4 ms.
+// (one core), a frame with 262,144 particles, repeated from the same ones so
+// that its handles settle, 11.0 -> 3.4 ms.
 namespace {
 
 // w[i] -= l[i] * y
