@@ -318,7 +318,8 @@ def neighbour_mode(asked, n, d):
     """The neighbour mode a scene of n particles with derived parameters d runs
     in (pbf_handle::effective_mode): asked if it is 4, else 8 where the dense
     window (the walls' box in cells, 6 more on each side) has at most 2^26 cells
-    and, for the automatic choice, as few per particle as the engine wants."""
+    and, for the automatic choice, as few per particle as the engine wants (its
+    walls at rest)."""
     if asked == 4 or d.enable_apbf or n >= 1 << 27 or (asked < 0 and n < 3 << 16):
         return 4
     lo, hi = (np.floor(np.float32(b)[:3] / np.float32(d.h)).astype(np.float64) for b in (d.bounds_min, d.bounds_max))

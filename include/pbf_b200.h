@@ -320,7 +320,9 @@ int pbf_set_use_graph(pbf_handle* h, int on);
  *                          2^18 when the window has at most 64 cells per
  *                          particle, from 3 * 2^16 when it has at most 16, else
  *                          mode 4 (where mode 8's launches and window cost
- *                          more than its walk saves); APBF and
+ *                          more than its walk saves), as it does below 2^19
+ *                          while the walls cross cells within 4 steps of the
+ *                          last time, unless the window is small; APBF and
  *                          windows over 2^26 cells run mode 4.  Modes 4 and 8 give
  *                          bit-identical results (same pairs, order and pair
  *                          arithmetic).  Other values: PBF_ERR_INVALID. */

@@ -428,12 +428,45 @@ int pbf_handle::effective_mode() const
 {
     if (pass_mode >= 0 && pass_mode != 8) return pass_mode;
     const bool automatic = pass_mode < 0;
+    if (automatic && window_wait && n < (1u << 19)) return 4;
     if ((automatic && n < 3u * (1u << 16)) || derived.enable_apbf || n >= (1u << 27)) return 4;
     int g0[3];
     uint32_t nd[3];
     if (!dense_window(g0, nd)) return 4;
     const bool roomy = (uint64_t)nd[0] * nd[1] * nd[2] > (n > (1u << 18) ? 64ull : 16ull) * n;
     return automatic && n < (1u << 19) && roomy ? 4 : 8;
+}
+
+// Called once a step.  A new window's tables (k_d_clean, k_d_dcol) take 1.1 us
+// per 1,000 cells, which mode 8 saves over a few steps: 373,248 particles at 15
+// cells a particle, tables 6.3 ms, a step 3.1 ms in mode 8 and 4.65 in mode 4,
+// so that walls that cross a cell every step took 9.4.  A window that changes
+// again within kWindowSteps steps is therefore not followed until it has stayed
+// for as many; one that changes less often is followed at once, and so is one of
+// up to 4 cells a particle where mode 4 runs one thread per particle (0.8 cells:
+// 3.3 ms with tables every step; 4.7: 4.9; with groups of lanes 262,144 particles
+// take 2.3 ms whatever the walls do, 2.8 and 4.1 with tables).
+void pbf_handle::watch_window()
+{
+    int g0[3] = {0, 0, 0};
+    uint32_t nd[3] = {0, 0, 0};
+    dense_window(g0, nd);
+    const bool small = !coop_lanes(n) && (uint64_t)nd[0] * nd[1] * nd[2] <= 4ull * n;
+    const bool was = window_wait;
+    if (std::equal(g0, g0 + 3, wanted_g0) && std::equal(nd, nd + 3, wanted_n)) {
+        window_steps = std::min(window_steps + 1, kWindowSteps);
+        if (window_steps == kWindowSteps) window_wait = false;
+    } else {
+        window_wait = window_wait || window_steps < kWindowSteps;
+        window_steps = wanted_n[0] ? 0 : kWindowSteps;  // (the first window is no change)
+        std::copy(g0, g0 + 3, wanted_g0);
+        std::copy(nd, nd + 3, wanted_n);
+    }
+    if (small) window_wait = false;
+    if (was != window_wait && pass_mode < 0 && n < (1u << 19)) {  // the mode may change
+        label_space = false;
+        invalidate_graph();
+    }
 }
 
 int pbf_handle::ensure_label_capacity()
@@ -885,6 +918,7 @@ int pbf_handle::step()
 {
     if (n == 0) return PBF_OK;  // PBFluids.cpp:325
     if (const int rc = ensure_capacity(n)) return rc;
+    watch_window();
     if (effective_mode() == 8) {
         const int rc = ensure_dense();  // allocation and slot flags before any capture
         if (rc) return rc;

@@ -107,6 +107,14 @@ struct pbf_handle {
     uint32_t *dsort = nullptr, *dsort_sums = nullptr;
     size_t cap_dsort = 0;
     int effective_mode() const;
+    // Steps since the window last changed (the walls' cells or h), and whether
+    // the automatic choice below 2^19 particles waits for it to settle.
+    static constexpr uint32_t kWindowSteps = 4;
+    uint32_t window_steps = kWindowSteps;
+    bool window_wait = false;
+    int wanted_g0[3] = {0, 0, 0};
+    uint32_t wanted_n[3] = {0, 0, 0};
+    void watch_window();
     int ensure_label_capacity();
     int unpermute_for_read(int which);
     // sorted order
